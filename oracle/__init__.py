@@ -48,10 +48,11 @@ def _ptr(a: np.ndarray):
 def build(ref_tree: str | None = None) -> None:
     """Compile liboracle.so (always) and oracle/_ref from the reference tree
     ``ref_tree`` (else the CELLSPE_REFERENCE_TREE environment variable) when
-    one is given and exists; without one only the restatement is built."""
+    one is given and holds anything; without one, or with an empty folder in
+    its place, only the restatement is built."""
     subprocess.run(["make", "-s", "-C", str(HERE), "liboracle.so"], check=True)
     ref_tree = ref_tree or os.environ.get("CELLSPE_REFERENCE_TREE")
-    if ref_tree and Path(ref_tree).is_dir():
+    if ref_tree and Path(ref_tree).is_dir() and any(Path(ref_tree).iterdir()):
         subprocess.run(["make", "-s", "-C", str(HERE), "ref", f"REF={ref_tree}"], check=True)
         (REF_DIR / "reference_tree.txt").write_text(str(Path(ref_tree).resolve()))
 
