@@ -85,13 +85,6 @@ const float2* rotator_table(int L, double off_hz, double fs_hz)
     return d;
 }
 
-CS_DEV float lut_pick4(const float (&l)[4], unsigned c)
-{
-    float lo = (c & 1u) ? l[1] : l[0];
-    float hi = (c & 1u) ? l[3] : l[2];
-    return (c & 2u) ? hi : lo;
-}
-
 // Samples s and s+1 (s even) of a plane word through a 16-entry table of
 // level pairs (one shared-memory read instead of two 4-way selects); blanked
 // samples (their bit in the validity mask clear) are 0.0, as mark5access
@@ -444,137 +437,267 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
     }
 }
 
-__global__ void k_spec_reduce(const float* __restrict__ partial, float* __restrict__ power, int rows, int nchunk,
-                              int nb, float scale)
+// power[row][k] = scale * sum of the row's chunk partials.  Bound by the read
+// of the partials.  A CTA takes blockDim.x bins of one row; each of its
+// blockDim.y slices adds every blockDim.y-th chunk and the slices' sums are
+// added in order, so the sum is deterministic.  Eight slices where a thread per
+// bin would leave the chip empty (spec_reduce_slices): a row with hundreds of
+// chunks is then not one thread's serial chain (16 rows x 512 chunks x 513 bins:
+// 46 us with a thread per bin, 10 us); one slice where there are bins enough
+// (16 rows x 32 chunks x 32769 bins: 13 us, 20 us with eight).
+constexpr int RED_THREADS = 256;
+__global__ void __launch_bounds__(RED_THREADS) k_spec_reduce(const float* __restrict__ partial, float* __restrict__ power,
+                                                             int nchunk, int nb, float scale)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)rows * nb) return;
-    int r = (int)(i / nb), k = (int)(i % nb);
+    __shared__ float part[RED_THREADS];
+    const int r = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
     const float* src = partial + (int64_t)r * nchunk * nb + k;
     float s = 0.f;
-    for (int c = 0; c < nchunk; c++) s += src[(int64_t)c * nb];
-    power[i] = s * scale;
+    if (k < nb)
+        for (int c = threadIdx.y; c < nchunk; c += blockDim.y) s += src[(int64_t)c * nb];
+    if (blockDim.y > 1) {
+        part[threadIdx.y * blockDim.x + threadIdx.x] = s;
+        __syncthreads();
+        for (int q = 1; q < blockDim.y; q++) s += part[q * blockDim.x + threadIdx.x];
+    }
+    if (threadIdx.y == 0 && k < nb) power[(int64_t)r * nb + k] = s * scale;
 }
 
-// PCal fold: thread-private accumulators in shared memory, [bin][thread].
-// TaskCoreIPP::doMaths folds the overlapped FFT windows whose running FFT
-// count is a multiple of the overlap factor (TaskCoreIPP.cpp:414-418).  The
-// count starts at 0 once per call (:358), runs on across the spectra of the
-// call and advances after every source's FFT (:434-435), so with ns sources
-// source rs folds window j of spectrum s when (ns (s novl + j) + rs) % ov == 0:
-// an arithmetic progression j0, j0 + step, ... (step = ov / gcd(ns, ov)),
-// possibly empty.  Each window is folded from its own start (the rotator
-// index restarts), N samples from j * hop.
+// one slice from about one full wave of threads (152 SMs x 1024) on
+int spec_reduce_slices(int64_t bins, int nchunk) { return bins < 152 * 1024 && nchunk >= 8 ? 8 : 1; }
+
+// PCal fold.  TaskCoreIPP::doMaths folds the overlapped FFT windows whose
+// running FFT count is a multiple of the overlap factor (TaskCoreIPP.cpp:
+// 414-418).  The count starts at 0 once per call (:358), runs on across the
+// spectra of the call and advances after every source's FFT (:434-435), so with
+// ns sources source rs folds window j of spectrum s when
+// (ns (s novl + j) + rs) % ov == 0: an arithmetic progression j0, j0 + step, ...
+// (step = ov / gcd(ns, ov)), possibly empty.  Each window is folded from its
+// own start (the rotator index restarts), N samples from j * hop.
+//
+// Samples whose rotator index l is equal are multiplied by the same value, so
+// the fold counts how often each of the four codes occurs per l and applies
+// levels and rotator to the counts: exact integers until the last step.  The
+// counting is bit-sliced: a plane word holds 16 two-bit codes, and words at
+// the same place in the rotator period are added as vertical counters (a
+// carry-save adder is two three-input logic operations for 32 positions), the
+// AND of a code's two bits in a second set.  About 9 logic operations per word
+// instead of 16 level selections and 32 multiply-adds, which bound the fold
+// per sample (16 rows x 2^25 samples: 610 us, 80 us now; the read of the planes
+// takes 20 us).
+// N, L and T are powers of two (L divides N, T divides L), so a thread that
+// strides by PCAL_BLOCKS * PCAL_THREADS = 4096 words (65536 samples >= L) keeps
+// its place in the rotator period.
 CS_DEV int gcd_int(int a, int b) { while (b) { int t = a % b; a = b; b = t; } return a; }
 
-__global__ void k_pcal_fold(const uint8_t* __restrict__ planes, int64_t bytes_per_sub, int nspec, int64_t samp_per_spec,
-                            int N, int ov, int novl, int ns, int rs, int T, int L, const float2* __restrict__ rot,
-                            float l0, float l1, float l2, float l3, const uint32_t* __restrict__ vmask,
-                            float2* __restrict__ partial, int nblk_per_row)
+constexpr int PCAL_THREADS = 128;
+constexpr int PCAL_BLOCKS = 32;
+constexpr int PCAL_POS = 16 * PCAL_THREADS;      // sample positions of a CTA's words
+constexpr int PCAL_PLANES = 12;                  // vertical counter planes above 1, 2 and 4
+
+// full adder on 32 positions: s = a ^ b ^ c, carry = majority
+CS_DEV void csa(uint32_t& carry, uint32_t& s, uint32_t a, uint32_t b)
 {
-    extern __shared__ float2 pacc[];                 // [T][blockDim]
+    const uint32_t u = s;
+    s = u ^ a ^ b;
+    carry = (u & a) | (u & b) | (a & b);
+}
+
+// Vertical counters of 32 positions: weights 1, 2, 4, then 8 2^i in q[i].
+struct VCount {
+    uint32_t one, two, four, q[PCAL_PLANES];
+    CS_DEV void clear()
+    {
+        one = two = four = 0;
+#pragma unroll
+        for (int i = 0; i < PCAL_PLANES; i++) q[i] = 0;
+    }
+    CS_DEV void add8(const uint32_t (&w)[8])
+    {
+        uint32_t t0, t1, f0, f1, e;
+        csa(t0, one, w[0], w[1]);
+        csa(t1, one, w[2], w[3]);
+        csa(f0, two, t0, t1);
+        csa(t0, one, w[4], w[5]);
+        csa(t1, one, w[6], w[7]);
+        csa(f1, two, t0, t1);
+        csa(e, four, f0, f1);
+#pragma unroll
+        for (int i = 0; i < PCAL_PLANES; i++) {
+            const uint32_t t = q[i] & e;
+            q[i] ^= e;
+            e = t;
+        }
+    }
+    CS_DEV int count(int pos) const
+    {
+        int c = (int)((one >> pos) & 1u) + 2 * (int)((two >> pos) & 1u) + 4 * (int)((four >> pos) & 1u);
+#pragma unroll
+        for (int i = 0; i < PCAL_PLANES; i++) c += (int)((q[i] >> pos) & 1u) << (3 + i);
+        return c;
+    }
+};
+// words a thread may add before its counters are emptied (a multiple of 8)
+constexpr int PCAL_BATCH = (8 << PCAL_PLANES) - 8;
+
+// the 16 validity bits of a plane word, each doubled to its code's two bits
+CS_DEV uint32_t double_bits(uint32_t v)
+{
+    v = (v | (v << 8)) & 0x00ff00ffu;
+    v = (v | (v << 4)) & 0x0f0f0f0fu;
+    v = (v | (v << 2)) & 0x33333333u;
+    v = (v | (v << 1)) & 0x55555555u;
+    return v | (v << 1);
+}
+
+template <bool MASK>
+__global__ void __launch_bounds__(PCAL_THREADS) k_pcal_fold(
+    const uint8_t* __restrict__ planes, int64_t bytes_per_sub, int nspec, int64_t samp_per_spec, int N, int ov, int novl,
+    int ns, int rs, int T, int L, const float2* __restrict__ rot, float l0, float l1, float l2, float l3,
+    const uint32_t* __restrict__ vmask, float2* __restrict__ partial)
+{
+    __shared__ int hist[4][PCAL_POS];                // count of each code per position in the period
+    __shared__ double2 sums[PCAL_THREADS];
     const int row = blockIdx.y, sub = row / nspec, spec = row % nspec;
-    const int nt = blockDim.x, tid = threadIdx.x;
-    for (int b = 0; b < T; b++) pacc[b * nt + tid] = make_float2(0.f, 0.f);
+    const int tid = threadIdx.x;
+    const int LB = min(L, PCAL_POS);                 // rotator positions this CTA touches
+    const int LW = max(1, LB / 16);                  // distinct word places among them
+    for (int i = tid; i < 4 * PCAL_POS; i += PCAL_THREADS) (&hist[0][0])[i] = 0;
+    __syncthreads();
     const uint32_t* plane = reinterpret_cast<const uint32_t*>(planes + (int64_t)sub * bytes_per_sub);
     const int step = ov / gcd_int(ns, ov);
     int j0 = -1;
     for (int j = 0; j < step && j < novl; j++)
         if (((int64_t)ns * ((int64_t)spec * novl + j) + rs) % ov == 0) { j0 = j; break; }
     const int cnt = j0 >= 0 ? (novl - 1 - j0) / step + 1 : 0;
-    const int hop = N / ov, wpw = N / 16;            // 32-bit words per window
+    const int wpw = N / 16, lg = 31 - __clz(wpw);    // 32-bit words per window
     const int64_t nwords = (int64_t)cnt * wpw;
-    const float lut[4] = {l0, l1, l2, l3};
-    // Sample j of word wi of a window has rotator index (16 wi + j) mod L and
-    // bin that mod T.  A thread keeps the 16 rotator values and bins of its
-    // current wi in registers and sums each j over the windows in a register,
-    // adding the sums into its shared-memory slots when wi changes (for
-    // N = 65536, whose windows have 4096 words like the 32 x 128 threads of
-    // a row, never: each thread owns one wi).
-    float2 acc[16], rj[16];
-    int bj[16];
-    int cur = -1;
-    auto flush = [&]() {
+    const int64_t base = ((int64_t)spec * samp_per_spec + (int64_t)max(j0, 0) * (N / ov)) / 16;
+    const int64_t win_words = (int64_t)step * (N / ov) / 16;
+    constexpr int STRIDE = PCAL_BLOCKS * PCAL_THREADS;
+    int64_t w = (int64_t)blockIdx.x * PCAL_THREADS + tid;
+    VCount bits, both, val;                          // code bits; their ANDs (two words a set); valid samples
+    while (__syncthreads_or(w < nwords)) {
+        bits.clear(), both.clear(), val.clear();
+        int added = 0;                               // words counted in this batch
+        for (int n = 0; n < PCAL_BATCH && w < nwords; n += 8) {
+            uint32_t x[8], m[8], av[8];
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            if (cur >= 0) {
-                float2& slot = pacc[bj[j] * nt + tid];
-                slot.x += acc[j].x;
-                slot.y += acc[j].y;
+            for (int u = 0; u < 8; u++) {
+                const int64_t wu = w + (int64_t)u * STRIDE;
+                const bool in = wu < nwords;
+                const int64_t wg = base + (wu >> lg) * win_words + (wu & (wpw - 1));
+                x[u] = in ? __ldg(plane + wg) : 0u;
+                m[u] = 0u;
+                if (MASK) {
+                    m[u] = in ? __ldg(vmask + (wg >> 1)) >> ((wg & 1) * 16) & 0xffffu : 0u;
+                } else {
+                    added += in;
+                }
             }
-            acc[j] = make_float2(0.f, 0.f);
-        }
-    };
-    flush();
-    for (int64_t w = (int64_t)blockIdx.x * nt + tid; w < nwords; w += (int64_t)nblk_per_row * nt) {
-        const int win = (int)(w / wpw), wi = (int)(w - (int64_t)win * wpw);
-        if (wi != cur) {
-            flush();
-            cur = wi;
-            int li = (wi * 16) % L, bi = li % T;
+            w += 8 * (int64_t)STRIDE;
+            if (MASK) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                rj[j] = __ldg(rot + li);
-                bj[j] = bi;
-                li++;
-                bi++;
-                if (li == L) li = 0, bi = 0;
-                else if (bi == T) bi = 0;
+                for (int u = 0; u < 8; u++) {
+                    const uint32_t d = double_bits(m[u]);
+                    x[u] &= d;
+                    m[u] = d & 0x55555555u;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) av[u] = u < 4 ? m[2 * u] | (m[2 * u + 1] << 1) : 0u;
+                val.add8(av);
             }
-        }
-        const int64_t wg = ((int64_t)spec * samp_per_spec + (int64_t)(j0 + win * step) * hop) / 16 + wi;
-        const uint32_t word = __ldg(plane + wg);
-        const uint32_t valid = vmask ? __ldg(vmask + (wg >> 1)) >> ((wg & 1) * 16) : 0xffffu;
+            bits.add8(x);
 #pragma unroll
+            for (int u = 0; u < 8; u++)
+                av[u] = u < 4 ? ((x[2 * u] & (x[2 * u] >> 1)) & 0x55555555u) | ((x[2 * u + 1] & (x[2 * u + 1] << 1)) & 0xaaaaaaaau)
+                              : 0u;
+            both.add8(av);
+        }
+        // counts per code, summed over the lanes of the warp at the same place
+        // in the period, then over the CTA
+#pragma unroll 1
         for (int j = 0; j < 16; j++) {
-            const float x = (valid >> j) & 1u ? lut_pick4(lut, (word >> (2 * j)) & 3u) : 0.f;
-            acc[j].x += x * rj[j].x;
-            acc[j].y += x * rj[j].y;
+            const int n01 = both.count(2 * j) + both.count(2 * j + 1);
+            const int n0 = bits.count(2 * j), n1 = bits.count(2 * j + 1);
+            const int nv = MASK ? val.count(2 * j) + val.count(2 * j + 1) : added;
+            int h[4] = {nv - n0 - n1 + n01, n0 - n01, n1 - n01, n01};
+            for (int o = 16; o >= LW; o >>= 1) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) h[c] += __shfl_xor_sync(0xffffffffu, h[c], o);
+            }
+            if ((tid & 31) < LW) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) atomicAdd(&hist[c][(16 * tid + j) & (LB - 1)], h[c]);
+            }
         }
     }
-    flush();
     __syncthreads();
-    for (int b = tid; b < T; b += nt) {
-        float2 s = make_float2(0.f, 0.f);
-        for (int u = 0; u < nt; u++) {
-            float2 v = pacc[b * nt + u];
-            s.x += v.x;
-            s.y += v.y;
+    // levels and rotator: thread t takes the positions t, t + 128, ... (all of
+    // them in bin t % T, as T divides 128), in FP64
+    const double lev[4] = {l0, l1, l2, l3};
+    double2 s = make_double2(0., 0.);
+    for (int i = tid; i < LB; i += PCAL_THREADS) {
+        double x = 0.;
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (hist[c][i]) x += (double)hist[c][i] * lev[c];
+        const float2 r = __ldg(rot + (((int)blockIdx.x * PCAL_POS + i) & (L - 1)));
+        s.x += x * r.x;
+        s.y += x * r.y;
+    }
+    sums[tid] = s;
+    __syncthreads();
+    if (tid < T) {
+        for (int u = tid + T; u < PCAL_THREADS; u += T) {
+            s.x += sums[u].x;
+            s.y += sums[u].y;
         }
-        partial[((int64_t)row * nblk_per_row + blockIdx.x) * T + b] = s;
+        partial[((int64_t)row * PCAL_BLOCKS + blockIdx.x) * T + tid] = make_float2((float)s.x, (float)s.y);
     }
 }
 
-__global__ void k_pcal_reduce(const float2* __restrict__ partial, int rows, int nblk, int T, int ntones,
-                              float2* __restrict__ bins, float2* __restrict__ tones)
+// A CTA per row: bins from the row's partials in CTA order, then the tones
+// DFT(bins)/T in FP64, a warp per tone with the T roots of unity in shared
+// memory.  (One thread per row for all of it, with a double-precision sine and
+// cosine per term, took 868 us at any size; 13 us now.)
+constexpr int PCAL_RED = 128;
+__global__ void __launch_bounds__(PCAL_RED) k_pcal_reduce(const float2* __restrict__ partial, int nblk, int T, int ntones,
+                                                          float2* __restrict__ bins, float2* __restrict__ tones)
 {
-    int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= rows) return;
-    for (int b = 0; b < T; b++) {
+    __shared__ float2 sb[PCAL_RED];
+    __shared__ double2 root[PCAL_RED];
+    const int row = blockIdx.x, tid = threadIdx.x;
+    if (tid < T) {
         float2 s = make_float2(0.f, 0.f);
         for (int u = 0; u < nblk; u++) {
-            float2 v = partial[((int64_t)row * nblk + u) * T + b];
+            const float2 v = partial[((int64_t)row * nblk + u) * T + tid];
             s.x += v.x;
             s.y += v.y;
         }
-        bins[(int64_t)row * T + b] = s;
+        bins[(int64_t)row * T + tid] = s;
+        sb[tid] = s;
+        double sn, cs;
+        sincospi(-2.0 * (double)tid / (double)T, &sn, &cs);
+        root[tid] = make_double2(cs, sn);
     }
     if (!tones) return;
-    for (int k = 0; k < ntones; k++) {
+    __syncthreads();
+    const int lane = tid & 31;
+    for (int k = tid >> 5; k < ntones; k += PCAL_RED / 32) {
         double re = 0, im = 0;
-        for (int n = 0; n < T; n++) {
-            float2 bv = bins[(int64_t)row * T + n];
-            double sn, cs;
-            sincospi(-2.0 * (double)(((int64_t)k * n) % T) / (double)T, &sn, &cs);
-            re += bv.x * cs - bv.y * sn;
-            im += bv.x * sn + bv.y * cs;
+        for (int n = lane; n < T; n += 32) {
+            const double2 w = root[(int)(((int64_t)k * n) % T)];
+            re += sb[n].x * w.x - sb[n].y * w.y;
+            im += sb[n].x * w.y + sb[n].y * w.x;
         }
-        tones[(int64_t)row * ntones + k] = make_float2((float)(re / T), (float)(im / T));
+        for (int o = 16; o; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lane == 0) tones[(int64_t)row * ntones + k] = make_float2((float)(re / T), (float)(im / T));
     }
 }
-
-constexpr int PCAL_THREADS = 128;
-constexpr int PCAL_BLOCKS = 32;
 
 // CELLSPE_SPEC_CTA_FFT=1 selects the shared-memory radix-16 kernel for N =
 // 32768 and 65536 instead of choosing between it and the warp four-step.
@@ -723,8 +846,8 @@ int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st)
     const int novl = a.overlap * a.ffts_per_spectrum - (a.overlap - 1);
     if (!a.skip_power) {
         const float scale = (float)(1.0 / (double)novl);
-        int64_t tot = (int64_t)rows * nb;
-        k_spec_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(a.partial, a.power, rows, nchunk, nb, scale),
+        const int slices = spec_reduce_slices((int64_t)rows * nb, nchunk), bins = RED_THREADS / slices;
+        k_spec_reduce<<<dim3((nb + bins - 1) / bins, rows), dim3(bins, slices), 0, st>>>(a.partial, a.power, nchunk, nb, scale),
             cs_count_launches(1);
         CS_CUDA_TRY(cudaGetLastError());
     }
@@ -736,16 +859,14 @@ int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st)
         if (!rot) return CS_ERR_ARG;
         float2* pp = reinterpret_cast<float2*>(a.partial + power_partial_floats(a));
         int64_t samp_per_spec = (int64_t)a.ffts_per_spectrum * a.N;
-        int nt = PCAL_THREADS;
-        size_t smem = (size_t)T * nt * sizeof(float2);
-        CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_pcal_fold), (int)smem));
         const int ns = a.pcal_sources > 0 ? a.pcal_sources : 1;
-        k_pcal_fold<<<dim3(PCAL_BLOCKS, rows), nt, smem, st>>>(a.planes, a.bytes_per_sub, a.nspec, samp_per_spec, a.N,
+        auto fold = a.valid_mask ? k_pcal_fold<true> : k_pcal_fold<false>;
+        fold<<<dim3(PCAL_BLOCKS, rows), PCAL_THREADS, 0, st>>>(a.planes, a.bytes_per_sub, a.nspec, samp_per_spec, a.N,
                                                                a.overlap, novl, ns, a.pcal_source, T, L, rot, a.lut[0],
-                                                               a.lut[1], a.lut[2], a.lut[3], a.valid_mask, pp,
-                                                               PCAL_BLOCKS), cs_count_launches(1);
+                                                               a.lut[1], a.lut[2], a.lut[3], a.valid_mask, pp),
+            cs_count_launches(1);
         CS_CUDA_TRY(cudaGetLastError());
-        k_pcal_reduce<<<(rows + 63) / 64, 64, 0, st>>>(pp, rows, PCAL_BLOCKS, T, a.ntones, a.pcal_bins, a.pcal_tones), cs_count_launches(1);
+        k_pcal_reduce<<<rows, PCAL_RED, 0, st>>>(pp, PCAL_BLOCKS, T, a.ntones, a.pcal_bins, a.pcal_tones), cs_count_launches(1);
         CS_CUDA_TRY(cudaGetLastError());
     }
     return 0;

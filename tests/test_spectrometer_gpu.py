@@ -219,3 +219,31 @@ def test_pcal_unit_test_recipe_through_the_gpu(cg, slope_deg):
     expect = -90.0 + slope_deg * np.arange(1, ntones)
     err = np.abs((phase - expect + 180) % 360 - 180)
     assert err.max() < 0.1, err
+
+
+@pytest.mark.parametrize("nsub,N,L,T,overlap,K,nspec", [
+    (1, 1024, 1, 1, 1, 3, 1),            # one position, one bin
+    (1, 1024, 8, 4, 2, 5, 2),            # a period shorter than a word
+    (4, 1024, 16, 16, 1, 130, 1),        # a period of one word, more words than one round
+    (1, 2048, 1024, 128, 4, 7, 3),       # more places than a warp has lanes, the most bins
+    (8, 8192, 4096, 32, 2, 9, 2),        # periods longer than a CTA's words
+    (1, 65536, 65536, 64, 2, 3, 1),      # the longest period
+    (1, 65536, 32, 32, 1, 9, 1),         # nine rounds of 4096 words: one past the carry-save group
+])
+def test_pcal_fold_places(cg, orc, nsub, N, L, T, overlap, K, nspec):
+    """Phase-cal bins for rotator lengths on both sides of a word, a warp and a CTA, and the tones of every bin."""
+    fs, ntones = 32e6, T
+    off = fs / L if L > T else 0.0
+    raw = np.random.default_rng(N + L).integers(0, 256, N * K * nspec * nsub // 4, dtype=np.uint8)
+    p = cg.spec_params(N, overlap, 2, K, nspec, nsub, raw.size, tonebins=T, rotatorlen=L, ntones=ntones,
+                       offset_hz=off, fs_hz=fs)
+    power = np.zeros((nsub, nspec, N // 2 + 1), np.float32)
+    bins = np.zeros((nsub, nspec, T), np.complex64)
+    tones = np.zeros((nsub, nspec, ntones), np.complex64)
+    cg.spectrometer(p, raw, power, bins, tones)
+    _, ref_b = _oracle(orc, raw, nsub, N, overlap, 2, K, T, L, off, fs)
+    assert np.linalg.norm(bins - ref_b) / np.linalg.norm(ref_b) < TOL
+    for c in range(nsub):
+        for s in range(nspec):
+            ref_t = orc.pcal_tones(ref_b[c, s], ntones)
+            assert np.linalg.norm(tones[c, s] - ref_t) / np.linalg.norm(ref_t) < TOL
