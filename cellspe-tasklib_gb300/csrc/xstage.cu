@@ -8,7 +8,9 @@
 // rank-K update, so it is tiled like a GEMM: a CTA owns a 64x64 block of
 // (i, j) for one channel and streams 16 time samples per stage through
 // shared memory; each of its 128 threads keeps 4x8 complex accumulators
-// (32x32 blocks of 32 threads when S <= 32).
+// (32x32 blocks of 32 threads when S <= 32).  Arrays of up to 8 inputs go to
+// k_xmac_f32_few, and FX jobs of more to cs_xmac_split (xstage_split.cu); the
+// tiles remain for spectra that the caller brings and for fewer than 24 segments.
 // Only blocks on or below the diagonal are launched.
 //
 // Layout in:  float2 spectra[C][S][K]   (time innermost)
@@ -133,6 +135,81 @@ __global__ void __launch_bounds__(XT * XT / 32) k_xmac_f32(const float2* __restr
     }
 }
 
+// A few inputs (S <= 8): all S(S+1)/2 products of a channel in one pass over
+// its rows, which are read once, coalesced along time.  Bound by that read
+// (2 inputs x 512 channels x 4096 segments: 33.5 MB), where the 32 x 32 tile
+// above would give one warp a channel and its whole time axis in turn (1020 us
+// for those; 9 us here).  NW warps share a channel's time axis; their sums are
+// added by shuffles and then in warp order, so the result is deterministic.
+constexpr int FEW_WARPS = 8;
+template <int S, int NW>
+__global__ void __launch_bounds__(32 * FEW_WARPS) k_xmac_f32_few(const float2* __restrict__ spec, int C, int K, int kp,
+                                                                 float2* __restrict__ vis, int accumulate)
+{
+    constexpr int P = S * (S + 1) / 2;
+    __shared__ float red[FEW_WARPS][2 * P];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x * (FEW_WARPS / NW) + warp / NW;
+    float re[P], im[P];
+#pragma unroll
+    for (int p = 0; p < P; p++) re[p] = im[p] = 0.f;
+    if (c < C) {
+        const float2* base = spec + (int64_t)c * S * kp;
+#pragma unroll(S <= 4 ? 4 : 2)
+        for (int k = (warp % NW) * 32 + lane; k < K; k += 32 * NW) {
+            float2 x[S];
+#pragma unroll
+            for (int s = 0; s < S; s++) x[s] = __ldg(base + (int64_t)s * kp + k);
+#pragma unroll
+            for (int i = 0; i < S; i++)
+#pragma unroll
+                for (int j = 0; j <= i; j++) {
+                    const int p = i * (i + 1) / 2 + j;
+                    re[p] = fmaf(x[i].x, x[j].x, re[p]);
+                    re[p] = fmaf(x[i].y, x[j].y, re[p]);
+                    im[p] = fmaf(x[i].y, x[j].x, im[p]);
+                    im[p] = fmaf(-x[i].x, x[j].y, im[p]);
+                }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            re[p] += __shfl_xor_sync(0xffffffffu, re[p], o);
+            im[p] += __shfl_xor_sync(0xffffffffu, im[p], o);
+        }
+        if (lane == 0) red[warp][2 * p] = re[p], red[warp][2 * p + 1] = im[p];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < (FEW_WARPS / NW) * P; t += 32 * FEW_WARPS) {
+        const int g = t / P, p = t % P, ch = blockIdx.x * (FEW_WARPS / NW) + g;
+        if (ch >= C) continue;
+        float2 v = make_float2(0.f, 0.f);
+        for (int w = g * NW; w < (g + 1) * NW; w++) {
+            v.x += red[w][2 * p];
+            v.y += red[w][2 * p + 1];
+        }
+        float2* o = vis + (int64_t)ch * P + p;
+        if (accumulate) {
+            v.x += o->x;
+            v.y += o->y;
+        }
+        *o = v;
+    }
+}
+
+template <int S>
+void launch_few(const float2* spectra, int C, int K, int kp, float2* vis, int accumulate, cudaStream_t st)
+{
+    // the whole CTA on a channel for long time axes, or where a warp per
+    // channel would not give every SM two CTAs
+    if (K >= 1024 || (K >= 256 && C < 152 * 2 * FEW_WARPS))
+        k_xmac_f32_few<S, FEW_WARPS><<<C, 32 * FEW_WARPS, 0, st>>>(spectra, C, K, kp, vis, accumulate);
+    else
+        k_xmac_f32_few<S, 1><<<(C + FEW_WARPS - 1) / FEW_WARPS, 32 * FEW_WARPS, 0, st>>>(spectra, C, K, kp, vis, accumulate);
+}
+
 __global__ void k_vis_transpose(const float2* __restrict__ in, float2* __restrict__ out, int C, int64_t P)
 {
     __shared__ float2 tile[32][33];
@@ -162,6 +239,20 @@ int cs_xmac_f32(const float2* spectra, int S, int C, int K, int kp, float2* vis,
     int64_t tiles = (int64_t)nb * (nb + 1) / 2;
     int64_t P = (int64_t)S * (S + 1) / 2;
     dim3 grid((unsigned)tiles, C);
+    switch (S) {
+        case 1: launch_few<1>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 2: launch_few<2>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 3: launch_few<3>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 4: launch_few<4>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 5: launch_few<5>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 6: launch_few<6>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 7: launch_few<7>(spectra, C, K, kp, vis, accumulate, st); break;
+        case 8: launch_few<8>(spectra, C, K, kp, vis, accumulate, st); break;
+    }
+    if (S <= 8) {
+        cs_count_launches(1);
+        return (int)cudaGetLastError();
+    }
     if (xt == 32)
         k_xmac_f32<32><<<grid, 32, 0, st>>>(spectra, S, K, kp, vis, P, accumulate);
     else

@@ -44,3 +44,20 @@ def test_xmac_accumulate(cg):
     v2 = v1.copy()
     cg.xmac(spec, S, C, K, v2, accumulate=True)
     assert np.allclose(v2, 2 * v1, rtol=1e-6, atol=1e-5)
+
+
+@pytest.mark.parametrize("C,K", [(1, 1), (9, 31), (17, 255), (16, 256), (3, 1023), (2, 1025), (2433, 257)])
+@pytest.mark.parametrize("S", range(1, 9))
+def test_xmac_few_inputs(cg, S, C, K):
+    """Up to eight inputs: a warp or a CTA per channel, time axes that fill neither, accumulation."""
+    rng = np.random.default_rng(S * 1000 + K)
+    spec = (rng.standard_normal((C, S, K)) + 1j * rng.standard_normal((C, S, K))).astype(np.complex64)
+    i, j = np.tril_indices(S)
+    a = spec.astype(np.complex128)
+    ref = np.matmul(a, a.conj().transpose(0, 2, 1))[:, i, j]
+    vis = np.zeros((C, S * (S + 1) // 2), np.complex64)
+    cg.xmac(spec, S, C, K, vis)
+    # K-term FP32 sums spread over 32 lanes at least: well under 2^-20
+    assert np.linalg.norm(vis - ref) / np.linalg.norm(ref) < 1e-6
+    cg.xmac(spec, S, C, K, vis, accumulate=True)
+    assert np.linalg.norm(vis - 2 * ref) / np.linalg.norm(ref) < 2e-6
