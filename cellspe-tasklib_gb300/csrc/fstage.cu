@@ -32,6 +32,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 
@@ -49,6 +50,57 @@ template <int M> struct FCfg {
     // then advances in lockstep on __syncthreads
     static constexpr bool CTA_BAR = (GROUPS == 1) || (T < 32);
 };
+
+// Eight FP32 values as FP16 terms hi = fp16(s x), lo = fp16(w (s x - hi)), 16 bytes each.
+CS_DEV void split8(const float (&x)[8], float s, float w, uint4& hi, uint4& lo)
+{
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float a = x[2 * u] * s, b = x[2 * u + 1] * s;
+        const __half2 hh = __floats2half2_rn(a, b);
+        const float2 hf = __half22float2(hh);
+        const __half2 ll = __floats2half2_rn(w * (a - hf.x), w * (b - hf.y));
+        h[u] = *reinterpret_cast<const uint32_t*>(&hh);
+        l[u] = *reinterpret_cast<const uint32_t*>(&ll);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// segments the split layout holds: K rounded up to whole 32-segment blocks
+__host__ CS_DEV int split_segments(int K) { return (K + 31) & ~31; }
+
+// segments the kernel's tiles cover
+inline int out_segments(const CsFStageArgs& a) { return a.split > 0.f ? split_segments(a.K) : a.K; }
+
+// Write-out of a FP32 staging tile [M channels][G + 1] (G segments of input s
+// from segment k0) as two FP16 terms in 32-segment blocks (CsFStageArgs::
+// split); segments past K are written as zeros.  A thread takes eight segments
+// of one channel's Re or Im: 16-byte stores, pairs of lanes filling a sector.
+template <int M, int G, int NT>
+CS_DEV void split_writeout(const CsFStageArgs& a, const unsigned char* stage, int s, int k0)
+{
+    constexpr int P8 = G / 8;
+    const int nvalid = max(0, min(G, a.K - k0)), nseg = min(G, split_segments(a.K) - k0);
+    const int S = out_rows(a), blocks = out_pitch(a) / 32;
+    const float* st = reinterpret_cast<const float*>(stage);
+    uint4* out = reinterpret_cast<uint4*>(a.out);
+    for (int idx = threadIdx.x; idx < M * 2 * P8; idx += NT) {
+        const int piece = idx % P8, comp = (idx / P8) & 1, c = idx / (2 * P8);
+        if (8 * piece >= nseg) continue;
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            x[u] = 8 * piece + u < nvalid ? st[2 * (c * (G + 1) + 8 * piece + u) + comp] : 0.f;
+        uint4 hi, lo;
+        split8(x, a.split, a.split_lo, hi, lo);
+        const int k = k0 + 8 * piece;
+        uint4* o = out + (((int64_t)c * S + s) * blocks + k / 32) * 16 + comp * 8 + (k % 32) / 8;
+        o[0] = hi;
+        o[4] = lo;
+    }
+}
 
 template <int M, int FMT>
 constexpr int stage_g()
@@ -278,6 +330,58 @@ int dispatch_fstage(const CsFStageArgs& a, cudaStream_t st)
     return dispatch_fstage2<M, false>(a, st);
 }
 
+// Corner-turned write-out of a staging tile [M channels][G + 1] (G segments of
+// input s from segment k0; FP32 float2 or FP16 half2 Re|Im) into the channel-
+// major layout: F32 float2 rows (c, s), F16 half rows (c, plane, s), pitch KP.
+template <int FMT, int M, int G, int NT>
+CS_DEV void stage_writeout(const CsFStageArgs& a, const unsigned char* stage, int s, int k0)
+{
+    const int nvalid = max(0, min(G, a.K - k0));
+    const int S = out_rows(a), KP = out_pitch(a);
+    if constexpr (FMT == CS_SPECTRA_F32) {
+        if (a.split > 0.f) {
+            split_writeout<M, G, NT>(a, stage, s, k0);
+            return;
+        }
+        const float2* st = reinterpret_cast<const float2*>(stage);
+        float2* out = reinterpret_cast<float2*>(a.out);
+        if (nvalid == G && KP % 2 == 0) {
+            for (int idx = threadIdx.x; idx < M * (G / 2); idx += NT) {
+                const int c = idx / (G / 2), l = 2 * (idx % (G / 2));
+                const float2 x0 = st[c * (G + 1) + l], x1 = st[c * (G + 1) + l + 1];
+                *reinterpret_cast<float4*>(out + ((int64_t)c * S + s) * KP + k0 + l) = make_float4(x0.x, x0.y, x1.x, x1.y);
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < M * G; idx += NT) {
+                const int c = idx / G, l = idx % G;
+                if (l < nvalid) out[((int64_t)c * S + s) * KP + k0 + l] = st[c * (G + 1) + l];
+            }
+        }
+    } else {
+        const __half2* st = reinterpret_cast<const __half2*>(stage);
+        __half* out = reinterpret_cast<__half*>(a.out);
+        if (nvalid == G && KP % 8 == 0) {
+            constexpr int P8 = G / 8;
+            for (int idx = threadIdx.x; idx < M * 2 * P8; idx += NT) {
+                const int piece = idx % P8, plane = (idx / P8) & 1, c = idx / (2 * P8);
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(st + c * (G + 1) + 8 * piece);
+                const uint32_t sel = plane ? 0x7632u : 0x5410u;
+                *reinterpret_cast<uint4*>(out + (((int64_t)c * 2 + plane) * S + s) * KP + k0 + 8 * piece) =
+                    make_uint4(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel),
+                               __byte_perm(w[4], w[5], sel), __byte_perm(w[6], w[7], sel));
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < M * 2 * G; idx += NT) {
+                const int l = idx % G, plane = (idx / G) & 1, c = idx / (2 * G);
+                if (l < nvalid) {
+                    const __half2 x = st[c * (G + 1) + l];
+                    out[(((int64_t)c * 2 + plane) * S + s) * KP + k0 + l] = plane ? __high2half(x) : __low2half(x);
+                }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // N = 2048 fast path: one warp per segment.
 // The 1024-point complex FFT of z[n] = x[2n] + i x[2n+1] runs as a 32 x 32
@@ -316,7 +420,7 @@ template <int N_PENDING>
 CS_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_PENDING) : "memory"); }
 
 template <int FMT, bool PHASE, int WARPS, int ROUNDS, int G>
-__global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16) ? 1 : (WARPS == 8) ? 2 : 3) k_fx_fstage_w2048(const __grid_constant__ CsFStageArgs a, const float2* __restrict__ tw)
+__global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16 || (FMT == CS_SPECTRA_F32 && G == 16)) ? 1 : (WARPS == 8) ? 2 : 3) k_fx_fstage_w2048(const __grid_constant__ CsFStageArgs a, const float2* __restrict__ tw)
 {
     constexpr int M = 1024, N = 2048, NT = 32 * WARPS, PER = G / WARPS;
     static_assert(G % WARPS == 0 && G % 8 == 0, "segments per CTA");
@@ -480,20 +584,7 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16) ? 1 : (WAR
     const int nvalid = max(0, min(G, a.K - k0));
     const int S = out_rows(a), KP = out_pitch(a);      // output layout
     if constexpr (FMT == CS_SPECTRA_F32) {
-        const float2* st = reinterpret_cast<const float2*>(stage);
-        float2* out = reinterpret_cast<float2*>(a.out);
-        if (nvalid == G && KP % 2 == 0) {
-            for (int idx = threadIdx.x; idx < M * (G / 2); idx += NT) {
-                const int c = idx / (G / 2), l = 2 * (idx % (G / 2));
-                const float2 x0 = st[c * (G + 1) + l], x1 = st[c * (G + 1) + l + 1];
-                *reinterpret_cast<float4*>(out + ((int64_t)c * S + s) * KP + k0 + l) = make_float4(x0.x, x0.y, x1.x, x1.y);
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < M * G; idx += NT) {
-                const int c = idx / G, l = idx % G;
-                if (l < nvalid) out[((int64_t)c * S + s) * KP + k0 + l] = st[c * (G + 1) + l];
-            }
-        }
+        stage_writeout<FMT, M, G, NT>(a, stage, s, k0);
     } else {
         const __half2* st = reinterpret_cast<const __half2*>(stage);
         __half* out = reinterpret_cast<__half*>(a.out);
@@ -535,7 +626,7 @@ int launch_w2048_variant(const CsFStageArgs& a, const float2* tw, cudaStream_t s
     size_t smem = w2048_smem<FMT, WARPS, G>();
     auto kern = k_fx_fstage_w2048<FMT, PHASE, WARPS, ROUNDS, G>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
-    dim3 grid((a.K + G * ROUNDS - 1) / (G * ROUNDS), a.S);
+    dim3 grid((out_segments(a) + G * ROUNDS - 1) / (G * ROUNDS), a.S);
     kern<<<grid, 32 * WARPS, smem, st>>>(a, tw), cs_count_launches(1);
     return (int)cudaGetLastError();
 }
@@ -624,6 +715,10 @@ int launch_w2048(const CsFStageArgs& a, cudaStream_t st)
 {
     const float2* tw = cs_twiddles(2048);
     if (!tw) return CS_ERR_ARG;
+    // two FP16 terms: 16 segments per CTA (8 warps, 2 each; the FP32 staging
+    // tile of 32 would not fit), so each plane's run of a block is a whole sector
+    if constexpr (FMT == CS_SPECTRA_F32)
+        if (a.split > 0.f) return launch_w2048_variant<FMT, PHASE, 8, 1, 16>(a, tw, st);
     const char* env = getenv("CELLSPE_FSTAGE_VARIANT");
     if (env && env[0] >= '1' && env[0] <= '0' + W_NVARIANTS)
         return launch_w2048_choice<FMT, PHASE>(env[0] - '0', a, tw, st);
@@ -921,54 +1016,6 @@ int dispatch_wbig(const CsFStageArgs& a, cudaStream_t st)
 // The two half-warps of a warp fill staging columns 16 apart, so their
 // stores fall in disjoint banks.  LSB-first input only.
 // ---------------------------------------------------------------------------
-// Corner-turned write-out of a staging tile [M channels][G + 1] (G segments of
-// input s from segment k0; FP32 float2 or FP16 half2 Re|Im) into the channel-
-// major layout: F32 float2 rows (c, s), F16 half rows (c, plane, s), pitch KP.
-template <int FMT, int M, int G, int NT>
-CS_DEV void stage_writeout(const CsFStageArgs& a, const unsigned char* stage, int s, int k0)
-{
-    const int nvalid = max(0, min(G, a.K - k0));
-    const int S = out_rows(a), KP = out_pitch(a);
-    if constexpr (FMT == CS_SPECTRA_F32) {
-        const float2* st = reinterpret_cast<const float2*>(stage);
-        float2* out = reinterpret_cast<float2*>(a.out);
-        if (nvalid == G && KP % 2 == 0) {
-            for (int idx = threadIdx.x; idx < M * (G / 2); idx += NT) {
-                const int c = idx / (G / 2), l = 2 * (idx % (G / 2));
-                const float2 x0 = st[c * (G + 1) + l], x1 = st[c * (G + 1) + l + 1];
-                *reinterpret_cast<float4*>(out + ((int64_t)c * S + s) * KP + k0 + l) = make_float4(x0.x, x0.y, x1.x, x1.y);
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < M * G; idx += NT) {
-                const int c = idx / G, l = idx % G;
-                if (l < nvalid) out[((int64_t)c * S + s) * KP + k0 + l] = st[c * (G + 1) + l];
-            }
-        }
-    } else {
-        const __half2* st = reinterpret_cast<const __half2*>(stage);
-        __half* out = reinterpret_cast<__half*>(a.out);
-        if (nvalid == G && KP % 8 == 0) {
-            constexpr int P8 = G / 8;
-            for (int idx = threadIdx.x; idx < M * 2 * P8; idx += NT) {
-                const int piece = idx % P8, plane = (idx / P8) & 1, c = idx / (2 * P8);
-                const uint32_t* w = reinterpret_cast<const uint32_t*>(st + c * (G + 1) + 8 * piece);
-                const uint32_t sel = plane ? 0x7632u : 0x5410u;
-                *reinterpret_cast<uint4*>(out + (((int64_t)c * 2 + plane) * S + s) * KP + k0 + 8 * piece) =
-                    make_uint4(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel),
-                               __byte_perm(w[4], w[5], sel), __byte_perm(w[6], w[7], sel));
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < M * 2 * G; idx += NT) {
-                const int l = idx % G, plane = (idx / G) & 1, c = idx / (2 * G);
-                if (l < nvalid) {
-                    const __half2 x = st[c * (G + 1) + l];
-                    out[(((int64_t)c * 2 + plane) * S + s) * KP + k0 + l] = plane ? __high2half(x) : __low2half(x);
-                }
-            }
-        }
-    }
-}
-
 constexpr int H_G = 64, H_TP = 17, H_RAWC = 512 / 64 + 2, H_RAWW = 4 * H_RAWC;
 
 template <int FMT>
@@ -1119,7 +1166,7 @@ int launch_w512(const CsFStageArgs& a, cudaStream_t st)
     const size_t smem = w512_smem<FMT>();
     auto kern = k_fx_fstage_w512<FMT, PHASE>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
-    kern<<<dim3((a.K + H_G - 1) / H_G, a.S), 256, smem, st>>>(a, nullptr), cs_count_launches(1);
+    kern<<<dim3((out_segments(a) + H_G - 1) / H_G, a.S), 256, smem, st>>>(a, nullptr), cs_count_launches(1);
     return (int)cudaGetLastError();
 }
 
@@ -1328,7 +1375,7 @@ int launch_w1024(const CsFStageArgs& a, cudaStream_t st)
     auto kern = k_fx_fstage_w1024<FMT, PHASE>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
     constexpr int G = w1024_g<FMT>();
-    kern<<<dim3((a.K + G - 1) / G, a.S), 256, smem, st>>>(a, nullptr), cs_count_launches(1);
+    kern<<<dim3((out_segments(a) + G - 1) / G, a.S), 256, smem, st>>>(a, nullptr), cs_count_launches(1);
     return (int)cudaGetLastError();
 }
 
@@ -1396,11 +1443,26 @@ int cs_fstage_layout(const CsFStageArgs& a)
     return e && (e[0] == '0' || e[0] == '1') ? 1 : 2;
 }
 
+float cs_fstage_split_scale(const CsFStageArgs& a)
+{
+    if (a.format != CS_SPECTRA_F32 || a.msb_first) return 0.f;
+    const char* gen = getenv("CELLSPE_FSTAGE_GENERIC");
+    if (gen && gen[0] == '1') return 0.f;
+    float m = 0.f;
+    for (float l : a.lut) {
+        if (!std::isfinite(l)) return 0.f;
+        m = std::max(m, std::fabs(l));
+    }
+    if (!(m > 1e-15f && m < 1e15f)) return 0.f;
+    return std::ldexp(1.f, (int)std::floor(std::log2(32768.0 / ((double)a.N * m))));
+}
+
 int cs_fx_fstage(const CsFStageArgs& a, cudaStream_t st)
 {
     if (!a.raw || !a.out || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
     if ((uintptr_t)a.raw % 16 || a.bytes_per_input % 16 || (uintptr_t)a.out % 16) return CS_ERR_ARG;
     if (a.kblock < 0 || a.kblock > 2 || (a.kblock && !cs_fstage_kblocked(a))) return CS_ERR_ARG;
+    if (a.split > 0.f && !a.seg_major && (!cs_fstage_split_scale(a) || (a.kp ? a.kp : a.K) % 32)) return CS_ERR_ARG;
     // channel-grouped k-blocked spectra: only the warp-specialised form writes them
     if (a.kblock == 2) return cs_fstage_tc32_supported(a) ? cs_fx_fstage_tc32(a, st, true) : CS_ERR_ARG;
     // The tensor-core F stage is opt-in (CELLSPE_FSTAGE_TC=1, read per call):
@@ -1541,14 +1603,55 @@ __global__ void __launch_bounds__(256) k_transpose_f32(const float2* __restrict_
     }
 }
 
+// [S][K][C] float2 -> two FP16 terms in 32-segment blocks (CsFStageArgs::
+// split).  Bound by the copy (8 bytes in and out per value).  A CTA takes 64
+// segments x 32 channels: 256-byte reads along the channels, and per channel
+// two blocks of 256 contiguous bytes, a thread writing eight segments of one
+// plane pair (hi, lo) in 16-byte stores.  Segments past K are written as zeros up
+// to the end of their block.
+constexpr int TC = 32;
+__global__ void __launch_bounds__(256) k_transpose_split(const float2* __restrict__ in, int K, int C, int kp, int S_out,
+                                                         uint4* __restrict__ out, float scale, float lo_weight)
+{
+    __shared__ float tile[2][TC][TT + 1];            // Re, Im: [channel][segment]
+    const int s = blockIdx.z, k0 = blockIdx.y * TT, c0 = blockIdx.x * TC;
+    for (int i = threadIdx.x; i < TT * TC; i += 256) {
+        const int cc = i % TC, kk = i / TC, k = k0 + kk, c = c0 + cc;
+        const float2 x = (k < K && c < C) ? in[((int64_t)s * K + k) * C + c] : make_float2(0.f, 0.f);
+        tile[0][cc][kk] = x.x;
+        tile[1][cc][kk] = x.y;
+    }
+    __syncthreads();
+    const int nseg = split_segments(K) - k0;
+    for (int i = threadIdx.x; i < TC * 2 * (TT / 8); i += 256) {
+        const int piece = i % (TT / 8), comp = (i / (TT / 8)) & 1, cc = i / (2 * (TT / 8)), c = c0 + cc;
+        if (c >= C || 8 * piece >= nseg) continue;
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = tile[comp][cc][8 * piece + u];
+        uint4 hi, lo;
+        split8(x, scale, lo_weight, hi, lo);
+        const int k = k0 + 8 * piece;
+        uint4* o = out + (((int64_t)c * S_out + s) * (kp / 32) + k / 32) * 16 + comp * 8 + (k % 32) / 8;
+        o[0] = hi;
+        o[4] = lo;
+    }
+}
+
 }  // namespace
 
-int cs_spectra_transpose(const void* tmp, int S, int K, int C, int kp, int S_out, int format, void* out, cudaStream_t st)
+int cs_spectra_transpose(const void* tmp, int S, int K, int C, int kp, int S_out, int format, void* out, cudaStream_t st,
+                         float split, float split_lo)
 {
     if (!tmp || !out || S <= 0 || K <= 0 || C <= 0 || kp < K || S_out < S || S > 65535) return CS_ERR_ARG;
     const dim3 grid((C + TT - 1) / TT, (K + TT - 1) / TT, S);
     if (grid.y > 65535) return CS_ERR_ARG;
-    if (format == CS_SPECTRA_F32) {
+    if (split > 0.f) {
+        if (format != CS_SPECTRA_F32 || kp % 32 || (uintptr_t)out % 16) return CS_ERR_ARG;
+        k_transpose_split<<<dim3((C + TC - 1) / TC, (K + TT - 1) / TT, S), 256, 0, st>>>((const float2*)tmp, K, C, kp, S_out,
+                                                                                       (uint4*)out, split, split_lo),
+            cs_count_launches(1);
+    } else if (format == CS_SPECTRA_F32) {
         k_transpose_f32<<<grid, 256, 0, st>>>((const float2*)tmp, K, C, kp, S_out, (float2*)out), cs_count_launches(1);
     } else {
         if ((uintptr_t)out % 4 || kp % 2) return CS_ERR_ARG;

@@ -73,6 +73,12 @@ struct CsFStageArgs {
                                 // makes the channel-major layout (the generic kernels only)
     int kblock;                 // F16 only: 1 k-blocked rows, 2 channel-grouped k-blocked
                                 // rows; see cs_fstage_layout
+    float split;                // F32 only: 0 float2 rows; else the power of two that scales
+                                // the spectra into two FP16 terms for cs_xmac_split: half
+                                // [C][S_out][kp/32][2][64] (kp % 32 == 0), planes Re and Im
+                                // of 32 hi and 32 lo halves, zero from segment K to the next
+                                // multiple of 32
+    float split_lo;             // weight of the lo term (cs_xmac_split_lo)
 };
 int cs_fx_fstage(const CsFStageArgs& a, cudaStream_t st);
 // Per host thread: whether the 2048-point F stage may time its schedules on
@@ -99,10 +105,16 @@ bool cs_fstage_kblocked(const CsFStageArgs& a);
 // starts at c0 * S_out * kp * 4 bytes in both k-blocked layouts.
 int cs_fstage_layout(const CsFStageArgs& a);
 // Segment-major spectra [S][K][C] (tmp) -> the X stage's layout at out:
-// F32 float2 rows (c, s), F16 half rows (c, plane, s); row pitch kp, S_out
+// F32 float2 rows (c, s) or, with split > 0, their two FP16 terms
+// (CsFStageArgs::split); F16 half rows (c, plane, s); row pitch kp, S_out
 // inputs per (c[, plane]) block (tmp and out already offset to the block).
 int cs_spectra_transpose(const void* tmp, int S, int K, int C, int kp, int S_out, int format, void* out,
-                         cudaStream_t st);
+                         cudaStream_t st, float split = 0.f, float split_lo = 1.f);
+// The scale for CsFStageArgs::split: the power of two that brings the largest
+// spectrum value N samples of these levels can give (N max|level|) just below
+// 2^15; 0 when the F stage cannot write the two terms for these arguments
+// (MSB-first input or the generic kernel), or the levels have no such scale.
+float cs_fstage_split_scale(const CsFStageArgs& a);
 // fstage_tc.cu: the N = 2048 FP16-output F stage on the tensor cores (both
 // DFT passes as tcgen05 MMAs).  cs_fx_fstage uses it for those arguments
 // when the environment sets CELLSPE_FSTAGE_TC=1.
@@ -125,6 +137,12 @@ int cs_fstage_tc32_status(unsigned* code);
 // [C][P], P = S(S+1)/2, p = i(i+1)/2 + j (j <= i), V = sum_k X_i conj(X_j).
 int cs_xmac_f32(const float2* spectra, int S, int C, int K, int kp, float2* vis, int accumulate,
                 cudaStream_t st);
+// FP32 X stage on the tensor cores from spectra as two FP16 terms
+// (CsFStageArgs::split, scale 1 / inv_scale) -> vis float2 [C][P].
+int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, cudaStream_t st);
+float cs_xmac_split_lo(int S);       // the lo term's weight it expects for S inputs
+// Error code of the last cs_xmac_split launch (0 = ok), after its stream has synchronised.
+int cs_xmac_split_status(unsigned* code);
 // Tensor-core (tcgen05, FP16 in, FP32 accumulate) X stage:
 // spectra __half [C][2][S][kp] (K used; kp % 8 == 0), or k-blocked
 // [C][S][kp/32][2][32] with kblock = 1 (K, kp % 32 == 0), or channel-grouped

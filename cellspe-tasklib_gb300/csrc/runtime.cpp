@@ -448,6 +448,14 @@ int op_xmac_i8(Workspace& ws, bool host, const void* planes, const float* scale,
 // for the X stage's TMA loads and costs at most 25% memory at K = 256 (1.6%
 // at K = 4096).
 long long spectra_pitch(long long K) { return K >= 256 ? K + 64 : K; }
+// FP32 jobs of at least SPLIT_MIN_K segments (whose X stage may take its spectra as
+// two FP16 terms in 32-segment blocks) round it up to whole blocks.
+constexpr int SPLIT_MIN_K = 24, SPLIT_MIN_S = 9;
+long long spectra_pitch(long long K, int x_mode)
+{
+    const long long kp = spectra_pitch(K);
+    return x_mode == CELLSPE_X_FP32 && K >= SPLIT_MIN_K ? (kp + 31) / 32 * 32 : kp;
+}
 
 long long fx_bytes(const cellspe_fx_params* p, bool with_poly)
 {
@@ -458,7 +466,7 @@ long long fx_bytes(const cellspe_fx_params* p, bool with_poly)
     if (host) b += align256(S * p->bytes_per_input);
     if (with_poly) b += align256(S * 32) + 3 * align256(S * K * 4);
     const bool f32 = p->x_mode != CELLSPE_X_TC_FP16;   // FP32 spectra (FP32 and INT8 X stages)
-    b += align256(C * S * spectra_pitch(K) * (f32 ? 8 : 4));
+    b += align256(C * S * spectra_pitch(K, p->x_mode) * (f32 ? 8 : 4));
     if (N >= 4096) b += align256(C * S * K * (f32 ? 8 : 4));   // segment-major spectra
     if (p->x_mode == CELLSPE_X_INT8) b += align256(C * 2 * S * spectra_pitch(K)) + align256(S * C * 4);
     bool stage_vis = host || p->vis_order == CELLSPE_VIS_BASELINE_MAJOR || p->accumulate;
@@ -558,8 +566,14 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         }
         d_inv_scale = inv;
     }
-    const int kp = (int)spectra_pitch(K);
+    const int kp = (int)spectra_pitch(K, p->x_mode);
     fa.kp = kp;
+    // FP32 X stage: on the tensor cores from spectra as two FP16 terms, except
+    // for arrays of a few inputs (cs_xmac_f32 reads each row once there: 2 inputs
+    // x 512 channels x 4096 segments 9 us) and for fewer segments than most of a
+    // 32-segment block
+    if (p->x_mode == CELLSPE_X_FP32 && S >= SPLIT_MIN_S && K >= SPLIT_MIN_K) fa.split = cs_fstage_split_scale(fa);
+    fa.split_lo = cs_xmac_split_lo(S);
     // FP16, N = 2048: 128-byte runs per 32 segments, k-blocked (1) or
     // channel-grouped k-blocked (2, the warp-specialised F stage)
     fa.kblock = cs_fstage_layout(fa);
@@ -590,12 +604,14 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         }
         void* rows_out = fb.out;
         if (segmaj) {
+            fb.split = 0.f;
             fb.seg_major = 1;
             fb.out = seg_tmp + s0 * K * C * seg_bytes;
         }
         int rc = map_rc(cs_fx_fstage(fb, ws.stream), "F stage");
         if (!rc && segmaj)
-            rc = map_rc(cs_spectra_transpose(fb.out, (int)(s1 - s0), K, C, kp, S, fa.format, rows_out, ws.stream),
+            rc = map_rc(cs_spectra_transpose(fb.out, (int)(s1 - s0), K, C, kp, S, fa.format, rows_out, ws.stream, fa.split,
+                                             fa.split_lo),
                         "spectra transpose");
         if (rc) j.err = rc;
     }
@@ -628,7 +644,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         const long long c0 = cbound(b), c1 = cbound(b + 1), cn = c1 - c0;
         if (cn <= 0) continue;
         int rc;
-        if (p->x_mode == CELLSPE_X_FP32)
+        if (fa.split > 0.f)
+            rc = cs_xmac_split((const char*)fa.out + c0 * S * kp * 8, S, (int)cn, K, kp, vis_cp + c0 * P, 1.f / fa.split,
+                               ws.stream);
+        else if (p->x_mode == CELLSPE_X_FP32)
             rc = cs_xmac_f32((const float2*)fa.out + c0 * S * kp, S, (int)cn, K, kp, vis_cp + c0 * P, 0, ws.stream);
         else if (p->x_mode == CELLSPE_X_INT8)
             rc = cs_xmac_i8(i8_planes + c0 * 2 * S * kp, S, (int)cn, K, kp, vis_cp + c0 * P, i8_scale + c0, C, 0,
@@ -691,6 +710,11 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         else if (cs_xmac_tc_status(&code) != 0 || code != 0)
             rc = set_err(CELLSPE_ERR_CUDA, "X stage: tensor-core pipeline wait timed out (code " +
                                                std::to_string(code) + ")");
+    }
+    if (sync && !rc && fa.split > 0.f) {
+        unsigned code = 0;
+        if (cs_xmac_split_status(&code) != 0 || code != 0)
+            rc = set_err(CELLSPE_ERR_CUDA, "X stage: tensor-core pipeline wait timed out (code " + std::to_string(code) + ")");
     }
     if (sync && !rc) {
         for (int i = 0; i < 4; i++) {

@@ -251,3 +251,55 @@ def test_fx_warp_fstages_delay_model(cg, orc, N, K, monkeypatch):
     cg.fx_correlate(cg.fx_params(S, N, K, raw.shape[1], x_mode=cg.X_TC_FP16, **kw), raw, gtc, delay_poly=poly)
     assert _rel(tc, gtc) < 1e-3
     assert _rel(tc, ref) < 1e-3
+
+
+def _vis_f64(orc, raw, S, N, K, start=0, state=(None, None, None), lut=None):
+    """[C][P] FP64 visibilities, channel-major."""
+    kw = {} if lut is None else {"lut": lut}
+    X = orc.fx_spectra_f64(raw, S, N, K, start, *state, **kw)             # [S][K][C]
+    A = np.ascontiguousarray(X.transpose(2, 0, 1))
+    i, j = np.tril_indices(S)
+    return np.matmul(A, A.conj().transpose(0, 2, 1))[:, i, j]
+
+
+@pytest.mark.parametrize("S,N,K", [
+    (8, 512, 96), (9, 512, 23),                      # a few inputs; fewer segments than the two-term form takes
+    (9, 512, 24), (16, 512, 33), (17, 1024, 64), (32, 2048, 65),      # one row quarter, partial 32-segment blocks
+    (33, 2048, 48), (64, 1024, 40), (65, 512, 100), (128, 512, 31),   # one tile of 64 and 128 rows
+    (129, 512, 40), (200, 2048, 32), (257, 512, 25),                  # off-diagonal tiles, ragged last rows
+    (40, 4096, 40), (12, 8192, 70), (10, 32768, 24)])                 # segment-major spectra
+def test_fx_fp32_split_sizes(cg, orc, S, N, K):
+    """FP32 jobs on both sides of every size the X stage's forms change at, against FP64."""
+    import synth
+
+    T = (N * K + 5 + 63) // 64 * 64
+    raw = synth.stations_offset_binary(S, T, rho=0.2, seed=S + N)
+    p = cg.fx_params(S, N, K, raw.shape[1], start_sample=5)
+    vis = np.zeros((N // 2, S * (S + 1) // 2), np.complex64)
+    cg.fx_correlate(p, raw, vis)
+    # FP32 rounding of an N-point transform and of K-term sums: a few 2^-24, 2e-6 at most
+    assert _rel(vis, _vis_f64(orc, raw, S, N, K, 5)) < 2e-6
+
+
+@pytest.mark.parametrize("N", [512, 1024, 2048, 4096])
+def test_fx_fp32_split_delay_levels(cg, orc, N):
+    """The same with a delay model, large custom levels and a full-scale tone (the largest spectrum value of these levels)."""
+    import synth
+
+    S, K, fs, lo, margin = 20, 70, 32e6, 1e6, 2048
+    T = N * K + 2 * margin
+    raw = synth.stations_offset_binary(S, T, rho=0.3, seed=N)
+    raw[3] = 0b11000011                              # codes 3, 0, 0, 3: +-level square wave, one channel takes N max|level| / sqrt 2
+    poly = np.zeros((S, 4))
+    rng = np.random.default_rng(N)
+    poly[:, 0] = rng.uniform(-30e-6, 30e-6, S)
+    poly[:, 1] = rng.uniform(-3e-6, 3e-6, S)
+    levels = np.array([-3.0e4, -1.1e4, 0.9e4, 3.1e4], np.float32)
+    p = cg.fx_params(S, N, K, raw.shape[1], start_sample=margin, fs_hz=fs, lo_hz=lo, custom_levels=levels)
+    vis = np.zeros((N // 2, S * (S + 1) // 2), np.complex64)
+    cg.fx_correlate(p, raw, vis, delay_poly=poly)
+    ref = _vis_f64(orc, raw, S, N, K, margin, orc.delay_state_f64(poly, N, K, fs, lo), levels)
+    i, j = np.tril_indices(S)
+    for q in (i != 3) & (j != 3), (i == 3) & (j != 3):        # the tone's own products do not hide the others
+        # the phasor's angle is FP32: up to N/2 dphase rad, 2^-24 of a few hundred rad
+        assert _rel(vis[:, q], ref[:, q]) < TOL
