@@ -73,7 +73,6 @@ constexpr int B_B1FULL0 = 0, B_B1FULL1 = 1, B_D1FULL = 2, B_EPI1 = 3, B_D2FULL =
 // error codes
 constexpr unsigned E_MMA_WAIT = 1, E_WORKER_WAIT = 2, E_STORE_WAIT = 3;
 
-__device__ unsigned g_fstc_error;
 
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 
@@ -188,9 +187,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
             const uint32_t id2 = tc::idesc_f16(128, 32, false, false, false);
             bool ok = true;
             for (int j = 0; j < nunits && ok; j++) {
-                ok = tc::mbar_wait(bar(j & 1), (uint32_t)(j >> 1) & 1, &g_fstc_error, E_MMA_WAIT, WAIT_CYCLES);
+                ok = tc::mbar_wait(bar(j & 1), (uint32_t)(j >> 1) & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 if (ok && j > 0)
-                    ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)(j - 1) & 1, &g_fstc_error, E_MMA_WAIT, WAIT_CYCLES);
+                    ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)(j - 1) & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 if (!ok) break;
                 tc::fence_after();
                 const uint32_t b1 = sbase + OFF_B1 + (uint32_t)(j & 1) * B1_BYTES;
@@ -202,9 +201,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
                     tc::mma_f16(tmem, da, db, id1, kk ? 1u : 0u);
                 }
                 tc::commit(bar(B_D1FULL));
-                ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)j & 1, &g_fstc_error, E_MMA_WAIT, WAIT_CYCLES);
+                ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)j & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 if (ok && j > 0)
-                    ok = tc::mbar_wait(bar(B_EPI2), (uint32_t)(j - 1) & 1, &g_fstc_error, E_MMA_WAIT, WAIT_CYCLES);
+                    ok = tc::mbar_wait(bar(B_EPI2), (uint32_t)(j - 1) & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 if (!ok) break;
                 tc::fence_after();
 #pragma unroll
@@ -220,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
             }
             // completes once every MMA issued above has finished
             tc::commit(bar(B_DRAIN));
-            tc::mbar_wait(bar(B_DRAIN), 0, &g_fstc_error, E_MMA_WAIT, WAIT_CYCLES);
+            tc::mbar_wait(bar(B_DRAIN), 0, a.err, E_MMA_WAIT, WAIT_CYCLES);
         }
         __syncwarp();
     } else if (warp == 9) {
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
         // rows); STORED completes once the buffer has been read.
         if (lane == 0) {
             for (int j = 0; j < nunits; j++) {
-                if (!tc::mbar_wait(bar(B_REPACK), (uint32_t)j & 1, &g_fstc_error, E_STORE_WAIT, WAIT_CYCLES)) break;
+                if (!tc::mbar_wait(bar(B_REPACK), (uint32_t)j & 1, a.err, E_STORE_WAIT, WAIT_CYCLES)) break;
                 const uint32_t u = blockIdx.x + (uint32_t)j * gridDim.x;      // 32-bit: no FP64-assisted division
                 const int s = (int)(u / (uint32_t)args.units_k), k0 = (int)(u % (uint32_t)args.units_k) * G;
                 const uint32_t src = sbase + OFF_B1 + (uint32_t)(j & 1) * B1_BYTES;
@@ -331,7 +330,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
             unit_of(j, s, k0);
 
             // ---- epilogue 1: Y -> Z = Y W_2048^(n2 k1) -> A2 (FP16) ----
-            ok = tc::mbar_wait(bar(B_D1FULL), (uint32_t)j & 1, &g_fstc_error, E_WORKER_WAIT, WAIT_CYCLES);
+            ok = tc::mbar_wait(bar(B_D1FULL), (uint32_t)j & 1, a.err, E_WORKER_WAIT, WAIT_CYCLES);
             if (!worker_vote(ok)) { ok = false; break; }
             tc::fence_after();
             {
@@ -381,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
 
             if (j + 1 < nunits) {
                 // sample buffer (j+1) & 1 held unit j-1's spectra for the store warp
-                ok = j == 0 || tc::mbar_wait(bar(B_STORED), (uint32_t)(j - 1) & 1, &g_fstc_error, E_WORKER_WAIT,
+                ok = j == 0 || tc::mbar_wait(bar(B_STORED), (uint32_t)(j - 1) & 1, a.err, E_WORKER_WAIT,
                                              WAIT_CYCLES);
                 if (!worker_vote(ok)) { ok = false; break; }
                 cp_async_wait_all();
@@ -393,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
             if (j + 2 < nunits) fetch(j + 2);
 
             // ---- epilogue 2: X -> phasor, scale -> FP16 staging ----
-            ok = tc::mbar_wait(bar(B_D2FULL), (uint32_t)j & 1, &g_fstc_error, E_WORKER_WAIT, WAIT_CYCLES);
+            ok = tc::mbar_wait(bar(B_D2FULL), (uint32_t)j & 1, a.err, E_WORKER_WAIT, WAIT_CYCLES);
             if (!worker_vote(ok)) { ok = false; break; }          // (also: staging is free again)
             tc::fence_after();
             __half2* stg = reinterpret_cast<__half2*>(sm + OFF_STG);
@@ -529,7 +528,7 @@ int cs_fx_fstage_tc(const CsFStageArgs& a, cudaStream_t st)
 {
     if (!cs_fstage_tc_supported(a)) return CS_ERR_UNSUPPORTED;
     if ((int64_t)a.S * ((a.K + G - 1) / G) >= (int64_t)1 << 31) return CS_ERR_UNSUPPORTED;   // 32-bit unit indices
-    if (!a.raw || !a.out || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
+    if (!a.raw || !a.out || !a.err || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
     if ((uintptr_t)a.raw % 16 || a.bytes_per_input % 16 || (uintptr_t)a.out % 16) return CS_ERR_ARG;
     const uint4* consts = tc_constants();
     if (!consts) return (int)cudaErrorMemoryAllocation;
@@ -554,9 +553,6 @@ int cs_fx_fstage_tc(const CsFStageArgs& a, cudaStream_t st)
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
         CUDA_SUCCESS)
         return CS_ERR_ARG;
-    void* errp = nullptr;
-    CS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_fstc_error));
-    CS_CUDA_TRY(cudaMemsetAsync(errp, 0, sizeof(unsigned), st));
     TcFArgs t{};
     t.f = a;
     t.consts = consts;
@@ -571,9 +567,4 @@ int cs_fx_fstage_tc(const CsFStageArgs& a, cudaStream_t st)
         k_fx_fstage_tc<false><<<grid, THREADS, SMEM_BYTES, st>>>(t, tm), cs_count_launches(1);
     }
     return (int)cudaGetLastError();
-}
-
-int cs_fstage_tc_status(unsigned* code)
-{
-    return (int)cudaMemcpyFromSymbol(code, g_fstc_error, sizeof(unsigned));
 }

@@ -103,7 +103,6 @@ constexpr int B_B1FULL = 0, B_D1FULL = 1, B_EPI1 = 2, B_D2FULL0 = 3, B_EPI2_0 = 
 // error codes
 constexpr unsigned E_MMA_WAIT = 1, E_WORKER_WAIT = 2;
 
-__device__ unsigned g_fst32_error;
 
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 static_assert(OFF_B1 % 1024 == 0 && OFF_A2 % 1024 == 0 && OFF_A2P % 1024 == 0 && A2P_REGION % 1024 == 0,
@@ -232,7 +231,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
                 const int b = j & 1;
                 // B1 holds quad j (decoded after epilogue 1 of quad j-1, which
                 // freed D1 buffer b of quad j-2)
-                ok = tc::mbar_wait(bar(B_B1FULL), (uint32_t)j & 1, &g_fst32_error, E_MMA_WAIT, WAIT_CYCLES);
+                ok = tc::mbar_wait(bar(B_B1FULL), (uint32_t)j & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 if (!ok) break;
                 tc::fence_after();
                 const uint32_t b1 = sbase + OFF_B1;
@@ -245,10 +244,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
                 }
                 tc::commit(bar(B_D1FULL));
                 // A2 buffer b (and the quad's A2' rows) written by epilogue 1 of quad j
-                ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)j & 1, &g_fst32_error, E_MMA_WAIT, WAIT_CYCLES);
+                ok = tc::mbar_wait(bar(B_EPI1), (uint32_t)j & 1, a.err, E_MMA_WAIT, WAIT_CYCLES);
                 // D2 buffer b free: epilogue 2 of quad j-2 done
                 if (ok && j >= 2)
-                    ok = tc::mbar_wait(bar(B_EPI2_0 + b), (uint32_t)((j - 2) >> 1) & 1, &g_fst32_error, E_MMA_WAIT,
+                    ok = tc::mbar_wait(bar(B_EPI2_0 + b), (uint32_t)((j - 2) >> 1) & 1, a.err, E_MMA_WAIT,
                                        WAIT_CYCLES);
                 if (!ok) break;
                 tc::fence_after();
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
                     // previous unit's epilogue 2' is done
                     const int u = j / QUADS;
                     if (u >= 1)
-                        ok = tc::mbar_wait(bar(B_EPI2P), (uint32_t)(u - 1) & 1, &g_fst32_error, E_MMA_WAIT,
+                        ok = tc::mbar_wait(bar(B_EPI2P), (uint32_t)(u - 1) & 1, a.err, E_MMA_WAIT,
                                            WAIT_CYCLES);
                     if (!ok) break;
                     tc::fence_after();
@@ -280,7 +279,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
             }
             // completes once every MMA issued above has finished
             tc::commit(bar(B_DRAIN));
-            tc::mbar_wait(bar(B_DRAIN), 0, &g_fst32_error, E_MMA_WAIT, WAIT_CYCLES);
+            tc::mbar_wait(bar(B_DRAIN), 0, a.err, E_MMA_WAIT, WAIT_CYCLES);
         }
         __syncwarp();
     } else {
@@ -410,12 +409,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
             cp_async_wait_all();
             ok = true;
             if (tid == 0) {
-                if (do1) ok = tc::mbar_wait(bar(B_D1FULL), (uint32_t)j & 1, &g_fst32_error, E_WORKER_WAIT, WAIT_CYCLES);
+                if (do1) ok = tc::mbar_wait(bar(B_D1FULL), (uint32_t)j & 1, a.err, E_WORKER_WAIT, WAIT_CYCLES);
                 if (ok && do2)
-                    ok = tc::mbar_wait(bar(B_D2FULL0 + (jj & 1)), (uint32_t)(jj >> 1) & 1, &g_fst32_error,
+                    ok = tc::mbar_wait(bar(B_D2FULL0 + (jj & 1)), (uint32_t)(jj >> 1) & 1, a.err,
                                        E_WORKER_WAIT, WAIT_CYCLES);
                 if (ok && uend)
-                    ok = tc::mbar_wait(bar(B_D2PFULL), (uint32_t)(jj / QUADS) & 1, &g_fst32_error, E_WORKER_WAIT,
+                    ok = tc::mbar_wait(bar(B_D2PFULL), (uint32_t)(jj / QUADS) & 1, a.err, E_WORKER_WAIT,
                                        WAIT_CYCLES);
             }
             if (!worker_vote(ok)) { ok = false; break; }
@@ -713,7 +712,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_fx_fstage_tc32ws(const __grid
     };
     // a group leader's bounded wait (the group then votes on the outcome)
     auto lwait = [&](int i, uint32_t parity) {
-        return tc::mbar_wait(bar(i), parity, &g_fst32_error, E_WORKER_WAIT, WAIT_CYCLES);
+        return tc::mbar_wait(bar(i), parity, a.err, E_WORKER_WAIT, WAIT_CYCLES);
     };
     // channel-grouped k-blocked spectra: the 128-byte run of (channel c,
     // input s, 32-segment block kb), in runs of 64 halves
@@ -747,7 +746,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_fx_fstage_tc32ws(const __grid
             const uint32_t id1 = tc::idesc_f16(128, 128, false, false, true);
             const uint32_t id2 = tc::idesc_f16(128, 64, false, false, false);
             auto w = [&](int i, uint32_t ph) {
-                return tc::mbar_wait(bar(i), ph, &g_fst32_error, E_MMA_WAIT, WAIT_CYCLES);
+                return tc::mbar_wait(bar(i), ph, a.err, E_MMA_WAIT, WAIT_CYCLES);
             };
             // pass 1 of quad j: B1 -> D1[j & 1].  D1[j & 1] was last read by
             // epilogue 1 for quad j - 2, whose completion pass 2 of quad j - 2
@@ -795,7 +794,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_fx_fstage_tc32ws(const __grid
                 }
             }
             tc::commit(bar(WB_DRAIN));
-            tc::mbar_wait(bar(WB_DRAIN), 0, &g_fst32_error, E_MMA_WAIT, WAIT_CYCLES);
+            tc::mbar_wait(bar(WB_DRAIN), 0, a.err, E_MMA_WAIT, WAIT_CYCLES);
         }
         __syncwarp();
     } else if (warp < WS_E2) {
@@ -1213,7 +1212,7 @@ int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised)
     // the warp-specialised form writes the channel-grouped layout, the lockstep form layout 1
     if (a.kblock != (specialised ? 2 : 1)) return CS_ERR_ARG;
     if ((int64_t)a.S * (a.K / US) >= (int64_t)1 << 31) return CS_ERR_UNSUPPORTED;   // unit indices are 32-bit
-    if (!a.raw || !a.out || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
+    if (!a.raw || !a.out || !a.err || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
     if ((uintptr_t)a.raw % 16 || a.bytes_per_input % 16 || (uintptr_t)a.out % 16) return CS_ERR_ARG;
     const uint4* consts = tc32_constants();
     if (!consts) return (int)cudaErrorMemoryAllocation;
@@ -1223,9 +1222,6 @@ int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised)
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         g_sms32 = n > 0 ? n : 148;
     }
-    void* errp = nullptr;
-    CS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_fst32_error));
-    CS_CUDA_TRY(cudaMemsetAsync(errp, 0, sizeof(unsigned), st));
     Tc32Args t{};
     t.f = a;
     t.consts = consts;
@@ -1248,9 +1244,4 @@ int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised)
         kern<<<grid, THREADS, SMEM_BYTES, st>>>(t), cs_count_launches(1);
     }
     return (int)cudaGetLastError();
-}
-
-int cs_fstage_tc32_status(unsigned* code)
-{
-    return (int)cudaMemcpyFromSymbol(code, g_fst32_error, sizeof(unsigned));
 }

@@ -41,6 +41,14 @@ int cs_rfft_batch(const float* in, float2* out, int n, int64_t batch, cudaStream
 int cs_perm_pack(const float2* bins, float* out, int n, int64_t batch, cudaStream_t st);
 
 // fstage.cu -----------------------------------------------------------------
+// Error record of a job's tensor-core kernels (bounded waits that ran out),
+// in device memory: kernels take the address of `code`, which they set once, and
+// copy it to *host (page-locked; may be null).  Zeroed again by whoever found an error.
+struct alignas(16) CsErrorWord {
+    unsigned code, pad;
+    unsigned* host;
+};
+
 struct CsDelayState {       // per (input, segment)
     int32_t* shift;         // integer sample shift
     float* phase0;          // fringe phase, radians in [0, 2 pi)
@@ -79,6 +87,7 @@ struct CsFStageArgs {
                                 // of 32 hi and 32 lo halves, zero from segment K to the next
                                 // multiple of 32
     float split_lo;             // weight of the lo term (cs_xmac_split_lo)
+    unsigned* err;              // CsErrorWord::code of the job (tensor-core F stages)
 };
 int cs_fx_fstage(const CsFStageArgs& a, cudaStream_t st);
 // Per host thread: whether the 2048-point F stage may time its schedules on
@@ -120,9 +129,6 @@ float cs_fstage_split_scale(const CsFStageArgs& a);
 // when the environment sets CELLSPE_FSTAGE_TC=1.
 bool cs_fstage_tc_supported(const CsFStageArgs& a);
 int cs_fx_fstage_tc(const CsFStageArgs& a, cudaStream_t st);
-// Error code of the last tensor-core F-stage launch (0 = ok; 1, 2 = a wait
-// timed out).  Call after the stream has synchronised.
-int cs_fstage_tc_status(unsigned* code);
 // fstage_tc32.cu: the N = 2048 tensor-core F stage with 32-segment units and
 // k-blocked FP16 output (kblock = 1, K and kp multiples of 32), real-input
 // symmetry halving the CUDA-core twiddle work; `specialised` selects the
@@ -130,7 +136,6 @@ int cs_fstage_tc_status(unsigned* code);
 // unless CELLSPE_FSTAGE_TC32 is 0 (the warp FFT) or 1 (the lockstep form).
 bool cs_fstage_tc32_supported(const CsFStageArgs& a);
 int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised = false);
-int cs_fstage_tc32_status(unsigned* code);
 
 // xstage.cu -----------------------------------------------------------------
 // FP32 CUDA-core X stage: spectra float2 [C][S][kp] (K used) -> vis float2
@@ -139,17 +144,16 @@ int cs_xmac_f32(const float2* spectra, int S, int C, int K, int kp, float2* vis,
                 cudaStream_t st);
 // FP32 X stage on the tensor cores from spectra as two FP16 terms
 // (CsFStageArgs::split, scale 1 / inv_scale) -> vis float2 [C][P].
-int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, cudaStream_t st);
+int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err,
+                  cudaStream_t st);
 float cs_xmac_split_lo(int S);       // the lo term's weight it expects for S inputs
-// Error code of the last cs_xmac_split launch (0 = ok), after its stream has synchronised.
-int cs_xmac_split_status(unsigned* code);
 // Tensor-core (tcgen05, FP16 in, FP32 accumulate) X stage:
 // spectra __half [C][2][S][kp] (K used; kp % 8 == 0), or k-blocked
 // [C][S][kp/32][2][32] with kblock = 1 (K, kp % 32 == 0), or channel-grouped
 // k-blocked with kblock = 2 (C % 16 == 0; see cs_fstage_layout) -> vis
 // float2 [C][P]; inv_scale [S*C] or null.
 int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis, const float* inv_scale,
-                   int scale_stride, int accumulate, cudaStream_t st,
+                   int scale_stride, int accumulate, unsigned* err, cudaStream_t st,
                    int kblock = 0);   // inv_scale[s * scale_stride + c]
 // INT8 X stage (legacy mma.sync IMMA: tcgen05 has no kind::i8 on sm_103a),
 // int32 accumulate: planes int8 [C][2][S][kp] (K, kp % 32 == 0, K <= 65536),
@@ -158,9 +162,6 @@ int cs_xmac_i8(const int8_t* planes, int S, int C, int K, int kp, float2* vis, c
                   int accumulate, cudaStream_t st);
 // FP32 spectra [C][S][kp] -> int8 planes [C][2][S][kp], per-row max-abs scale [S][C].
 int cs_quantise_i8(const float2* spectra, int S, int C, int K, int kp, int8_t* planes, float* scale, cudaStream_t st);
-// Error code of the last tensor-core X-stage launch (0 = ok; 1..3 = a
-// pipeline wait timed out).  Call after the launching stream has synchronised.
-int cs_xmac_tc_status(unsigned* code);
 // Batched service jobs: job b's inputs are rows off .. off + S - 1 of a stacked
 // job whose channel-major triangle is src [C][P_stacked]; its own triangle goes to
 // dst ([C][P] or, baseline_major, [P][C]).

@@ -171,6 +171,10 @@ struct Workspace {
     cudaEvent_t ev_legacy = nullptr;  // ordering after the legacy default stream
     Arena arena;
     bool own_stream = true;
+    // error records of the job's tensor-core kernels, F stage and X stage, in
+    // device memory, and the page-locked words they reach the host through
+    CsErrorWord* d_err = nullptr;
+    volatile unsigned* h_err = nullptr;
     struct Out { void* host; const void* dev; size_t bytes; };
     std::vector<Out> outs;
     int init()
@@ -187,7 +191,41 @@ struct Workspace {
         for (auto& ev : cev)
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_legacy, cudaEventDisableTiming);
-        return e == cudaSuccess ? 0 : cuda_fail(e, "stream setup");
+        if (e == cudaSuccess) e = init_errors();
+        if (e == cudaSuccess) return 0;
+        destroy();
+        return cuda_fail(e, "stream setup");
+    }
+    cudaError_t init_errors()
+    {
+        void *d = nullptr, *h = nullptr, *hd = nullptr;
+        cudaError_t e = cudaHostAlloc(&h, 2 * sizeof(unsigned), cudaHostAllocMapped);
+        if (e != cudaSuccess) return e;
+        h_err = static_cast<unsigned*>(h);
+        h_err[0] = h_err[1] = 0;
+        e = cudaMalloc(&d, 2 * sizeof(CsErrorWord));
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&hd, h, 0);
+        d_err = static_cast<CsErrorWord*>(d);
+        const CsErrorWord w[2] = {{0, 0, static_cast<unsigned*>(hd)}, {0, 0, static_cast<unsigned*>(hd) + 1}};
+        if (e == cudaSuccess) e = cudaMemcpy(d, w, sizeof w, cudaMemcpyHostToDevice);
+        return e;
+    }
+    unsigned* f_err() const { return &d_err[0].code; }
+    unsigned* x_err() const { return &d_err[1].code; }
+    // Before a job: clears what an earlier one that was not waited for may have left.
+    void clear_errors()
+    {
+        if (!h_err[0] && !h_err[1]) return;
+        for (int i = 0; i < 2; i++) cudaMemsetAsync(&d_err[i].code, 0, sizeof(unsigned), stream), h_err[i] = 0;
+    }
+    // After a job's stream has synchronised: the error of its tensor-core kernels, cleared.
+    int check_errors(const std::string& who)
+    {
+        const unsigned f = h_err[0], x = h_err[1];
+        if (!f && !x) return 0;
+        clear_errors();
+        return set_err(CELLSPE_ERR_CUDA, who + (f ? "F stage" : "X stage") + ": tensor-core pipeline wait timed out (code " +
+                                             std::to_string(f ? f : x) + ")");
     }
     // The library's streams are non-blocking, so a call that reads device
     // buffers first waits (on the device, not the host) for everything issued
@@ -214,6 +252,8 @@ struct Workspace {
             if (ev) cudaEventDestroy(ev), ev = nullptr;
         for (auto& ev : cev)
             if (ev) cudaEventDestroy(ev), ev = nullptr;
+        if (d_err) cudaFree(d_err), d_err = nullptr;
+        if (h_err) cudaFreeHost(const_cast<unsigned*>(h_err)), h_err = nullptr;
         if (copy) cudaStreamSynchronize(copy), cudaStreamDestroy(copy), copy = nullptr;
         if (stream && own_stream) cudaStreamDestroy(stream);
         stream = nullptr;
@@ -222,7 +262,19 @@ struct Workspace {
 };
 
 thread_local std::unique_ptr<Workspace> t_ws;
-thread_local float t_stage_ms[4] = {0, 0, 0, 0};   // delay model, F stage, X stage, output
+// Stage times of the thread's last blocking FX job (delay model, F stage, X
+// stage, output), read from the events of its workspace when they are asked for.
+thread_local float t_stage_ms[4] = {0, 0, 0, 0};
+thread_local Workspace* t_stage_ws = nullptr;      // set while the events have not been read
+void read_stage_times()
+{
+    if (!t_stage_ws) return;
+    for (int i = 0; i < 4; i++) {
+        float ms = 0.f;
+        t_stage_ms[i] = cudaEventElapsedTime(&ms, t_stage_ws->sev[i], t_stage_ws->sev[i + 1]) == cudaSuccess ? ms : -1.f;
+    }
+    t_stage_ws = nullptr;
+}
 
 Workspace* thread_ws(int* rc)
 {
@@ -241,12 +293,18 @@ long long budget_bytes()
 }
 
 // Admission limit for one job: an explicit budget is a hard per-job cap;
-// otherwise 90% of free device memory plus what this workspace already holds.
-long long job_limit(const Workspace& ws)
+// otherwise 90% of free device memory plus what this workspace already holds,
+// so a job of `need` bytes that the workspace already has room for is within it
+// without asking the driver (which takes longer than a small job).
+bool over_limit(const Workspace& ws, long long need, long long* limit = nullptr)
 {
-    long long b = g_budget.load();
-    if (b > 0) return b;
-    return budget_bytes() + (long long)ws.arena.capacity();
+    long long lim = g_budget.load();
+    if (lim <= 0) {
+        if (need <= (long long)ws.arena.capacity()) return false;
+        lim = budget_bytes() + (long long)ws.arena.capacity();
+    }
+    if (limit) *limit = lim;
+    return need > lim;
 }
 
 // Staging helper: host buffers are copied through the workspace; device
@@ -410,17 +468,13 @@ int op_xmac_f16(Workspace& ws, bool host, const void* spectra, int S, int C, int
     Job j(ws, host);
     const void* d_sp = j.in(spectra, (size_t)C * 2 * S * K * 2);
     void* d_vis = j.out(vis, (size_t)C * P * 8, accumulate != 0);
+    ws.clear_errors();
     if (!j.err) {
-        int rc = map_rc(cs_xmac_tc_f16(d_sp, S, C, K, K, (float2*)d_vis, nullptr, 0, accumulate, ws.stream), "xmac_f16");
+        int rc = map_rc(cs_xmac_tc_f16(d_sp, S, C, K, K, (float2*)d_vis, nullptr, 0, accumulate, ws.x_err(), ws.stream), "xmac_f16");
         if (rc) j.err = rc;
     }
     int rc = j.finish();
-    if (!rc) {
-        unsigned code = 0;
-        if (cs_xmac_tc_status(&code) != 0 || code != 0)
-            rc = set_err(CELLSPE_ERR_CUDA, "xmac_f16: tensor-core pipeline wait timed out (code " + std::to_string(code) + ")");
-    }
-    return rc;
+    return rc ? rc : ws.check_errors("xmac_f16: ");
 }
 
 int op_xmac_i8(Workspace& ws, bool host, const void* planes, const float* scale, int S, int C, int K, void* vis,
@@ -493,8 +547,8 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     float lut[4];
     if (!pick_levels(p->levels, p->custom_levels, lut)) return set_err(CELLSPE_ERR_ARG, "fx: unknown level table");
     long long need = fx_bytes(p, poly != nullptr);
-    long long budget = job_limit(ws);
-    if (need > budget)
+    long long budget = 0;
+    if (over_limit(ws, need, &budget))
         return set_err(CELLSPE_ERR_NOMEM, "fx: job needs " + std::to_string(need) + " device bytes, budget " +
                                               std::to_string(budget));
     const bool host = p->memory == CELLSPE_MEM_HOST;
@@ -533,8 +587,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             ws.chain->valid = cudaEventRecord(ws.chain->in_done, ws.copy) == cudaSuccess;
         }
     }
+    ws.clear_errors();
     if (sync) cudaEventRecord(ws.sev[0], ws.stream);
     CsFStageArgs fa{};
+    fa.err = ws.f_err();
     fa.raw = d_raw;
     fa.bytes_per_input = p->bytes_per_input;
     fa.S = S; fa.N = N; fa.K = K;
@@ -646,7 +702,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         int rc;
         if (fa.split > 0.f)
             rc = cs_xmac_split((const char*)fa.out + c0 * S * kp * 8, S, (int)cn, K, kp, vis_cp + c0 * P, 1.f / fa.split,
-                               ws.stream);
+                               ws.x_err(), ws.stream);
         else if (p->x_mode == CELLSPE_X_FP32)
             rc = cs_xmac_f32((const float2*)fa.out + c0 * S * kp, S, (int)cn, K, kp, vis_cp + c0 * P, 0, ws.stream);
         else if (p->x_mode == CELLSPE_X_INT8)
@@ -654,7 +710,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
                             ws.stream);
         else
             rc = cs_xmac_tc_f16((const uint16_t*)fa.out + c0 * 2 * S * kp, S, (int)cn, K, kp, vis_cp + c0 * P,
-                                d_inv_scale ? d_inv_scale + c0 : nullptr, C, 0, ws.stream, fa.kblock);
+                                d_inv_scale ? d_inv_scale + c0 : nullptr, C, 0, ws.x_err(), ws.stream, fa.kblock);
         rc = map_rc(rc, "X stage");
         if (!rc && stream_out) {
             cudaError_t e = cudaEventRecord(ws.cev[PIPE_IN + b], ws.stream);
@@ -675,7 +731,8 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     if (!direct && !stream_out && !j.err) {
         float2* result = vis_cp;
         if (p->vis_order == CELLSPE_VIS_BASELINE_MAJOR) {
-            float2* t = (float2*)j.scratch((size_t)C * P * 8);
+            // straight into the caller's device buffer where nothing is added to it
+            float2* t = !host && !p->accumulate ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
             if (!j.err) {
                 int rc = map_rc(cs_vis_to_baseline_major(vis_cp, t, C, P, ws.stream), "transpose");
                 if (rc) j.err = rc;
@@ -691,9 +748,6 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
                 }
             } else if (host) {
                 ws.outs.push_back({vis, result, (size_t)C * P * 8});
-            } else {
-                cudaError_t e = cudaMemcpyAsync(vis, result, (size_t)C * P * 8, cudaMemcpyDeviceToDevice, ws.stream);
-                if (e != cudaSuccess) j.err = cuda_fail(e, "result copy");
             }
         }
     }
@@ -701,27 +755,8 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     // after a failure the copy stream may still hold copies into the workspace
     if (nsc > 1 && j.err) cudaStreamSynchronize(ws.copy);
     int rc = j.finish(sync);
-    if (sync && !rc && p->x_mode == CELLSPE_X_TC_FP16) {
-        unsigned code = 0;
-        unsigned code32 = 0;
-        if (cs_fstage_tc_status(&code) != 0 || code != 0 || cs_fstage_tc32_status(&code32) != 0 || code32 != 0)
-            rc = set_err(CELLSPE_ERR_CUDA, "F stage: tensor-core pipeline wait timed out (code " +
-                                               std::to_string(code | code32) + ")");
-        else if (cs_xmac_tc_status(&code) != 0 || code != 0)
-            rc = set_err(CELLSPE_ERR_CUDA, "X stage: tensor-core pipeline wait timed out (code " +
-                                               std::to_string(code) + ")");
-    }
-    if (sync && !rc && fa.split > 0.f) {
-        unsigned code = 0;
-        if (cs_xmac_split_status(&code) != 0 || code != 0)
-            rc = set_err(CELLSPE_ERR_CUDA, "X stage: tensor-core pipeline wait timed out (code " + std::to_string(code) + ")");
-    }
-    if (sync && !rc) {
-        for (int i = 0; i < 4; i++) {
-            float ms = 0.f;
-            t_stage_ms[i] = cudaEventElapsedTime(&ms, ws.sev[i], ws.sev[i + 1]) == cudaSuccess ? ms : -1.f;
-        }
-    }
+    if (sync && !rc) rc = ws.check_errors("");
+    if (sync && !rc) t_stage_ws = &ws;
     return rc;
 }
 
@@ -948,7 +983,7 @@ int op_mark5b_decode(Workspace& ws, bool host, const void* framed, long long byt
     if (int rc = m5b_check(framed, bytes, nchan, "mark5b_decode")) return rc;
     if (!out || nsamp <= 0) return set_err(CELLSPE_ERR_ARG, "mark5b_decode: bad output");
     const long long need = (host ? align256(bytes) + align256(nsamp * nchan * 4) : 0) + align256(bytes / M5B_FRAME * 8) + 512;
-    if (need > job_limit(ws)) return set_err(CELLSPE_ERR_NOMEM, "mark5b_decode: job exceeds the device memory budget");
+    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "mark5b_decode: job exceeds the device memory budget");
     cellspe_mark5b_info tmp{};
     if (!info) info = &tmp;
     Job j(ws, host);
@@ -970,7 +1005,7 @@ int op_vdif_decode(Workspace& ws, bool host, const void* framed, long long bytes
     if (nchan < 4 && nchan > 0 && nsamp % (4 / nchan))
         return set_err(CELLSPE_ERR_ARG, "vdif_decode: nsamp must be a multiple of the samples per byte");
     const long long need = (host ? align256(bytes) + align256(nsamp * nchan * 4) : 0) + align256(bytes / 24 * 8) + 768;
-    if (need > job_limit(ws)) return set_err(CELLSPE_ERR_NOMEM, "vdif_decode: job exceeds the device memory budget");
+    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "vdif_decode: job exceeds the device memory budget");
     cellspe_vdif_info tmp{};
     if (!info) info = &tmp;
     Job j(ws, host);
@@ -1026,7 +1061,7 @@ int op_mark5b_deframe(Workspace& ws, bool host, const void* framed, long long by
     const long long mwords_max = (nmax * spf + 31) / 32;
     const long long need = (host ? align256(bytes) + align256(nmax * M5B_PAYLOAD) + align256(mwords_max * 4) : 0) +
                            align256(nmax * 8) + 256;
-    if (need > job_limit(ws)) return set_err(CELLSPE_ERR_NOMEM, "mark5b_deframe: job exceeds the device memory budget");
+    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "mark5b_deframe: job exceeds the device memory budget");
     cellspe_mark5b_info tmp{};
     if (!info) info = &tmp;
     Job j(ws, host);
@@ -1042,7 +1077,7 @@ int op_vdif_deframe(Workspace& ws, bool host, const void* framed, long long byte
     if (!framed) return set_err(CELLSPE_ERR_ARG, "vdif_deframe: null input");
     if (frames < 0) return set_err(CELLSPE_ERR_ARG, "vdif_deframe: negative frame count");
     const long long need = (host ? 2 * align256(bytes) + align256(bytes / 4 + 4) : 0) + align256(bytes / 24 * 8) + 512;
-    if (need > job_limit(ws)) return set_err(CELLSPE_ERR_NOMEM, "vdif_deframe: job exceeds the device memory budget");
+    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "vdif_deframe: job exceeds the device memory budget");
     cellspe_vdif_info tmp{};
     if (!info) info = &tmp;
     Job j(ws, host);
@@ -1221,8 +1256,7 @@ int op_spectrometer(Workspace& ws, const cellspe_spec_params* p, const void* raw
     float lut[4];
     if (!pick_levels(p->levels, p->custom_levels, lut)) return set_err(CELLSPE_ERR_ARG, "spectrometer: unknown level table");
     long long need = spec_bytes(p);
-    long long budget = job_limit(ws);
-    if (need > budget) return set_err(CELLSPE_ERR_NOMEM, "spectrometer: job exceeds the device memory budget");
+    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "spectrometer: job exceeds the device memory budget");
     const bool host = p->memory == CELLSPE_MEM_HOST;
     Job j(ws, host);
     const SpecPlanes sp = spec_planes(ws, j, p, raw);
@@ -1268,7 +1302,7 @@ int op_spectrometer_xpol(Workspace& ws, const cellspe_spec_params* p, const void
     if (p->pcal_tonebins > 0 && !pcal_bins) return set_err(CELLSPE_ERR_ARG, "spectrometer_xpol: pcal enabled without pcal_bins");
     float lut[4];
     if (!pick_levels(p->levels, p->custom_levels, lut)) return set_err(CELLSPE_ERR_ARG, "spectrometer_xpol: unknown level table");
-    if (spec_xpol_bytes(p) > job_limit(ws))
+    if (over_limit(ws, spec_xpol_bytes(p)))
         return set_err(CELLSPE_ERR_NOMEM, "spectrometer_xpol: job exceeds the device memory budget");
     const bool host = p->memory == CELLSPE_MEM_HOST;
     const int N = p->fft_points, nb = N / 2 + 1, nspec = p->n_spectra;
@@ -2184,6 +2218,7 @@ long long cellspe_kernel_launches(void) { return cs_launch_count(); }
 int cellspe_last_stage_times(float* ms, int n)
 {
     if (!ms || n < 0) return CELLSPE_ERR_ARG;
+    read_stage_times();
     for (int i = 0; i < n && i < 4; i++) ms[i] = t_stage_ms[i];
     return 0;
 }
@@ -2369,6 +2404,7 @@ int cellspe_fx_correlate_async(const cellspe_fx_params* p, const void* raw, cons
 int cellspe_release_workspace(void)
 {
     if (t_ws) {
+        read_stage_times();
         t_ws->destroy();
         t_ws.reset();
     }

@@ -53,6 +53,19 @@ __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t par
     return ok != 0;
 }
 
+// Error record of a launch (CsErrorWord): the first code stays in the device
+// word, and reaches the host through its page-locked mirror, so that a launch
+// without an error costs neither a reset nor a copy.
+__device__ __forceinline__ void record_error(unsigned* err, unsigned code)
+{
+    atomicCAS(err, 0u, code);
+    unsigned* host = *reinterpret_cast<unsigned* const*>(err + 2);
+    if (host) {
+        *reinterpret_cast<volatile unsigned*>(host) = code;
+        __threadfence_system();
+    }
+}
+
 // Bounded wait on phase `parity`: false (and `code` recorded in *err) after
 // `limit` cycles.  Between checks of the bound the thread sleeps in
 // try_wait (at most 0.1 ms at a time) instead of spinning.
@@ -63,7 +76,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
     const long long t0 = clock64();
     while (!mbar_try_wait_suspend(bar, parity, 100000u)) {
         if (clock64() - t0 > limit) {
-            atomicCAS(err, 0u, code);
+            record_error(err, code);
             return false;
         }
     }

@@ -67,13 +67,6 @@ constexpr long long WAIT_CYCLES = 4000000000LL;     // ~2 s at 2 GHz
 constexpr float GRAM_BIAS = 1.30e-7f, TILE_BIAS = 2.17e-7f;
 constexpr unsigned ERR_FULL_WAIT = 1, ERR_EMPTY_WAIT = 2, ERR_ACC_WAIT = 3, ERR_DRAIN_WAIT = 4;
 
-__device__ unsigned g_split_error;
-
-CS_DEV bool mbar_wait(uint32_t bar, uint32_t parity, unsigned code)
-{
-    return tc::mbar_wait(bar, parity, &g_split_error, code, WAIT_CYCLES);
-}
-
 // K-major operand of 128-byte rows; a descriptor's low 14 bits hold the address / 16,
 // so an offset within the operand ring is added to them
 CS_DEV uint64_t sw128_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 8 * ROW_BYTES, tc::SW128); }
@@ -102,6 +95,7 @@ struct SplitArgs {
     float2* vis;
     float inv;                  // 1 / s: every product is scaled by inv twice
     int stages;
+    unsigned* err;              // CsErrorWord::code of the job
     uint32_t plane_bytes;       // k_xmac_split: one plane of an operand, box rows x 128 bytes
 };
 
@@ -110,17 +104,19 @@ constexpr int BAR_BYTES = (2 * MAX_STAGES + 5) * 8 + 16;
 
 // The barriers and TMEM of a CTA, and the two roles both kernels share.
 struct Pipe {
+    unsigned* err;                                   // CsErrorWord::code of the job
     uint32_t full0, empty0, accf, acce, done, tmem;
     int stages;
 };
 
 // One CTA's set-up: barriers (E epilogue warps release an accumulator), TMEM.
 template <int E, int ISSUERS>
-CS_DEV Pipe pipe_open(unsigned char* after, int stages, uint32_t tmem_cols, const CUtensorMap* tmap)
+CS_DEV Pipe pipe_open(unsigned char* after, int stages, uint32_t tmem_cols, unsigned* err, const CUtensorMap* tmap)
 {
     uint64_t* bars = reinterpret_cast<uint64_t*>(after);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 5);
     Pipe p;
+    p.err = err;
     p.stages = stages;
     p.full0 = tc::smem_u32(bars);
     p.empty0 = p.full0 + 8 * MAX_STAGES;
@@ -155,7 +151,7 @@ CS_DEV void produce(const Pipe& p, int nk, uint32_t bytes, Load load)
     int issued = 0, s = 0;
     uint32_t ph = 1;
     for (int kc = 0; kc < nk; kc++) {
-        if (!mbar_wait(p.empty0 + 8 * s, ph, ERR_EMPTY_WAIT)) break;
+        if (!tc::mbar_wait(p.empty0 + 8 * s, ph, p.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) break;
         tc::mbar_expect_tx(p.full0 + 8 * s, bytes);
         load(kc, s, p.full0 + 8 * s);
         issued = kc + 1;
@@ -163,7 +159,7 @@ CS_DEV void produce(const Pipe& p, int nk, uint32_t bytes, Load load)
     }
     // every stage this thread filled must have landed before the CTA exits
     for (int kc = (issued > p.stages ? issued - p.stages : 0); kc < issued; kc++)
-        mbar_wait(p.full0 + 8 * (kc % p.stages), (kc / p.stages) & 1, ERR_DRAIN_WAIT);
+        tc::mbar_wait(p.full0 + 8 * (kc % p.stages), (kc / p.stages) & 1, p.err, ERR_DRAIN_WAIT, WAIT_CYCLES);
 }
 
 // MMA issuer (one thread): `mmas(stage, buffer)` issues the MMAs of the chunks
@@ -173,8 +169,8 @@ CS_DEV void issue(const Pipe& p, int nk, int first, int step, Mmas mmas)
 {
     for (int kc = first; kc < nk; kc += step) {
         const int b = kc & 1, s = kc % p.stages;
-        if (!mbar_wait(p.acce + 8 * b, ((kc >> 1) & 1) ^ 1, ERR_ACC_WAIT)) break;
-        if (!mbar_wait(p.full0 + 8 * s, (kc / p.stages) & 1, ERR_FULL_WAIT)) break;
+        if (!tc::mbar_wait(p.acce + 8 * b, ((kc >> 1) & 1) ^ 1, p.err, ERR_ACC_WAIT, WAIT_CYCLES)) break;
+        if (!tc::mbar_wait(p.full0 + 8 * s, (kc / p.stages) & 1, p.err, ERR_FULL_WAIT, WAIT_CYCLES)) break;
         tc::fence_after();
         mmas(s, b);
         tc::commit(p.empty0 + 8 * s);
@@ -182,7 +178,7 @@ CS_DEV void issue(const Pipe& p, int nk, int first, int step, Mmas mmas)
     }
     // TMEM is freed only after every MMA issued has finished
     tc::commit(p.done);
-    mbar_wait(p.done, 0, ERR_DRAIN_WAIT);
+    tc::mbar_wait(p.done, 0, p.err, ERR_DRAIN_WAIT, WAIT_CYCLES);
 }
 
 // Epilogue warp: adds each chunk's columns [0, ncol) of `lanes` (TMEM address of
@@ -196,7 +192,7 @@ CS_DEV bool accumulate(const Pipe& p, int nk, uint32_t lanes, uint32_t step, int
     bool ok = true;
     for (int kc = 0; kc < nk; kc++) {
         const int b = kc & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(p.accf + 8 * b, (kc >> 1) & 1, ERR_ACC_WAIT));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(p.accf + 8 * b, (kc >> 1) & 1, p.err, ERR_ACC_WAIT, WAIT_CYCLES));
         if (!ok) break;
         tc::fence_after();
 #pragma unroll
@@ -217,7 +213,7 @@ CS_DEV bool accumulate(const Pipe& p, int nk, uint32_t lanes, uint32_t step, int
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(p.acce + 8 * b);
     }
-    ok = ok && (*reinterpret_cast<volatile unsigned*>(&g_split_error) == 0u);
+    ok = ok && (*reinterpret_cast<volatile unsigned*>(p.err) == 0u);
     return __all_sync(0xffffffffu, ok);
 }
 
@@ -243,7 +239,7 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
     unsigned char* smem = align1k(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x, S = a.S, nk = (a.K + BK - 1) / BK;
-    const Pipe p = pipe_open<E, 1>(smem + a.stages * STAGE + gram_slack<R>(), a.stages, COLS, &tmap);
+    const Pipe p = pipe_open<E, 1>(smem + a.stages * STAGE + gram_slack<R>(), a.stages, COLS, a.err, &tmap);
     const uint32_t sbase = tc::smem_u32(smem);
     if (warp == E) {
         if (lane == 0)
@@ -313,7 +309,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
     // 128 rows of a plane of fewer (lanes never stored)
     const uint32_t stage_bytes = gridDim.x == 1 ? op_bytes : 2 * op_bytes;
     const uint32_t slack = BM * ROW_BYTES - a.plane_bytes;
-    const Pipe p = pipe_open<T_E, 2>(smem + a.stages * stage_bytes + slack, a.stages, T_COLS, &tmap);
+    const Pipe p = pipe_open<T_E, 2>(smem + a.stages * stage_bytes + slack, a.stages, T_COLS, a.err, &tmap);
     const uint32_t sbase = tc::smem_u32(smem);
     if (warp == T_E) {
         if (lane == 0)
@@ -366,7 +362,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
         bool ok = true;
         for (int kc = 0; kc < nk; kc++) {
             const int b = kc & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(p.accf + 8 * b, (kc >> 1) & 1, ERR_ACC_WAIT));
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(p.accf + 8 * b, (kc >> 1) & 1, p.err, ERR_ACC_WAIT, WAIT_CYCLES));
             if (!ok) break;
             tc::fence_after();
 #pragma unroll
@@ -387,7 +383,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(p.acce + 8 * b);
         }
-        ok = ok && (*reinterpret_cast<volatile unsigned*>(&g_split_error) == 0u);
+        ok = ok && (*reinterpret_cast<volatile unsigned*>(p.err) == 0u);
         // all or none of the epilogue warps go on: M - M^T needs every row.  The last
         // chunk's MMAs are done, so the operand ring is free: a 32 x 17 block
         // per warp, then (diagonal tile) M
@@ -454,9 +450,9 @@ int launch_gram(const CUtensorMap& tm, SplitArgs a, int C, cudaStream_t st)
 
 float cs_xmac_split_lo(int S) { return S <= 64 ? 2.f : 1.f; }
 
-int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, cudaStream_t st)
+int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err, cudaStream_t st)
 {
-    if (!spectra || !vis || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp % BK || kp < K || (uintptr_t)spectra % 16)
+    if (!spectra || !vis || !err || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp % BK || kp < K || (uintptr_t)spectra % 16)
         return CS_ERR_ARG;
     CsEncodeTiledFn enc = cs_encode_tiled();
     if (!enc) return CS_ERR_UNSUPPORTED;
@@ -473,11 +469,7 @@ int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return CS_ERR_ARG;
-    void* errp = nullptr;
-    CS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_split_error));
-    CS_CUDA_TRY(cudaMemsetAsync(errp, 0, sizeof(unsigned), st));
-
-    SplitArgs a{S, K, (int64_t)S * (S + 1) / 2, vis, inv_scale, 0, (uint32_t)rows * ROW_BYTES};
+    SplitArgs a{S, K, (int64_t)S * (S + 1) / 2, vis, inv_scale, 0, err, (uint32_t)rows * ROW_BYTES};
     if (S <= 16) return launch_gram<16>(tm, a, C, st);
     if (S <= 32) return launch_gram<32>(tm, a, C, st);
     if (S <= 64) return launch_gram<64>(tm, a, C, st);
@@ -487,9 +479,4 @@ int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis,
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_split), (int)smem));
     k_xmac_split<<<dim3(tiles, C), 32 * (T_E + 3), smem, st>>>(tm, a), cs_count_launches(1);
     return (int)cudaGetLastError();
-}
-
-int cs_xmac_split_status(unsigned* code)
-{
-    return (int)cudaMemcpyFromSymbol(code, g_split_error, sizeof(unsigned));
 }

@@ -52,18 +52,10 @@ static_assert(EPI_STG_BYTES + BM * MP * 4 <= STAGES * STAGE_BYTES, "epilogue M s
 constexpr uint32_t TMEM_COLS = 256;
 constexpr long long WAIT_CYCLES = 4000000000LL;     // ~2 s at 2 GHz
 
-// error codes written to g_tc_error
+// error codes
 constexpr unsigned ERR_FULL_WAIT = 1, ERR_EMPTY_WAIT = 2, ERR_ACC_WAIT = 3;
 
-__device__ unsigned g_tc_error;
-
 using tc::smem_u32;
-
-// Bounded wait: false (and the error code recorded in g_tc_error) after WAIT_CYCLES.
-CS_DEV bool mbar_wait(uint32_t bar, uint32_t parity, unsigned code)
-{
-    return tc::mbar_wait(bar, parity, &g_tc_error, code, WAIT_CYCLES);
-}
 
 // K-major operand in shared memory with 64-byte swizzle: 8-row x 64-byte
 // atoms stacked along M/N every 512 bytes (stride byte offset).
@@ -99,6 +91,7 @@ struct TcArgs {
     uint32_t tmem_cols;         // TMEM columns: Re V in [0, cols/2), Im V in [cols/2, cols)
     int kblock;                 // spectra k-blocked: 1 [C][S][kp/32][2][32] (4-D tensor map),
                                 // 2 channel-grouped [C/16][S][kp/32][16][2][32] (5-D)
+    unsigned* err;              // CsErrorWord::code of the job
 };
 
 __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant__ CUtensorMap tmap,
@@ -174,7 +167,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             for (int kc = 0; kc < nk && ok; kc++) {
                 const int s = kc % STAGES;
                 const uint32_t ph = (kc / STAGES) & 1;
-                if (!mbar_wait(empty0 + 8 * s, ph ^ 1, ERR_EMPTY_WAIT)) { ok = false; break; }
+                if (!tc::mbar_wait(empty0 + 8 * s, ph ^ 1, a.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) { ok = false; break; }
                 const uint32_t st = sbase + s * stage_bytes;
                 const uint32_t fb = full0 + 8 * s;
                 tc::mbar_expect_tx(fb, stage_tx);
@@ -192,7 +185,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             }
             // drain: every stage this thread filled must have landed before the CTA exits
             for (int kc = (issued > STAGES ? issued - STAGES : 0); kc < issued; kc++)
-                mbar_wait(full0 + 8 * (kc % STAGES), (kc / STAGES) & 1, ERR_FULL_WAIT);
+                tc::mbar_wait(full0 + 8 * (kc % STAGES), (kc / STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -202,7 +195,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             bool ok = true;
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % STAGES;
-                if (!mbar_wait(full0 + 8 * s, (kc / STAGES) & 1, ERR_FULL_WAIT)) { ok = false; break; }
+                if (!tc::mbar_wait(full0 + 8 * s, (kc / STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) { ok = false; break; }
                 tc::fence_after();
                 const uint32_t st = sbase + s * stage_bytes;
 #pragma unroll
@@ -222,7 +215,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             // Always commit: the barrier then completes only after every MMA
             // issued so far has finished, so TMEM is never freed under one.
             tc::commit(accb);
-            if (!ok) atomicCAS(&g_tc_error, 0u, ERR_FULL_WAIT);
+            if (!ok) tc::record_error(a.err, ERR_FULL_WAIT);
         }
         __syncwarp();
     } else {
@@ -230,8 +223,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
         const int q = warp & 3;                                    // TMEM lane quarter
         const int r = 32 * q + lane;
         const int i = i0 + r;
-        bool ok = mbar_wait(accb, 0, ERR_ACC_WAIT);
-        ok = ok && (*reinterpret_cast<volatile unsigned*>(&g_tc_error) == 0u);
+        bool ok = tc::mbar_wait(accb, 0, a.err, ERR_ACC_WAIT, WAIT_CYCLES);
+        ok = ok && (*reinterpret_cast<volatile unsigned*>(a.err) == 0u);
         __syncwarp();
         // M - M^T needs the other warps' rows: the four epilogue warps agree
         // (one vote, so all of them or none reach the barrier below)
@@ -350,9 +343,9 @@ CsEncodeTiledFn cs_encode_tiled()
 }
 
 int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis, const float* inv_scale,
-                   int scale_stride, int accumulate, cudaStream_t st, int kblock)
+                   int scale_stride, int accumulate, unsigned* err, cudaStream_t st, int kblock)
 {
-    if (!spectra || !vis || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp < K) return CS_ERR_ARG;
+    if (!spectra || !vis || !err || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp < K) return CS_ERR_ARG;
     if (K % 8 != 0 || kp % 8 != 0 || (uintptr_t)spectra % 16) return CS_ERR_ARG;   // TMA: 16-byte pitch and base
     if (kblock < 0 || kblock > 2 || (kblock && (K % 32 != 0 || kp % 32 != 0)) || (kblock == 2 && C % 16 != 0))
         return CS_ERR_ARG;
@@ -399,10 +392,6 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     }
     if (r != CUDA_SUCCESS) return CS_ERR_ARG;
 
-    void* errp = nullptr;
-    CS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_tc_error));
-    CS_CUDA_TRY(cudaMemsetAsync(errp, 0, sizeof(unsigned), st));
-
     // S <= 128: one diagonal tile per channel, B = A, 16 KB stages and only the
     // TMEM columns the tile needs, so several CTAs share an SM
     const int small = S <= BM ? 1 : 0;
@@ -413,17 +402,10 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
         while (cols < 2 * n_eff) cols *= 2;
     }
     TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, tiles, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
-             accumulate, box_rows, small, cols, kblock};
+             accumulate, box_rows, small, cols, kblock, err};
     const size_t smem = (size_t)STAGES * (small ? 2 * A_BYTES : STAGE_BYTES) + 1024 + 256;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc), (int)smem));
     dim3 grid(ntiles, C);
     k_xmac_tc<<<grid, TC_THREADS, smem, st>>>(tm, a), cs_count_launches(1);
     return (int)cudaGetLastError();
-}
-
-// Error code of the last tensor-core launch on this device (0 = ok); the
-// caller must have synchronised the launching stream.
-int cs_xmac_tc_status(unsigned* code)
-{
-    return (int)cudaMemcpyFromSymbol(code, g_tc_error, sizeof(unsigned));
 }
