@@ -4,12 +4,15 @@
 // (minicorrelator/fft_1d_r2_modified.h:81-534, cellspe-tasklib-dsp.cpp:
 // 519-602): complex forward transform, interleaved {re, im}, unscaled.
 // cs_rfft_batch replaces genericFFTexec_R (architecture.h:563-578, FFTW r2c
-// layout: N/2+1 bins).  Both run CtaFft<M> groups (M/16 threads per
-// transform, several transforms per CTA).  Twiddle tables are computed once
+// layout: N/2+1 bins).  Transforms of 64 to 1024 complex points run in the
+// registers of a warp or part of one (k_fft_warp), others as CtaFft<M> groups
+// (M/16 threads per transform, several transforms per CTA).  Twiddle tables are computed once
 // per size in FP64 on the host, rounded to FP32 and kept on the device.
 #include "common.cuh"
 #include "kernels.h"
+#include "warpfft.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <map>
@@ -180,17 +183,100 @@ int launch_batch(const void* in, float2* out, int64_t batch, float scale, cudaSt
     return (int)cudaGetLastError();
 }
 
+// 64 to 1024 complex points: L lanes per transform, read and written straight from
+// and to global memory (256-byte runs per load of a warp of 1024 points), one
+// shared-memory transpose, nothing else shared between warps.  Bound by the copy:
+// 65536 real transforms of 2048 points take 181 us a call (1.07 GB, 158 us at the
+// copy rate); the shared-memory radix-16 passes, three of them with CTA barriers,
+// took 346.  2^27 floats as complex transforms of 512 and 1024 points 503 -> 362 and
+// 632 -> 361 us, real ones of 1024 points 282 -> 185.
+constexpr int FW_NT = 256;
+template <int L, int R, bool REAL, bool INV>
+__global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict__ in, float2* __restrict__ out, int64_t batch,
+                                                       const float2* __restrict__ tw, float scale)
+{
+    using W = WarpFft<L, R>;
+    constexpr int M = W::M, GROUPS = FW_NT / L;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2* tab = reinterpret_cast<float2*>(smem);
+    const int g = threadIdx.x / L, lane = threadIdx.x % L;
+    float2* tile = tab + W::TWIDDLES + g * W::TILE;
+    W::fill(tab, tw, 2);
+    float2 wh[W::CPL];
+#pragma unroll
+    for (int c = 0; c < W::CPL; c++) wh[c] = cscale(__ldg(tw + lane + L * c), 0.5f);
+    __syncthreads();
+    // whole rounds, so that every lane of a warp takes part in its shuffles
+    for (int64_t b0 = (int64_t)blockIdx.x * GROUPS; b0 < batch; b0 += (int64_t)gridDim.x * GROUPS) {
+        const int64_t b = b0 + g;
+        const bool valid = b < batch;
+        const float2* src = in + (valid ? b : b0) * M;
+        float2 v[R];
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            v[j] = __ldg(src + lane + L * j);                // REAL: {x[2n], x[2n+1]}
+            if (INV) v[j].y = -v[j].y;
+        }
+        W::run(v, tile, lane, tab);
+        if constexpr (REAL) {
+            float2* o = out + b * (M + 1);
+            W::split(
+                v, lane, wh,
+                [&](int, int k, float2 X1, float2 X2) {
+                    if (!valid) return;
+                    if (k == 0) X1.y = X2.y = 0.f;           // DC and Nyquist
+                    o[k] = X1;
+                    o[M - k] = X2;
+                },
+                [&](float2 X) {
+                    if (valid) o[M / 2] = X;
+                });
+        } else {
+            float2* o = out + b * M;
+#pragma unroll
+            for (int c = 0; c < W::CPL; c++)
+#pragma unroll
+                for (int k2 = 0; k2 < L; k2++) {
+                    float2 z = v[c * L + k2];
+                    if (INV) z = make_float2(z.x * scale, -z.y * scale);
+                    if (valid) o[lane + L * c + R * k2] = z;
+                }
+        }
+    }
+}
+
+template <int L, int R, bool REAL, bool INV>
+int launch_warp(const void* in, float2* out, int64_t batch, float scale, cudaStream_t st)
+{
+    using W = WarpFft<L, R>;
+    const float2* tw = cs_twiddles(2 * W::M);
+    if (!tw) return CS_ERR_ARG;
+    const size_t smem = (size_t)(W::TWIDDLES + FW_NT / L * W::TILE) * sizeof(float2);
+    auto kern = k_fft_warp<L, R, REAL, INV>;
+    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
+    const int64_t blocks = (batch + FW_NT / L - 1) / (FW_NT / L);
+    kern<<<(unsigned)std::min<int64_t>(blocks, 152 * 4), FW_NT, smem, st>>>(static_cast<const float2*>(in), out, batch, tw, scale),
+        cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
+
+// Complex transforms of 128 and 256 points stay with the radix-16 groups, whose two
+// passes already run at the copy rate (2^27 floats: 355 and 359 us against 385 and 360).
 template <bool REAL, bool INV>
 int dispatch(const void* in, float2* out, int m, int64_t batch, float scale, cudaStream_t st)
 {
     switch (m) {
         case 16: return launch_batch<16, REAL, INV>(in, out, batch, scale, st);
         case 32: return launch_batch<32, REAL, INV>(in, out, batch, scale, st);
-        case 64: return launch_batch<64, REAL, INV>(in, out, batch, scale, st);
-        case 128: return launch_batch<128, REAL, INV>(in, out, batch, scale, st);
-        case 256: return launch_batch<256, REAL, INV>(in, out, batch, scale, st);
-        case 512: return launch_batch<512, REAL, INV>(in, out, batch, scale, st);
-        case 1024: return launch_batch<1024, REAL, INV>(in, out, batch, scale, st);
+        case 64: return launch_warp<8, 8, REAL, INV>(in, out, batch, scale, st);
+        case 128:
+            if constexpr (!REAL) return launch_batch<128, REAL, INV>(in, out, batch, scale, st);
+            return launch_warp<8, 16, REAL, INV>(in, out, batch, scale, st);
+        case 256:
+            if constexpr (!REAL) return launch_batch<256, REAL, INV>(in, out, batch, scale, st);
+            return launch_warp<16, 16, REAL, INV>(in, out, batch, scale, st);
+        case 512: return launch_warp<16, 32, REAL, INV>(in, out, batch, scale, st);
+        case 1024: return launch_warp<32, 32, REAL, INV>(in, out, batch, scale, st);
         case 2048: return launch_batch<2048, REAL, INV>(in, out, batch, scale, st);
         case 4096: return launch_batch<4096, REAL, INV>(in, out, batch, scale, st);
         case 8192: return launch_batch<8192, REAL, INV>(in, out, batch, scale, st);

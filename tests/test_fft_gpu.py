@@ -78,3 +78,28 @@ def test_fft_r2c_perm_packing(cg, n, batch):
     xd, od = torch.from_numpy(x).cuda(), torch.zeros((batch, n), dtype=torch.float32, device="cuda")
     cg.fft_r2c_perm(xd, od)
     assert np.array_equal(od.cpu().numpy(), out)
+
+
+@pytest.mark.parametrize("n", [64, 128, 256, 512, 1024])
+@pytest.mark.parametrize("batch", [1, 5, 33, 20011])
+def test_fft_lane_groups(cg, n, batch):
+    """Transforms held in a warp or part of one: batches that fill no warp and no CTA, and more than one round of CTAs."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n + batch)
+    x = torch.randn((batch, n, 2), generator=g, device="cuda")
+    z = torch.view_as_complex(x)
+    out = torch.full((batch, n), float("nan"), dtype=torch.complex64, device="cuda")
+    cg.fft_c2c(z, out, n, batch)
+    ref = torch.fft.fft(z.to(torch.complex128))
+    # FP32 rounding through log2 n levels: about 2^-24 sqrt(log2 n)
+    assert float((out - ref).norm() / ref.norm()) < 1e-6
+    r = torch.full((batch, n + 1), float("nan"), dtype=torch.complex64, device="cuda")
+    cg.fft_r2c(x.view(batch, 2 * n), r, 2 * n, batch)
+    ref = torch.fft.rfft(x.view(batch, 2 * n).double())
+    assert float((r - ref).norm() / ref.norm()) < 1e-6
+    assert float(r[:, 0].imag.abs().max()) == 0.0 and float(r[:, n].imag.abs().max()) == 0.0
+    lags = torch.empty_like(out)
+    cg.vis_lags(z, lags, 0.5)
+    ref = torch.fft.ifft(z.to(torch.complex128)) * (0.5 * n)
+    assert float((lags - ref).norm() / ref.norm()) < 1e-6
