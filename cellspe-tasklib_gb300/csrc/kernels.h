@@ -209,6 +209,9 @@ struct CsSpecArgs {
     int pcal_source;            // this source's index among them
     int skip_power;             // 1: phase-cal only (no power spectra)
 };
+// FFTs per partial spectrum that a job whose default scratch does not fit its
+// budget falls back to.
+constexpr int CS_SPEC_CHUNK = 32;
 int64_t cs_spectrometer_scratch_floats(const CsSpecArgs& a);
 int64_t cs_spectrometer_pcal_floats(const CsSpecArgs& a);   // the phase-cal part of it
 int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st);

@@ -1102,9 +1102,10 @@ int vdif_spec_mbps(const cellspe_spec_params* p)
     return (r > 0 && r < INT32_MAX && std::fabs(mbps - (double)r) < 1e-6) ? (int)r : 0;
 }
 
-long long spec_bytes(const cellspe_spec_params* p)
+long long spec_bytes(const cellspe_spec_params* p, int ffts_per_chunk = 0)
 {
     CsSpecArgs a{};
+    a.ffts_per_chunk = ffts_per_chunk;
     a.nsub = p->n_subbands; a.N = p->fft_points; a.overlap = p->overlap;
     a.ffts_per_spectrum = p->ffts_per_spectrum; a.nspec = p->n_spectra; a.tonebins = p->pcal_tonebins;
     long long b = align256(cs_spectrometer_scratch_floats(a) * 4);
@@ -1255,12 +1256,17 @@ int op_spectrometer(Workspace& ws, const cellspe_spec_params* p, const void* raw
     if (p->pcal_tonebins > 0 && !pcal_bins) return set_err(CELLSPE_ERR_ARG, "spectrometer: pcal enabled without pcal_bins");
     float lut[4];
     if (!pick_levels(p->levels, p->custom_levels, lut)) return set_err(CELLSPE_ERR_ARG, "spectrometer: unknown level table");
-    long long need = spec_bytes(p);
-    if (over_limit(ws, need)) return set_err(CELLSPE_ERR_NOMEM, "spectrometer: job exceeds the device memory budget");
+    int chunk = 0;                      // the default, or fewer and larger partial spectra where those do not fit
+    if (over_limit(ws, spec_bytes(p))) {
+        chunk = CS_SPEC_CHUNK;
+        if (over_limit(ws, spec_bytes(p, chunk)))
+            return set_err(CELLSPE_ERR_NOMEM, "spectrometer: job exceeds the device memory budget");
+    }
     const bool host = p->memory == CELLSPE_MEM_HOST;
     Job j(ws, host);
     const SpecPlanes sp = spec_planes(ws, j, p, raw);
     CsSpecArgs a = spec_args(p, sp, lut);
+    a.ffts_per_chunk = chunk;
     const long long rows = (long long)p->n_subbands * p->n_spectra;
     a.power = (float*)j.out(power, (size_t)rows * (p->fft_points / 2 + 1) * 4, false);
     if (a.tonebins > 0) {
@@ -1283,7 +1289,7 @@ long long spec_xpol_bytes(const cellspe_spec_params* p)
     const long long nwin = (long long)p->n_spectra * (p->overlap * p->ffts_per_spectrum - (p->overlap - 1));
     cellspe_spec_params one = *p;
     one.n_subbands = p->n_subbands;
-    long long b = 2 * spec_bytes(&one);
+    long long b = 2 * spec_bytes(&one, CS_SPEC_CHUNK);
     b += align256(nwin * N * 4) + 2 * align256(nwin * nb * 8);
     b += align256(3LL * p->n_spectra * nb * 8);
     return b;

@@ -27,7 +27,9 @@
 // bins.  Tones = DFT(bins)/T, first ntones (PCal.cpp:280-300, getFinalPCal).
 #include "common.cuh"
 #include "kernels.h"
+#include "warpfft.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <map>
@@ -37,7 +39,7 @@
 
 namespace {
 
-constexpr int SPEC_CH = 32;   // FFTs per chunk (one partial spectrum each)
+constexpr int SPEC_CH = CS_SPEC_CHUNK;   // most FFTs per chunk (one partial spectrum each) for N >= 4096
 
 template <int MC> struct SCfg {
     static constexpr int T = MC / 16;
@@ -62,6 +64,27 @@ const float* window_table(int type, int n)
     if (cudaMalloc(&d, sizeof(float) * n) != cudaSuccess) return nullptr;
     cudaMemcpy(d, h.data(), sizeof(float) * n, cudaMemcpyHostToDevice);
     g_win[key] = d;
+    return d;
+}
+
+// The same window in the order of k_spec_power_m's warps: pairs (2 n, 2 n + 1),
+// n = n1 + m1 m, as [m1][1024].
+std::map<std::tuple<int, int, int>, float2*> g_winp;
+const float2* window_pairs(int type, int n, int m1)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(g_win_mu);
+    auto key = std::make_tuple(dev, type, n);
+    auto it = g_winp.find(key);
+    if (it != g_winp.end()) return it->second;
+    std::vector<float2> h(n / 2);
+    for (int i = 0; i < n / 2; i++)
+        h[(i % m1) * 1024 + i / m1] = make_float2((float)cs_window_value(type, 2 * i, n), (float)cs_window_value(type, 2 * i + 1, n));
+    float2* d = nullptr;
+    if (cudaMalloc(&d, sizeof(float2) * (n / 2)) != cudaSuccess) return nullptr;
+    cudaMemcpy(d, h.data(), sizeof(float2) * (n / 2), cudaMemcpyHostToDevice);
+    g_winp[key] = d;
     return d;
 }
 
@@ -196,6 +219,317 @@ __global__ void __launch_bounds__(SCfg<MC>::NT) k_spec_power(const __grid_consta
 #pragma unroll
         for (int gg = 0; gg < GROUPS; gg++) s += acc_all[gg * NACC + l];
         prow[k] = s;
+    }
+}
+
+// The FFTs of one chunk: the plane words of FFT j as a thread group's cp.async
+// copies into its shared buffer, in 16-byte pieces where the FFTs start on
+// 16-byte boundaries (hop a multiple of 64 samples), in words otherwise.
+CS_DEV void spec_fetch(uint32_t* dst, const uint32_t* __restrict__ plane, int64_t start, int words, int t, int nt, bool vec)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const uint32_t* src = plane + (start >> 4);
+    if (vec) {
+        for (int i = t; i < words / 4; i += nt)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(src + 4 * i) : "memory");
+    } else {
+        for (int i = t; i < words; i += nt)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * i), "l"(src + i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int PENDING> CS_DEV void spec_fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+// Whether any sample of the window [start, start + N) is blanked, as far as
+// thread t of nt sees (start a multiple of 16).
+CS_DEV bool spec_blanked(const uint32_t* __restrict__ vmask, int64_t start, int N, int t, int nt)
+{
+    bool any = false;
+    if (start & 31) {
+        for (int i = t; i < N / 16; i += nt) {
+            const int64_t s = start + 16 * i;
+            any |= ((__ldg(vmask + (s >> 5)) >> (s & 31)) & 0xffffu) != 0xffffu;
+        }
+    } else {
+        for (int i = t; i < N / 32; i += nt) any |= __ldg(vmask + (start >> 5) + i) != 0xffffffffu;
+    }
+    return any;
+}
+
+// N = 1024 and 2048: a FFT in the registers of L lanes (WarpFft), its powers
+// added to registers of the lanes that own the bins, so a group's only shared
+// memory traffic is the plane words, the level pairs, the twiddles and one transpose, and
+// no group waits on another until the chunk ends.  Bound by instruction issue
+// (16 warps per SM; registers).  16 rows x 16383 FFTs of 1024 points: 247 us;
+// the radix-16 groups with shared-memory accumulators and CTA barriers took 608.
+constexpr int SP_NT = 256;
+template <int L, int R, bool MASK>
+__global__ void __launch_bounds__(SP_NT, 2) k_spec_power_s(const __grid_constant__ CsSpecArgs a, const float2* __restrict__ tw,
+                                                           const float* __restrict__ win, int nchunk, int ch)
+{
+    using W = WarpFft<L, R>;
+    constexpr int M = W::M, N = 2 * M, GROUPS = SP_NT / L, WARPS = SP_NT / 32, WORDS = N / 16;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2* tab = reinterpret_cast<float2*>(smem);
+    float2* tiles = tab + W::TWIDDLES;
+    uint32_t* raw = reinterpret_cast<uint32_t*>(tiles + GROUPS * W::TILE);
+    __shared__ float2 lut16[16];
+    const int g = threadIdx.x / L, lane = threadIdx.x % L;
+    float2* tile = tiles + g * W::TILE;
+    uint32_t* rw = raw + g * 2 * WORDS;
+    const int chunk = blockIdx.x, row = blockIdx.y;
+    const int sub = row / a.nspec, spec = row % a.nspec;
+    const int novl = a.overlap * a.ffts_per_spectrum - (a.overlap - 1);
+    const int hop = N / a.overlap;
+    const bool vec = hop % 64 == 0;
+    const uint32_t* plane = reinterpret_cast<const uint32_t*>(a.planes + (int64_t)sub * a.bytes_per_sub);
+    const int64_t first = (int64_t)spec * a.ffts_per_spectrum * N;
+    const int j_begin = chunk * ch, j_end = min(novl, j_begin + ch);
+    // a group past the chunk's end transforms its first FFT again and drops it
+    auto start_of = [&](int j) { return first + (int64_t)(j < j_end ? j : j_begin) * hop; };
+    spec_fetch(rw, plane, start_of(j_begin + g), WORDS, lane, L, vec);
+    if (threadIdx.x < 16) lut16[threadIdx.x] = make_float2(a.lut[threadIdx.x & 3], a.lut[threadIdx.x >> 2]);
+    W::fill(tab, tw, 2);
+    float2 wh[W::CPL];
+#pragma unroll
+    for (int c = 0; c < W::CPL; c++) wh[c] = cscale(__ldg(tw + lane + L * c), 0.5f);
+    float acc[R], mid = 0.f;
+#pragma unroll
+    for (int i = 0; i < R; i++) acc[i] = 0.f;
+    __syncthreads();
+    const float2* win2 = reinterpret_cast<const float2*>(win) + lane;
+    const int sh = 4 * (lane & 7);                   // a pair's four bits within its word
+    // the mask of the next FFT is looked at while this one is transformed
+    bool blank_next = MASK && spec_blanked(a.valid_mask, start_of(j_begin + g), N, lane, L);
+    int u = 0;
+    for (int j0 = j_begin; j0 < j_end; j0 += GROUPS, u ^= 1) {
+        const int j = j0 + g;
+        const int64_t start = start_of(j);
+        bool blanked = false;
+        if constexpr (MASK) blanked = __any_sync(0xffffffffu, blank_next);
+        if (j0 + GROUPS < j_end) {
+            spec_fetch(rw + (u ^ 1) * WORDS, plane, start_of(j + GROUPS), WORDS, lane, L, vec);
+            if constexpr (MASK) blank_next = spec_blanked(a.valid_mask, start_of(j + GROUPS), N, lane, L);
+            spec_fetch_wait<1>();
+        } else {
+            spec_fetch_wait<0>();
+        }
+        __syncwarp();
+        const uint32_t* w = rw + u * WORDS + (lane >> 3);
+        float2 v[R];
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            float2 x = lut16[(w[q * (L / 8)] >> sh) & 15u];
+            if (MASK && blanked) {
+                const int64_t t = start + 2 * (lane + L * q);
+                const uint32_t m = __ldg(a.valid_mask + (t >> 5)) >> (t & 31);
+                x = make_float2((m & 1u) ? x.x : 0.f, (m & 2u) ? x.y : 0.f);
+            }
+            const float2 wn = __ldg(win2 + L * q);
+            v[q] = make_float2(x.x * wn.x, x.y * wn.y);
+        }
+        W::run(v, tile, lane, tab);
+        const bool valid = j < j_end;
+        W::split(
+            v, lane, wh,
+            [&](int i, int, float2 X1, float2 X2) {
+                if (!valid) return;
+                acc[2 * i] += X1.x * X1.x + X1.y * X1.y;
+                acc[2 * i + 1] += X2.x * X2.x + X2.y * X2.y;
+            },
+            [&](float2 X) {
+                if (valid) mid += X.x * X.x + X.y * X.y;
+            });
+    }
+    // the groups' sums: over the warp's groups by shuffles, then over the warps in order
+#pragma unroll
+    for (int o = L; o < 32; o *= 2) {
+#pragma unroll
+        for (int i = 0; i < R; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        mid += __shfl_xor_sync(0xffffffffu, mid, o);
+    }
+    __syncthreads();
+    float* red = reinterpret_cast<float*>(tiles);    // [WARPS][M + 1]
+    if ((threadIdx.x & 31) < L) {
+        float* r = red + (threadIdx.x >> 5) * (M + 1);
+#pragma unroll
+        for (int c = 0; c < W::CPL; c++)
+#pragma unroll
+            for (int k2 = 0; k2 < L / 2; k2++) {
+                const int i = c * (L / 2) + k2, k = lane + L * c + R * k2;
+                r[k] = acc[2 * i];
+                r[M - k] = acc[2 * i + 1];
+            }
+        if (lane == 0) r[M / 2] = mid;
+    }
+    __syncthreads();
+    float* prow = a.partial + ((int64_t)row * nchunk + chunk) * (M + 1);
+    for (int k = threadIdx.x; k <= M; k += SP_NT) {
+        float t = red[k];
+#pragma unroll
+        for (int q = 1; q < WARPS; q++) t += red[q * (M + 1) + k];
+        prow[k] = t;
+    }
+}
+
+// N = 4096, 8192 and 16384: M1 = N / 2048 warps per FFT, decimation in time by
+// M1.  Warp n1 transforms z[n1 + M1 m], m < 1024, in registers (WarpFft) and
+// parks the result Y_n1 in its tile; after one CTA barrier each thread takes
+// mirrored columns kA and 1024 - kA (kA = thread + 32 M1 i; thread 0 also
+// columns 0 and 512, each its own mirror):
+//     Z[k2 + 1024 k1] = sum_n1 W_M1^(n1 k1) (W_M^(n1 k2) Y_n1[k2]),
+// two M1-point DFTs, the second rotated by one as W_M^(n1 (1024 - k2)) =
+// W_M1^n1 conj(W_M^(n1 k2)), which holds both ends of every real-FFT pair, and
+// adds the powers to its own registers.  The window table is read in the
+// warps' order (winp: [M1][1024] pairs).  Bound by instruction issue; 12 rows x
+// 1999 FFTs of 8192 points: 323 us (with some blanked windows), the radix-16 groups 430.
+template <int M1, bool MASK>
+__global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_constant__ CsSpecArgs a,
+                                                                   const float2* __restrict__ tw,
+                                                                   const float2* __restrict__ winp, int nchunk, int ch)
+{
+    using W = WarpFft<32, 32>;
+    constexpr int M = 1024 * M1, N = 2 * M, NT = 32 * M1, WORDS = N / 16, TASKS = 512 / NT;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2* tab = reinterpret_cast<float2*>(smem);
+    float2* tiles = tab + W::TWIDDLES;
+    uint32_t* raw = reinterpret_cast<uint32_t*>(tiles + M1 * W::TILE);
+    __shared__ float2 lut16[16];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float2* tile = tiles + warp * W::TILE;
+    const int chunk = blockIdx.x, row = blockIdx.y;
+    const int sub = row / a.nspec, spec = row % a.nspec;
+    const int novl = a.overlap * a.ffts_per_spectrum - (a.overlap - 1);
+    const int hop = N / a.overlap;
+    const bool vec = hop % 64 == 0;
+    const uint32_t* plane = reinterpret_cast<const uint32_t*>(a.planes + (int64_t)sub * a.bytes_per_sub);
+    const int64_t first = (int64_t)spec * a.ffts_per_spectrum * N;
+    const int j_begin = chunk * ch, j_end = min(novl, j_begin + ch);
+    spec_fetch(raw, plane, first + (int64_t)j_begin * hop, WORDS, tid, NT, vec);
+    if (tid < 16) lut16[tid] = make_float2(a.lut[tid & 3], a.lut[tid >> 2]);
+    W::fill(tab, tw, 2 * M1);
+    float acc[TASKS][2 * M1], extra = 0.f;
+#pragma unroll
+    for (int i = 0; i < TASKS; i++)
+#pragma unroll
+        for (int q = 0; q < 2 * M1; q++) acc[i][q] = 0.f;
+    const float2* win2 = winp + 1024 * warp + lane;
+    const int n0 = warp + M1 * lane;                 // this lane's first pair; pair q is 32 M1 further on
+    const int w0 = n0 >> 3, sh = 4 * (n0 & 7);
+    auto power = [](float2 X) { return X.x * X.x + X.y * X.y; };
+    // the mask of the next FFT is looked at while this one is transformed
+    bool blank_next = MASK && spec_blanked(a.valid_mask, first + (int64_t)j_begin * hop, N, tid, NT);
+    int u = 0;
+    for (int j = j_begin; j < j_end; j++, u ^= 1) {
+        const int64_t start = first + (int64_t)j * hop;
+        const bool blank = blank_next;
+        if (j + 1 < j_end) {
+            spec_fetch(raw + (u ^ 1) * WORDS, plane, start + hop, WORDS, tid, NT, vec);
+            if constexpr (MASK) blank_next = spec_blanked(a.valid_mask, start + hop, N, tid, NT);
+            spec_fetch_wait<1>();
+        } else {
+            spec_fetch_wait<0>();
+        }
+        bool blanked = false;
+        // this FFT's words are in, the previous one's columns are read
+        if constexpr (MASK) blanked = __syncthreads_or(blank) != 0;
+        else __syncthreads();
+        {
+            const uint32_t* w = raw + u * WORDS + w0;
+            float2 v[32];
+#pragma unroll
+            for (int q = 0; q < 32; q++) {
+                float2 x = lut16[(w[4 * M1 * q] >> sh) & 15u];
+                if (MASK && blanked) {
+                    const int64_t t = start + 2 * (n0 + 32 * M1 * q);
+                    const uint32_t m = __ldg(a.valid_mask + (t >> 5)) >> (t & 31);
+                    x = make_float2((m & 1u) ? x.x : 0.f, (m & 2u) ? x.y : 0.f);
+                }
+                const float2 wn = __ldg(win2 + 32 * q);
+                v[q] = make_float2(x.x * wn.x, x.y * wn.y);
+            }
+            W::run(v, tile, lane, tab);
+#pragma unroll
+            for (int k2 = 0; k2 < 32; k2++) tile[lane + 32 * k2] = v[k2];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TASKS; i++) {
+            const int kA = tid + NT * i;
+            if (kA == 0) {
+                // columns 0 and 512 (W_M^512 = W_(2 M1)), each paired with itself
+                float2 y0[M1], y5[M1];
+#pragma unroll
+                for (int n1 = 0; n1 < M1; n1++) {
+                    y0[n1] = tiles[n1 * W::TILE];
+                    y5[n1] = cmul(tiles[n1 * W::TILE + 512], w32((16 / M1) * n1));
+                }
+                Dft<M1>::run(y0);
+                Dft<M1>::run(y5);
+                const float2 w512 = __ldg(tw + 512);
+#pragma unroll
+                for (int k1 = 0; k1 <= M1 / 2; k1++) {
+                    float2 Xk, Xm;
+                    r2c_pair(y0[k1], y0[(M1 - k1) % M1], w32((16 / M1) * k1), Xk, Xm);
+                    if (k1 == 0) {                   // DC and Nyquist are real
+                        acc[i][0] += Xk.x * Xk.x;
+                        acc[i][1] += Xm.x * Xm.x;
+                    } else if (k1 < M1 / 2) {
+                        acc[i][2 * k1] += power(Xk);
+                        acc[i][2 * k1 + 1] += power(Xm);
+                    } else {
+                        extra += power(Xk);
+                    }
+                }
+#pragma unroll
+                for (int k1 = 0; k1 < M1 / 2; k1++) {
+                    float2 Xk, Xm;
+                    r2c_pair(y5[k1], y5[M1 - 1 - k1], cmul(w512, w32((16 / M1) * k1)), Xk, Xm);
+                    acc[i][M1 + 2 * k1] += power(Xk);
+                    acc[i][M1 + 2 * k1 + 1] += power(Xm);
+                }
+                continue;
+            }
+            float2 ya[M1], yb[M1];
+            const float2 u1 = __ldg(tw + 2 * kA);    // W_M^kA
+            float2 pw = make_float2(1.f, 0.f);
+#pragma unroll
+            for (int n1 = 0; n1 < M1; n1++) {
+                const float2 za = tiles[n1 * W::TILE + kA], zb = tiles[n1 * W::TILE + 1024 - kA];
+                ya[n1] = n1 ? cmul(za, pw) : za;
+                yb[n1] = n1 ? cmul_conj(zb, pw) : zb;
+                pw = n1 ? cmul(pw, u1) : u1;
+            }
+            Dft<M1>::run(ya);                        // ya[k1] = Z[kA + 1024 k1]
+            Dft<M1>::run(yb);                        // yb[(k1 + 1) % M1] = Z[1024 - kA + 1024 k1]
+            const float2 wA = __ldg(tw + kA);        // W_N^kA
+#pragma unroll
+            for (int k1 = 0; k1 < M1; k1++) {
+                float2 Xk, Xm;
+                r2c_pair(ya[k1], yb[(M1 - k1) % M1], k1 ? cmul(wA, w32((16 / M1) * k1)) : wA, Xk, Xm);
+                acc[i][2 * k1] += power(Xk);
+                acc[i][2 * k1 + 1] += power(Xm);
+            }
+        }
+    }
+    // every bin has one owner
+    float* prow = a.partial + ((int64_t)row * nchunk + chunk) * (M + 1);
+#pragma unroll
+    for (int i = 0; i < TASKS; i++) {
+        const int kA = tid + NT * i;
+#pragma unroll
+        for (int k1 = 0; k1 < M1; k1++) {
+            if (kA) {
+                prow[kA + 1024 * k1] = acc[i][2 * k1];
+                prow[M - kA - 1024 * k1] = acc[i][2 * k1 + 1];
+            } else if (k1 < M1 / 2) {
+                prow[1024 * k1] = acc[i][2 * k1];
+                prow[M - 1024 * k1] = acc[i][2 * k1 + 1];
+                prow[512 + 1024 * k1] = acc[i][M1 + 2 * k1];
+                prow[M - 512 - 1024 * k1] = acc[i][M1 + 2 * k1 + 1];
+            }
+        }
+        if (kA == 0) prow[M / 2] = extra;
     }
 }
 
@@ -438,29 +772,35 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
 }
 
 // power[row][k] = scale * sum of the row's chunk partials.  Bound by the read
-// of the partials.  A CTA takes blockDim.x bins of one row; each of its
-// blockDim.y slices adds every blockDim.y-th chunk and the slices' sums are
-// added in order, so the sum is deterministic.  Eight slices where a thread per
-// bin would leave the chip empty (spec_reduce_slices): a row with hundreds of
-// chunks is then not one thread's serial chain (16 rows x 512 chunks x 513 bins:
-// 46 us with a thread per bin, 10 us); one slice where there are bins enough
-// (16 rows x 32 chunks x 32769 bins: 13 us, 20 us with eight).
+// of the partials.  A CTA takes 256 / SLICES bins of one row; each slice adds
+// every SLICES-th chunk and the slices' sums are added in order, so the sum is
+// deterministic.  Eight slices where a thread per bin would leave the chip empty
+// (spec_reduce_slices): a row with hundreds of chunks is then not one thread's
+// serial chain (16 rows x 512 chunks x 513 bins: 46 us with a thread per bin, 10 us);
+// one slice where there are bins enough (16 rows x 32 chunks x 32769 bins: 13 us,
+// 20 us with eight).
 constexpr int RED_THREADS = 256;
+template <int SLICES>
 __global__ void __launch_bounds__(RED_THREADS) k_spec_reduce(const float* __restrict__ partial, float* __restrict__ power,
                                                              int nchunk, int nb, float scale)
 {
-    __shared__ float part[RED_THREADS];
-    const int r = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int BINS = RED_THREADS / SLICES;
+    __shared__ float part[SLICES][BINS];
+    const int bin = threadIdx.x % BINS, slice = threadIdx.x / BINS;
+    const int r = blockIdx.y, k = blockIdx.x * BINS + bin;
     const float* src = partial + (int64_t)r * nchunk * nb + k;
     float s = 0.f;
-    if (k < nb)
-        for (int c = threadIdx.y; c < nchunk; c += blockDim.y) s += src[(int64_t)c * nb];
-    if (blockDim.y > 1) {
-        part[threadIdx.y * blockDim.x + threadIdx.x] = s;
-        __syncthreads();
-        for (int q = 1; q < blockDim.y; q++) s += part[q * blockDim.x + threadIdx.x];
+    if (k < nb) {
+#pragma unroll 8
+        for (int c = slice; c < nchunk; c += SLICES) s += __ldg(src + (int64_t)c * nb);
     }
-    if (threadIdx.y == 0 && k < nb) power[(int64_t)r * nb + k] = s * scale;
+    if constexpr (SLICES > 1) {
+        part[slice][bin] = s;
+        __syncthreads();
+#pragma unroll
+        for (int q = 1; q < SLICES; q++) s += part[q][bin];
+    }
+    if (slice == 0 && k < nb) power[(int64_t)r * nb + k] = s * scale;
 }
 
 // one slice from about one full wave of threads (152 SMs x 1024) on
@@ -483,7 +823,7 @@ int spec_reduce_slices(int64_t bins, int nchunk) { return bins < 152 * 1024 && n
 // carry-save adder is two three-input logic operations for 32 positions), the
 // AND of a code's two bits in a second set.  About 9 logic operations per word
 // instead of 16 level selections and 32 multiply-adds, which bound the fold
-// per sample (16 rows x 2^25 samples: 610 us, 80 us now; the read of the planes
+// per sample (16 rows x 2^25 samples: 610 us, 61 us now; the read of the planes
 // takes 20 us).
 // N, L and T are powers of two (L divides N, T divides L), so a thread that
 // strides by PCAL_BLOCKS * PCAL_THREADS = 4096 words (65536 samples >= L) keeps
@@ -529,11 +869,13 @@ struct VCount {
             e = t;
         }
     }
-    CS_DEV int count(int pos) const
+    // the count of a position; planes from `np` on are known to be empty
+    CS_DEV int count(int pos, int np) const
     {
         int c = (int)((one >> pos) & 1u) + 2 * (int)((two >> pos) & 1u) + 4 * (int)((four >> pos) & 1u);
 #pragma unroll
-        for (int i = 0; i < PCAL_PLANES; i++) c += (int)((q[i] >> pos) & 1u) << (3 + i);
+        for (int i = 0; i < PCAL_PLANES; i++)
+            if (i < np) c += (int)((q[i] >> pos) & 1u) << (3 + i);
         return c;
     }
 };
@@ -579,23 +921,9 @@ __global__ void __launch_bounds__(PCAL_THREADS) k_pcal_fold(
     VCount bits, both, val;                          // code bits; their ANDs (two words a set); valid samples
     while (__syncthreads_or(w < nwords)) {
         bits.clear(), both.clear(), val.clear();
-        int added = 0;                               // words counted in this batch
-        for (int n = 0; n < PCAL_BATCH && w < nwords; n += 8) {
-            uint32_t x[8], m[8], av[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int64_t wu = w + (int64_t)u * STRIDE;
-                const bool in = wu < nwords;
-                const int64_t wg = base + (wu >> lg) * win_words + (wu & (wpw - 1));
-                x[u] = in ? __ldg(plane + wg) : 0u;
-                m[u] = 0u;
-                if (MASK) {
-                    m[u] = in ? __ldg(vmask + (wg >> 1)) >> ((wg & 1) * 16) & 0xffffu : 0u;
-                } else {
-                    added += in;
-                }
-            }
-            w += 8 * (int64_t)STRIDE;
+        int added = 0, rounds = 0;                   // words and groups of eight counted in this batch
+        auto add = [&](uint32_t (&x)[8], uint32_t (&m)[8]) {
+            uint32_t av[8];
             if (MASK) {
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
@@ -613,14 +941,60 @@ __global__ void __launch_bounds__(PCAL_THREADS) k_pcal_fold(
                 av[u] = u < 4 ? ((x[2 * u] & (x[2 * u] >> 1)) & 0x55555555u) | ((x[2 * u + 1] & (x[2 * u + 1] << 1)) & 0xaaaaaaaau)
                               : 0u;
             both.add8(av);
+            rounds++;
+            w += 8 * (int64_t)STRIDE;
+        };
+        // windows back to back (one source): no index arithmetic per word, and
+        // the next eight words on their way while eight are added
+        if (win_words == wpw && w + 7 * (int64_t)STRIDE < nwords) {
+            const uint32_t* p = plane + base;
+            const uint32_t* q = vmask + (base >> 1);
+            const int half = (int)((base + w) & 1) * 16;
+            uint32_t xn[8], mn[8];
+            auto load = [&](int64_t at) {
+                if (at + 7 * (int64_t)STRIDE >= nwords) return;
+#pragma unroll
+                for (int u = 0; u < 8; u++) xn[u] = __ldg(p + at + u * STRIDE);
+                if (MASK) {
+#pragma unroll
+                    for (int u = 0; u < 8; u++) mn[u] = __ldg(q + (((base & 1) + at) >> 1) + u * (STRIDE / 2));
+                }
+            };
+            load(w);
+            while (rounds < PCAL_BATCH / 8 && w + 7 * (int64_t)STRIDE < nwords) {
+                uint32_t x[8], m[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    x[u] = xn[u];
+                    m[u] = MASK ? mn[u] >> half & 0xffffu : 0u;
+                }
+                load(w + 8 * (int64_t)STRIDE);
+                added += 8;
+                add(x, m);
+            }
         }
+        while (rounds < PCAL_BATCH / 8 && w < nwords) {
+            uint32_t x[8], m[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int64_t wu = w + (int64_t)u * STRIDE;
+                const bool in = wu < nwords;
+                const int64_t wg = base + (wu >> lg) * win_words + (wu & (wpw - 1));
+                x[u] = in ? __ldg(plane + wg) : 0u;
+                m[u] = MASK && in ? __ldg(vmask + (wg >> 1)) >> ((wg & 1) * 16) & 0xffffu : 0u;
+                added += in;
+            }
+            add(x, m);
+        }
+        // planes in use: `rounds` groups of eight at most in any lane
+        const int np = 32 - __clz(__reduce_max_sync(0xffffffffu, rounds));
         // counts per code, summed over the lanes of the warp at the same place
         // in the period, then over the CTA
 #pragma unroll 1
         for (int j = 0; j < 16; j++) {
-            const int n01 = both.count(2 * j) + both.count(2 * j + 1);
-            const int n0 = bits.count(2 * j), n1 = bits.count(2 * j + 1);
-            const int nv = MASK ? val.count(2 * j) + val.count(2 * j + 1) : added;
+            const int n01 = both.count(2 * j, np) + both.count(2 * j + 1, np);
+            const int n0 = bits.count(2 * j, np), n1 = bits.count(2 * j + 1, np);
+            const int nv = MASK ? val.count(2 * j, np) + val.count(2 * j + 1, np) : added;
             int h[4] = {nv - n0 - n1 + n01, n0 - n01, n1 - n01, n01};
             for (int o = 16; o >= LW; o >>= 1) {
 #pragma unroll
@@ -710,7 +1084,57 @@ bool spec_cta_fft()
     return v;
 }
 
-int spec_chunk(const CsSpecArgs& a) { return a.ffts_per_chunk > 0 ? a.ffts_per_chunk : SPEC_CH; }
+// FFTs per chunk (one CTA, one partial spectrum; N = 65536: two CTAs): as many
+// as leave about three waves of CTAs on the chip.  Fewer, larger chunks share a
+// CTA's start and the writing of its partial spectrum between more FFTs; a small
+// job in chunks of 32 would leave most SMs idle (16 rows x 256 FFTs of 4096 points:
+// 220 us with 32, 95 with 4).  Not under 16 where a CTA's 16 or 8 groups
+// take one FFT each, nor under 4; not above 512, and 32 for N >= 4096, whose
+// partial spectra are the larger part of the scratch.
+int spec_chunk(const CsSpecArgs& a)
+{
+    if (a.ffts_per_chunk > 0) return a.ffts_per_chunk;
+    const int ctas = a.N <= 2048 ? 2 : a.N == 4096 ? 8 : a.N == 8192 ? 4 : a.N == 16384 ? 2 : 1;   // per SM
+    const int64_t waves = (int64_t)152 * 3 * ctas / (a.N == 65536 ? 2 : 1);
+    const int64_t total = (int64_t)(a.overlap * (int64_t)a.ffts_per_spectrum - (a.overlap - 1)) * a.nsub * a.nspec;
+    const int64_t ch = (total + waves - 1) / waves;
+    if (a.N <= 2048) return (int)(std::min<int64_t>(512, std::max<int64_t>(16, ch) + 15) / 16 * 16);
+    return (int)std::min<int64_t>(SPEC_CH, std::max<int64_t>(4, ch));
+}
+
+template <int L, int R>
+int launch_power_s(const CsSpecArgs& a, int nchunk, cudaStream_t st)
+{
+    using W = WarpFft<L, R>;
+    constexpr int N = 2 * W::M, GROUPS = SP_NT / L;
+    const float2* tw = a.tw_table ? a.tw_table : cs_twiddles(N);
+    const float* win = a.win_table ? a.win_table : window_table(a.window, N);
+    if (!tw || !win) return CS_ERR_ARG;
+    const size_t smem = (size_t)(W::TWIDDLES + GROUPS * W::TILE) * sizeof(float2) + (size_t)GROUPS * 2 * (N / 16) * 4;
+    auto kern = a.valid_mask ? k_spec_power_s<L, R, true> : k_spec_power_s<L, R, false>;
+    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
+    kern<<<dim3(nchunk, a.nsub * a.nspec), SP_NT, smem, st>>>(a, tw, win, nchunk, spec_chunk(a)), cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
+
+template <int MC, int P> int launch_power(const CsSpecArgs& a, int nchunk, cudaStream_t st);
+
+template <int M1>
+int launch_power_m(const CsSpecArgs& a, int nchunk, cudaStream_t st)
+{
+    using W = WarpFft<32, 32>;
+    constexpr int N = 2048 * M1;
+    // a caller's own tables come in natural order and without allocation
+    if (a.win_table) return launch_power<1024 * M1, 1>(a, nchunk, st);
+    const float2* tw = a.tw_table ? a.tw_table : cs_twiddles(N);
+    const float2* winp = window_pairs(a.window, N, M1);
+    if (!tw || !winp) return CS_ERR_ARG;
+    const size_t smem = (size_t)(W::TWIDDLES + M1 * W::TILE) * sizeof(float2) + (size_t)2 * (N / 16) * 4;
+    auto kern = a.valid_mask ? k_spec_power_m<M1, true> : k_spec_power_m<M1, false>;
+    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
+    kern<<<dim3(nchunk, a.nsub * a.nspec), 32 * M1, smem, st>>>(a, tw, winp, nchunk, spec_chunk(a)), cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
 
 template <int MC, int P>
 int launch_power(const CsSpecArgs& a, int nchunk, cudaStream_t st)
@@ -832,11 +1256,11 @@ int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st)
     const int nchunk = spec_nchunk(a);
     int rc = 0;
     if (!a.skip_power) switch (a.N) {
-        case 1024: rc = launch_power<512, 1>(a, nchunk, st); break;
-        case 2048: rc = launch_power<1024, 1>(a, nchunk, st); break;
-        case 4096: rc = launch_power<2048, 1>(a, nchunk, st); break;
-        case 8192: rc = launch_power<4096, 1>(a, nchunk, st); break;
-        case 16384: rc = launch_power<8192, 1>(a, nchunk, st); break;
+        case 1024: rc = launch_power_s<16, 32>(a, nchunk, st); break;
+        case 2048: rc = launch_power_s<32, 32>(a, nchunk, st); break;
+        case 4096: rc = launch_power_m<2>(a, nchunk, st); break;
+        case 8192: rc = launch_power_m<4>(a, nchunk, st); break;
+        case 16384: rc = launch_power_m<8>(a, nchunk, st); break;
         case 32768: rc = launch_power_long<1>(a, nchunk, st); break;
         case 65536: rc = launch_power_long<2>(a, nchunk, st); break;
         default: return CS_ERR_UNSUPPORTED;
@@ -847,7 +1271,8 @@ int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st)
     if (!a.skip_power) {
         const float scale = (float)(1.0 / (double)novl);
         const int slices = spec_reduce_slices((int64_t)rows * nb, nchunk), bins = RED_THREADS / slices;
-        k_spec_reduce<<<dim3((nb + bins - 1) / bins, rows), dim3(bins, slices), 0, st>>>(a.partial, a.power, nchunk, nb, scale),
+        (slices == 8 ? k_spec_reduce<8> : k_spec_reduce<1>)<<<dim3((nb + bins - 1) / bins, rows), RED_THREADS, 0, st>>>(
+            a.partial, a.power, nchunk, nb, scale),
             cs_count_launches(1);
         CS_CUDA_TRY(cudaGetLastError());
     }

@@ -247,3 +247,38 @@ def test_pcal_fold_places(cg, orc, nsub, N, L, T, overlap, K, nspec):
         for s in range(nspec):
             ref_t = orc.pcal_tones(ref_b[c, s], ntones)
             assert np.linalg.norm(tones[c, s] - ref_t) / np.linalg.norm(ref_t) < TOL
+
+
+@pytest.mark.parametrize("N,overlap,K,nspec,nsub", [
+    (1024, 1, 1, 1, 1),                  # one FFT
+    (1024, 64, 5, 2, 1),                 # starts every 16 samples: word copies
+    (1024, 32, 3, 1, 1),                 # starts every 32 samples
+    (1024, 2, 300, 2, 4),                # several rounds and chunks, a ragged last one
+    (2048, 4, 9, 3, 1), (2048, 128, 2, 1, 1), (2048, 2, 70, 1, 8),
+    (4096, 1, 33, 1, 4), (4096, 256, 2, 1, 1), (4096, 2, 17, 2, 1),
+    (8192, 4, 9, 1, 1), (8192, 2, 20, 1, 4), (16384, 2, 17, 1, 1), (16384, 1, 3, 2, 4)])
+@pytest.mark.parametrize("framed", [False, True])
+def test_power_sizes(cg, orc, N, overlap, K, nspec, nsub, framed):
+    """Every power kernel on odd counts of FFTs, from plain planes and from a VDIF recording with invalid frames."""
+    import synth
+
+    T, db, fs = N * K * nspec, 1000, 32e6
+    rng = np.random.default_rng(N + overlap + K)
+    if framed:
+        mbps = int(fs * 2 * nsub / 1e6)
+        nf = max(4, -(-T * nsub // (4 * db)) + 1)
+        raw = synth.vdif_frames(rng.integers(0, 256, nf * db, dtype=np.uint8), db, nsub, mbps)
+        for f in range(1, nf, 3):
+            synth.vdif_set_invalid(raw, f, db + 32)
+        planes = orc.vdif_decode_framed(raw, nsub, mbps, T)[1]
+        p = cg.spec_params(N, overlap, 3, K, nspec, nsub, raw.size, layout=cg.SPEC_VDIF_FRAMED, levels=cg.LEVELS_VDIF,
+                           fs_hz=fs)
+    else:
+        raw = rng.integers(0, 256, (T // 4 * nsub + 16 * nsub - 1) // (16 * nsub) * 16 * nsub, dtype=np.uint8)
+        planes = orc.unpack2bit(raw, T, nsub, orc.MARK5B_LUT)
+        p = cg.spec_params(N, overlap, 3, K, nspec, nsub, raw.size)
+    power = np.full((nsub, nspec, N // 2 + 1), np.nan, np.float32)
+    cg.spectrometer(p, raw, power)
+    for c in range(nsub):
+        ref, _ = orc.spectrometer(planes[c][:T], N, overlap, 3, K)
+        assert np.linalg.norm(power[c] - ref) / np.linalg.norm(ref) < TOL
