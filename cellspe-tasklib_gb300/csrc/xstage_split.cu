@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = align1k(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x, S = a.S, nk = (a.K + BK - 1) / BK;
+    const int c = blockIdx.x, nk = (a.K + BK - 1) / BK;
     const Pipe p = pipe_open<E, 1>(smem + a.stages * STAGE + gram_slack<R>(), a.stages, COLS, a.err, &tmap);
     const uint32_t sbase = tc::smem_u32(smem);
     if (warp == E) {
@@ -272,12 +272,15 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
             for (int j = 0; j < NC; j++) g[(32 * warp + lane) * GP + j] = acc[j];
             epi_vote(true, 32 * E);
             float2* out = a.vis + (int64_t)c * a.P;
-            for (int i = warp; i < S; i += E)
-                for (int j = lane; j <= i; j += 32) {
-                    const float re = (g[i * GP + j] + g[j * GP + i]) + (g[(R + i) * GP + R + j] + g[(R + j) * GP + R + i]);
-                    const float im = (g[(R + i) * GP + j] - g[(R + j) * GP + i]) + (g[j * GP + R + i] - g[i * GP + R + j]);
-                    out[(int64_t)i * (i + 1) / 2 + j] = make_float2(unscale(re, GRAM_BIAS, a.inv) * 0.5f, unscale(im, GRAM_BIAS, a.inv) * 0.5f);
-                }
+            for (int t = threadIdx.x; t < (int)a.P; t += 32 * E) {
+                int i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+                if ((i + 1) * (i + 2) / 2 <= t) i++;
+                else if (i * (i + 1) / 2 > t) i--;
+                const int j = t - i * (i + 1) / 2;
+                const float re = (g[i * GP + j] + g[j * GP + i]) + (g[(R + i) * GP + R + j] + g[(R + j) * GP + R + i]);
+                const float im = (g[(R + i) * GP + j] - g[(R + j) * GP + i]) + (g[j * GP + R + i] - g[i * GP + R + j]);
+                out[t] = make_float2(unscale(re, GRAM_BIAS, a.inv) * 0.5f, unscale(im, GRAM_BIAS, a.inv) * 0.5f);
+            }
         }
         tc::fence_before();
     }

@@ -33,6 +33,7 @@
 #include "tcgen05.cuh"
 #include "tma.h"
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -64,19 +65,20 @@ CS_DEV uint64_t sw64_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 512,
 // the four epilogue warps (2..5): named barrier 1 over their 128 threads, and
 // an AND vote on it that every one of them reaches
 CS_DEV void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-CS_DEV bool epi_vote(bool ok)
+CS_DEV bool group_vote(bool ok, int nthreads)
 {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.and.pred q, 1, 128, p;\n\t"
+        "bar.red.and.pred q, 1, %2, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"(ok ? 1u : 0u)
+        : "r"(ok ? 1u : 0u), "r"(nthreads)
         : "memory");
     return r != 0;
 }
+CS_DEV bool epi_vote(bool ok) { return group_vote(ok, 128); }
 
 struct TcArgs {
     int S, C, K;
@@ -301,6 +303,207 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
+// S <= 64: every product of a channel from a few MMAs per 16 segments.
+//   Planes: Z = [Xr; Xi], RI rows each (S rounded up to 8), is one operand; one
+//     MMA of 2 RI columns gives G = Z Z^T, Re V = Grr + Gii, Im V = Gir - Gri.
+//   k-blocked (BLK): an operand row holds a block's 32 Re and 32 Im halves; Re V
+//     takes two MMAs, M = Xi Xr^T one, Im V = M - M^T.
+// The parts are put together at the end through shared memory.  One TMA copy brings a
+// chunk of 128-byte rows (64 segments of both planes, or 32 of both parts): a
+// copy costs the SM's TMA unit about 125 cycles however small it is, which
+// bound the form with a copy per plane and 32 segments (521 us), and four MMAs
+// of S columns, at least 32 cycles each, the one before (622 us): 32 inputs x 4096
+// channels x 4096 segments, 310 us here (2.15 GB, 318 us at the copy rate).  The
+// accumulators are one TMEM buffer of COLS columns for the whole time axis.  Warps: E = COLS / 32
+// epilogue warps, the TMA producer, the MMA issuer and TMEM owner.
+// ---------------------------------------------------------------------------
+constexpr int G_ROW = 128;                          // operand row bytes
+template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : COLS == 32 ? 6 : COLS == 64 ? 5 : 4; }
+
+CS_DEV uint64_t sw128_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 8 * G_ROW, tc::SW128); }
+
+template <int COLS, bool BLK>
+__global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constant__ CUtensorMap tmap,
+                                                            const __grid_constant__ TcArgs a)
+{
+    constexpr int E = COLS / 32, ST = gram_stages<COLS, BLK>(), SEGS = BLK ? 32 : 64;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x, S = a.S, RI = a.box_rows, nk = (a.K + SEGS - 1) / SEGS;
+    const uint32_t stage_bytes = (uint32_t)(BLK ? RI : 2 * RI) * G_ROW;
+    // columns of an accumulator: all of G, or Re V and M side by side
+    const uint32_t n = BLK ? (uint32_t)((S + 15) & ~15) : 2 * (uint32_t)RI;
+    // barriers in front, so that the ring and the rows past it end the buffer
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem);                   // full[], empty[], acc
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
+    unsigned char* ring = smem + 1024;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * ST, accb = full0 + 16 * ST;
+    const uint32_t sbase = smem_u32(ring);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; s++) {
+            tc::mbar_init(full0 + 8 * s, 1);
+            tc::mbar_init(empty0 + 8 * s, 1);
+        }
+        tc::mbar_init(accb, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    }
+    if (warp == E + 1) tc::tmem_alloc(smem_u32(tmem_slot), COLS);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tmem_slot;
+    if (warp == E) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int kc = 0; kc < nk; kc++) {
+                const int s = kc % ST;
+                if (!tc::mbar_wait(empty0 + 8 * s, ((kc / ST) & 1) ^ 1, a.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) break;
+                const uint32_t st = sbase + s * stage_bytes, fb = full0 + 8 * s;
+                tc::mbar_expect_tx(fb, stage_bytes);
+                if constexpr (BLK) tc::tma_load_5d(st, &tmap, 0, a.kblock == 2 ? c & 15 : 0, kc, 0, a.kblock == 2 ? c >> 4 : c, fb);
+                else tc::tma_load_4d(st, &tmap, kc * SEGS, 0, 0, c, fb);
+                issued = kc + 1;
+            }
+            // drain: every stage this thread filled must have landed before the CTA exits
+            for (int kc = (issued > ST ? issued - ST : 0); kc < issued; kc++)
+                tc::mbar_wait(full0 + 8 * (kc % ST), (kc / ST) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
+        }
+    } else if (warp == E + 1) {
+        if (lane == 0) {
+            const uint32_t id = tc::idesc_f16(BM, n, false, false, false);
+            const uint64_t d0 = sw128_desc(sbase);
+            for (int kc = 0; kc < nk; kc++) {
+                const int s = kc % ST;
+                if (!tc::mbar_wait(full0 + 8 * s, (kc / ST) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) break;
+                tc::fence_after();
+                const uint64_t d = d0 + s * (stage_bytes / 16);
+                const uint32_t acc = kc ? 1u : 0u;
+                if constexpr (BLK) {
+                    // 16 segments are 32 bytes; the Im halves start at byte 64
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++) {
+                        const uint64_t re = d + 2 * kk, im = d + 4 + 2 * kk;
+                        tc::mma_f16(tmem, re, re, id, kk ? 1u : acc);
+                        tc::mma_f16(tmem + n, im, re, id, kk ? 1u : acc);
+                        tc::mma_f16(tmem, im, im, id, 1u);
+                    }
+                } else {
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++) tc::mma_f16(tmem, d + 2 * kk, d + 2 * kk, id, kk ? 1u : acc);
+                }
+                tc::commit(empty0 + 8 * s);
+            }
+            // always: the barrier then completes only after every MMA issued has finished
+            tc::commit(accb);
+        }
+        __syncwarp();
+    } else {
+        bool ok = tc::mbar_wait(accb, 0, a.err, ERR_ACC_WAIT, WAIT_CYCLES);
+        ok = ok && (*reinterpret_cast<volatile unsigned*>(a.err) == 0u);
+        // all or none of the epilogue warps go on (a product needs several rows)
+        if (group_vote(__all_sync(0xffffffffu, ok), 32 * E)) {
+            tc::fence_after();
+            float* g = reinterpret_cast<float*>(ring);           // free: the accumulators are final
+            const int rows = BLK ? RI : 2 * RI, cols = BLK ? 2 * (int)n : (int)n, GP = cols + 1;
+            if (32 * warp < rows) {
+                for (int cb = 0; cb < cols; cb += 16) {
+                    uint32_t v[16];
+                    tc::tmem_ld_32x32b_x16(tmem + ((uint32_t)(32 * warp) << 16) + cb, v);
+                    tc::tmem_ld_wait();
+                    if (32 * warp + lane < rows)
+#pragma unroll
+                        for (int j = 0; j < 16; j++) g[(32 * warp + lane) * GP + cb + j] = __uint_as_float(v[j]);
+                }
+            }
+            group_vote(true, 32 * E);
+            float2* out = a.vis + (int64_t)c * a.P;
+            for (int p = threadIdx.x; p < (int)a.P; p += 32 * E) {
+                int i = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);
+                if ((i + 1) * (i + 2) / 2 <= p) i++;
+                else if (i * (i + 1) / 2 > p) i--;
+                const int j = p - i * (i + 1) / 2;
+                float2 v;
+                if constexpr (BLK) v = make_float2(g[i * GP + j], g[i * GP + n + j] - g[j * GP + n + i]);
+                else v = make_float2(g[i * GP + j] + g[(RI + i) * GP + RI + j], g[(RI + i) * GP + j] - g[i * GP + RI + j]);
+                if (a.inv_scale) {
+                    const float f = __ldg(a.inv_scale + (int64_t)i * a.scale_stride + c) *
+                                    __ldg(a.inv_scale + (int64_t)j * a.scale_stride + c);
+                    v = make_float2(v.x * f, v.y * f);
+                }
+                if (a.accumulate) {
+                    const float2 old = out[p];
+                    v.x += old.x;
+                    v.y += old.y;
+                }
+                out[p] = v;
+            }
+        }
+        tc::fence_before();
+    }
+    __syncthreads();
+    if (warp == E + 1) {
+        tc::fence_after();
+        tc::tmem_dealloc(tmem, COLS);
+    }
+}
+
+template <int COLS, bool BLK>
+int launch_gram(const CUtensorMap& tm, const TcArgs& a, cudaStream_t st)
+{
+    // the ring, the rows past it that an MMA of 128 rows reads (lanes never
+    // stored), and after the last MMA the accumulators [rows][columns + 1]
+    const size_t rows = (BLK ? 1 : 2) * (size_t)a.box_rows, stage = rows * G_ROW;
+    const size_t cols = BLK ? 2 * (((size_t)a.S + 15) / 16 * 16) : rows;
+    const size_t ring = gram_stages<COLS, BLK>() * stage + BM * G_ROW - stage;
+    const size_t smem = 2048 + std::max(ring, rows * (cols + 1) * sizeof(float));
+    auto kern = k_xmac_tc_gram<COLS, BLK>;
+    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
+    kern<<<a.C, COLS + 64, smem, st>>>(tm, a), cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
+
+// S <= 64: tensor maps whose one box is a chunk's rows, 128 bytes each; inputs
+// past S and segments past K read as zeros.
+int xmac_gram(CsEncodeTiledFn enc, const void* spectra, int kp, TcArgs a, cudaStream_t st)
+{
+    const cuuint64_t S = a.S, C = a.C, K = a.K, rows = a.box_rows, pitch = (cuuint64_t)kp * 2;
+    const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+    CUtensorMap tm;
+    CUresult r;
+    auto encode = [&](int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
+        return enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(spectra), dim, stride, box, one,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    if (!a.kblock) {
+        // [C][2][S][kp] -> (64 segments, inputs, planes, channel)
+        const cuuint64_t dim[4] = {K, S, 2, C}, stride[3] = {pitch, S * pitch, 2 * S * pitch};
+        const cuuint32_t box[4] = {64, (cuuint32_t)rows, 2, 1};
+        r = encode(4, dim, stride, box);
+    } else if (a.kblock == 2) {
+        // [C/16][S][kp/32][16][64] -> (64 halves, channel of the group, block, inputs, group)
+        const cuuint64_t dim[5] = {64, 16, K / 32, S, C / 16};
+        const cuuint64_t stride[4] = {128, 2048, (cuuint64_t)kp / 32 * 2048, S * (kp / 32) * 2048};
+        const cuuint32_t box[5] = {64, 1, 1, (cuuint32_t)rows, 1};
+        r = encode(5, dim, stride, box);
+    } else {
+        // [C][S][kp/32][64] -> (64 halves, -, block, inputs, channel)
+        const cuuint64_t dim[5] = {64, 1, K / 32, S, C};
+        const cuuint64_t stride[4] = {128, 128, (cuuint64_t)kp / 32 * 128, S * (kp / 32) * 128};
+        const cuuint32_t box[5] = {64, 1, 1, (cuuint32_t)rows, 1};
+        r = encode(5, dim, stride, box);
+    }
+    if (r != CUDA_SUCCESS) return CS_ERR_ARG;
+    if (a.kblock)
+        return a.S <= 16 ? launch_gram<32, true>(tm, a, st)
+               : a.S <= 32 ? launch_gram<64, true>(tm, a, st) : launch_gram<128, true>(tm, a, st);
+    return a.S <= 16 ? launch_gram<32, false>(tm, a, st)
+           : a.S <= 32 ? launch_gram<64, false>(tm, a, st) : launch_gram<128, false>(tm, a, st);
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 std::mutex g_tiles_mu;
@@ -351,6 +554,11 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
         return CS_ERR_ARG;
     CsEncodeTiledFn enc = cs_encode_tiled();
     if (!enc) return CS_ERR_UNSUPPORTED;
+    if (S <= 64) {
+        const TcArgs g{S, C, K, (int64_t)S * (S + 1) / 2, nullptr, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
+                       accumulate, (S + 7) / 8 * 8, 1, 0, kblock, err};
+        return xmac_gram(enc, spectra, kp, g, st);
+    }
     int ntiles = 0;
     const int2* tiles = tile_list(S, &ntiles);
     if (!tiles) return CS_ERR_ARG;
@@ -392,7 +600,7 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     }
     if (r != CUDA_SUCCESS) return CS_ERR_ARG;
 
-    // S <= 128: one diagonal tile per channel, B = A, 16 KB stages and only the
+    // S <= 64: k_xmac_tc_gram; S <= 128: one diagonal tile per channel, B = A, 16 KB stages and only the
     // TMEM columns the tile needs, so several CTAs share an SM
     const int small = S <= BM ? 1 : 0;
     uint32_t cols = TMEM_COLS;

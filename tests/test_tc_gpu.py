@@ -38,6 +38,25 @@ def test_xmac_f16_exact_inputs(cg, S, C, K):
     assert np.abs(autos.imag).max() <= 1e-5 * np.abs(autos.real).max()
 
 
+@pytest.mark.parametrize("K", [8, 32, 40, 296])
+@pytest.mark.parametrize("S", [1, 2, 7, 8, 9, 16, 17, 31, 32, 33, 63, 64, 65])
+def test_xmac_f16_gram_sizes(cg, S, K):
+    """Up to 64 inputs one Gram matrix holds every product: row counts on both sides of its operand sizes, time axes of
+    part of a chunk, one and more than the ring holds; overwriting and accumulating."""
+    rng = np.random.default_rng(100 * S + K)
+    C = 5
+    spec = rng.standard_normal((C, 2, S, K)).astype(np.float16)
+    X = spec[:, 0].astype(np.float64) + 1j * spec[:, 1].astype(np.float64)
+    i, j = np.tril_indices(S)
+    ref = np.matmul(X, X.conj().transpose(0, 2, 1))[:, i, j]
+    vis = np.full((C, i.size), np.nan, np.complex64)
+    cg.xmac_f16(spec, S, C, K, vis)
+    # FP16 products are exact in FP32; K-term FP32 sums without rounding to nearest
+    assert np.linalg.norm(vis - ref) / np.linalg.norm(ref) < 1e-5
+    cg.xmac_f16(spec, S, C, K, vis, accumulate=True)
+    assert np.linalg.norm(vis - 2 * ref) / np.linalg.norm(ref) < 2e-5
+
+
 @pytest.mark.parametrize("S", [40, 200])
 def test_xmac_f16_accumulate(cg, S):
     """accumulate adds to the visibilities; S = 200 has diagonal tiles past the
