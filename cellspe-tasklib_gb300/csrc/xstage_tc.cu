@@ -10,9 +10,9 @@
 // SM's TMEM and one's epilogue overlaps the other's MMAs.  Each k-step issues
 // four kind::f16 MMAs (M=128, N=128, K=16); the minus sign of the last product
 // is the instruction descriptor's negate-A bit, so no negated copy of the data
-// exists.  Operands are K-major (time innermost), loaded by TMA with 64-byte
-// swizzle into a 3-stage shared-memory ring (32 KB stages) guarded by
-// mbarriers.  A diagonal tile (i0 = j0) loads its rows once and uses them as
+// exists.  Operands are K-major (time innermost), loaded by TMA into a 3-stage
+// shared-memory ring (32 KB stages) guarded by mbarriers, one copy per operand
+// bringing its Re and Im parts.  A diagonal tile (i0 = j0) loads its rows once and uses them as
 // both operands, and needs three MMAs per k-step: its Im columns accumulate
 // M = Xi Xr^T and the epilogue forms Im V = M - M^T through shared memory.
 //
@@ -23,8 +23,8 @@
 // and returns, and the host reports the failure.
 //
 // Layout in:  __half spectra[C][2][S][K]  (plane 0 = Re, plane 1 = Im), or
-//             k-blocked [C][S][K/32][2][32] (4-D tensor map), or channel-grouped
-//             k-blocked [C/16][S][K/32][16][2][32] (5-D tensor map)
+//             k-blocked [C][S][K/32][2][32], or channel-grouped k-blocked
+//             [C/16][S][K/32][16][2][32]
 // Layout out: float2 vis[C][P], p = i(i+1)/2 + j, j <= i
 #include <cuda.h>
 
@@ -61,6 +61,8 @@ using tc::smem_u32;
 // K-major operand in shared memory with 64-byte swizzle: 8-row x 64-byte
 // atoms stacked along M/N every 512 bytes (stride byte offset).
 CS_DEV uint64_t sw64_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 512, tc::SW64); }
+// the same with 128-byte rows (32 Re and 32 Im halves, or 64 segments of one part)
+CS_DEV uint64_t sw128_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 1024, tc::SW128); }
 
 // the four epilogue warps (2..5): named barrier 1 over their 128 threads, and
 // an AND vote on it that every one of them reaches
@@ -91,8 +93,8 @@ struct TcArgs {
     int box_rows;               // rows per TMA box: BM, or S rounded up to 8 when S < BM
     int small;                  // S <= BM: one tile per channel whose B operand is its A operand
     uint32_t tmem_cols;         // TMEM columns: Re V in [0, cols/2), Im V in [cols/2, cols)
-    int kblock;                 // spectra k-blocked: 1 [C][S][kp/32][2][32] (4-D tensor map),
-                                // 2 channel-grouped [C/16][S][kp/32][16][2][32] (5-D)
+    int kblock;                 // spectra k-blocked: 1 [C][S][kp/32][2][32],
+                                // 2 channel-grouped [C/16][S][kp/32][16][2][32]
     unsigned* err;              // CsErrorWord::code of the job
 };
 
@@ -119,7 +121,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
     // columns this tile needs: j < min(j0 + BN, i0 + BM, S), rounded up to 16
     const int n_need = min(min(j0 + BN, i0 + BM), S) - j0;
     const uint32_t n_eff = (uint32_t)((n_need + 15) & ~15);
-    const bool half_b = n_eff <= (uint32_t)BM;      // only the first 128 B rows are loaded
     // a diagonal tile (i0 == j0) multiplies its rows by themselves: B is A, so
     // its stages load A only (as every tile does when S <= BM)
     const bool diag = a.small || i0 == j0;
@@ -130,8 +131,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
     // S < 128: the boxes hold the S (rounded up to 8) rows that exist, so a
     // channel's planes are read once; the rows of the operand tiles past them
     // only feed accumulator rows and columns that are never stored
-    const uint32_t stage_tx = diag ? 2u * (uint32_t)a.box_rows * BK * 2
-                              : half_b ? 4u * (uint32_t)a.box_rows * BK * 2 : STAGE_BYTES;
+    const uint32_t stage_tx = (diag ? 2u : 4u) * (uint32_t)a.box_rows * BK * 2;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -153,16 +153,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            const int rowA_re = (c * 2 + 0) * S + i0, rowA_im = (c * 2 + 1) * S + i0;
-            const int rowB_re = (c * 2 + 0) * S + j0, rowB_im = (c * 2 + 1) * S + j0;
-            // k-blocked: rows (c, s) with the plane a coordinate of its own;
-            // channel-grouped: the input s a coordinate, the channel split
-            // into (c % 16, c / 16), the plane as x = 32 plane halves (64 B)
-            const int krowA = a.kblock == 2 ? i0 : c * S + i0, krowB = a.kblock == 2 ? j0 : c * S + j0;
-            auto load = [&](uint32_t dst, int kc, int plane, int row2d, int rowk, uint32_t bar) {
-                if (a.kblock == 2) tc::tma_load_5d(dst, &tmap, 32 * plane, c & 15, kc, rowk, c >> 4, bar);
-                else if (a.kblock) tc::tma_load_4d(dst, &tmap, 0, plane, kc, rowk, bar);
-                else tc::tma_load_2d(dst, &tmap, kc * BK, row2d, bar);
+            // one copy per operand brings both parts of its rows: planes as Re rows
+            // then Im rows of 64 bytes, k-blocked as rows of 32 Re and 32 Im halves
+            auto load = [&](uint32_t dst, int kc, int row, uint32_t bar) {
+                if (a.kblock) tc::tma_load_5d(dst, &tmap, 0, a.kblock == 2 ? c & 15 : 0, kc, row, a.kblock == 2 ? c >> 4 : c, bar);
+                else tc::tma_load_4d(dst, &tmap, kc * BK, row, 0, c, bar);
             };
             int issued = 0;
             bool ok = true;
@@ -173,16 +168,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
                 const uint32_t st = sbase + s * stage_bytes;
                 const uint32_t fb = full0 + 8 * s;
                 tc::mbar_expect_tx(fb, stage_tx);
-                load(st, kc, 0, rowA_re, krowA, fb);
-                load(st + A_BYTES, kc, 1, rowA_im, krowA, fb);
-                if (!diag) {
-                    load(st + 2 * A_BYTES, kc, 0, rowB_re, krowB, fb);
-                    load(st + 2 * A_BYTES + B_BYTES, kc, 1, rowB_im, krowB, fb);
-                }
-                if (!half_b) {
-                    load(st + 2 * A_BYTES + A_BYTES, kc, 0, rowB_re + BM, krowB + BM, fb);
-                    load(st + 2 * A_BYTES + B_BYTES + A_BYTES, kc, 1, rowB_im + BM, krowB + BM, fb);
-                }
+                load(st, kc, i0, fb);
+                if (!diag) load(st + 2 * A_BYTES, kc, j0, fb);
                 issued = kc + 1;
             }
             // drain: every stage this thread filled must have landed before the CTA exits
@@ -194,18 +181,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
         if (lane == 0) {
             const uint32_t id_pos = tc::idesc_f16(BM, n_eff, false, false, false), id_neg = tc::idesc_f16(BM, n_eff, true, false, false);
             const uint32_t d_re = tmem, d_im = tmem + a.tmem_cols / 2;
+            const uint64_t d0 = a.kblock ? sw128_desc(sbase) : sw64_desc(sbase);
+            const uint32_t im16 = a.kblock ? 4 : (uint32_t)a.box_rows * BK * 2 / 16;   // Im after Re, in 16 bytes
             bool ok = true;
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % STAGES;
                 if (!tc::mbar_wait(full0 + 8 * s, (kc / STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) { ok = false; break; }
                 tc::fence_after();
-                const uint32_t st = sbase + s * stage_bytes;
+                const uint64_t da = d0 + s * (stage_bytes / 16), db = diag ? da : da + 2 * A_BYTES / 16;
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
-                    const uint32_t off = kk * 32;                  // 16 FP16 along K
-                    const uint64_t ar = sw64_desc(st + off), ai = sw64_desc(st + A_BYTES + off);
-                    const uint64_t br = diag ? ar : sw64_desc(st + 2 * A_BYTES + off);
-                    const uint64_t bi = diag ? ai : sw64_desc(st + 2 * A_BYTES + B_BYTES + off);
+                    // 16 FP16 along K are 32 bytes
+                    const uint64_t ar = da + 2 * kk, ai = ar + im16, br = db + 2 * kk, bi = br + im16;
                     const uint32_t acc = (kc | kk) ? 1u : 0u;
                     tc::mma_f16(d_re, ar, br, id_pos, acc);           // Re += Ar Br^T
                     tc::mma_f16(d_re, ai, bi, id_pos, 1u);            // Re += Ai Bi^T
@@ -319,8 +306,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
 // ---------------------------------------------------------------------------
 constexpr int G_ROW = 128;                          // operand row bytes
 template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : COLS == 32 ? 6 : COLS == 64 ? 5 : 4; }
-
-CS_DEV uint64_t sw128_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 8 * G_ROW, tc::SW128); }
 
 template <int COLS, bool BLK>
 __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constant__ CUtensorMap tmap,
@@ -464,38 +449,39 @@ int launch_gram(const CUtensorMap& tm, const TcArgs& a, cudaStream_t st)
     return (int)cudaGetLastError();
 }
 
-// S <= 64: tensor maps whose one box is a chunk's rows, 128 bytes each; inputs
-// past S and segments past K read as zeros.
-int xmac_gram(CsEncodeTiledFn enc, const void* spectra, int kp, TcArgs a, cudaStream_t st)
+// Tensor map whose one box is an operand's rows of one chunk, both parts: planes
+// [C][2][S][kp] as (segments, inputs, planes, channel) with `segs` segments
+// (64-byte rows of 32, 128-byte rows of 64), k-blocked as (64 halves, ...).
+// Inputs past S and segments past K read as zeros.
+bool encode_map(CsEncodeTiledFn enc, const void* spectra, int kp, int segs, const TcArgs& a, CUtensorMap* tm)
 {
-    const cuuint64_t S = a.S, C = a.C, K = a.K, rows = a.box_rows, pitch = (cuuint64_t)kp * 2;
-    const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-    CUtensorMap tm;
-    CUresult r;
+    const cuuint64_t S = a.S, C = a.C, K = a.K, pitch = (cuuint64_t)kp * 2, blocks = (cuuint64_t)kp / 32;
+    const cuuint32_t rows = a.box_rows, one[5] = {1, 1, 1, 1, 1};
     auto encode = [&](int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
-        return enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(spectra), dim, stride, box, one,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        return enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(spectra), dim, stride, box, one,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
     if (!a.kblock) {
-        // [C][2][S][kp] -> (64 segments, inputs, planes, channel)
         const cuuint64_t dim[4] = {K, S, 2, C}, stride[3] = {pitch, S * pitch, 2 * S * pitch};
-        const cuuint32_t box[4] = {64, (cuuint32_t)rows, 2, 1};
-        r = encode(4, dim, stride, box);
-    } else if (a.kblock == 2) {
-        // [C/16][S][kp/32][16][64] -> (64 halves, channel of the group, block, inputs, group)
-        const cuuint64_t dim[5] = {64, 16, K / 32, S, C / 16};
-        const cuuint64_t stride[4] = {128, 2048, (cuuint64_t)kp / 32 * 2048, S * (kp / 32) * 2048};
-        const cuuint32_t box[5] = {64, 1, 1, (cuuint32_t)rows, 1};
-        r = encode(5, dim, stride, box);
-    } else {
-        // [C][S][kp/32][64] -> (64 halves, -, block, inputs, channel)
-        const cuuint64_t dim[5] = {64, 1, K / 32, S, C};
-        const cuuint64_t stride[4] = {128, 128, (cuuint64_t)kp / 32 * 128, S * (kp / 32) * 128};
-        const cuuint32_t box[5] = {64, 1, 1, (cuuint32_t)rows, 1};
-        r = encode(5, dim, stride, box);
+        const cuuint32_t box[4] = {(cuuint32_t)segs, rows, 2, 1};
+        return encode(4, dim, stride, box);
     }
-    if (r != CUDA_SUCCESS) return CS_ERR_ARG;
+    const cuuint32_t box[5] = {64, 1, 1, rows, 1};
+    if (a.kblock == 2) {
+        // [C/16][S][kp/32][16][64]: (64 halves, channel of the group, block, inputs, group)
+        const cuuint64_t dim[5] = {64, 16, K / 32, S, C / 16}, stride[4] = {128, 2048, blocks * 2048, S * blocks * 2048};
+        return encode(5, dim, stride, box);
+    }
+    // [C][S][kp/32][64]: (64 halves, -, block, inputs, channel)
+    const cuuint64_t dim[5] = {64, 1, K / 32, S, C}, stride[4] = {128, 128, blocks * 128, S * blocks * 128};
+    return encode(5, dim, stride, box);
+}
+
+int xmac_gram(CsEncodeTiledFn enc, const void* spectra, int kp, const TcArgs& a, cudaStream_t st)
+{
+    CUtensorMap tm;
+    if (!encode_map(enc, spectra, kp, 64, a, &tm)) return CS_ERR_ARG;
     if (a.kblock)
         return a.S <= 16 ? launch_gram<32, true>(tm, a, st)
                : a.S <= 32 ? launch_gram<64, true>(tm, a, st) : launch_gram<128, true>(tm, a, st);
@@ -563,43 +549,7 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     const int2* tiles = tile_list(S, &ntiles);
     if (!tiles) return CS_ERR_ARG;
 
-    CUtensorMap tm;
-    cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)C * 2 * S};
-    cuuint64_t gstride[1] = {(cuuint64_t)kp * 2};
     const int box_rows = S < BM ? (S + 7) / 8 * 8 : BM;
-    cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r;
-    if (!kblock) {
-        r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(spectra), gdim, gstride, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (kblock == 2) {
-        // [C/16 groups][S inputs][K/32 used of kp/32 blocks][16 channels][64
-        // halves (Re 32, Im 32)]: a box of (32 halves, 1 channel, 1 block,
-        // box_rows inputs, 1 group) lands as the same [rows][32] tile; inputs
-        // past S read as zeros
-        cuuint64_t g5[5] = {64, 16, (cuuint64_t)K / 32, (cuuint64_t)S, (cuuint64_t)C / 16};
-        cuuint64_t s5[4] = {128, 2048, (cuuint64_t)kp / 32 * 2048, (cuuint64_t)S * (kp / 32) * 2048};
-        cuuint32_t b5[5] = {32, 1, 1, (cuuint32_t)box_rows, 1};
-        cuuint32_t e5[5] = {1, 1, 1, 1, 1};
-        r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(spectra), g5, s5, b5, e5,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-        // [C*S rows][K/32 used of kp/32 blocks][2 planes][32 halves]: a box of
-        // (32 halves, 1 plane, 1 block, box_rows rows) lands in shared memory as
-        // the same [rows][32] tile as the channel-major map's box
-        cuuint64_t g4[4] = {32, 2, (cuuint64_t)K / 32, (cuuint64_t)C * S};
-        cuuint64_t s4[3] = {64, 128, (cuuint64_t)kp / 32 * 128};
-        cuuint32_t b4[4] = {32, 1, 1, (cuuint32_t)box_rows};
-        cuuint32_t e4[4] = {1, 1, 1, 1};
-        r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(spectra), g4, s4, b4, e4,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (r != CUDA_SUCCESS) return CS_ERR_ARG;
-
     // S <= 64: k_xmac_tc_gram; S <= 128: one diagonal tile per channel, B = A, 16 KB stages and only the
     // TMEM columns the tile needs, so several CTAs share an SM
     const int small = S <= BM ? 1 : 0;
@@ -611,6 +561,8 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     }
     TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, tiles, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
              accumulate, box_rows, small, cols, kblock, err};
+    CUtensorMap tm;
+    if (!encode_map(enc, spectra, kp, BK, a, &tm)) return CS_ERR_ARG;
     const size_t smem = (size_t)STAGES * (small ? 2 * A_BYTES : STAGE_BYTES) + 1024 + 256;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc), (int)smem));
     dim3 grid(ntiles, C);
