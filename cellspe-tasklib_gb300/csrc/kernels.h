@@ -142,11 +142,24 @@ int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised =
 // [C][P], P = S(S+1)/2, p = i(i+1)/2 + j (j <= i), V = sum_k X_i conj(X_j).
 int cs_xmac_f32(const float2* spectra, int S, int C, int K, int kp, float2* vis, int accumulate,
                 cudaStream_t st);
+// Mean relative loss of a Gram matrix's positive sums to the truncation of its
+// one-chunk accumulators, and an accumulated product in the spectra's own scale
+// with that loss given back (xstage_split.cu says how it was measured).
+constexpr float CS_GRAM_BIAS = 1.30e-7f;
+#ifdef __CUDACC__
+__device__ __forceinline__ float cs_split_unscale(float v, float bias, float inv) { return fmaf(v, bias, v) * inv * inv; }
+#endif
 // FP32 X stage on the tensor cores from spectra as two FP16 terms
 // (CsFStageArgs::split, scale 1 / inv_scale) -> vis float2 [C][P].
 int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err,
                   cudaStream_t st);
 float cs_xmac_split_lo(int S);       // the lo term's weight it expects for S inputs
+// X stage of small arrays straight from segment-major spectra [S][K][c_pitch]
+// (half2, or float2 taken as two FP16 terms of scale `split`), C channels from
+// `spectra` on -> vis float2 [C][P]; C and c_pitch multiples of 8.
+bool cs_xmac_seg_supported(int S);
+int cs_xmac_seg(const void* spectra, int format, int S, int C, int c_pitch, int K, float2* vis, const float* inv_scale,
+                int scale_stride, float split, unsigned* err, cudaStream_t st);
 // Tensor-core (tcgen05, FP16 in, FP32 accumulate) X stage:
 // spectra __half [C][2][S][kp] (K used; kp % 8 == 0), or k-blocked
 // [C][S][kp/32][2][32] with kblock = 1 (K, kp % 32 == 0), or channel-grouped

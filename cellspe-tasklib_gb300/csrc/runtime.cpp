@@ -633,7 +633,6 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     // FP16, N = 2048: 128-byte runs per 32 segments, k-blocked (1) or
     // channel-grouped k-blocked (2, the warp-specialised F stage)
     fa.kblock = cs_fstage_layout(fa);
-    fa.out = j.scratch((size_t)C * S * kp * (fa.format == CS_SPECTRA_F32 ? 8 : 4));
     if (sync) cudaEventRecord(ws.sev[1], ws.stream);
     // bytes of one spectra element: F32 rows [C][S][kp] of float2, F16 rows [C][2][S][kp] of half
     const long long el_bytes = fa.format == CS_SPECTRA_F32 ? 8 : 2;
@@ -641,7 +640,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     // their spectra are written segment-major and transposed in 64 x 64 tiles
     const bool segmaj = N >= 4096;
     const long long seg_bytes = fa.format == CS_SPECTRA_F32 ? 8 : 4;       // one channel of one segment
+    // small arrays: the X stage reads the segment-major spectra itself
+    const bool seg_x = segmaj && (fa.format == CS_SPECTRA_F16 || fa.split > 0.f) && cs_xmac_seg_supported(S);
     char* seg_tmp = segmaj ? (char*)j.scratch((size_t)((long long)S * K * C * seg_bytes)) : nullptr;
+    fa.out = seg_x ? seg_tmp : j.scratch((size_t)C * S * kp * (fa.format == CS_SPECTRA_F32 ? 8 : 4));
     for (int i = 0; i < nsc && !j.err; i++) {
         CsFStageArgs fb = fa;
         long long s0 = 0, s1 = S;
@@ -665,7 +667,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             fb.out = seg_tmp + s0 * K * C * seg_bytes;
         }
         int rc = map_rc(cs_fx_fstage(fb, ws.stream), "F stage");
-        if (!rc && segmaj)
+        if (!rc && segmaj && !seg_x)
             rc = map_rc(cs_spectra_transpose(fb.out, (int)(s1 - s0), K, C, kp, S, fa.format, rows_out, ws.stream, fa.split,
                                              fa.split_lo),
                         "spectra transpose");
@@ -689,18 +691,21 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     for (int b = 0; b < ncb && !j.err; b++) {
         // streamed output: a small first block (1/16 of the channels) starts the
         // copy out early; the rest in equal blocks
-        // (channel-grouped spectra: block bounds on whole groups of 16 channels)
+        // (channel-grouped and segment-major spectra: block bounds on whole groups of 16 channels)
         auto cbound = [&](int i) -> long long {
             if (ncb == 1) return i ? C : 0;
             if (i == ncb) return C;
             const long long first = std::max(1LL, (long long)C / 16);
             const long long c = i == 0 ? 0 : first + (long long)(C - first) * (i - 1) / (ncb - 1);
-            return fa.kblock == 2 ? c / 16 * 16 : c;
+            return fa.kblock == 2 || seg_x ? c / 16 * 16 : c;
         };
         const long long c0 = cbound(b), c1 = cbound(b + 1), cn = c1 - c0;
         if (cn <= 0) continue;
         int rc;
-        if (fa.split > 0.f)
+        if (seg_x)
+            rc = cs_xmac_seg(seg_tmp + c0 * seg_bytes, fa.format, S, (int)cn, C, K, vis_cp + c0 * P,
+                             d_inv_scale ? d_inv_scale + c0 : nullptr, C, fa.split, ws.x_err(), ws.stream);
+        else if (fa.split > 0.f)
             rc = cs_xmac_split((const char*)fa.out + c0 * S * kp * 8, S, (int)cn, K, kp, vis_cp + c0 * P, 1.f / fa.split,
                                ws.x_err(), ws.stream);
         else if (p->x_mode == CELLSPE_X_FP32)
@@ -2436,7 +2441,9 @@ cellspe_service* cellspe_service_create(const cellspe_service_config* cfg)
     sv->priority_samples = !cfg || cfg->priority_samples == 0 ? (1LL << 24) : cfg->priority_samples;
     sv->large_samples = cfg ? cfg->large_samples : 0;
     // batching is on by default (64 inputs); a negative batch_inputs turns it off
-    sv->batch_inputs = !cfg || cfg->batch_inputs == 0 ? 64 : std::max(0, std::min(cfg->batch_inputs, 128));
+    // (the X stage's forms for more than 64 inputs add in another order than those a
+    // small job runs alone, and a batched job's values are to equal its solo run's)
+    sv->batch_inputs = !cfg || cfg->batch_inputs == 0 ? 64 : std::max(0, std::min(cfg->batch_inputs, 64));
     for (int i = 0; i < n; i++) sv->workers.emplace_back(service_worker, sv);
     return sv;
 }

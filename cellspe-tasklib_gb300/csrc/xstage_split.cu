@@ -64,7 +64,7 @@ constexpr long long WAIT_CYCLES = 4000000000LL;     // ~2 s at 2 GHz
 // truncation, given back at the end: measured as the mean error of the autos
 // against FP64 less that of the FP32 transform alone, the same to 0.1e-7 at N = 512,
 // 2048 and 8192, K = 24 .. 1024 (two hi hi' MMAs per chunk and accumulator, four for a tile).
-constexpr float GRAM_BIAS = 1.30e-7f, TILE_BIAS = 2.17e-7f;
+constexpr float GRAM_BIAS = CS_GRAM_BIAS, TILE_BIAS = 2.17e-7f;
 constexpr unsigned ERR_FULL_WAIT = 1, ERR_EMPTY_WAIT = 2, ERR_ACC_WAIT = 3, ERR_DRAIN_WAIT = 4;
 
 // K-major operand of 128-byte rows; a descriptor's low 14 bits hold the address / 16,
@@ -217,9 +217,6 @@ CS_DEV bool accumulate(const Pipe& p, int nk, uint32_t lanes, uint32_t step, int
     return __all_sync(0xffffffffu, ok);
 }
 
-// an accumulated product in the spectra's own scale
-CS_DEV float unscale(float v, float bias, float inv) { return fmaf(v, bias, v) * inv * inv; }
-
 CS_DEV unsigned char* align1k(unsigned char* p) { return p + ((1024u - (tc::smem_u32(p) & 1023u)) & 1023u); }
 
 // ---- S <= 64: the Gram matrix of Z = [Xr; Xi], 2 R rows -----------------------
@@ -279,7 +276,7 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
                 const int j = t - i * (i + 1) / 2;
                 const float re = (g[i * GP + j] + g[j * GP + i]) + (g[(R + i) * GP + R + j] + g[(R + j) * GP + R + i]);
                 const float im = (g[(R + i) * GP + j] - g[(R + j) * GP + i]) + (g[j * GP + R + i] - g[i * GP + R + j]);
-                out[t] = make_float2(unscale(re, GRAM_BIAS, a.inv) * 0.5f, unscale(im, GRAM_BIAS, a.inv) * 0.5f);
+                out[t] = make_float2(cs_split_unscale(re, GRAM_BIAS, a.inv) * 0.5f, cs_split_unscale(im, GRAM_BIAS, a.inv) * 0.5f);
             }
         }
         tc::fence_before();
@@ -410,7 +407,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
                     for (int j = 0; j < 16; j++) {
                         float im = acci[cb * 16 + j];
                         if (diag) im -= msh[(col0 + cb * 16 + j) * MP + r];
-                        stg[lane * 17 + j] = make_float2(unscale(accr[cb * 16 + j], TILE_BIAS, a.inv), unscale(im, TILE_BIAS, a.inv));
+                        stg[lane * 17 + j] = make_float2(cs_split_unscale(accr[cb * 16 + j], TILE_BIAS, a.inv), cs_split_unscale(im, TILE_BIAS, a.inv));
                     }
                     __syncwarp();
 #pragma unroll 4

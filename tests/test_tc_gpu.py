@@ -269,3 +269,24 @@ def test_fx_tc32_fstage_delay_model_and_scale(cg, orc, fstage32):
     vs = np.zeros_like(vis)
     cg.fx_correlate(ps, raw, vs, delay_poly=poly)
     assert np.linalg.norm(vs - vis) / np.linalg.norm(vis) < 1e-3
+
+
+@pytest.mark.parametrize("mode", ["tc", "fp32"])
+@pytest.mark.parametrize("S,N,K", [(1, 4096, 8), (8, 4096, 72), (9, 4096, 24), (16, 8192, 136), (17, 4096, 40),
+                                   (32, 4096, 264), (32, 16384, 24), (33, 4096, 40), (64, 4096, 96), (65, 4096, 32)])
+def test_fx_segment_major_sizes(cg, orc, S, N, K, mode):
+    """Long transforms: the X stage that reads segment-major spectra itself on both sides of its input counts, with
+    time axes of part of a chunk, one chunk and more than its ring; the tensor-core form with a channel scale."""
+    import synth
+
+    raw = synth.stations_offset_binary(S, N * K, rho=0.3, seed=S + K)
+    C, tc = N // 2, mode == "tc"
+    scale = np.random.default_rng(S).uniform(0.5, 2.0, (S, C)).astype(np.float32) if tc else None
+    p = cg.fx_params(S, N, K, raw.shape[1], x_mode=cg.X_TC_FP16 if tc else cg.X_FP32, channel_scale=scale)
+    vis = np.full((C, S * (S + 1) // 2), np.nan, np.complex64)
+    cg.fx_correlate(p, raw, vis)
+    X = np.ascontiguousarray(orc.fx_spectra_f64(raw, S, N, K).transpose(2, 0, 1))
+    i, j = np.tril_indices(S)
+    ref = np.matmul(X, X.conj().transpose(0, 2, 1))[:, i, j]
+    # FP16 spectra: 2^-12 per value, less over K; FP32: a few 2^-24
+    assert np.linalg.norm(vis - ref) / np.linalg.norm(ref) < (1e-3 if tc else 2e-6)
