@@ -10,9 +10,8 @@
 // segment of a chunk (32 KB), and each of eight warps' threads turns eight
 // segments of its channels into 16-byte pieces of the swizzled operand rows, up
 // to three chunks behind the copies.  The spectra are read once and
-// nothing is written.  Products as in k_xmac_tc_gram and k_xmac_gram: the rows
-// Z = [Xr; Xi] of a channel multiply themselves, Re V and Im V are parts of
-// G = Z Z^T put together at the end.  Bound by the read of the spectra: those 32
+// nothing is written.  The arithmetic is k_xmac_tc_gram's (FP16: rows Xr, Xi and
+// zeros, Re V and M in one accumulator) and k_xmac_gram's (FP32).  Bound by the read of the spectra: those 32
 // inputs take 436 us in FP16 (2.15 GB, 318 us at the copy rate; 512 CTAs of 3.4
 // waves) and 831 us in FP32, with the transpose 1040 and 2300.  (Register loads instead of TMA: 614 and 1285 us, cp.async 1030 and 1700; the F
 // stage writing blocks of channels for 128-byte TMA rows: 420 and 825, but its
@@ -102,22 +101,21 @@ CS_DEV void product(int p, int& i, int& j)
 }
 
 // ---- FP16 ------------------------------------------------------------------
-// RI: inputs rounded up to 16 or 32; eight channels per CTA, whose accumulators
-// of 2 RI columns fill half (RI = 16, two CTAs per SM) or all of TMEM.  A chunk of SEGS
-// segments gives each loader one task: 8 segments of 4 channels of an input.
+// RI: inputs rounded up to 16 or 32; eight channels per CTA, with accumulators of
+// RI columns.  A chunk of SEGS segments gives each loader one task: 8 segments of 4
+// channels of an input.
 template <int RI> struct F16Cfg {
     static constexpr int CB = 8, SEGS = RI == 16 ? 64 : 32, ROWB = 2 * SEGS, KG = SEGS / 8;
     using R = Raw<RI, SEGS>;
-    static constexpr int CTAS = RI == 16 ? 2 : 1, COLS = CB * 2 * RI;
-    static constexpr uint32_t TILE = 2 * RI * ROWB, STAGE = CB * TILE;      // 32 KB
-    static constexpr int STAGES = RI == 16 ? 1 : 3, DEPTH = RI == 16 ? 2 : 3;
+    static constexpr int COLS = CB * RI;
+    static constexpr uint32_t TILE = 3 * RI * ROWB, STAGE = CB * TILE;      // 48 KB
+    static constexpr int STAGES = 2, DEPTH = 3;
     static constexpr uint32_t SLACK = (BM - 2 * RI) * ROWB;                 // operand rows an MMA reads past the ring
-    static constexpr int GCH = RI == 32 ? 4 : 8;                            // channels put together at a time
     static_assert(RI * KG * 2 == LOADERS, "one task per loader");
 };
 
 template <int RI>
-__global__ void __launch_bounds__(LOADERS + 64, F16Cfg<RI>::CTAS)
+__global__ void __launch_bounds__(LOADERS + 96, 1)
     k_xmac_seg_f16(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ SegArgs a)
 {
     using F = F16Cfg<RI>;
@@ -134,38 +132,49 @@ __global__ void __launch_bounds__(LOADERS + 64, F16Cfg<RI>::CTAS)
     if (tid == 0) {
         for (int s = 0; s < F::STAGES; s++) {
             tc::mbar_init(full0 + 8 * s, LOADERS / 32);
-            tc::mbar_init(empty0 + 8 * s, 1);
+            tc::mbar_init(empty0 + 8 * s, 2);
         }
         for (int r = 0; r < F::DEPTH; r++) {
             tc::mbar_init(rfull + 8 * r, 1);
             tc::mbar_init(rempty + 8 * r, LOADERS / 32);
         }
-        tc::mbar_init(accb, 1);
+        tc::mbar_init(accb, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // the zero rows of every tile
+    constexpr uint32_t ZB = RI * F::ROWB;
+    for (uint32_t i = tid; i < F::STAGES * F::CB * ZB / 16; i += LOADERS + 96)
+        *reinterpret_cast<uint4*>(ring + i / (ZB / 16) * F::TILE + 2 * ZB + i % (ZB / 16) * 16) = make_uint4(0, 0, 0, 0);
+    tc::fence_proxy_async();
     if (warp == LOADERS / 32) tc::tmem_alloc(tc::smem_u32(slot), F::COLS);
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *slot;
 
-    if (warp == LOADERS / 32 + 1) {
+    if (warp == LOADERS / 32 + 2) {
         if (lane == 0)
             feed<F::DEPTH, F::SEGS>(&tmap, tc::smem_u32(raw), F::R::BYTES, rfull, rempty, nk, a.err);
-    } else if (warp == LOADERS / 32) {
+    } else if (warp >= LOADERS / 32) {
+        // two issuers, four channels each: one thread's instructions took as long
+        // as the MMAs (611 us with one, 512 unrolled, SEG2_NEW with two)
+        const int ca = (warp - LOADERS / 32) * (F::CB / 2);
         if (lane == 0) {
-            const uint32_t id = tc::idesc_f16(BM, 2 * RI, false, false, false);
+            const uint32_t id = tc::idesc_f16(BM, RI, false, false, false);
             const uint64_t d0 = tc::smem_desc(tc::smem_u32(ring), 16, 8 * F::ROWB, F::ROWB == 128 ? tc::SW128 : tc::SW64);
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % F::STAGES;
                 if (!tc::mbar_wait(full0 + 8 * s, (kc / F::STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) break;
                 tc::fence_after();
-#pragma unroll 1
-                for (int c = 0; c < F::CB; c++) {
-                    const uint64_t d = d0 + (s * F::STAGE + c * F::TILE) / 16;
 #pragma unroll
-                    for (int kk = 0; kk < F::SEGS / 16; kk++)
-                        tc::mma_f16(tmem + c * 2 * RI, d + 2 * kk, d + 2 * kk, id, (kc | kk) ? 1u : 0u);
+                for (int q = 0; q < F::CB / 2; q++) {
+                    const int c = ca + q;
+                    const uint64_t d = d0 + (s * F::STAGE + c * F::TILE) / 16, di = d + RI * F::ROWB / 16;
+#pragma unroll
+                    for (int kk = 0; kk < F::SEGS / 16; kk++) {
+                        tc::mma_f16(tmem + c * RI, d + 2 * kk, d + 2 * kk, id, (kc | kk) ? 1u : 0u);
+                        tc::mma_f16(tmem + c * RI, di + 2 * kk, di + 2 * kk, id, 1u);
+                    }
                 }
                 tc::commit(empty0 + 8 * s);
             }
@@ -218,40 +227,37 @@ __global__ void __launch_bounds__(LOADERS + 64, F16Cfg<RI>::CTAS)
         ok = ok && (*reinterpret_cast<volatile unsigned*>(a.err) == 0u);
         if (vote(__all_sync(0xffffffffu, ok), LOADERS)) {
             tc::fence_after();
-            // the ring is free: GCH channels' G at a time, [2 RI][2 RI + 1]
-            constexpr int N2 = 2 * RI, GP = N2 + 1, Q = N2 / 32;           // Q: lane quarters in use
+            // the ring is free: every channel's Re V rows, then M rows, [2 RI][RI + 1]
+            constexpr int GP = RI + 1, Q = 2 * RI / 32;                     // Q: lane quarters in use
             float* g0 = reinterpret_cast<float*>(ring);
             const int q = warp & 3;
-            for (int cb = 0; cb < F::CB; cb += F::GCH) {
-                if (q < Q)
-                    // two warps read each quarter, every other 16 columns
-                    for (int t = (warp >> 2) * 16; t < F::GCH * N2; t += 32) {
-                        const int c = t / N2, col = t % N2;
-                        uint32_t v[16];
-                        tc::tmem_ld_32x32b_x16(tmem + ((uint32_t)(32 * q) << 16) + (cb + c) * N2 + col, v);
-                        tc::tmem_ld_wait();
-                        float* g = g0 + (c * N2 + 32 * q + lane) * GP + col;
+            if (q < Q)
+                // two warps read each quarter, every other 16 columns
+                for (int t = (warp >> 2) * 16; t < F::CB * RI; t += 32) {
+                    const int c = t / RI, col = t % RI;
+                    uint32_t v[16];
+                    tc::tmem_ld_32x32b_x16(tmem + ((uint32_t)(32 * q) << 16) + t, v);
+                    tc::tmem_ld_wait();
+                    float* g = g0 + (c * 2 * RI + 32 * q + lane) * GP + col;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) g[j] = __uint_as_float(v[j]);
-                    }
-                vote(true, LOADERS);
-                for (int c = 0; c < F::GCH; c++) {
-                    const int cg = c0 + cb + c;
-                    const float* g = g0 + c * N2 * GP;
-                    float2* out = a.vis + (int64_t)cg * a.P;
-                    for (int p = tid; p < (int)a.P; p += LOADERS) {
-                        int i, j;
-                        product(p, i, j);
-                        float2 v = make_float2(g[i * GP + j] + g[(RI + i) * GP + RI + j], g[(RI + i) * GP + j] - g[i * GP + RI + j]);
-                        if (a.inv_scale) {
-                            const float f = __ldg(a.inv_scale + (int64_t)i * a.scale_stride + cg) *
-                                            __ldg(a.inv_scale + (int64_t)j * a.scale_stride + cg);
-                            v = make_float2(v.x * f, v.y * f);
-                        }
-                        out[p] = v;
-                    }
+                    for (int j = 0; j < 16; j++) g[j] = __uint_as_float(v[j]);
                 }
-                vote(true, LOADERS);
+            vote(true, LOADERS);
+            for (int c = 0; c < F::CB; c++) {
+                const int cg = c0 + c;
+                const float* g = g0 + c * 2 * RI * GP;
+                float2* out = a.vis + (int64_t)cg * a.P;
+                for (int p = tid; p < (int)a.P; p += LOADERS) {
+                    int i, j;
+                    product(p, i, j);
+                    float2 v = make_float2(g[i * GP + j], g[(RI + i) * GP + j] - g[(RI + j) * GP + i]);
+                    if (a.inv_scale) {
+                        const float f = __ldg(a.inv_scale + (int64_t)i * a.scale_stride + cg) *
+                                        __ldg(a.inv_scale + (int64_t)j * a.scale_stride + cg);
+                        v = make_float2(v.x * f, v.y * f);
+                    }
+                    out[p] = v;
+                }
             }
         }
         tc::fence_before();
@@ -473,10 +479,10 @@ int launch_f16(const void* spectra, int64_t pitch, const SegArgs& a, cudaStream_
     using F = F16Cfg<RI>;
     CUtensorMap tm;
     if (!encode_map<F>(spectra, a, a.C, pitch, RI, &tm)) return CS_ERR_ARG;
-    const size_t ring = F::STAGES * F::STAGE + F::SLACK + F::DEPTH * F::R::BYTES, g = (size_t)F::GCH * 2 * RI * (2 * RI + 1) * 4;
+    const size_t ring = F::STAGES * F::STAGE + F::SLACK + F::DEPTH * F::R::BYTES, g = (size_t)F::CB * 2 * RI * (RI + 1) * 4;
     const size_t smem = 2048 + std::max(ring, g);
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_seg_f16<RI>), (int)smem));
-    k_xmac_seg_f16<RI><<<a.C / F::CB, LOADERS + 64, smem, st>>>(tm, a), cs_count_launches(1);
+    k_xmac_seg_f16<RI><<<a.C / F::CB, LOADERS + 96, smem, st>>>(tm, a), cs_count_launches(1);
     return (int)cudaGetLastError();
 }
 

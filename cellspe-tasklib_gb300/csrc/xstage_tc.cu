@@ -291,18 +291,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
 
 // ---------------------------------------------------------------------------
 // S <= 64: every product of a channel from a few MMAs per 16 segments.
-//   Planes: Z = [Xr; Xi], RI rows each (S rounded up to 8), is one operand; one
-//     MMA of 2 RI columns gives G = Z Z^T, Re V = Grr + Gii, Im V = Gir - Gri.
+//   Planes: a stage holds Xr, Xi and zeros, RI rows each (S rounded up to 8).
+//     [Xr; Xi] Xr^T and [Xi; 0] Xi^T go into one accumulator, whose upper rows
+//     are then Re V, added in the order of the tiles below (Re, Im, Re, ... : the
+//     accumulator truncates, so another order would move every auto by parts in
+//     10^5 at thousands of segments), and whose lower rows are M = Xi Xr^T.
 //   k-blocked (BLK): an operand row holds a block's 32 Re and 32 Im halves; Re V
-//     takes two MMAs, M = Xi Xr^T one, Im V = M - M^T.
-// The parts are put together at the end through shared memory.  One TMA copy brings a
-// chunk of 128-byte rows (64 segments of both planes, or 32 of both parts): a
-// copy costs the SM's TMA unit about 125 cycles however small it is, which
-// bound the form with a copy per plane and 32 segments (521 us), and four MMAs
-// of S columns, at least 32 cycles each, the one before (622 us): 32 inputs x 4096
-// channels x 4096 segments, 310 us here (2.15 GB, 318 us at the copy rate).  The
-// accumulators are one TMEM buffer of COLS columns for the whole time axis.  Warps: E = COLS / 32
-// epilogue warps, the TMA producer, the MMA issuer and TMEM owner.
+//     takes two MMAs, M one.
+// Im V = M - M^T is put together at the end through shared memory.  One TMA copy
+// brings a chunk of 128-byte rows (64 segments of both planes, or 32 of both
+// parts): a copy costs the SM's TMA unit about 125 cycles however small it is,
+// which bound a form with a copy per plane and 32 segments; four MMAs of S columns per
+// 16 segments, at least 32 cycles each, bound the tiles.  32 inputs x 4096
+// channels x 4096 segments (2.15 GB, 318 us at the copy rate) take 352 us a call
+// where the tiles took 643, 64 x 2048 x 4096 341 where they took 462; for 16 inputs and
+// fewer the MMAs' least cost still bounds it (8 x 4096 x 4096: 618 -> 307 us).  The
+// accumulators are one TMEM buffer of COLS columns for the whole time axis.  Warps:
+// E = COLS / 32 epilogue warps, the TMA producer, the MMA issuer and TMEM owner.
 // ---------------------------------------------------------------------------
 constexpr int G_ROW = 128;                          // operand row bytes
 template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : COLS == 32 ? 6 : COLS == 64 ? 5 : 4; }
@@ -316,9 +321,9 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x, S = a.S, RI = a.box_rows, nk = (a.K + SEGS - 1) / SEGS;
-    const uint32_t stage_bytes = (uint32_t)(BLK ? RI : 2 * RI) * G_ROW;
-    // columns of an accumulator: all of G, or Re V and M side by side
-    const uint32_t n = BLK ? (uint32_t)((S + 15) & ~15) : 2 * (uint32_t)RI;
+    const uint32_t plane = (uint32_t)RI * G_ROW, stage_bytes = BLK ? plane : 3 * plane;
+    // columns of an accumulator (BLK: Re V and M side by side)
+    const uint32_t n = (uint32_t)((S + 15) & ~15);
     // barriers in front, so that the ring and the rows past it end the buffer
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);                   // full[], empty[], acc
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
@@ -334,6 +339,11 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
     }
+    if constexpr (!BLK) {
+        for (uint32_t i = threadIdx.x; i < ST * plane / 16; i += COLS + 64)
+            *reinterpret_cast<uint4*>(ring + i / (plane / 16) * stage_bytes + 2 * plane + i % (plane / 16) * 16) = make_uint4(0, 0, 0, 0);
+        tc::fence_proxy_async();
+    }
     if (warp == E + 1) tc::tmem_alloc(smem_u32(tmem_slot), COLS);
     tc::fence_before();
     __syncthreads();
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
                 const int s = kc % ST;
                 if (!tc::mbar_wait(empty0 + 8 * s, ((kc / ST) & 1) ^ 1, a.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) break;
                 const uint32_t st = sbase + s * stage_bytes, fb = full0 + 8 * s;
-                tc::mbar_expect_tx(fb, stage_bytes);
+                tc::mbar_expect_tx(fb, BLK ? plane : 2 * plane);
                 if constexpr (BLK) tc::tma_load_5d(st, &tmap, 0, a.kblock == 2 ? c & 15 : 0, kc, 0, a.kblock == 2 ? c >> 4 : c, fb);
                 else tc::tma_load_4d(st, &tmap, kc * SEGS, 0, 0, c, fb);
                 issued = kc + 1;
@@ -375,8 +385,12 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
                         tc::mma_f16(tmem, im, im, id, 1u);
                     }
                 } else {
+                    const uint64_t di = d + plane / 16;
 #pragma unroll
-                    for (int kk = 0; kk < 4; kk++) tc::mma_f16(tmem, d + 2 * kk, d + 2 * kk, id, kk ? 1u : acc);
+                    for (int kk = 0; kk < 4; kk++) {
+                        tc::mma_f16(tmem, d + 2 * kk, d + 2 * kk, id, kk ? 1u : acc);
+                        tc::mma_f16(tmem, di + 2 * kk, di + 2 * kk, id, 1u);
+                    }
                 }
                 tc::commit(empty0 + 8 * s);
             }
@@ -411,7 +425,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
                 const int j = p - i * (i + 1) / 2;
                 float2 v;
                 if constexpr (BLK) v = make_float2(g[i * GP + j], g[i * GP + n + j] - g[j * GP + n + i]);
-                else v = make_float2(g[i * GP + j] + g[(RI + i) * GP + RI + j], g[(RI + i) * GP + j] - g[i * GP + RI + j]);
+                else v = make_float2(g[i * GP + j], g[(RI + i) * GP + j] - g[(RI + j) * GP + i]);
                 if (a.inv_scale) {
                     const float f = __ldg(a.inv_scale + (int64_t)i * a.scale_stride + c) *
                                     __ldg(a.inv_scale + (int64_t)j * a.scale_stride + c);
@@ -439,9 +453,10 @@ int launch_gram(const CUtensorMap& tm, const TcArgs& a, cudaStream_t st)
 {
     // the ring, the rows past it that an MMA of 128 rows reads (lanes never
     // stored), and after the last MMA the accumulators [rows][columns + 1]
-    const size_t rows = (BLK ? 1 : 2) * (size_t)a.box_rows, stage = rows * G_ROW;
-    const size_t cols = BLK ? 2 * (((size_t)a.S + 15) / 16 * 16) : rows;
-    const size_t ring = gram_stages<COLS, BLK>() * stage + BM * G_ROW - stage;
+    const size_t plane = (size_t)a.box_rows * G_ROW, rows = (BLK ? 1 : 2) * (size_t)a.box_rows;
+    const size_t cols = (BLK ? 2 : 1) * (((size_t)a.S + 15) / 16 * 16);
+    // an operand of 128 rows from the last stage's Xr (BLK) or Xi on
+    const size_t ring = gram_stages<COLS, BLK>() * (BLK ? plane : 3 * plane) + BM * G_ROW - (BLK ? plane : 2 * plane);
     const size_t smem = 2048 + std::max(ring, rows * (cols + 1) * sizeof(float));
     auto kern = k_xmac_tc_gram<COLS, BLK>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
