@@ -195,7 +195,7 @@ template <int L, int R, bool REAL, bool INV>
 __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict__ in, float2* __restrict__ out, int64_t batch,
                                                        const float2* __restrict__ tw, float scale)
 {
-    using W = WarpFft<L, R>;
+    using W = WarpFft<L, R, false>;     // bound by the copy, and by registers: no packed sums
     constexpr int M = W::M, GROUPS = FW_NT / L;
     extern __shared__ __align__(16) unsigned char smem[];
     float2* tab = reinterpret_cast<float2*>(smem);
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict_
 template <int L, int R, bool REAL, bool INV>
 int launch_warp(const void* in, float2* out, int64_t batch, float scale, cudaStream_t st)
 {
-    using W = WarpFft<L, R>;
+    using W = WarpFft<L, R, false>;     // bound by the copy, and by registers: no packed sums
     const float2* tw = cs_twiddles(2 * W::M);
     if (!tw) return CS_ERR_ARG;
     const size_t smem = (size_t)(W::TWIDDLES + FW_NT / L * W::TILE) * sizeof(float2);

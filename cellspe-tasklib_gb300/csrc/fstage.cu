@@ -791,6 +791,7 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
     constexpr int M = 1024 * M1, N = 2 * M, NT = 32 * M1;
     constexpr int RAWC = N / 64 + 2;             // 16-byte chunks of one segment (+ alignment slack)
     constexpr int SEGS = wbig_segs<M1, PHASE>(), BUFS = SEGS > 1 ? 2 : 1;
+    constexpr bool PK = M1 < 16;                 // 512 threads leave no registers for aligned pairs
     extern __shared__ __align__(16) unsigned char smem[];
     float2* tiles = reinterpret_cast<float2*>(smem);
     uint32_t* rw_all = reinterpret_cast<uint32_t*>(tiles + M1 * B_TILE);
@@ -856,7 +857,7 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
             const uint32_t bits = __funnelshift_r(rw[wb + 4 * M1 * j], rw[wb + 4 * M1 * j + 1], sh);
             v[j] = lut16[bits & 15u];
         }
-        Dft<32>::run(v);
+        Dft<32, PK>::run(v);
         float2 q = make_float2(1.f, 0.f);
 #pragma unroll
         for (int b = 0; b < 4; b++) {
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
 #pragma unroll
         for (int e = 0; e < 32; e++) v[e] = tb[lane * W_TP + e];
         __syncwarp();
-        Dft<32>::run(v);                                         // v[k2] = Y_n1[lane + 32 k2]
+        Dft<32, PK>::run(v);                                         // v[k2] = Y_n1[lane + 32 k2]
 #pragma unroll
         for (int e = 0; e < 32; e++) tb[lane + 32 * e] = v[e];
     }
@@ -914,13 +915,13 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
                 y5[n1] = cmul(tiles[n1 * B_TILE + 512], p);
                 p = cmul(p, u);
             }
-            Dft<M1>::run(y0);
-            Dft<M1>::run(y5);
+            Dft<M1, PK>::run(y0);
+            Dft<M1, PK>::run(y5);
             float2 w = make_float2(1.f, 0.f);                    // W_N^(1024 k1)
 #pragma unroll
             for (int k1 = 0; k1 <= M1 / 2; k1++) {
                 float2 Xk, Xm;
-                r2c_pair(y0[k1], y0[(M1 - k1) % M1], w, Xk, Xm);
+                r2c_pair<PK>(y0[k1], y0[(M1 - k1) % M1], w, Xk, Xm);
                 const int c = 1024 * k1;
                 if constexpr (PHASE) Xk = cmul(Xk, phasor(c)), Xm = cmul(Xm, phasor(M - c));
                 emit(c, Xk);
@@ -931,7 +932,7 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
 #pragma unroll
             for (int k1 = 0; k1 < M1 / 2; k1++) {
                 float2 Xk, Xm;
-                r2c_pair(y5[k1], y5[M1 - 1 - k1], w, Xk, Xm);
+                r2c_pair<PK>(y5[k1], y5[M1 - 1 - k1], w, Xk, Xm);
                 const int c = 512 + 1024 * k1;
                 if constexpr (PHASE) Xk = cmul(Xk, phasor(c)), Xm = cmul(Xm, phasor(M - c));
                 emit(c, Xk);
@@ -952,8 +953,8 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
                 p = cmul(p, u);
             }
         }
-        Dft<M1>::run(ya);                                         // ya[k1] = Z[kA + 1024 k1]
-        Dft<M1>::run(yb);                                         // yb[(k1 + 1) % M1] = Z[kB + 1024 k1]
+        Dft<M1, PK>::run(ya);                                         // ya[k1] = Z[kA + 1024 k1]
+        Dft<M1, PK>::run(yb);                                         // yb[(k1 + 1) % M1] = Z[kB + 1024 k1]
         float2 w = __ldg(tw + kA);                                // W_N^(kA + 1024 k1)
         float2 BA = make_float2(1.f, 0.f), BB = BA;
         if constexpr (PHASE) {
@@ -963,7 +964,7 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
 #pragma unroll
         for (int k1 = 0; k1 < M1; k1++) {
             float2 Xk, Xm;
-            r2c_pair(ya[k1], yb[(M1 - k1) % M1], w, Xk, Xm);
+            r2c_pair<PK>(ya[k1], yb[(M1 - k1) % M1], w, Xk, Xm);
             const int c = kA + 1024 * k1;
             if constexpr (PHASE) {
                 Xk = cmul(Xk, BA);

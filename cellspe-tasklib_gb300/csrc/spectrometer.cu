@@ -260,7 +260,7 @@ CS_DEV bool spec_blanked(const uint32_t* __restrict__ vmask, int64_t start, int 
 // added to registers of the lanes that own the bins, so a group's only shared
 // memory traffic is the plane words, the level pairs, the twiddles and one transpose, and
 // no group waits on another until the chunk ends.  Bound by instruction issue
-// (16 warps per SM; registers).  16 rows x 16383 FFTs of 1024 points: 247 us;
+// (16 warps per SM; registers).  16 rows x 16383 FFTs of 1024 points: 235 us;
 // the radix-16 groups with shared-memory accumulators and CTA barriers took 608.
 constexpr int SP_NT = 256;
 template <int L, int R, bool MASK>
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(SP_NT, 2) k_spec_power_s(const __grid_constant
 // W_M1^n1 conj(W_M^(n1 k2)), which holds both ends of every real-FFT pair, and
 // adds the powers to its own registers.  The window table is read in the
 // warps' order (winp: [M1][1024] pairs).  Bound by instruction issue; 12 rows x
-// 1999 FFTs of 8192 points: 323 us (with some blanked windows), the radix-16 groups 430.
+// 1999 FFTs of 8192 points: 285 us (with some blanked windows), the radix-16 groups 430.
 template <int M1, bool MASK>
 __global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_constant__ CsSpecArgs a,
                                                                    const float2* __restrict__ tw,
@@ -654,10 +654,10 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
                     const float2 wb = (a.window == 2) ? make_float2(1.f - wa.x, 1.f - wa.y) : __ldg(win2 + n2);
                     const float2 z2 = make_float2(x2.x * wb.x, x2.y * wb.y);
                     // y_1[n] = (z[n] - z[n + MC]) W_M^n, W_M^(1024 n1 + m) = W_32^n1 W_M^m
-                    v[n1] = p ? cmul(csub(z1, z2), rot32(tm, n1)) : cadd(z1, z2);
+                    v[n1] = p ? cmul(csub<false>(z1, z2), rot32(tm, n1)) : cadd<false>(z1, z2);
                 }
             }
-            Dft<16>::run(v);
+            Dft<16, false>::run(v);
             // W_MC^(m k1): powers of u = W_MC^m by a balanced recurrence
             const float2 u = c ? umc[1] : umc[0];
             float2 wk[16];
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
             float2 x[32];
 #pragma unroll
             for (int e = 0; e < 32; e++) x[e] = rowp[lane + 34 * e];          // m = lane + 32 e
-            Dft<32>::run(x);
+            Dft<32, false>::run(x);
             float2 q = make_float2(1.f, 0.f);
             const float2 w8 = wps[8][lane];
 #pragma unroll
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
             __syncwarp();
 #pragma unroll
             for (int e = 0; e < 32; e++) x[e] = rowp[lane * 33 + e];
-            Dft<32>::run(x);                                                    // x[e] = Y[warp][lane + 32 e]
+            Dft<32, false>::run(x);                                                    // x[e] = Y[warp][lane + 32 e]
             __syncwarp();
 #pragma unroll
             for (int e = 0; e < 32; e++) rowp[lane + 34 * e] = x[e];          // k2 = lane + 32 e
@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
             const int mp = k1 + 16 * k2;                   // index in the CTA's transform
             const int k = P * mp + p;                      // bin of the full real FFT
             float2 Xk, Xm;
-            r2c_pair(za, zb, cmul(ck[k1], b), Xk, Xm);          // W_N^k
+            r2c_pair<false>(za, zb, cmul(ck[k1], b), Xk, Xm);          // W_N^k
             if (special && k == 0) {
                 slots[s * SW_NT + tid] += Xk.x * Xk.x;
                 slots[(s + 1) * SW_NT + tid] += Xm.x * Xm.x;

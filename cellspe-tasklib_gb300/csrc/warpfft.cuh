@@ -9,7 +9,8 @@
 #pragma once
 #include "common.cuh"
 
-template <int L, int R> struct WarpFft {
+// PK: packed sums (common.cuh).
+template <int L, int R, bool PK = true> struct WarpFft {
     static_assert(R % L == 0 && L >= 8 && L <= 32 && R <= 32, "lanes and points per lane");
     static constexpr int M = L * R, CPL = R / L;
     static constexpr int TILE = R * (L + 1);         // float2 per group; the odd row keeps both passes conflict-free
@@ -23,7 +24,7 @@ template <int L, int R> struct WarpFft {
 
     static CS_DEV void run(float2 (&v)[R], float2* tile, int lane, const float2* tab)
     {
-        Dft<R>::run(v);
+        Dft<R, PK>::run(v);
 #pragma unroll
         for (int e = 1; e < R; e++) v[e] = cmul(v[e], tab[e * L + lane]);
 #pragma unroll
@@ -35,7 +36,7 @@ template <int L, int R> struct WarpFft {
             for (int n = 0; n < L; n++) v[c * L + n] = tile[(lane + L * c) * (L + 1) + n];
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < CPL; c++) Dft<L>::run(v + c * L);
+        for (int c = 0; c < CPL; c++) Dft<L, PK>::run(v + c * L);
     }
 
     // Real-FFT split of the result (z[n] = x[2n] + i x[2n+1], N = 2 M): calls
