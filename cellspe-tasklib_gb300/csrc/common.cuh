@@ -299,3 +299,11 @@ template <bool PACKED = true> CS_DEV void r2c_pair(float2 a, float2 b, float2 w,
     float2 d = csub<PACKED>(E, wO);
     Xmk = make_float2(d.x, -d.y);
 }
+// The same with wh = w / 2, which leaves four multiplications out.
+CS_DEV void r2c_pair_h(float2 a, float2 b, float2 wh, float2& Xk, float2& Xmk)
+{
+    const float2 s = make_float2(a.x + b.x, a.y - b.y);
+    const float2 t = cmul(wh, make_float2(a.x - b.x, a.y + b.y));     // w O = -i t
+    Xk = make_float2(fmaf(0.5f, s.x, t.y), fmaf(0.5f, s.y, -t.x));
+    Xmk = make_float2(fmaf(0.5f, s.x, -t.y), -fmaf(0.5f, s.y, t.x));
+}

@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 namespace {
 
@@ -757,25 +758,38 @@ int launch_w2048(const CsFStageArgs& a, cudaStream_t st)
 // shared memory (the warp's own transpose tile) and, after one CTA barrier,
 //     Z[k2 + 1024 k1] = sum_n1 W_M1^(n1 k1) (W_M^(n1 k2) Y_n1[k2]).
 // Each thread takes the mirrored columns k2 and 1024 - k2 (k2 = 1 ... 511;
-// thread 0 also columns 0 and 512): twiddled by powers of u = W_M^k2 (the
+// the last warp's lanes columns 0 and 512): twiddled by powers of u = W_M^k2 (the
 // second column by conj(u)^n1, whose DFT comes out rotated by one since
 // W_M^(n1 (1024 - k2)) = W_M1^n1 conj(u)^n1), two M1-point DFTs, and the
 // real-FFT split pairs Z[k2 + 1024 k1] with Z[M - k2 - 1024 k1] =
 // Z[(1024 - k2) + 1024 (M1 - 1 - k1)], so the split needs no data exchange.
 // Channels then get the phasor exp(i (phase0 + c dphase)) and the optional
 // scale and are written segment-major ([S][K][C], coalesced along c) for
-// cs_spectra_transpose.  LSB-first input only.  A CTA that fills an SM on its
-// own (16 warps, or 8 warps with the phasor's registers) takes SEGS = 4
-// consecutive segments and fetches the next one's raw words (cp.async) while
-// it transforms the current one; the other forms take one segment and leave
-// the overlap to the other CTAs on the SM.
+// cs_spectra_transpose.  LSB-first input only.  The 16-warp form, which fills
+// an SM on its own, takes SEGS = 4 consecutive segments and fetches the next
+// one's raw words (cp.async) while it transforms the current one; the others
+// take one segment and leave the overlap to the other CTAs on the SM.  Bound by
+// instruction issue.  32 inputs of 2^25 samples: 8192 points with the phasor
+// 1648 -> 1260 us in FP16 (the self-paired columns in one warp's lanes
+// instead of one thread's, two sincosf a segment, the scale tested once, one word a
+// pair at even offsets); 32768 points, 200 inputs of 2^24 samples, 5.2 -> 4.8 ms (one
+// CTA's phases do not overlap: 65 % of the issue slots).
 // ---------------------------------------------------------------------------
 constexpr int B_TILE = 32 * W_TP;               // float2 per warp: transpose tile, then Y_n1
 
 template <int M1, bool PHASE>
 constexpr int wbig_segs()
 {
-    return (M1 == 16 || (M1 == 8 && PHASE)) ? 4 : 1;
+    return M1 == 16 ? 4 : 1;
+}
+
+// CTAs on an SM: 24 warps of 80 registers where that gains (16384 points 642 -> 583
+// us, with the phasor 711 -> 657; 8192 with it 638 -> 632; the plain forms of up to
+// 8192 points keep 20 warps of 96, which take 540 us and not 549)
+template <int M1, bool PHASE>
+constexpr int wbig_blocks()
+{
+    return M1 == 16 ? 1 : (M1 == 8 || PHASE) ? 24 / M1 : 20 / M1;
 }
 
 template <int M1, bool PHASE>
@@ -786,7 +800,7 @@ size_t wbig_smem()
 }
 
 template <int M1, int FMT, bool PHASE>
-__global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constant__ CsFStageArgs a, const float2* __restrict__ tw)
+__global__ void __launch_bounds__(32 * M1, wbig_blocks<M1, PHASE>()) k_fx_fstage_wbig(const __grid_constant__ CsFStageArgs a, const float2* __restrict__ tw)
 {
     constexpr int M = 1024 * M1, N = 2 * M, NT = 32 * M1;
     constexpr int RAWC = N / 64 + 2;             // 16-byte chunks of one segment (+ alignment slack)
@@ -830,7 +844,8 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
     }
     const float2 w8 = cmul(wp[4], wp[4]);
     float2* tb = tiles + warp * B_TILE;
-    const float2 c2 = __ldg(tw + 1024);                          // W_N^1024 = W_(2 M1)
+    __shared__ float2 w2m[2 * M1];                               // W_(2 M1)^i
+    if (threadIdx.x < 2 * M1) w2m[threadIdx.x] = __ldg(tw + 1024 * threadIdx.x);
 
 #pragma unroll 1
     for (int i = 0; i < SEGS; i++) {
@@ -852,10 +867,22 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
         const int f0 = off + 2 * (warp + M1 * lane);            // sample offset of this lane's first pair
         const int wb = f0 >> 4, sh = 2 * (f0 & 15);
         float2 v[32];
+        // pair j is 64 M1 samples = 4 M1 words further on; at an even offset (all jobs
+        // without delays) no pair crosses a word, and the word turned by the pair's
+        // place holds the table's byte offset
+        if (off & 1) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) {                           // pair j is 64 M1 samples = 4 M1 words further on
-            const uint32_t bits = __funnelshift_r(rw[wb + 4 * M1 * j], rw[wb + 4 * M1 * j + 1], sh);
-            v[j] = lut16[bits & 15u];
+            for (int j = 0; j < 32; j++) {
+                const uint32_t bits = __funnelshift_r(rw[wb + 4 * M1 * j], rw[wb + 4 * M1 * j + 1], sh);
+                v[j] = lut16[bits & 15u];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const uint32_t x = rw[wb + 4 * M1 * j];
+                v[j] = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(lut16) +
+                                                        (__funnelshift_r(x, x, (sh - 3) & 31) & 0x78u));
+            }
         }
         Dft<32, PK>::run(v);
         float2 q = make_float2(1.f, 0.f);
@@ -881,66 +908,58 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
     __syncthreads();
 
     // ---- mirrored column pairs: radix-M1 step, real-FFT split, phasor, write ----
-    float2 D = make_float2(1.f, 0.f);
+    // phasors exp(i (ph0 + c dph)): P0 exp(i c dph) and PM exp(-i (M - c) dph) from
+    // four constants of the segment (one lane each), a thread's first column and
+    // products of these, so a thread takes two sincosf a segment and not two a task
+    float2 P0, PM, D, DT, E;
     float ph0 = 0.f, dph = 0.f;
     if constexpr (PHASE) {
         ph0 = __ldg(a.phase0 + sk);
         dph = __ldg(a.dphase + sk);
         float sn, cs;
-        sincosf(1024.f * dph, &sn, &cs);
-        D = make_float2(cs, sn);
+        sincosf(lane == 0 ? ph0 : lane == 1 ? ph0 + (float)M * dph : lane == 2 ? 1024.f * dph : (float)NT * dph, &sn, &cs);
+        auto of = [&](int l) { return make_float2(__shfl_sync(0xffffffffu, cs, l), __shfl_sync(0xffffffffu, sn, l)); };
+        P0 = of(0), PM = of(1), D = of(2), DT = of(3);
+        sincosf((float)threadIdx.x * dph, &sn, &cs);
+        E = make_float2(cs, sn);                                  // exp(i kA dph)
     }
-    const float* scl = a.scale ? a.scale + (int64_t)s * M : nullptr;
     const int64_t obase = sk * M;
+    auto columns = [&](auto scaled) {
+    const float* scl = decltype(scaled)::value ? a.scale + (int64_t)s * M : nullptr;
     auto emit = [&](int c, float2 X) {
-        if (scl) X = cscale(X, __ldg(scl + c));
+        if constexpr (decltype(scaled)::value) X = cscale(X, __ldg(scl + c));
         if constexpr (FMT == CS_SPECTRA_F32) reinterpret_cast<float2*>(a.out)[obase + c] = X;
         else reinterpret_cast<__half2*>(a.out)[obase + c] = __floats2half2_rn(X.x, X.y);
     };
-    auto phasor = [&](int c) -> float2 {
-        float sn, cs;
-        sincosf(ph0 + (float)c * dph, &sn, &cs);
-        return make_float2(cs, sn);
-    };
+    if (warp == M1 - 1) {
+        // columns 0 and 512, each paired with itself: channel c = 512 l is lane l's,
+        // Z[c] = sum_n1 Y_n1[512 (l & 1)] W_2M1^(l n1), its pair lane 2 M1 - l's.  (As
+        // another pair of one thread's columns they cost as many instructions again
+        // as a whole warp's columns, while the other warps waited at the barrier.)
+        const int l = lane & (2 * M1 - 1);
+        float2 z = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int n1 = 0; n1 < M1; n1++) {
+            const float2 y = tiles[n1 * B_TILE + 512 * (l & 1)], w = w2m[(l * n1) & (2 * M1 - 1)];
+            z.x = fmaf(y.x, w.x, fmaf(-y.y, w.y, z.x));
+            z.y = fmaf(y.x, w.y, fmaf(y.y, w.x, z.y));
+        }
+        const int lp = (2 * M1 - l) & (2 * M1 - 1);
+        const float2 zp = make_float2(__shfl_sync(0xffffffffu, z.x, lp), __shfl_sync(0xffffffffu, z.y, lp));
+        if (lane < 2 * M1) {
+            float2 Xk, Xm;
+            r2c_pair_h(z, zp, cscale(__ldg(tw + 512 * l), 0.5f), Xk, Xm);
+            if constexpr (PHASE) {
+                float sn, cs;
+                sincosf(ph0 + (float)(512 * l) * dph, &sn, &cs);
+                Xk = cmul(Xk, make_float2(cs, sn));
+            }
+            emit(512 * l, Xk);
+        }
+    }
 #pragma unroll 1
     for (int task = threadIdx.x; task < 512; task += NT) {
-        if (task == 0) {
-            // column 0 (u = 1) and column 512 (u = W_M^512), each paired with itself
-            float2 y0[M1], y5[M1];
-            const float2 u = __ldg(tw + 1024);
-            float2 p = make_float2(1.f, 0.f);
-#pragma unroll
-            for (int n1 = 0; n1 < M1; n1++) {
-                y0[n1] = tiles[n1 * B_TILE];
-                y5[n1] = cmul(tiles[n1 * B_TILE + 512], p);
-                p = cmul(p, u);
-            }
-            Dft<M1, PK>::run(y0);
-            Dft<M1, PK>::run(y5);
-            float2 w = make_float2(1.f, 0.f);                    // W_N^(1024 k1)
-#pragma unroll
-            for (int k1 = 0; k1 <= M1 / 2; k1++) {
-                float2 Xk, Xm;
-                r2c_pair<PK>(y0[k1], y0[(M1 - k1) % M1], w, Xk, Xm);
-                const int c = 1024 * k1;
-                if constexpr (PHASE) Xk = cmul(Xk, phasor(c)), Xm = cmul(Xm, phasor(M - c));
-                emit(c, Xk);
-                if (k1 > 0 && k1 < M1 / 2) emit(M - c, Xm);
-                w = cmul(w, c2);
-            }
-            w = __ldg(tw + 512);                                  // W_N^(512 + 1024 k1)
-#pragma unroll
-            for (int k1 = 0; k1 < M1 / 2; k1++) {
-                float2 Xk, Xm;
-                r2c_pair<PK>(y5[k1], y5[M1 - 1 - k1], w, Xk, Xm);
-                const int c = 512 + 1024 * k1;
-                if constexpr (PHASE) Xk = cmul(Xk, phasor(c)), Xm = cmul(Xm, phasor(M - c));
-                emit(c, Xk);
-                emit(M - c, Xm);
-                w = cmul(w, c2);
-            }
-            continue;
-        }
+        if (task) {
         const int kA = task, kB = 1024 - task;
         float2 ya[M1], yb[M1];
         {
@@ -955,16 +974,16 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
         }
         Dft<M1, PK>::run(ya);                                         // ya[k1] = Z[kA + 1024 k1]
         Dft<M1, PK>::run(yb);                                         // yb[(k1 + 1) % M1] = Z[kB + 1024 k1]
-        float2 w = __ldg(tw + kA);                                // W_N^(kA + 1024 k1)
-        float2 BA = make_float2(1.f, 0.f), BB = BA;
+        const float2 w = cscale(__ldg(tw + kA), 0.5f);            // W_N^(kA + 1024 k1) / 2 = w W_2M1^k1
+        float2 BA, BB;
         if constexpr (PHASE) {
-            BA = phasor(kA);                                      // channel kA + 1024 k1
-            BB = phasor(M - kA);                                  // channel M - kA - 1024 k1
+            BA = cmul(P0, E);                                     // channel kA + 1024 k1
+            BB = cmul_conj(PM, E);                                // channel M - kA - 1024 k1
         }
 #pragma unroll
         for (int k1 = 0; k1 < M1; k1++) {
             float2 Xk, Xm;
-            r2c_pair<PK>(ya[k1], yb[(M1 - k1) % M1], w, Xk, Xm);
+            r2c_pair_h(ya[k1], yb[(M1 - k1) % M1], rot32(w, (16 / M1) * k1), Xk, Xm);
             const int c = kA + 1024 * k1;
             if constexpr (PHASE) {
                 Xk = cmul(Xk, BA);
@@ -974,9 +993,13 @@ __global__ void __launch_bounds__(32 * M1) k_fx_fstage_wbig(const __grid_constan
             }
             emit(c, Xk);
             emit(M - c, Xm);
-            w = cmul(w, c2);
         }
+        }
+        if constexpr (PHASE) E = cmul(E, DT);
     }
+    };
+    if (a.scale) columns(std::true_type{});
+    else columns(std::false_type{});
     }
 }
 
