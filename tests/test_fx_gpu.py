@@ -281,6 +281,32 @@ def test_fx_fp32_split_sizes(cg, orc, S, N, K):
     assert _rel(vis, _vis_f64(orc, raw, S, N, K, 5)) < 2e-6
 
 
+@pytest.mark.parametrize("start", [4, 5])
+@pytest.mark.parametrize("N", [4096, 8192, 16384, 32768])
+def test_fx_long_transforms(cg, orc, N, start):
+    """Long transforms at even and odd first samples against FP64, every channel; with a channel scale against without."""
+    import synth
+
+    S, K = 9, 5                                      # a remainder of the 32768-point form's four segments a block
+    raw = synth.stations_offset_binary(S, (N * K + start + 63) // 64 * 64, rho=0.3, seed=N + start)
+    C, P = N // 2, S * (S + 1) // 2
+    vis = np.zeros((C, P), np.complex64)
+    cg.fx_correlate(cg.fx_params(S, N, K, raw.shape[1], start_sample=start), raw, vis)
+    ref = _vis_f64(orc, raw, S, N, K, start)
+    # FP32 rounding of an N-point transform and of a few sums: a few 2^-24, 2e-6 at most
+    assert _rel(vis, ref) < 2e-6
+    for c in (0, 1, 512, 1024, C // 2, C // 2 + 512, C - 512, C - 1):     # the mirrored columns' special cases
+        assert _rel(vis[c], ref[c]) < 1e-5, c
+    # FP16 spectra under a scale of powers of two are the same but for halves too small to be normal
+    raw, K8 = np.concatenate([raw, raw], axis=1), 8
+    scale = np.exp2(np.random.default_rng(N).integers(-1, 2, (S, C))).astype(np.float32)
+    out = []
+    for sc in (None, scale):
+        out.append(np.zeros((C, P), np.complex64))
+        cg.fx_correlate(cg.fx_params(S, N, K8, raw.shape[1], start_sample=start, x_mode=cg.X_TC_FP16, channel_scale=sc), raw, out[-1])
+    assert _rel(out[1], out[0]) < 1e-5
+
+
 @pytest.mark.parametrize("N", [512, 1024, 2048, 4096])
 def test_fx_fp32_split_delay_levels(cg, orc, N):
     """The same with a delay model, large custom levels and a full-scale tone (the largest spectrum value of these levels)."""
