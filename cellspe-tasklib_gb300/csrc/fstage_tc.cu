@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc(const __grid_consta
 
     if (warp == 8) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id1 = tc::idesc_f16(128, 256, false, false, true);    // B1 MN-major
             const uint32_t id2 = tc::idesc_f16(128, 32, false, false, false);
             bool ok = true;

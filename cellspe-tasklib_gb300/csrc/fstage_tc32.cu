@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_fstage_tc32(const __grid_cons
 
     if (warp == MMA_WARP) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id1 = tc::idesc_f16(128, 128, false, false, true);    // B1 MN-major
             const uint32_t id2 = tc::idesc_f16(128, 64, false, false, false);
             bool ok = true;
@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_fx_fstage_tc32ws(const __grid
         if (SCALE) X = cscale(X, __ldg(scl + (c_)));
     if (warp == WS_MMA) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id1 = tc::idesc_f16(128, 128, false, false, true);
             const uint32_t id2 = tc::idesc_f16(128, 64, false, false, false);
             auto w = [&](int i, uint32_t ph) {

@@ -110,6 +110,20 @@ __device__ __forceinline__ uint32_t idesc_f16(uint32_t m, uint32_t n, bool neg_a
            ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// One lane of a converged warp.  A branch on it, not on the lane's number, tells the
+// compiler that one thread runs it: a tcgen05.mma then takes its descriptors from
+// uniform registers and not through a loop over the active lanes.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r));
+    return r != 0;
+}
+
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
 {
     asm volatile(

@@ -155,13 +155,13 @@ __global__ void __launch_bounds__(LOADERS + 96, 1)
     const uint32_t tmem = *slot;
 
     if (warp == LOADERS / 32 + 2) {
-        if (lane == 0)
+        if (tc::elect_one())
             feed<F::DEPTH, F::SEGS>(&tmap, tc::smem_u32(raw), F::R::BYTES, rfull, rempty, nk, a.err);
     } else if (warp >= LOADERS / 32) {
         // two issuers, four channels each: one thread's instructions took as long
         // as the MMAs (611 us with one, 512 unrolled, 487 with two)
         const int ca = (warp - LOADERS / 32) * (F::CB / 2);
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, RI, false, false, false);
             const uint64_t d0 = tc::smem_desc(tc::smem_u32(ring), 16, 8 * F::ROWB, F::ROWB == 128 ? tc::SW128 : tc::SW64);
             for (int kc = 0; kc < nk; kc++) {
@@ -326,10 +326,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     const uint32_t tmem = *slot;
 
     if (warp == 17) {
-        if (lane == 0)
+        if (tc::elect_one())
             feed<F::DEPTH, F::SEGS>(&tmap, tc::smem_u32(raw), F::R::BYTES, rfull, rempty, nk, a.err);
     } else if (warp == 16) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, F::N2, false, false, false);
             const uint64_t d0 = tc::smem_desc(tc::smem_u32(ring), 16, 8 * F::ROWB, tc::SW128);
             for (int kc = 0; kc < nk; kc++) {

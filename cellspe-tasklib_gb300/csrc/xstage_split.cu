@@ -239,12 +239,12 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
     const Pipe p = pipe_open<E, 1>(smem + a.stages * STAGE + gram_slack<R>(), a.stages, COLS, a.err, &tmap);
     const uint32_t sbase = tc::smem_u32(smem);
     if (warp == E) {
-        if (lane == 0)
+        if (tc::elect_one())
             produce(p, nk, STAGE, [&](int kc, int s, uint32_t bar) {
                 tc::tma_load_5d(sbase + s * STAGE, &tmap, 0, 0, 0, kc, c, bar);
             });
     } else if (warp == E + 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, NC, false, false, false);
             const uint64_t d0 = sw128_desc(sbase);
             issue(p, nk, 0, 1, [&](int s, int b) {
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
     const Pipe p = pipe_open<T_E, 2>(smem + a.stages * stage_bytes + slack, a.stages, T_COLS, a.err, &tmap);
     const uint32_t sbase = tc::smem_u32(smem);
     if (warp == T_E) {
-        if (lane == 0)
+        if (tc::elect_one())
             produce(p, nk, diag ? op_bytes : 2 * op_bytes, [&](int kc, int s, uint32_t bar) {
                 const uint32_t st = sbase + s * stage_bytes;
                 tc::tma_load_5d(st, &tmap, 0, i0, 0, kc, c, bar);
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
     } else if (warp > T_E) {
         // two issuers, each with its own TMEM buffer (even and odd chunks): one's
         // waits and commits, about 500 cycles of a chunk, pass behind the other's MMAs
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t pos = tc::idesc_f16(BM, n_eff, false, false, false);
             const uint32_t neg = tc::idesc_f16(BM, n_eff, true, false, false);
             const uint64_t d0 = sw128_desc(sbase);
