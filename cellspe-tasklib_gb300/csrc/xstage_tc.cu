@@ -4,23 +4,33 @@
 // of the S x K spectra matrix X = Xr + i Xi (the conjugate MAC of
 // genericAddProduct_32fc_conj, architecture.h:427-433, for every product):
 //     Re V = Xr Xr^T + Xi Xi^T,      Im V = Xi Xr^T - Xr Xi^T.
-// A CTA owns one 128 (i) x 128 (j) tile of one channel that touches the lower
-// triangle.  Its two FP32 accumulators live in tensor memory (TMEM): columns
-// 0..127 hold Re V, 128..255 hold Im V, lane = row i, so two CTAs share an
-// SM's TMEM and one's epilogue overlaps the other's MMAs.  Each k-step issues
-// four kind::f16 MMAs (M=128, N=128, K=16); the minus sign of the last product
-// is the instruction descriptor's negate-A bit, so no negated copy of the data
-// exists.  Operands are K-major (time innermost), loaded by TMA into a 3-stage
-// shared-memory ring (32 KB stages) guarded by mbarriers, one copy per operand
-// bringing its Re and Im parts.  A diagonal tile (i0 = j0) loads its rows once and uses them as
-// both operands, and needs three MMAs per k-step: its Im columns accumulate
+// Work is one 128 (i) x 128 (j) tile of one channel that touches the lower
+// triangle.  Its two FP32 accumulators live in tensor memory (TMEM): 128 columns
+// Re V, 128 columns Im V, lane = row i.  Each k-step issues four kind::f16 MMAs
+// (M=128, N=128, K=16); the minus sign of the last product is the instruction
+// descriptor's negate-A bit, so no negated copy of the data exists.  Operands are
+// K-major (time innermost), loaded by TMA into a shared-memory ring (32 KB
+// stages) guarded by mbarriers, one copy per operand bringing its Re and Im
+// parts.  A diagonal tile (i0 = j0) loads its rows once and uses them as both
+// operands, and needs three MMAs per k-step: its Im columns accumulate
 // M = Xi Xr^T and the epilogue forms Im V = M - M^T through shared memory.
 //
-// Warp roles (6 warps): warp 0 = TMA producer, warp 1 = TMEM owner and MMA
-// issuer, warps 2..5 = epilogue (TMEM -> registers -> global; warp w reads
-// TMEM lanes 32*(w%4)..+31).  Every mbarrier wait is bounded: on timeout the
-// kernel records an error code, drains its own copies (bounded), frees TMEM
-// and returns, and the host reports the failure.
+// k_xmac_tc, one persistent CTA an SM: warp 0 = TMA producer, running ahead into
+// the next tile, warps 1 and 2 = MMA issuers of Re V and Im V (a single one's
+// instructions took longer than the MMAs), warp 3 = TMEM owner, warps 4..11 =
+// epilogue (TMEM -> registers -> global, a quarter of the lanes and every other
+// column block each) of one half of TMEM while the MMAs fill the other.  Bound by
+// the MMAs' reads of shared memory and, in short integrations, by the stores of
+// the visibilities.  200 inputs: 4096 channels of 128, 512 and 960 segments 243,
+// 372 and 522 us with a tile a CTA, 172, 270 and 463 so; 16384 channels of 512
+// 2.83 -> 2.1 ms.  Up to 128 inputs (one diagonal tile): 100 inputs, 2048 channels
+// of 512 150 -> 92 us.
+//
+// k_xmac_tc_pair: a tile a CTA, two CTAs an SM, for long integrations.
+//
+// Every mbarrier wait is bounded: on timeout the kernel records an error code,
+// drains its own copies (bounded), frees TMEM and returns, and the host reports
+// the failure.
 //
 // Layout in:  __half spectra[C][2][S][K]  (plane 0 = Re, plane 1 = Im), or
 //             k-blocked [C][S][K/32][2][32], or channel-grouped k-blocked
@@ -35,22 +45,20 @@
 
 #include <algorithm>
 #include <mutex>
-#include <vector>
 
 namespace {
 
 constexpr int BM = 128, BN = 128, BK = 32;          // tile and k-chunk (64 B of FP16 = one swizzle row)
-constexpr int STAGES = 3;
 constexpr int A_BYTES = BM * BK * 2;                // 8 KB
 constexpr int B_BYTES = BN * BK * 2;                // 8 KB
+constexpr int STAGES = 4;                           // twice as many of half the size when S <= BM
 constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;   // Ar, Ai, Br, Bi = 32 KB
-constexpr int TC_THREADS = 192;
-// epilogue shared memory: four warps' 32 x 17 float2 staging blocks, then (on
-// a diagonal tile) M as [BM][MP] floats; both inside the operand ring
-constexpr int EPI_STG_BYTES = 4 * 32 * 17 * 8;
-constexpr int MP = BM + 1;
-static_assert(EPI_STG_BYTES + BM * MP * 4 <= STAGES * STAGE_BYTES, "epilogue M staging inside the ring");
-constexpr uint32_t TMEM_COLS = 256;
+constexpr int EPI_WARPS = 8;
+constexpr int TC_THREADS = 128 + 32 * EPI_WARPS;
+constexpr uint32_t ACC_COLS = 256;                  // TMEM columns of one tile: Re V, then Im V or M
+constexpr int MP = BM + 1;                          // pitch of M in shared memory
+constexpr size_t TC_SMEM = 1024 + STAGES * STAGE_BYTES + EPI_WARPS * 32 * 16 * 8 + BM * MP * 4 + (4 * STAGES + 6) * 8;
+static_assert(TC_SMEM <= 227 * 1024, "shared memory of one SM");
 constexpr long long WAIT_CYCLES = 4000000000LL;     // ~2 s at 2 GHz
 
 // error codes
@@ -64,9 +72,8 @@ CS_DEV uint64_t sw64_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 512,
 // the same with 128-byte rows (32 Re and 32 Im halves, or 64 segments of one part)
 CS_DEV uint64_t sw128_desc(uint32_t saddr) { return tc::smem_desc(saddr, 16, 1024, tc::SW128); }
 
-// the four epilogue warps (2..5): named barrier 1 over their 128 threads, and
-// an AND vote on it that every one of them reaches
-CS_DEV void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// named barrier 1 over the epilogue warps, with an AND vote that every one of
+// them reaches
 CS_DEV bool group_vote(bool ok, int nthreads)
 {
     uint32_t r;
@@ -80,23 +87,48 @@ CS_DEV bool group_vote(bool ok, int nthreads)
         : "memory");
     return r != 0;
 }
-CS_DEV bool epi_vote(bool ok) { return group_vote(ok, 128); }
 
 struct TcArgs {
     int S, C, K;
     int64_t P;
-    const int2* tiles;          // (i0, j0) per tile
+    int64_t ntiles;             // tiles of a channel's lower triangle
+    int turn;                   // of the CTAs' order, per round
     float2* vis;
     const float* inv_scale;     // [S][scale_stride] or null
     int scale_stride;
     int accumulate;
     int box_rows;               // rows per TMA box: BM, or S rounded up to 8 when S < BM
     int small;                  // S <= BM: one tile per channel whose B operand is its A operand
-    uint32_t tmem_cols;         // TMEM columns: Re V in [0, cols/2), Im V in [cols/2, cols)
     int kblock;                 // spectra k-blocked: 1 [C][S][kp/32][2][32],
                                 // 2 channel-grouped [C/16][S][kp/32][16][2][32]
     unsigned* err;              // CsErrorWord::code of the job
 };
+
+// Tile `round` of this CTA: row and column block and channel, or false.  The CTAs
+// take the tiles (a channel's together, so its rows stay in L2) in rounds of one
+// each; their order turns by `turn` a round, which gives every CTA diagonal and
+// full tiles alike.
+struct Tile {
+    int i0, j0, c;
+};
+// columns a tile needs: j < min(j0 + BN, i0 + BM, S), rounded up to 16
+CS_DEV uint32_t tile_cols(int S, const Tile& t) { return (uint32_t)((min(min(t.j0 + BN, t.i0 + BM), S) - t.j0 + 15) & ~15); }
+CS_DEV Tile tile_at(int n)                                         // n = i(i+1)/2 + j, j <= i
+{
+    int i = (int)((sqrtf(8.f * (float)n + 1.f) - 1.f) * 0.5f);
+    while ((int64_t)i * (i + 1) / 2 > n) i--;
+    while ((int64_t)(i + 1) * (i + 2) / 2 <= n) i++;
+    return Tile{i * BM, (n - i * (i + 1) / 2) * BN, 0};
+}
+CS_DEV bool tile_of(const TcArgs& a, int64_t round, Tile& t)
+{
+    const int64_t w = round * gridDim.x + (int)((blockIdx.x + round * a.turn) % gridDim.x);
+    if (w >= (int64_t)a.C * a.ntiles) return false;
+    const int c = (int)(w / a.ntiles);
+    t = tile_at((int)(w - (int64_t)c * a.ntiles));
+    t.c = c;
+    return true;
+}
 
 __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant__ CUtensorMap tmap,
                                                            const __grid_constant__ TcArgs a)
@@ -106,35 +138,246 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
     // the compiler keeps shared-space 32-bit addressing for every access
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     // S <= BM: a stage holds Ar and Ai only (the tile is diagonal, B = A)
-    const uint32_t stage_bytes = a.small ? 2 * A_BYTES : STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * stage_bytes);   // full[S], empty[S], acc
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
+    const uint32_t stage_bytes = a.small ? STAGE_BYTES / 2 : STAGE_BYTES;
+    const int stages = a.small ? 2 * STAGES : STAGES;
+    float2* stg_all = reinterpret_cast<float2*>(smem + STAGES * STAGE_BYTES);        // [EPI_WARPS][32][16]
+    float* msh = reinterpret_cast<float*>(stg_all + EPI_WARPS * 32 * 16);            // [BM][MP]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(msh + BM * MP);   // full[2 STAGES], empty[2 STAGES], accf[2], acce[2], done
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * STAGES + 5);
     const uint32_t sbase = smem_u32(smem);
-    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES, accb = full0 + 16 * STAGES;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 16 * STAGES, accf = empty0 + 16 * STAGES, acce = accf + 16;
+    const uint32_t done = acce + 16;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int2 tile = a.tiles[blockIdx.x];
-    const int c = blockIdx.y;
-    const int i0 = tile.x, j0 = tile.y;
     const int S = a.S;
     const int nk = (a.K + BK - 1) / BK;
-    // columns this tile needs: j < min(j0 + BN, i0 + BM, S), rounded up to 16
-    const int n_need = min(min(j0 + BN, i0 + BM), S) - j0;
-    const uint32_t n_eff = (uint32_t)((n_need + 15) & ~15);
-    // a diagonal tile (i0 == j0) multiplies its rows by themselves: B is A, so
-    // its stages load A only (as every tile does when S <= BM)
-    const bool diag = a.small || i0 == j0;
-    // and, when its stages span the full ring, its imaginary part is M - M^T
-    // with M = Ai Ar^T: three MMAs per k-step instead of four, M staged through
-    // shared memory for the transpose in the epilogue
-    const bool mtr = diag && !a.small;
-    // S < 128: the boxes hold the S (rounded up to 8) rows that exist, so a
-    // channel's planes are read once; the rows of the operand tiles past them
-    // only feed accumulator rows and columns that are never stored
-    const uint32_t stage_tx = (diag ? 2u : 4u) * (uint32_t)a.box_rows * BK * 2;
+    const int64_t rounds = ((int64_t)a.C * a.ntiles + gridDim.x - 1) / gridDim.x;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) {
+        for (int s = 0; s < stages; s++) {
+            tc::mbar_init(full0 + 8 * s, 1);
+            tc::mbar_init(empty0 + 8 * s, 2);
+        }
+        for (int b = 0; b < 2; b++) {
+            tc::mbar_init(accf + 8 * b, 2);
+            tc::mbar_init(acce + 8 * b, EPI_WARPS);
+        }
+        tc::mbar_init(done, 2);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    }
+    if (warp == 3) tc::tmem_alloc(smem_u32(tmem_slot), 2 * ACC_COLS);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        // ---------------- TMA producer ----------------
+        if (tc::elect_one()) {
+            // one copy per operand brings both parts of its rows: planes as Re rows
+            // then Im rows of 64 bytes, k-blocked as rows of 32 Re and 32 Im halves
+            auto load = [&](uint32_t dst, int c, int kc, int row, uint32_t bar) {
+                if (a.kblock) tc::tma_load_5d(dst, &tmap, 0, a.kblock == 2 ? c & 15 : 0, kc, row, a.kblock == 2 ? c >> 4 : c, bar);
+                else tc::tma_load_4d(dst, &tmap, kc * BK, row, 0, c, bar);
+            };
+            int s = 0, filled = 0;
+            uint32_t ph = 0;                               // of the ring's current turn
+            bool ok = true;
+            Tile t;
+            for (int64_t n = 0; n < rounds && ok && tile_of(a, n, t); n++) {
+                const bool diag = t.i0 == t.j0;            // B is A
+                // S < 128: the boxes hold the S (rounded up to 8) rows that exist, so a
+                // channel's planes are read once; the rows of the operand tiles past them
+                // only feed accumulator rows and columns that are never stored
+                const uint32_t tx = (diag ? 2u : 4u) * (uint32_t)a.box_rows * BK * 2;
+                for (int kc = 0; kc < nk; kc++) {
+                    if (!tc::mbar_wait(empty0 + 8 * s, ph ^ 1, a.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) { ok = false; break; }
+                    const uint32_t st = sbase + s * stage_bytes, fb = full0 + 8 * s;
+                    tc::mbar_expect_tx(fb, tx);
+                    load(st, t.c, kc, t.i0, fb);
+                    if (!diag) load(st + 2 * A_BYTES, t.c, kc, t.j0, fb);
+                    filled = min(filled + 1, stages);
+                    if (++s == stages) s = 0, ph ^= 1;
+                }
+            }
+            // drain: every stage this thread filled must have landed before the CTA exits
+            for (; filled > 0; filled--) {
+                if (--s < 0) s = stages - 1, ph ^= 1;
+                tc::mbar_wait(full0 + 8 * s, ph, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
+            }
+        }
+    } else if (warp <= 2) {
+        // ---------------- MMA issuers: warp 1 Re V, warp 2 Im V (or M) ----------------
+        if (tc::elect_one()) {
+            const uint64_t d0 = a.kblock ? sw128_desc(sbase) : sw64_desc(sbase);
+            const uint32_t im16 = a.kblock ? 4 : (uint32_t)a.box_rows * BK * 2 / 16;   // Im after Re, in 16 bytes
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            Tile t;
+            for (int64_t n = 0; n < rounds && ok && tile_of(a, n, t); n++) {
+                const bool diag = t.i0 == t.j0;
+                const uint32_t n_eff = tile_cols(S, t);
+                const uint32_t id_pos = tc::idesc_f16(BM, n_eff, false, false, false), id_neg = tc::idesc_f16(BM, n_eff, true, false, false);
+                const int b = (int)(n & 1);
+                if (!tc::mbar_wait(acce + 8 * b, (uint32_t)((n >> 1) & 1) ^ 1, a.err, ERR_ACC_WAIT, WAIT_CYCLES)) break;
+                tc::fence_after();
+                const uint32_t d = tmem + b * ACC_COLS + (warp == 2 ? ACC_COLS / 2 : 0);
+                for (int kc = 0; kc < nk; kc++) {
+                    if (!tc::mbar_wait(full0 + 8 * s, ph, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) { ok = false; break; }
+                    tc::fence_after();
+                    const uint64_t da = d0 + s * (stage_bytes / 16), db = diag ? da : da + 2 * A_BYTES / 16;
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; kk++) {
+                        // 16 FP16 along K are 32 bytes
+                        const uint64_t ar = da + 2 * kk, ai = ar + im16, br = db + 2 * kk, bi = br + im16;
+                        const uint32_t acc = (kc | kk) ? 1u : 0u;
+                        if (warp == 1) {
+                            tc::mma_f16(d, ar, br, id_pos, acc);           // Re += Ar Br^T
+                            tc::mma_f16(d, ai, bi, id_pos, 1u);            // Re += Ai Bi^T
+                        } else {
+                            tc::mma_f16(d, ai, br, id_pos, acc);           // Im += Ai Br^T  (M on a diagonal tile)
+                            if (!diag) tc::mma_f16(d, ar, bi, id_neg, 1u); // Im -= Ar Bi^T
+                        }
+                    }
+                    tc::commit(empty0 + 8 * s);                   // stage free once these MMAs finish
+                    if (++s == stages) s = 0, ph ^= 1;
+                }
+                if (ok) tc::commit(accf + 8 * b);
+            }
+            // `done` completes only after every MMA issued has finished, so TMEM is
+            // never freed under one
+            tc::commit(done);
+        }
+        __syncwarp();
+    } else if (warp >= 4) {
+        // ---------------- epilogue: TMEM -> global ----------------
+        const int q = warp & 3, half = (warp - 4) >> 2;            // TMEM lane quarter; even or odd column blocks
+        const int r = 32 * q + lane;
+        // 32-row x 16-column blocks through shared memory, so that a store
+        // instruction writes two 128-byte runs of one output row (columns XORed
+        // with the row: conflict-free both ways)
+        float2* stg = stg_all + (warp - 4) * 32 * 16;
+        Tile t;
+        for (int64_t n = 0; n < rounds && tile_of(a, n, t); n++) {
+            const int b = (int)(n & 1);
+            const bool ok = tc::mbar_wait(accf + 8 * b, (uint32_t)((n >> 1) & 1), a.err, ERR_ACC_WAIT, WAIT_CYCLES);
+            // the warps go on together or not at all; the last tile's M is read by now
+            if (!group_vote(__all_sync(0xffffffffu, ok), 32 * EPI_WARPS)) break;
+            tc::fence_after();
+            const bool diag = t.i0 == t.j0;
+            const int i = t.i0 + r;
+            const uint32_t acc = tmem + b * ACC_COLS + ((uint32_t)(32 * q) << 16);
+            const float si = (a.inv_scale && i < S) ? __ldg(a.inv_scale + (int64_t)i * a.scale_stride + t.c) : 1.f;
+            const int ncb = (int)(tile_cols(S, t) / 16);
+            if (diag) {
+                for (int cb = half; cb < ncb; cb += 2) {
+                    uint32_t mm[16];
+                    tc::tmem_ld_32x32b_x16(acc + ACC_COLS / 2 + cb * 16, mm);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int jj = 0; jj < 16; jj++) msh[r * MP + cb * 16 + jj] = __uint_as_float(mm[jj]);
+                }
+                group_vote(true, 32 * EPI_WARPS);
+            }
+            // this warp's rows end before the diagonal's later column blocks
+            const int last = diag ? min(ncb, 2 * q + 2) : ncb;
+            for (int cb = half; cb < last; cb += 2) {
+                uint32_t re[16], im[16];
+                tc::tmem_ld_32x32b_x16(acc + cb * 16, re);
+                if (!diag) tc::tmem_ld_32x32b_x16(acc + ACC_COLS / 2 + cb * 16, im);
+                tc::tmem_ld_wait();
+                if (diag) {
+#pragma unroll
+                    for (int jj = 0; jj < 16; jj++) {
+                        const int jl = cb * 16 + jj;                   // column within the tile
+                        im[jj] = __float_as_uint(msh[r * MP + jl] - msh[jl * MP + r]);
+                    }
+                }
+#pragma unroll
+                for (int jj = 0; jj < 16; jj++) {
+                    float f = si;
+                    if (a.inv_scale) {
+                        const int j = t.j0 + cb * 16 + jj;
+                        f *= (j < S) ? __ldg(a.inv_scale + (int64_t)j * a.scale_stride + t.c) : 0.f;
+                    }
+                    stg[lane * 16 + (jj ^ (lane & 15))] = make_float2(__uint_as_float(re[jj]) * f, __uint_as_float(im[jj]) * f);
+                }
+                __syncwarp();
+                const int col = lane & 15, j = t.j0 + cb * 16 + col;
+                int ii = t.i0 + 32 * q + (lane >> 4);
+                float2* o = a.vis + (int64_t)t.c * a.P + (int64_t)ii * (ii + 1) / 2 + j;
+#pragma unroll 4
+                for (int it = 0; it < 16; it++) {
+                    const int rr = 2 * it + (lane >> 4);
+                    if (ii < S && j <= ii) {
+                        float2 v = stg[rr * 16 + (col ^ (rr & 15))];
+                        if (a.accumulate) {
+                            const float2 old = *o;
+                            v.x += old.x;
+                            v.y += old.y;
+                        }
+                        *o = v;
+                    }
+                    o += 2 * ii + 3;                               // two rows on
+                    ii += 2;
+                }
+                __syncwarp();
+            }
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(acce + 8 * b);
+        }
+        tc::fence_before();
+    }
+    __syncthreads();
+    if (warp == 3) {
+        tc::mbar_wait(done, 0, a.err, ERR_ACC_WAIT, WAIT_CYCLES);
+        __syncwarp();
+        tc::fence_after();
+        tc::tmem_dealloc(tmem, 2 * ACC_COLS);
+    }
+}
+
+// The same with one tile a CTA, two CTAs an SM and one issuer each (6 warps: TMA
+// producer, TMEM owner and issuer, epilogue): tiles of long integrations, where a
+// ring of three stages each and chunk boundaries that do not meet keep the MMAs
+// busier than one CTA does and the epilogue is a small part.  From where it is
+// faster: 200 inputs of 4096 segments 829 us against 897 (512 inputs 2.97 ms, 3.04),
+// 132 inputs of 960 428 against 402, 300 inputs of 2048 875 against 863.
+constexpr int PAIR_MIN_K = 1536;
+constexpr int P_STAGES = 3, P_THREADS = 192;
+constexpr size_t P_SMEM = 1024 + P_STAGES * STAGE_BYTES + 256;
+// epilogue shared memory: four warps' 32 x 17 float2 staging blocks, then (on
+// a diagonal tile) M as [BM][MP] floats; both inside the operand ring
+constexpr int EPI_STG_BYTES = 4 * 32 * 17 * 8;
+static_assert(EPI_STG_BYTES + BM * MP * 4 <= P_STAGES * STAGE_BYTES, "epilogue M staging inside the ring");
+
+__global__ void __launch_bounds__(P_THREADS, 1) k_xmac_tc_pair(const __grid_constant__ CUtensorMap tmap,
+                                                           const __grid_constant__ TcArgs a)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    // offset from the shared array itself (not an integer round trip), so that
+    // the compiler keeps shared-space 32-bit addressing for every access
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P_STAGES * STAGE_BYTES);   // full[S], empty[S], acc
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * P_STAGES + 1);
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * P_STAGES, accb = full0 + 16 * P_STAGES;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Tile t = tile_at(blockIdx.x);
+    const int c = blockIdx.y;
+    const int i0 = t.i0, j0 = t.j0;
+    const int S = a.S;
+    const int nk = (a.K + BK - 1) / BK;
+    const uint32_t n_eff = tile_cols(S, t);
+    const bool diag = i0 == j0;                        // B is A, Im V = M - M^T
+    const uint32_t stage_tx = (diag ? 2u : 4u) * BM * BK * 2;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < P_STAGES; s++) {
             tc::mbar_init(full0 + 8 * s, 1);
             tc::mbar_init(empty0 + 8 * s, 1);
         }
@@ -143,7 +386,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
     }
     if (warp == 1) {
-        tc::tmem_alloc(smem_u32(tmem_slot), a.tmem_cols);
+        tc::tmem_alloc(smem_u32(tmem_slot), ACC_COLS);
     }
     tc::fence_before();
     __syncthreads();
@@ -152,7 +395,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             // one copy per operand brings both parts of its rows: planes as Re rows
             // then Im rows of 64 bytes, k-blocked as rows of 32 Re and 32 Im halves
             auto load = [&](uint32_t dst, int kc, int row, uint32_t bar) {
@@ -162,10 +405,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             int issued = 0;
             bool ok = true;
             for (int kc = 0; kc < nk && ok; kc++) {
-                const int s = kc % STAGES;
-                const uint32_t ph = (kc / STAGES) & 1;
+                const int s = kc % P_STAGES;
+                const uint32_t ph = (kc / P_STAGES) & 1;
                 if (!tc::mbar_wait(empty0 + 8 * s, ph ^ 1, a.err, ERR_EMPTY_WAIT, WAIT_CYCLES)) { ok = false; break; }
-                const uint32_t st = sbase + s * stage_bytes;
+                const uint32_t st = sbase + s * STAGE_BYTES;
                 const uint32_t fb = full0 + 8 * s;
                 tc::mbar_expect_tx(fb, stage_tx);
                 load(st, kc, i0, fb);
@@ -173,22 +416,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
                 issued = kc + 1;
             }
             // drain: every stage this thread filled must have landed before the CTA exits
-            for (int kc = (issued > STAGES ? issued - STAGES : 0); kc < issued; kc++)
-                tc::mbar_wait(full0 + 8 * (kc % STAGES), (kc / STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
+            for (int kc = (issued > P_STAGES ? issued - P_STAGES : 0); kc < issued; kc++)
+                tc::mbar_wait(full0 + 8 * (kc % P_STAGES), (kc / P_STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id_pos = tc::idesc_f16(BM, n_eff, false, false, false), id_neg = tc::idesc_f16(BM, n_eff, true, false, false);
-            const uint32_t d_re = tmem, d_im = tmem + a.tmem_cols / 2;
+            const uint32_t d_re = tmem, d_im = tmem + ACC_COLS / 2;
             const uint64_t d0 = a.kblock ? sw128_desc(sbase) : sw64_desc(sbase);
-            const uint32_t im16 = a.kblock ? 4 : (uint32_t)a.box_rows * BK * 2 / 16;   // Im after Re, in 16 bytes
+            const uint32_t im16 = a.kblock ? 4 : BM * BK * 2 / 16;   // Im after Re, in 16 bytes
             bool ok = true;
             for (int kc = 0; kc < nk; kc++) {
-                const int s = kc % STAGES;
-                if (!tc::mbar_wait(full0 + 8 * s, (kc / STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) { ok = false; break; }
+                const int s = kc % P_STAGES;
+                if (!tc::mbar_wait(full0 + 8 * s, (kc / P_STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) { ok = false; break; }
                 tc::fence_after();
-                const uint64_t da = d0 + s * (stage_bytes / 16), db = diag ? da : da + 2 * A_BYTES / 16;
+                const uint64_t da = d0 + s * (STAGE_BYTES / 16), db = diag ? da : da + 2 * A_BYTES / 16;
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; kk++) {
                     // 16 FP16 along K are 32 bytes
@@ -197,7 +440,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
                     tc::mma_f16(d_re, ar, br, id_pos, acc);           // Re += Ar Br^T
                     tc::mma_f16(d_re, ai, bi, id_pos, 1u);            // Re += Ai Bi^T
                     tc::mma_f16(d_im, ai, br, id_pos, acc);           // Im += Ai Br^T  (M on a diagonal tile)
-                    if (!mtr) tc::mma_f16(d_im, ar, bi, id_neg, 1u);  // Im -= Ar Bi^T
+                    if (!diag) tc::mma_f16(d_im, ar, bi, id_neg, 1u);  // Im -= Ar Bi^T
                 }
                 tc::commit(empty0 + 8 * s);                       // stage free once these MMAs finish
             }
@@ -218,7 +461,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
         // M - M^T needs the other warps' rows: the four epilogue warps agree
         // (one vote, so all of them or none reach the barrier below)
         bool go = __all_sync(0xffffffffu, ok);
-        if (mtr) go = epi_vote(go);
+        if (diag) go = group_vote(go, 128);
         if (go) {
             tc::fence_after();
             // Stage each 32-row x 16-column block through shared memory (the
@@ -230,22 +473,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
             const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
             const float si = (a.inv_scale && i < S) ? __ldg(a.inv_scale + (int64_t)i * a.scale_stride + c) : 1.f;
             const int ncb = (int)(n_eff / 16);
-            if (mtr) {
+            if (diag) {
                 for (int cb = 0; cb < ncb; cb++) {
                     uint32_t mm[16];
-                    tc::tmem_ld_32x32b_x16(lane_base + a.tmem_cols / 2 + cb * 16, mm);
+                    tc::tmem_ld_32x32b_x16(lane_base + ACC_COLS / 2 + cb * 16, mm);
                     tc::tmem_ld_wait();
 #pragma unroll
                     for (int jj = 0; jj < 16; jj++) msh[r * MP + cb * 16 + jj] = __uint_as_float(mm[jj]);
                 }
-                epi_bar();
+                group_vote(true, 128);
             }
             for (int cb = 0; cb < ncb; cb++) {
                 uint32_t re[16], im[16];
                 tc::tmem_ld_32x32b_x16(lane_base + cb * 16, re);
-                if (!mtr) tc::tmem_ld_32x32b_x16(lane_base + a.tmem_cols / 2 + cb * 16, im);
+                if (!diag) tc::tmem_ld_32x32b_x16(lane_base + ACC_COLS / 2 + cb * 16, im);
                 tc::tmem_ld_wait();
-                if (mtr) {
+                if (diag) {
 #pragma unroll
                     for (int jj = 0; jj < 16; jj++) {
                         const int jl = cb * 16 + jj;                   // column within the tile
@@ -285,7 +528,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
     __syncthreads();
     if (warp == 1) {
         tc::fence_after();
-        tc::tmem_dealloc(tmem, a.tmem_cols);
+        tc::tmem_dealloc(tmem, ACC_COLS);
     }
 }
 
@@ -350,7 +593,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
     tc::fence_after();
     const uint32_t tmem = *tmem_slot;
     if (warp == E) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int issued = 0;
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % ST;
@@ -366,7 +609,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
                 tc::mbar_wait(full0 + 8 * (kc % ST), (kc / ST) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES);
         }
     } else if (warp == E + 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, n, false, false, false);
             const uint64_t d0 = sw128_desc(sbase);
             for (int kc = 0; kc < nk; kc++) {
@@ -504,31 +747,6 @@ int xmac_gram(CsEncodeTiledFn enc, const void* spectra, int kp, const TcArgs& a,
            : a.S <= 32 ? launch_gram<64, false>(tm, a, st) : launch_gram<128, false>(tm, a, st);
 }
 
-// ---------------------------------------------------------------------------
-// host side
-// ---------------------------------------------------------------------------
-std::mutex g_tiles_mu;
-std::vector<std::pair<std::pair<int, int>, int2*>> g_tiles;   // ((device, S) -> device tile list)
-
-const int2* tile_list(int S, int* ntiles)
-{
-    std::vector<int2> h;
-    for (int i0 = 0; i0 < S; i0 += BM)
-        for (int j0 = 0; j0 < S; j0 += BN)
-            if (j0 <= i0 + BM - 1) h.push_back(make_int2(i0, j0));
-    *ntiles = (int)h.size();
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(g_tiles_mu);
-    for (auto& e : g_tiles)
-        if (e.first.first == dev && e.first.second == S) return e.second;
-    int2* d = nullptr;
-    if (cudaMalloc(&d, sizeof(int2) * h.size()) != cudaSuccess) return nullptr;
-    cudaMemcpy(d, h.data(), sizeof(int2) * h.size(), cudaMemcpyHostToDevice);
-    g_tiles.push_back({{dev, S}, d});
-    return d;
-}
-
 }  // namespace
 
 CsEncodeTiledFn cs_encode_tiled()
@@ -556,31 +774,27 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     CsEncodeTiledFn enc = cs_encode_tiled();
     if (!enc) return CS_ERR_UNSUPPORTED;
     if (S <= 64) {
-        const TcArgs g{S, C, K, (int64_t)S * (S + 1) / 2, nullptr, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
-                       accumulate, (S + 7) / 8 * 8, 1, 0, kblock, err};
+        const TcArgs g{S, C, K, (int64_t)S * (S + 1) / 2, 1, 0, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
+                       accumulate, (S + 7) / 8 * 8, 1, kblock, err};
         return xmac_gram(enc, spectra, kp, g, st);
     }
-    int ntiles = 0;
-    const int2* tiles = tile_list(S, &ntiles);
-    if (!tiles) return CS_ERR_ARG;
-
-    const int box_rows = S < BM ? (S + 7) / 8 * 8 : BM;
-    // S <= 64: k_xmac_tc_gram; S <= 128: one diagonal tile per channel, B = A, 16 KB stages and only the
-    // TMEM columns the tile needs, so several CTAs share an SM
-    const int small = S <= BM ? 1 : 0;
-    uint32_t cols = TMEM_COLS;
-    if (small) {
-        const uint32_t n_eff = (uint32_t)((S + 15) & ~15);
-        cols = 32;
-        while (cols < 2 * n_eff) cols *= 2;
-    }
-    TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, tiles, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
-             accumulate, box_rows, small, cols, kblock, err};
+    const int64_t nt = (S + BM - 1) / BM, ntiles = nt * (nt + 1) / 2;
+    int dev = 0, sms = 0;
+    CS_CUDA_TRY(cudaGetDevice(&dev));
+    CS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int grid = (int)std::min<int64_t>(sms, ntiles * C);
+    // grid + turn = 1 modulo the tiles of a channel: from one round to the next a CTA's tile moves on by one
+    const int turn = (int)(((1 - grid) % ntiles + ntiles) % ntiles);
+    const TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, ntiles, turn, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
+                   accumulate, S < BM ? (S + 7) / 8 * 8 : BM, S <= BM ? 1 : 0, kblock, err};
     CUtensorMap tm;
     if (!encode_map(enc, spectra, kp, BK, a, &tm)) return CS_ERR_ARG;
-    const size_t smem = (size_t)STAGES * (small ? 2 * A_BYTES : STAGE_BYTES) + 1024 + 256;
-    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc), (int)smem));
-    dim3 grid(ntiles, C);
-    k_xmac_tc<<<grid, TC_THREADS, smem, st>>>(tm, a), cs_count_launches(1);
+    if (S > BM && K >= PAIR_MIN_K) {
+        CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc_pair), (int)P_SMEM));
+        k_xmac_tc_pair<<<dim3((unsigned)ntiles, C), P_THREADS, P_SMEM, st>>>(tm, a), cs_count_launches(1);
+        return (int)cudaGetLastError();
+    }
+    CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc), (int)TC_SMEM));
+    k_xmac_tc<<<grid, TC_THREADS, TC_SMEM, st>>>(tm, a), cs_count_launches(1);
     return (int)cudaGetLastError();
 }

@@ -57,6 +57,24 @@ def test_xmac_f16_gram_sizes(cg, S, K):
     assert np.linalg.norm(vis - 2 * ref) / np.linalg.norm(ref) < 2e-5
 
 
+@pytest.mark.parametrize("S,C,K", [(65, 400, 40), (127, 310, 264), (128, 160, 8), (129, 60, 72), (200, 52, 1528),
+                                   (200, 3, 1536), (300, 60, 264), (513, 2, 1600)])
+def test_xmac_f16_tile_rounds(cg, S, C, K):
+    """Tiles of 128: several of them in turn on one SM and a partial last round, rows of part of a tile, time axes of
+    part of a chunk and of more than the ring holds, and both sides of the line to a tile a block."""
+    rng = np.random.default_rng(S + C)
+    spec = rng.integers(-3, 4, (C, 2, S, K)).astype(np.float16)
+    X = spec[:, 0].astype(np.float64) + 1j * spec[:, 1].astype(np.float64)
+    i, j = np.tril_indices(S)
+    ref = np.matmul(X, X.conj().transpose(0, 2, 1))[:, i, j]
+    vis = np.full((C, i.size), np.nan, np.complex64)
+    cg.xmac_f16(spec, S, C, K, vis)
+    # whole numbers, sums below 2^24: exact in FP32 whatever the order
+    assert np.array_equal(vis, ref)
+    cg.xmac_f16(spec, S, C, K, vis, accumulate=True)
+    assert np.array_equal(vis, 2 * ref)
+
+
 @pytest.mark.parametrize("S", [40, 200])
 def test_xmac_f16_accumulate(cg, S):
     """accumulate adds to the visibilities; S = 200 has diagonal tiles past the
