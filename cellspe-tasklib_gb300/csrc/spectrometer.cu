@@ -408,7 +408,10 @@ __global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_
     spec_fetch(raw, plane, first + (int64_t)j_begin * hop, WORDS, tid, NT, vec);
     if (tid < 16) lut16[tid] = make_float2(a.lut[tid & 3], a.lut[tid >> 2]);
     W::fill(tab, tw, 2 * M1);
-    float acc[TASKS][2 * M1], extra = 0.f;
+    __shared__ float2 w2m[2 * M1];                   // W_(2 M1)^i
+    if (tid < 2 * M1) w2m[tid] = __ldg(tw + 1024 * tid);
+    const float2 w512 = cscale(__ldg(tw + 512 * (lane & (2 * M1 - 1))), 0.5f);
+    float acc[TASKS][2 * M1], extra = 0.f, nyquist = 0.f;
 #pragma unroll
     for (int i = 0; i < TASKS; i++)
 #pragma unroll
@@ -453,43 +456,29 @@ __global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_
             for (int k2 = 0; k2 < 32; k2++) tile[lane + 32 * k2] = v[k2];
         }
         __syncthreads();
+        if (warp == M1 - 1) {
+            // columns 0 and 512, each paired with itself: bin 512 l is lane l's,
+            // Z = sum_n1 Y_n1[512 (l & 1)] W_2M1^(l n1), its pair lane 2 M1 - l's (one
+            // thread's pair of columns kept the other warps at the barrier)
+            const int l = lane & (2 * M1 - 1);
+            float2 z = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int n1 = 0; n1 < M1; n1++) {
+                const float2 y = tiles[n1 * W::TILE + 512 * (l & 1)], w = w2m[(l * n1) & (2 * M1 - 1)];
+                z.x = fmaf(y.x, w.x, fmaf(-y.y, w.y, z.x));
+                z.y = fmaf(y.x, w.y, fmaf(y.y, w.x, z.y));
+            }
+            const int lp = (2 * M1 - l) & (2 * M1 - 1);
+            const float2 zp = make_float2(__shfl_sync(0xffffffffu, z.x, lp), __shfl_sync(0xffffffffu, z.y, lp));
+            float2 Xk, Xm;
+            r2c_pair_h(z, zp, w512, Xk, Xm);
+            extra += l ? power(Xk) : Xk.x * Xk.x;    // DC and Nyquist are real
+            nyquist += Xm.x * Xm.x;
+        }
 #pragma unroll
         for (int i = 0; i < TASKS; i++) {
             const int kA = tid + NT * i;
-            if (kA == 0) {
-                // columns 0 and 512 (W_M^512 = W_(2 M1)), each paired with itself
-                float2 y0[M1], y5[M1];
-#pragma unroll
-                for (int n1 = 0; n1 < M1; n1++) {
-                    y0[n1] = tiles[n1 * W::TILE];
-                    y5[n1] = cmul(tiles[n1 * W::TILE + 512], w32((16 / M1) * n1));
-                }
-                Dft<M1>::run(y0);
-                Dft<M1>::run(y5);
-                const float2 w512 = __ldg(tw + 512);
-#pragma unroll
-                for (int k1 = 0; k1 <= M1 / 2; k1++) {
-                    float2 Xk, Xm;
-                    r2c_pair(y0[k1], y0[(M1 - k1) % M1], w32((16 / M1) * k1), Xk, Xm);
-                    if (k1 == 0) {                   // DC and Nyquist are real
-                        acc[i][0] += Xk.x * Xk.x;
-                        acc[i][1] += Xm.x * Xm.x;
-                    } else if (k1 < M1 / 2) {
-                        acc[i][2 * k1] += power(Xk);
-                        acc[i][2 * k1 + 1] += power(Xm);
-                    } else {
-                        extra += power(Xk);
-                    }
-                }
-#pragma unroll
-                for (int k1 = 0; k1 < M1 / 2; k1++) {
-                    float2 Xk, Xm;
-                    r2c_pair(y5[k1], y5[M1 - 1 - k1], cmul(w512, w32((16 / M1) * k1)), Xk, Xm);
-                    acc[i][M1 + 2 * k1] += power(Xk);
-                    acc[i][M1 + 2 * k1 + 1] += power(Xm);
-                }
-                continue;
-            }
+            if (kA == 0) continue;                   // columns 0 and 512: above
             float2 ya[M1], yb[M1];
             const float2 u1 = __ldg(tw + 2 * kA);    // W_M^kA
             float2 pw = make_float2(1.f, 0.f);
@@ -502,11 +491,11 @@ __global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_
             }
             Dft<M1>::run(ya);                        // ya[k1] = Z[kA + 1024 k1]
             Dft<M1>::run(yb);                        // yb[(k1 + 1) % M1] = Z[1024 - kA + 1024 k1]
-            const float2 wA = __ldg(tw + kA);        // W_N^kA
+            const float2 wA = cscale(__ldg(tw + kA), 0.5f);     // W_N^kA / 2
 #pragma unroll
             for (int k1 = 0; k1 < M1; k1++) {
                 float2 Xk, Xm;
-                r2c_pair(ya[k1], yb[(M1 - k1) % M1], k1 ? cmul(wA, w32((16 / M1) * k1)) : wA, Xk, Xm);
+                r2c_pair_h(ya[k1], yb[(M1 - k1) % M1], rot32(wA, (16 / M1) * k1), Xk, Xm);
                 acc[i][2 * k1] += power(Xk);
                 acc[i][2 * k1 + 1] += power(Xm);
             }
@@ -522,14 +511,12 @@ __global__ void __launch_bounds__(32 * M1, 16 / M1) k_spec_power_m(const __grid_
             if (kA) {
                 prow[kA + 1024 * k1] = acc[i][2 * k1];
                 prow[M - kA - 1024 * k1] = acc[i][2 * k1 + 1];
-            } else if (k1 < M1 / 2) {
-                prow[1024 * k1] = acc[i][2 * k1];
-                prow[M - 1024 * k1] = acc[i][2 * k1 + 1];
-                prow[512 + 1024 * k1] = acc[i][M1 + 2 * k1];
-                prow[M - 512 - 1024 * k1] = acc[i][M1 + 2 * k1 + 1];
             }
         }
-        if (kA == 0) prow[M / 2] = extra;
+    }
+    if (warp == M1 - 1 && lane < 2 * M1) {
+        prow[512 * lane] = extra;
+        if (lane == 0) prow[M] = nyquist;
     }
 }
 
@@ -600,7 +587,7 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
     // the split twiddle W_N^k of item (k1, k2), k = P (k1 + 16 k2) + p, as
     // ck[k1] = W_N^(P k1 + p) (shared, broadcast) times W_N^(16 P k2) of k2 = t, t + 512
     __shared__ float2 ck[16];
-    if (tid < 16) ck[tid] = __ldg(tw + P * tid + p);
+    if (tid < 16) ck[tid] = cscale(__ldg(tw + P * tid + p), 0.5f);
     float2 tmc[2], umc[2], bk[2];
 #pragma unroll
     for (int c = 0; c < 2; c++) {
@@ -725,7 +712,7 @@ __global__ void __launch_bounds__(SW_NT, 1) k_spec_power_w(const __grid_constant
             const int mp = k1 + 16 * k2;                   // index in the CTA's transform
             const int k = P * mp + p;                      // bin of the full real FFT
             float2 Xk, Xm;
-            r2c_pair<false>(za, zb, cmul(ck[k1], b), Xk, Xm);          // W_N^k
+            r2c_pair_h(za, zb, cmul(ck[k1], b), Xk, Xm);         // W_N^k / 2
             if (special && k == 0) {
                 slots[s * SW_NT + tid] += Xk.x * Xk.x;
                 slots[(s + 1) * SW_NT + tid] += Xm.x * Xm.x;
