@@ -411,6 +411,14 @@ size_t w2048_smem()
            + (size_t)1024 * (G + 1) * elem;         // staging tile
 }
 
+// The pair of samples `sh` bits (a multiple of 4) into `word`: the word turned so
+// that the table entry's byte offset stands in place.
+CS_DEV float2 pair_at(const float2* lut16, uint32_t word, int sh)
+{
+    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(lut16) +
+                                            (__funnelshift_r(word, word, (sh - 3) & 31) & 0x78u));
+}
+
 CS_DEV void cp_async16(uint32_t dst, const void* src, bool valid)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
@@ -503,10 +511,15 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16 || (FMT == 
             const int f0 = off + 2 * lane;
             const int wb = f0 >> 4, sh = 2 * (f0 & 15);
             float2 v[32];
+            if (off & 1) {                                      // as in the longer transforms' kernel
 #pragma unroll
-            for (int n2 = 0; n2 < 32; n2++) {
-                const uint32_t bits = __funnelshift_r(rw[wb + 4 * n2], rw[wb + 4 * n2 + 1], sh);
-                v[n2] = lut16[bits & 15u];
+                for (int n2 = 0; n2 < 32; n2++) {
+                    const uint32_t bits = __funnelshift_r(rw[wb + 4 * n2], rw[wb + 4 * n2 + 1], sh);
+                    v[n2] = lut16[bits & 15u];
+                }
+            } else {
+#pragma unroll
+                for (int n2 = 0; n2 < 32; n2++) v[n2] = pair_at(lut16, rw[wb + 4 * n2], sh);
             }
             Dft<32>::run(v);                                    // over n2 -> k1
             // v[k1] *= W_1024^(lane k1), the powers formed once per thread
@@ -544,9 +557,10 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16 || (FMT == 
                 sincosf(32.f * dph, &sn, &cs);
                 D = make_float2(cs, sn);
             }
-            const float* scl = a.scale ? a.scale + (int64_t)s * M : nullptr;
+            auto split = [&](auto scaled) {
+            const float* scl = decltype(scaled)::value ? a.scale + (int64_t)s * M : nullptr;
             auto put = [&](int c, float2 X) {
-                if (scl) X = cscale(X, __ldg(scl + c));
+                if constexpr (decltype(scaled)::value) X = cscale(X, __ldg(scl + c));
                 if constexpr (FMT == CS_SPECTRA_F32)
                     reinterpret_cast<float2*>(stage)[c * (G + 1) + ls] = X;
                 else
@@ -577,6 +591,9 @@ __global__ void __launch_bounds__(32 * WARPS, (WARPS == 16 || G > 16 || (FMT == 
                 put(c1, X1);
                 if (k2 < 16 && c1 != 0) put(c2, X2);
             }
+            };
+            if (a.scale) split(std::true_type{});
+            else split(std::false_type{});
         }
     }
     __syncthreads();
@@ -868,8 +885,7 @@ __global__ void __launch_bounds__(32 * M1, wbig_blocks<M1, PHASE>()) k_fx_fstage
         const int wb = f0 >> 4, sh = 2 * (f0 & 15);
         float2 v[32];
         // pair j is 64 M1 samples = 4 M1 words further on; at an even offset (all jobs
-        // without delays) no pair crosses a word, and the word turned by the pair's
-        // place holds the table's byte offset
+        // without delays) no pair crosses a word
         if (off & 1) {
 #pragma unroll
             for (int j = 0; j < 32; j++) {
@@ -878,11 +894,7 @@ __global__ void __launch_bounds__(32 * M1, wbig_blocks<M1, PHASE>()) k_fx_fstage
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const uint32_t x = rw[wb + 4 * M1 * j];
-                v[j] = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(lut16) +
-                                                        (__funnelshift_r(x, x, (sh - 3) & 31) & 0x78u));
-            }
+            for (int j = 0; j < 32; j++) v[j] = pair_at(lut16, rw[wb + 4 * M1 * j], sh);
         }
         Dft<32, PK>::run(v);
         float2 q = make_float2(1.f, 0.f);
