@@ -42,7 +42,8 @@ extern "C" {
 #define CELLSPE_UNPACK_MSB_FIRST     0x100  /* single channel: sample 0 in bits 7:6 */
 
 /* X-stage arithmetic */
-#define CELLSPE_X_FP32     0   /* FP32 CUDA cores                                   */
+#define CELLSPE_X_FP32     0   /* FP32 precision: CUDA cores, or tensor cores on two FP16 terms a value (FX jobs
+                                * of 9 inputs and 24 segments or more), with no larger error */
 #define CELLSPE_X_TC_FP16  1   /* tcgen05 tensor cores, FP16 inputs, FP32 accumulate */
 #define CELLSPE_X_INT8     2   /* int8 spectra (per input and channel max-abs scale),
                                   mma.sync IMMA, int32 accumulate; K % 16 == 0.
