@@ -1128,10 +1128,17 @@ __global__ void __launch_bounds__(256, FMT == CS_SPECTRA_F32 ? 1 : 2) k_fx_fstag
         const int f0 = off + 2 * hl;
         const int wb = f0 >> 4, sh = 2 * (f0 & 15);
         float2 v[16];
+        // pair j is 32 samples = 2 words further on; at even offsets (of both half-warps)
+        // no pair crosses a word
+        if (__any_sync(0xffffffffu, off & 1)) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) {                           // pair j is 32 samples = 2 words further on
-            const uint32_t bits = __funnelshift_r(rw[wb + 2 * j], rw[wb + 2 * j + 1], sh);
-            v[j] = lut16[bits & 15u];
+            for (int j = 0; j < 16; j++) {
+                const uint32_t bits = __funnelshift_r(rw[wb + 2 * j], rw[wb + 2 * j + 1], sh);
+                v[j] = lut16[bits & 15u];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[j] = pair_at(lut16, rw[wb + 2 * j], sh);
         }
         Dft<16>::run(v);
 #pragma unroll
@@ -1158,9 +1165,10 @@ __global__ void __launch_bounds__(256, FMT == CS_SPECTRA_F32 ? 1 : 2) k_fx_fstag
             sincosf(16.f * dph, &sn, &cs);
             D = make_float2(cs, sn);
         }
-        const float* scl = a.scale ? a.scale + (int64_t)s * M : nullptr;
+        auto write = [&](auto scaled) {
+        const float* scl = decltype(scaled)::value ? a.scale + (int64_t)s * M : nullptr;
         auto put = [&](int c, float2 X) {
-            if (scl) X = cscale(X, __ldg(scl + c));
+            if constexpr (decltype(scaled)::value) X = cscale(X, __ldg(scl + c));
             if constexpr (FMT == CS_SPECTRA_F32)
                 reinterpret_cast<float2*>(stage)[c * (G + 1) + ls] = X;
             else
@@ -1191,6 +1199,9 @@ __global__ void __launch_bounds__(256, FMT == CS_SPECTRA_F32 ? 1 : 2) k_fx_fstag
             put(c1, X1);
             if (k2 < 8 && c1 != 0) put(c2, X2);
         }
+        };
+        if (a.scale) write(std::true_type{});
+        else write(std::false_type{});
     }
     __syncthreads();
     stage_writeout<FMT, M, G, NT>(a, stage, s, k0);
@@ -1302,10 +1313,17 @@ __global__ void __launch_bounds__(256, 1) k_fx_fstage_w1024(const __grid_constan
         const int f0 = off + 2 * hl;
         const int wb = f0 >> 4, sh = 2 * (f0 & 15);
         float2 v[32];
+        // pair j is 32 samples = 2 words further on; at even offsets (of both half-warps)
+        // no pair crosses a word
+        if (__any_sync(0xffffffffu, off & 1)) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) {                           // pair j is 32 samples = 2 words further on
-            const uint32_t bits = __funnelshift_r(rw[wb + 2 * j], rw[wb + 2 * j + 1], sh);
-            v[j] = lut16[bits & 15u];
+            for (int j = 0; j < 32; j++) {
+                const uint32_t bits = __funnelshift_r(rw[wb + 2 * j], rw[wb + 2 * j + 1], sh);
+                v[j] = lut16[bits & 15u];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = pair_at(lut16, rw[wb + 2 * j], sh);
         }
         Dft<32>::run(v);
         {
@@ -1338,15 +1356,22 @@ __global__ void __launch_bounds__(256, 1) k_fx_fstage_w1024(const __grid_constan
         if constexpr (PHASE) {
             const float ph0 = __ldg(a.phase0 + sk), dph = __ldg(a.dphase + sk);
             float sn, cs;
-            sincosf(ph0 + (float)hl * dph, &sn, &cs);            A1 = make_float2(cs, sn);
-            sincosf(ph0 + (float)(M - hl) * dph, &sn, &cs);      A2 = make_float2(cs, sn);
-            sincosf(ph0 + (float)(hl + 16) * dph, &sn, &cs);     B1 = make_float2(cs, sn);
-            sincosf(ph0 + (float)(M - hl - 16) * dph, &sn, &cs); B2 = make_float2(cs, sn);
-            sincosf(32.f * dph, &sn, &cs);                       D = make_float2(cs, sn);
+            // two sincosf a thread, as in the longer transforms' kernel
+            sincosf(hl == 0 ? ph0 : hl == 1 ? ph0 + (float)M * dph : (hl == 2 ? 16.f : 32.f) * dph, &sn, &cs);
+            auto of = [&](int l) { return make_float2(__shfl_sync(0xffffffffu, cs, l, 16), __shfl_sync(0xffffffffu, sn, l, 16)); };
+            const float2 P0 = of(0), PM = of(1), D16 = of(2);
+            D = of(3);
+            sincosf((float)hl * dph, &sn, &cs);
+            const float2 E = make_float2(cs, sn);
+            A1 = cmul(P0, E);                                    // channel hl + 32 k2
+            A2 = cmul_conj(PM, E);                               // channel M - hl - 32 k2
+            B1 = cmul(A1, D16);
+            B2 = cmul_conj(A2, D16);
         }
-        const float* scl = a.scale ? a.scale + (int64_t)s * M : nullptr;
+        auto write = [&](auto scaled) {
+        const float* scl = decltype(scaled)::value ? a.scale + (int64_t)s * M : nullptr;
         auto put = [&](int c, float2 X) {
-            if (scl) X = cscale(X, __ldg(scl + c));
+            if constexpr (decltype(scaled)::value) X = cscale(X, __ldg(scl + c));
             if constexpr (FMT == CS_SPECTRA_F32)
                 reinterpret_cast<float2*>(stage)[c * (G + 1) + ls] = X;
             else
@@ -1399,6 +1424,9 @@ __global__ void __launch_bounds__(256, 1) k_fx_fstage_w1024(const __grid_constan
                 put(M - cB, X2);
             }
         }
+        };
+        if (a.scale) write(std::true_type{});
+        else write(std::false_type{});
     }
     __syncthreads();
     stage_writeout<FMT, M, G, NT>(a, stage, s, k0);
