@@ -93,6 +93,7 @@ struct TcArgs {
     int64_t P;
     int64_t ntiles;             // tiles of a channel's lower triangle
     int turn;                   // of the CTAs' order, per round
+    int stages;                 // of k_xmac_tc_gram's ring
     float2* vis;
     const float* inv_scale;     // [S][scale_stride] or null
     int scale_stride;
@@ -553,13 +554,16 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_xmac_tc_pair(const __grid_cons
 // E = COLS / 32 epilogue warps, the TMA producer, the MMA issuer and TMEM owner.
 // ---------------------------------------------------------------------------
 constexpr int G_ROW = 128;                          // operand row bytes
-template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : COLS == 32 ? 6 : COLS == 64 ? 5 : 4; }
+// Planes take two stages, which leave room for the most CTAs on an SM: 64 inputs, 8192
+// channels of 200 segments 206 us with four stages, 139 with two; 48 inputs 168 and 102.
+template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : 2; }
 
 template <int COLS, bool BLK>
 __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constant__ CUtensorMap tmap,
                                                             const __grid_constant__ TcArgs a)
 {
-    constexpr int E = COLS / 32, ST = gram_stages<COLS, BLK>(), SEGS = BLK ? 32 : 64;
+    constexpr int E = COLS / 32, MAX_ST = gram_stages<COLS, BLK>(), SEGS = BLK ? 32 : 64;
+    const int ST = a.stages;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -569,7 +573,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
     const uint32_t n = (uint32_t)((S + 15) & ~15);
     // barriers in front, so that the ring and the rows past it end the buffer
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);                   // full[], empty[], acc
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 1);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_ST + 1);
     unsigned char* ring = smem + 1024;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * ST, accb = full0 + 16 * ST;
     const uint32_t sbase = smem_u32(ring);
@@ -692,14 +696,16 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
 }
 
 template <int COLS, bool BLK>
-int launch_gram(const CUtensorMap& tm, const TcArgs& a, cudaStream_t st)
+int launch_gram(const CUtensorMap& tm, TcArgs a, cudaStream_t st)
 {
+    const int chunks = (a.K + (BLK ? 32 : 64) - 1) / (BLK ? 32 : 64);
+    a.stages = std::min(chunks, gram_stages<COLS, BLK>());
     // the ring, the rows past it that an MMA of 128 rows reads (lanes never
     // stored), and after the last MMA the accumulators [rows][columns + 1]
     const size_t plane = (size_t)a.box_rows * G_ROW, rows = (BLK ? 1 : 2) * (size_t)a.box_rows;
     const size_t cols = (BLK ? 2 : 1) * (((size_t)a.S + 15) / 16 * 16);
     // an operand of 128 rows from the last stage's Xr (BLK) or Xi on
-    const size_t ring = gram_stages<COLS, BLK>() * (BLK ? plane : 3 * plane) + BM * G_ROW - (BLK ? plane : 2 * plane);
+    const size_t ring = a.stages * (BLK ? plane : 3 * plane) + BM * G_ROW - (BLK ? plane : 2 * plane);
     const size_t smem = 2048 + std::max(ring, rows * (cols + 1) * sizeof(float));
     auto kern = k_xmac_tc_gram<COLS, BLK>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
@@ -774,7 +780,7 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     CsEncodeTiledFn enc = cs_encode_tiled();
     if (!enc) return CS_ERR_UNSUPPORTED;
     if (S <= 64) {
-        const TcArgs g{S, C, K, (int64_t)S * (S + 1) / 2, 1, 0, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
+        const TcArgs g{S, C, K, (int64_t)S * (S + 1) / 2, 1, 0, 0, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
                        accumulate, (S + 7) / 8 * 8, 1, kblock, err};
         return xmac_gram(enc, spectra, kp, g, st);
     }
@@ -785,7 +791,7 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     const int grid = (int)std::min<int64_t>(sms, ntiles * C);
     // grid + turn = 1 modulo the tiles of a channel: from one round to the next a CTA's tile moves on by one
     const int turn = (int)(((1 - grid) % ntiles + ntiles) % ntiles);
-    const TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, ntiles, turn, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
+    const TcArgs a{S, C, K, (int64_t)S * (S + 1) / 2, ntiles, turn, 0, vis, inv_scale, scale_stride > 0 ? scale_stride : C,
                    accumulate, S < BM ? (S + 7) / 8 * 8 : BM, S <= BM ? 1 : 0, kblock, err};
     CUtensorMap tm;
     if (!encode_map(enc, spectra, kp, BK, a, &tm)) return CS_ERR_ARG;
