@@ -43,7 +43,8 @@ int cs_perm_pack(const float2* bins, float* out, int n, int64_t batch, cudaStrea
 // fstage.cu -----------------------------------------------------------------
 // Error record of a job's tensor-core kernels (bounded waits that ran out),
 // in device memory: kernels take the address of `code`, which they set once, and
-// copy it to *host (page-locked; may be null).  Zeroed again by whoever found an error.
+// copy it to *host (page-locked; may be null).  Kernels whose result needs every
+// warp's part store nothing while the code is set, so a job starts with it zero.
 struct alignas(16) CsErrorWord {
     unsigned code, pad;
     unsigned* host;
@@ -154,6 +155,9 @@ __device__ __forceinline__ float cs_split_unscale(float v, float bias, float inv
 int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err,
                   cudaStream_t st);
 float cs_xmac_split_lo(int S);       // the lo term's weight it expects for S inputs
+// A kernel whose one wait runs out after about a millisecond (xstage_tc.cu): the
+// error record's path to the host, for tests.
+int cs_wait_timeout(unsigned* err, cudaStream_t st);
 // X stage of small arrays straight from segment-major spectra [S][K][c_pitch]
 // (half2, or float2 taken as two FP16 terms of scale `split`), C channels from
 // `spectra` on -> vis float2 [C][P]; C and c_pitch multiples of 8.

@@ -175,6 +175,7 @@ struct Workspace {
     // device memory, and the page-locked words they reach the host through
     CsErrorWord* d_err = nullptr;
     volatile unsigned* h_err = nullptr;
+    bool err_async = false;           // asynchronous jobs were issued since the words were last known clear
     struct Out { void* host; const void* dev; size_t bytes; };
     std::vector<Out> outs;
     int init()
@@ -212,18 +213,24 @@ struct Workspace {
     }
     unsigned* f_err() const { return &d_err[0].code; }
     unsigned* x_err() const { return &d_err[1].code; }
-    // Before a job: clears what an earlier one that was not waited for may have left.
-    void clear_errors()
+    // Before a job: the words become this job's own.  An asynchronous job is
+    // queued, or replayed from a graph, when nobody can tell what an earlier
+    // one will have left, so its reset runs on its own stream and is captured
+    // with it.  A blocking job needs one only after asynchronous jobs, or where
+    // the last error's page-locked words still stand.
+    void clear_errors(bool sync)
     {
-        if (!h_err[0] && !h_err[1]) return;
-        for (int i = 0; i < 2; i++) cudaMemsetAsync(&d_err[i].code, 0, sizeof(unsigned), stream), h_err[i] = 0;
+        if (sync && !err_async && !h_err[0] && !h_err[1]) return;
+        cudaMemset2DAsync(d_err, sizeof(CsErrorWord), 0, sizeof(unsigned), 2, stream);
+        if (sync) h_err[0] = h_err[1] = 0;
+        err_async = !sync;
     }
     // After a job's stream has synchronised: the error of its tensor-core kernels, cleared.
     int check_errors(const std::string& who)
     {
         const unsigned f = h_err[0], x = h_err[1];
         if (!f && !x) return 0;
-        clear_errors();
+        clear_errors(true);
         return set_err(CELLSPE_ERR_CUDA, who + (f ? "F stage" : "X stage") + ": tensor-core pipeline wait timed out (code " +
                                              std::to_string(f ? f : x) + ")");
     }
@@ -468,7 +475,7 @@ int op_xmac_f16(Workspace& ws, bool host, const void* spectra, int S, int C, int
     Job j(ws, host);
     const void* d_sp = j.in(spectra, (size_t)C * 2 * S * K * 2);
     void* d_vis = j.out(vis, (size_t)C * P * 8, accumulate != 0);
-    ws.clear_errors();
+    ws.clear_errors(true);
     if (!j.err) {
         int rc = map_rc(cs_xmac_tc_f16(d_sp, S, C, K, K, (float2*)d_vis, nullptr, 0, accumulate, ws.x_err(), ws.stream), "xmac_f16");
         if (rc) j.err = rc;
@@ -587,7 +594,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             ws.chain->valid = cudaEventRecord(ws.chain->in_done, ws.copy) == cudaSuccess;
         }
     }
-    ws.clear_errors();
+    ws.clear_errors(sync);
     if (sync) cudaEventRecord(ws.sev[0], ws.stream);
     CsFStageArgs fa{};
     fa.err = ws.f_err();
@@ -2410,6 +2417,18 @@ int cellspe_fx_correlate_async(const cellspe_fx_params* p, const void* raw, cons
     int rc = op_fx(*ws, p, raw, delay_poly, vis, false);
     ws->stream = saved;
     return rc;
+}
+
+int cellspe_debug_wait_timeout(int stage, int async, void* stream)
+{
+    DIRECT_WORKSPACE
+    if (stage < 0 || stage > 1) return set_err(CELLSPE_ERR_ARG, "debug_wait_timeout: stage must be 0 (F) or 1 (X)");
+    unsigned* word = stage ? ws->x_err() : ws->f_err();
+    if (async) return map_rc(cs_wait_timeout(word, (cudaStream_t)stream), "debug_wait_timeout");
+    ws->clear_errors(true);
+    if (int rc = map_rc(cs_wait_timeout(word, ws->stream), "debug_wait_timeout")) return rc;
+    cudaError_t e = cudaStreamSynchronize(ws->stream);
+    return e == cudaSuccess ? ws->check_errors("debug_wait_timeout: ") : cuda_fail(e, "kernel execution");
 }
 
 int cellspe_release_workspace(void)

@@ -753,6 +753,15 @@ int xmac_gram(CsEncodeTiledFn enc, const void* spectra, int kp, const TcArgs& a,
            : a.S <= 32 ? launch_gram<64, false>(tm, a, st) : launch_gram<128, false>(tm, a, st);
 }
 
+// One thread, one barrier that nothing arrives at.
+__global__ void k_wait_timeout(unsigned* err)
+{
+    __shared__ __align__(8) uint64_t bar;
+    tc::mbar_init(smem_u32(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_wait(smem_u32(&bar), 0, err, ERR_FULL_WAIT, 2000000LL);
+}
+
 }  // namespace
 
 CsEncodeTiledFn cs_encode_tiled()
@@ -802,5 +811,12 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
     }
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc), (int)TC_SMEM));
     k_xmac_tc<<<grid, TC_THREADS, TC_SMEM, st>>>(tm, a), cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
+
+int cs_wait_timeout(unsigned* err, cudaStream_t st)
+{
+    if (!err) return CS_ERR_ARG;
+    k_wait_timeout<<<1, 1, 0, st>>>(err), cs_count_launches(1);
     return (int)cudaGetLastError();
 }

@@ -66,6 +66,12 @@ int  cellspe_memcpy(void* dst, const void* src, size_t bytes, int kind); /* 1 H2
 /* Fault injection for tests: the next `count` tasks or calls on `slot`
  * (-1 = direct calls) fail with CELLSPE_ERR_INJECTED before touching the GPU. */
 int  cellspe_debug_inject_failure(int slot, int count);
+/* For tests: a kernel whose one wait, on a barrier that nothing arrives at, gives
+ * up after about a millisecond and is recorded as an error of the calling thread's
+ * F stage (0) or X stage (1).  async = 0: waits for it and returns the error as a
+ * blocking job would (CELLSPE_ERR_CUDA).  async = 1: issued on `stream`, as the part
+ * of an asynchronous job that timed out there. */
+int  cellspe_debug_wait_timeout(int stage, int async, void* stream);
 /* Kernels this library has launched since it was loaded (all threads). */
 long long cellspe_kernel_launches(void);
 /* Device time in ms of the calling thread's last blocking FX job, measured
