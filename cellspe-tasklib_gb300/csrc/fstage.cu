@@ -79,27 +79,57 @@ inline int out_segments(const CsFStageArgs& a) { return a.split > 0.f ? split_se
 // from segment k0) as two FP16 terms in 32-segment blocks (CsFStageArgs::
 // split); segments past K are written as zeros.  A thread takes eight segments
 // of one channel's Re or Im: 16-byte stores, pairs of lanes filling a sector.
+// The autos are summed here, from the FP32 values, and not by the tensor cores
+// (xstage_split.cu): the 2 P8 threads of a channel add their squares.  Four
+// channels at a time, each lane keeping one of them, so that they take three
+// shuffles and a store and not eight and four (this is bound by instruction issue:
+// 200 inputs x 2048 segments of 2048 points 1510 us without, 1590 so done one by one).
+CS_DEV float squares8(const float (&x)[8])
+{
+    float2 p = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) p = __ffma2_rn(make_float2(x[u], x[u + 1]), make_float2(x[u], x[u + 1]), p);
+    return p.x + p.y;
+}
 template <int M, int G, int NT>
 CS_DEV void split_writeout(const CsFStageArgs& a, const unsigned char* stage, int s, int k0)
 {
-    constexpr int P8 = G / 8;
+    constexpr int P8 = G / 8, CSTEP = NT / (2 * P8);
+    static_assert(P8 >= 2 && 2 * P8 <= 32 && NT % (2 * P8) == 0 && M % (4 * CSTEP) == 0, "whole warps of whole channels");
     const int nvalid = max(0, min(G, a.K - k0)), nseg = min(G, split_segments(a.K) - k0);
     const int S = out_rows(a), blocks = out_pitch(a) / 32;
-    const float* st = reinterpret_cast<const float*>(stage);
-    uint4* out = reinterpret_cast<uint4*>(a.out);
-    for (int idx = threadIdx.x; idx < M * 2 * P8; idx += NT) {
-        const int piece = idx % P8, comp = (idx / P8) & 1, c = idx / (2 * P8);
-        if (8 * piece >= nseg) continue;
-        float x[8];
+    // a thread's piece and part are the same in every channel it takes
+    const int piece = threadIdx.x % P8, comp = (threadIdx.x / P8) & 1, c0 = threadIdx.x / (2 * P8), k = k0 + 8 * piece;
+    const bool store = 8 * piece < nseg, sums = threadIdx.x % (2 * P8) < 4 && nvalid > 0;
+    const bool b0 = threadIdx.x & 1, b1 = threadIdx.x & 2;
+    const float* st = reinterpret_cast<const float*>(stage) + 2 * (c0 * (G + 1) + 8 * piece) + comp;
+    uint4* o = reinterpret_cast<uint4*>(a.out) + (((int64_t)c0 * S + s) * blocks + k / 32) * 16 + comp * 8 + (k % 32) / 8;
+    const int64_t step = (int64_t)CSTEP * S * blocks * 16;
+    float* sq = a.squares + ((int64_t)(k0 / G) * S + s) * M + c0 + (threadIdx.x & 3) * CSTEP;
+#pragma unroll 1
+    for (int n = 0; n < M / CSTEP; n += 4) {
+        float q[4];
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            x[u] = 8 * piece + u < nvalid ? st[2 * (c * (G + 1) + 8 * piece + u) + comp] : 0.f;
-        uint4 hi, lo;
-        split8(x, a.split, a.split_lo, hi, lo);
-        const int k = k0 + 8 * piece;
-        uint4* o = out + (((int64_t)c * S + s) * blocks + k / 32) * 16 + comp * 8 + (k % 32) / 8;
-        o[0] = hi;
-        o[4] = lo;
+        for (int i = 0; i < 4; i++) {
+            float x[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) x[u] = 8 * piece + u < nvalid ? st[2 * u] : 0.f;
+            q[i] = squares8(x);
+            if (store) {
+                uint4 hi, lo;
+                split8(x, a.split, a.split_lo, hi, lo);
+                o[0] = hi;
+                o[4] = lo;
+            }
+            st += 2 * CSTEP * (G + 1);
+            o += step;
+        }
+        const float r0 = (b0 ? q[1] : q[0]) + __shfl_xor_sync(0xffffffffu, b0 ? q[0] : q[1], 1);
+        const float r1 = (b0 ? q[3] : q[2]) + __shfl_xor_sync(0xffffffffu, b0 ? q[2] : q[3], 1);
+        float r = (b1 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b1 ? r0 : r1, 2);
+#pragma unroll
+        for (int d = 4; d < 2 * P8; d *= 2) r += __shfl_xor_sync(0xffffffffu, r, d);
+        if (sums) sq[n * CSTEP] = r;
     }
 }
 
@@ -340,10 +370,11 @@ CS_DEV void stage_writeout(const CsFStageArgs& a, const unsigned char* stage, in
     const int nvalid = max(0, min(G, a.K - k0));
     const int S = out_rows(a), KP = out_pitch(a);
     if constexpr (FMT == CS_SPECTRA_F32) {
-        if (a.split > 0.f) {
-            split_writeout<M, G, NT>(a, stage, s, k0);
-            return;
-        }
+        if constexpr (G >= 16)
+            if (a.split > 0.f) {
+                split_writeout<M, G, NT>(a, stage, s, k0);
+                return;
+            }
         const float2* st = reinterpret_cast<const float2*>(stage);
         float2* out = reinterpret_cast<float2*>(a.out);
         if (nvalid == G && KP % 2 == 0) {
@@ -398,6 +429,7 @@ CS_DEV void stage_writeout(const CsFStageArgs& a, const unsigned char* stage, in
 // Input must be LSB-first (sample j of a 32-bit word at bits 2j).
 // ---------------------------------------------------------------------------
 constexpr int W_G = 8, W_TP = 33;
+constexpr int W_SPLIT_G = 16;                   // segments per CTA where the output is two FP16 terms
 constexpr int W_RAWC = 2048 / 64 + 2;          // 16-byte chunks staged per segment (34 = 136 words)
 constexpr int W_RAWW = 4 * W_RAWC;
 
@@ -736,7 +768,7 @@ int launch_w2048(const CsFStageArgs& a, cudaStream_t st)
     // two FP16 terms: 16 segments per CTA (8 warps, 2 each; the FP32 staging
     // tile of 32 would not fit), so each plane's run of a block is a whole sector
     if constexpr (FMT == CS_SPECTRA_F32)
-        if (a.split > 0.f) return launch_w2048_variant<FMT, PHASE, 8, 1, 16>(a, tw, st);
+        if (a.split > 0.f) return launch_w2048_variant<FMT, PHASE, 8, 1, W_SPLIT_G>(a, tw, st);
     const char* env = getenv("CELLSPE_FSTAGE_VARIANT");
     if (env && env[0] >= '1' && env[0] <= '0' + W_NVARIANTS)
         return launch_w2048_choice<FMT, PHASE>(env[0] - '0', a, tw, st);
@@ -1526,7 +1558,7 @@ int cs_fx_fstage(const CsFStageArgs& a, cudaStream_t st)
     if (!a.raw || !a.out || a.S <= 0 || a.K <= 0) return CS_ERR_ARG;
     if ((uintptr_t)a.raw % 16 || a.bytes_per_input % 16 || (uintptr_t)a.out % 16) return CS_ERR_ARG;
     if (a.kblock < 0 || a.kblock > 2 || (a.kblock && !cs_fstage_kblocked(a))) return CS_ERR_ARG;
-    if (a.split > 0.f && !a.seg_major && (!cs_fstage_split_scale(a) || (a.kp ? a.kp : a.K) % 32)) return CS_ERR_ARG;
+    if (a.split > 0.f && !a.seg_major && (!cs_fstage_split_scale(a) || !a.squares || (a.kp ? a.kp : a.K) % 32)) return CS_ERR_ARG;
     // channel-grouped k-blocked spectra: only the warp-specialised form writes them
     if (a.kblock == 2) return cs_fstage_tc32_supported(a) ? cs_fx_fstage_tc32(a, st, true) : CS_ERR_ARG;
     // The tensor-core F stage is opt-in (CELLSPE_FSTAGE_TC=1, read per call):
@@ -1675,7 +1707,8 @@ __global__ void __launch_bounds__(256) k_transpose_f32(const float2* __restrict_
 // to the end of their block.
 constexpr int TC = 32;
 __global__ void __launch_bounds__(256) k_transpose_split(const float2* __restrict__ in, int K, int C, int kp, int S_out,
-                                                         uint4* __restrict__ out, float scale, float lo_weight)
+                                                         uint4* __restrict__ out, float scale, float lo_weight,
+                                                         float* __restrict__ squares)
 {
     __shared__ float tile[2][TC][TT + 1];            // Re, Im: [channel][segment]
     const int s = blockIdx.z, k0 = blockIdx.y * TT, c0 = blockIdx.x * TC;
@@ -1689,10 +1722,14 @@ __global__ void __launch_bounds__(256) k_transpose_split(const float2* __restric
     const int nseg = split_segments(K) - k0;
     for (int i = threadIdx.x; i < TC * 2 * (TT / 8); i += 256) {
         const int piece = i % (TT / 8), comp = (i / (TT / 8)) & 1, cc = i / (2 * (TT / 8)), c = c0 + cc;
-        if (c >= C || 8 * piece >= nseg) continue;
         float x[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) x[u] = tile[comp][cc][8 * piece + u];
+        float q = squares8(x);
+#pragma unroll
+        for (int d = 1; d < 2 * (TT / 8); d *= 2) q += __shfl_xor_sync(0xffffffffu, q, d);
+        if (c < C && i % (2 * (TT / 8)) == 0) squares[((int64_t)blockIdx.y * S_out + s) * C + c] = q;
+        if (c >= C || 8 * piece >= nseg) continue;
         uint4 hi, lo;
         split8(x, scale, lo_weight, hi, lo);
         const int k = k0 + 8 * piece;
@@ -1704,16 +1741,18 @@ __global__ void __launch_bounds__(256) k_transpose_split(const float2* __restric
 
 }  // namespace
 
+int cs_squares_segs(int N) { return N == 512 ? H_G : N == 1024 ? w1024_g<CS_SPECTRA_F32>() : N == 2048 ? W_SPLIT_G : TT; }
+
 int cs_spectra_transpose(const void* tmp, int S, int K, int C, int kp, int S_out, int format, void* out, cudaStream_t st,
-                         float split, float split_lo)
+                         float split, float split_lo, float* squares)
 {
     if (!tmp || !out || S <= 0 || K <= 0 || C <= 0 || kp < K || S_out < S || S > 65535) return CS_ERR_ARG;
     const dim3 grid((C + TT - 1) / TT, (K + TT - 1) / TT, S);
     if (grid.y > 65535) return CS_ERR_ARG;
     if (split > 0.f) {
-        if (format != CS_SPECTRA_F32 || kp % 32 || (uintptr_t)out % 16) return CS_ERR_ARG;
+        if (format != CS_SPECTRA_F32 || !squares || kp % 32 || (uintptr_t)out % 16) return CS_ERR_ARG;
         k_transpose_split<<<dim3((C + TC - 1) / TC, (K + TT - 1) / TT, S), 256, 0, st>>>((const float2*)tmp, K, C, kp, S_out,
-                                                                                       (uint4*)out, split, split_lo),
+                                                                                       (uint4*)out, split, split_lo, squares),
             cs_count_launches(1);
     } else if (format == CS_SPECTRA_F32) {
         k_transpose_f32<<<grid, 256, 0, st>>>((const float2*)tmp, K, C, kp, S_out, (float2*)out), cs_count_launches(1);

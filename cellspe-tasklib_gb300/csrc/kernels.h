@@ -88,6 +88,7 @@ struct CsFStageArgs {
                                 // of 32 hi and 32 lo halves, zero from segment K to the next
                                 // multiple of 32
     float split_lo;             // weight of the lo term (cs_xmac_split_lo)
+    float* squares;             // split: sums of |X|^2 over cs_squares_segs(N) segments, [block][S_out][C]
     unsigned* err;              // CsErrorWord::code of the job (tensor-core F stages)
 };
 int cs_fx_fstage(const CsFStageArgs& a, cudaStream_t st);
@@ -119,7 +120,8 @@ int cs_fstage_layout(const CsFStageArgs& a);
 // (CsFStageArgs::split); F16 half rows (c, plane, s); row pitch kp, S_out
 // inputs per (c[, plane]) block (tmp and out already offset to the block).
 int cs_spectra_transpose(const void* tmp, int S, int K, int C, int kp, int S_out, int format, void* out,
-                         cudaStream_t st, float split = 0.f, float split_lo = 1.f);
+                         cudaStream_t st, float split = 0.f, float split_lo = 1.f, float* squares = nullptr);
+int cs_squares_segs(int N);          // segments of a partial sum of CsFStageArgs::squares
 // The scale for CsFStageArgs::split: the power of two that brings the largest
 // spectrum value N samples of these levels can give (N max|level|) just below
 // 2^15; 0 when the F stage cannot write the two terms for these arguments
@@ -143,17 +145,15 @@ int cs_fx_fstage_tc32(const CsFStageArgs& a, cudaStream_t st, bool specialised =
 // [C][P], P = S(S+1)/2, p = i(i+1)/2 + j (j <= i), V = sum_k X_i conj(X_j).
 int cs_xmac_f32(const float2* spectra, int S, int C, int K, int kp, float2* vis, int accumulate,
                 cudaStream_t st);
-// Mean relative loss of a Gram matrix's positive sums to the truncation of its
-// one-chunk accumulators, and an accumulated product in the spectra's own scale
-// with that loss given back (xstage_split.cu says how it was measured).
-constexpr float CS_GRAM_BIAS = 1.30e-7f;
-#ifdef __CUDACC__
-__device__ __forceinline__ float cs_split_unscale(float v, float bias, float inv) { return fmaf(v, bias, v) * inv * inv; }
-#endif
+// Inputs and segments from which an FX job's FP32 X stage takes its spectra as two
+// FP16 terms: with fewer segments the CUDA cores' serial sums are the more accurate
+// ones (xstage_split.cu has the figures).
+constexpr int CS_SPLIT_MIN_S = 9, CS_SPLIT_MIN_K = 64;
 // FP32 X stage on the tensor cores from spectra as two FP16 terms
-// (CsFStageArgs::split, scale 1 / inv_scale) -> vis float2 [C][P].
-int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err,
-                  cudaStream_t st);
+// (CsFStageArgs::split, scale 1 / inv_scale) -> vis float2 [C][P], the autos from
+// the F stage's `blocks` squares of these channels (inputs c_pitch floats apart).
+int cs_xmac_split(const void* spectra, const float* squares, int blocks, int S, int C, int c_pitch, int K, int kp,
+                  float2* vis, float inv_scale, unsigned* err, cudaStream_t st);
 float cs_xmac_split_lo(int S);       // the lo term's weight it expects for S inputs
 // A kernel whose one wait runs out after about a millisecond (xstage_tc.cu): the
 // error record's path to the host, for tests.

@@ -509,14 +509,17 @@ int op_xmac_i8(Workspace& ws, bool host, const void* planes, const float* scale,
 // for the X stage's TMA loads and costs at most 25% memory at K = 256 (1.6%
 // at K = 4096).
 long long spectra_pitch(long long K) { return K >= 256 ? K + 64 : K; }
-// FP32 jobs of at least SPLIT_MIN_K segments (whose X stage may take its spectra as
-// two FP16 terms in 32-segment blocks) round it up to whole blocks.
-constexpr int SPLIT_MIN_K = 24, SPLIT_MIN_S = 9;
+// FP32 jobs of 64 segments and more (whose X stage may take its spectra as two
+// FP16 terms in 32-segment blocks) round it up to whole blocks.
 long long spectra_pitch(long long K, int x_mode)
 {
     const long long kp = spectra_pitch(K);
-    return x_mode == CELLSPE_X_FP32 && K >= SPLIT_MIN_K ? (kp + 31) / 32 * 32 : kp;
+    return x_mode == CELLSPE_X_FP32 && K >= CS_SPLIT_MIN_K ? (kp + 31) / 32 * 32 : kp;
 }
+
+// CsFStageArgs::squares of a job
+long long squares_blocks(int N, int K) { return (K + cs_squares_segs(N) - 1) / cs_squares_segs(N); }
+long long squares_bytes(int S, int N, int K) { return squares_blocks(N, K) * S * (N / 2) * 4; }
 
 long long fx_bytes(const cellspe_fx_params* p, bool with_poly)
 {
@@ -529,6 +532,7 @@ long long fx_bytes(const cellspe_fx_params* p, bool with_poly)
     const bool f32 = p->x_mode != CELLSPE_X_TC_FP16;   // FP32 spectra (FP32 and INT8 X stages)
     b += align256(C * S * spectra_pitch(K, p->x_mode) * (f32 ? 8 : 4));
     if (N >= 4096) b += align256(C * S * K * (f32 ? 8 : 4));   // segment-major spectra
+    if (p->x_mode == CELLSPE_X_FP32 && S >= CS_SPLIT_MIN_S && K >= CS_SPLIT_MIN_K) b += align256(squares_bytes(p->n_inputs, p->fft_points, p->n_segments));
     if (p->x_mode == CELLSPE_X_INT8) b += align256(C * 2 * S * spectra_pitch(K)) + align256(S * C * 4);
     bool stage_vis = host || p->vis_order == CELLSPE_VIS_BASELINE_MAJOR || p->accumulate;
     if (stage_vis) b += 3 * align256(C * P * 8);
@@ -633,9 +637,9 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     fa.kp = kp;
     // FP32 X stage: on the tensor cores from spectra as two FP16 terms, except
     // for arrays of a few inputs (cs_xmac_f32 reads each row once there: 2 inputs
-    // x 512 channels x 4096 segments 9 us) and for fewer segments than most of a
-    // 32-segment block
-    if (p->x_mode == CELLSPE_X_FP32 && S >= SPLIT_MIN_S && K >= SPLIT_MIN_K) fa.split = cs_fstage_split_scale(fa);
+    // x 512 channels x 4096 segments 9 us) and for integrations so short that the
+    // CUDA cores' serial sums are the more accurate ones
+    if (p->x_mode == CELLSPE_X_FP32 && S >= CS_SPLIT_MIN_S && K >= CS_SPLIT_MIN_K) fa.split = cs_fstage_split_scale(fa);
     fa.split_lo = cs_xmac_split_lo(S);
     // FP16, N = 2048: 128-byte runs per 32 segments, k-blocked (1) or
     // channel-grouped k-blocked (2, the warp-specialised F stage)
@@ -651,6 +655,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     const bool seg_x = segmaj && (fa.format == CS_SPECTRA_F16 || fa.split > 0.f) && cs_xmac_seg_supported(S);
     char* seg_tmp = segmaj ? (char*)j.scratch((size_t)((long long)S * K * C * seg_bytes)) : nullptr;
     fa.out = seg_x ? seg_tmp : j.scratch((size_t)C * S * kp * (fa.format == CS_SPECTRA_F32 ? 8 : 4));
+    if (fa.split > 0.f && !seg_x) fa.squares = (float*)j.scratch((size_t)squares_bytes(S, N, K));
     for (int i = 0; i < nsc && !j.err; i++) {
         CsFStageArgs fb = fa;
         long long s0 = 0, s1 = S;
@@ -666,6 +671,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             if (fa.shift) fb.shift = fa.shift + s0 * K;
             if (fa.phase0) fb.phase0 = fa.phase0 + s0 * K, fb.dphase = fa.dphase + s0 * K;
             if (fa.scale) fb.scale = fa.scale + s0 * C;
+            if (fa.squares) fb.squares = fa.squares + s0 * C;
         }
         void* rows_out = fb.out;
         if (segmaj) {
@@ -676,7 +682,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         int rc = map_rc(cs_fx_fstage(fb, ws.stream), "F stage");
         if (!rc && segmaj && !seg_x)
             rc = map_rc(cs_spectra_transpose(fb.out, (int)(s1 - s0), K, C, kp, S, fa.format, rows_out, ws.stream, fa.split,
-                                             fa.split_lo),
+                                             fa.split_lo, fb.squares),
                         "spectra transpose");
         if (rc) j.err = rc;
     }
@@ -713,8 +719,8 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             rc = cs_xmac_seg(seg_tmp + c0 * seg_bytes, fa.format, S, (int)cn, C, K, vis_cp + c0 * P,
                              d_inv_scale ? d_inv_scale + c0 : nullptr, C, fa.split, ws.x_err(), ws.stream);
         else if (fa.split > 0.f)
-            rc = cs_xmac_split((const char*)fa.out + c0 * S * kp * 8, S, (int)cn, K, kp, vis_cp + c0 * P, 1.f / fa.split,
-                               ws.x_err(), ws.stream);
+            rc = cs_xmac_split((const char*)fa.out + c0 * S * kp * 8, fa.squares + c0, (int)squares_blocks(N, K), S, (int)cn, C, K, kp,
+                               vis_cp + c0 * P, 1.f / fa.split, ws.x_err(), ws.stream);
         else if (p->x_mode == CELLSPE_X_FP32)
             rc = cs_xmac_f32((const float2*)fa.out + c0 * S * kp, S, (int)cn, K, kp, vis_cp + c0 * P, 0, ws.stream);
         else if (p->x_mode == CELLSPE_X_INT8)

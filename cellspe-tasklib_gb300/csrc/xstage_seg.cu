@@ -283,6 +283,7 @@ template <int RI> struct SplitCfg {
     static constexpr int COLS = 2 * CB * N2, STAGES = RI == 16 ? 4 : 3, DEPTH = RI == 16 ? 6 : 3;
     static constexpr uint32_t SLACK = (BM - N2) * ROWB;
     static constexpr int GROUPS = LOADERS / (RI * 8);                       // loaders work on GROUPS chunks at once
+    static constexpr int PARTS = GROUPS * SEGS / 8;                         // loaders that share an input's squares
     static constexpr int E = CB * Q;                                        // epilogue warps
 };
 constexpr int SPLIT_THREADS = 18 * 32;
@@ -297,7 +298,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
     // full[], empty[], accf[2], acce[2], done, raw full[], raw empty[]
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2 * F::STAGES + 5 + 2 * F::DEPTH);
-    unsigned char* ring = smem + 1024;                       // operands, then (past the rows an MMA may read) raw chunks
+    float* sq = reinterpret_cast<float*>(smem + 1024);       // [PARTS][CB][RI], 2 KB
+    unsigned char* ring = smem + 3072;                       // operands, then (past the rows an MMA may read) raw chunks
     unsigned char* raw = ring + F::STAGES * F::STAGE + F::SLACK;
     const uint32_t full0 = tc::smem_u32(bars), empty0 = full0 + 8 * F::STAGES, accf = empty0 + 8 * F::STAGES, acce = accf + 16,
                    done = acce + 16, rfull = done + 8, rempty = rfull + 8 * F::DEPTH;
@@ -356,13 +358,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
         }
         __syncwarp();
     } else if (warp & 2) {
-        // loader: channels 2 ch and 2 ch + 1, segments 8 kg ..+7 of an input
+        // loader: channels 2 ch and 2 ch + 1, segments 8 kg ..+7 of an input, and the
+        // sums of their squares: the autos are formed from the FP32 values (see
+        // xstage_split.cu), a chunk's eight segments first
         const int t = ((warp >> 2) * 2 + (warp & 1)) * 32 + lane;          // 0 .. 255
         const int grp = t / (RI * 8), u0 = t % (RI * 8);
         const int ch = u0 & 1, si = (u0 >> 1) % RI, kg = (u0 >> 1) / RI;
         const int sw = si & 7;
         const uint32_t row = (uint32_t)(2 * ch) * F::TILE + si * F::ROWB;
         const uint32_t hi_at = row + ((kg ^ sw) * 16), lo_at = row + (((kg + 4) ^ sw) * 16);
+        float squares[2] = {0.f, 0.f};
         bool ok = true;
         for (int kc = grp; kc < nk && ok; kc += F::GROUPS) {
             const int s = kc % F::STAGES, r = kc % F::DEPTH;
@@ -376,7 +381,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
             if (ok) {
                 unsigned char* st = ring + s * F::STAGE;
 #pragma unroll
-                for (int x = 0; x < 2; x++)
+                for (int x = 0; x < 2; x++) {
+                    float part = 0.f;
 #pragma unroll
                     for (int im = 0; im < 2; im++) {
                         uint32_t h[4], l[4];
@@ -385,6 +391,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
                             const uint4 e = v[2 * q], o = v[2 * q + 1];
                             const float fa = __uint_as_float(x ? (im ? e.w : e.z) : (im ? e.y : e.x)) * a.split;
                             const float fb = __uint_as_float(x ? (im ? o.w : o.z) : (im ? o.y : o.x)) * a.split;
+                            part = fmaf(fa, fa, part);
+                            part = fmaf(fb, fb, part);
                             const __half2 hh = __floats2half2_rn(fa, fb);
                             const float2 hf = __half22float2(hh);
                             const __half2 ll = __floats2half2_rn(2.f * (fa - hf.x), 2.f * (fb - hf.y));
@@ -395,6 +403,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
                         *reinterpret_cast<uint4*>(st + hi_at + at) = make_uint4(h[0], h[1], h[2], h[3]);
                         *reinterpret_cast<uint4*>(st + lo_at + at) = make_uint4(l[0], l[1], l[2], l[3]);
                     }
+                    squares[x] += part;
+                }
                 tc::fence_proxy_async();
             }
             __syncwarp();
@@ -405,6 +415,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
                 tc::mbar_arrive(rempty + 8 * r);
             }
         }
+#pragma unroll
+        for (int x = 0; x < 2; x++) sq[((grp * (F::SEGS / 8) + kg) * F::CB + 2 * ch + x) * RI + si] = squares[x];
+        asm volatile("bar.arrive 2, %0;" ::"n"(LOADERS + 32 * F::E) : "memory");
     } else if ((warp & 1) < F::Q) {
         // epilogue: channel warp / 4, rows 32 q ..+31 of its G
         const int c = warp >> 2, q = warp & 1;
@@ -434,6 +447,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(acce + 8 * b);
         }
+        // every loader arrives here, whatever became of its waits
+        asm volatile("bar.sync 2, %0;" ::"n"(LOADERS + 32 * F::E) : "memory");
         ok = ok && (*reinterpret_cast<volatile unsigned*>(a.err) == 0u);
         if (vote(__all_sync(0xffffffffu, ok), 32 * F::E)) {
             // the last chunk's MMAs are done, so the ring is free
@@ -446,10 +461,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1)
             for (int p = 32 * q + lane; p < (int)a.P; p += 32 * F::Q) {
                 int i, j;
                 product(p, i, j);
-                const float re = (g[i * GP + j] + g[j * GP + i]) + (g[(RI + i) * GP + RI + j] + g[(RI + j) * GP + RI + i]);
-                const float im = (g[(RI + i) * GP + j] - g[(RI + j) * GP + i]) + (g[j * GP + RI + i] - g[i * GP + RI + j]);
-                out[p] = make_float2(cs_split_unscale(re, CS_GRAM_BIAS, a.inv) * 0.5f,
-                                     cs_split_unscale(im, CS_GRAM_BIAS, a.inv) * 0.5f);
+                float re = 0.5f * ((g[i * GP + j] + g[j * GP + i]) + (g[(RI + i) * GP + RI + j] + g[(RI + j) * GP + RI + i]));
+                if (i == j) {
+                    re = 0.f;
+#pragma unroll
+                    for (int t = 0; t < F::PARTS; t++) re += sq[(t * F::CB + c) * RI + i];
+                }
+                const float im = 0.5f * ((g[(RI + i) * GP + j] - g[(RI + j) * GP + i]) + (g[j * GP + RI + i] - g[i * GP + RI + j]));
+                out[p] = make_float2(re * a.inv * a.inv, im * a.inv * a.inv);
             }
         }
         tc::fence_before();
@@ -495,7 +514,8 @@ int launch_split(const void* spectra, int64_t pitch, const SegArgs& a, cudaStrea
     CUtensorMap tm;
     if (!encode_map<F>(spectra, a, 2 * a.C, pitch, RI, &tm)) return CS_ERR_ARG;
     const size_t ring = F::STAGES * F::STAGE + F::SLACK + F::DEPTH * F::R::BYTES, g = (size_t)F::CB * F::N2 * (F::N2 + 1) * 4;
-    const size_t smem = 2048 + std::max(ring, g);
+    static_assert(F::PARTS * F::CB * RI * 4 == 2048, "squares");
+    const size_t smem = 4096 + std::max(ring, g);
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_seg_split<RI>), (int)smem));
     k_xmac_seg_split<RI><<<a.C / F::CB, SPLIT_THREADS, smem, st>>>(tm, a), cs_count_launches(1);
     return (int)cudaGetLastError();

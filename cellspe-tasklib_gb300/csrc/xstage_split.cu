@@ -31,10 +31,23 @@
 // grows with the number of MMAs on positive sums.  So an accumulator lives for
 // one 32-segment chunk only: the small cross terms go in first, then the hi hi'
 // terms, and the epilogue warps add the chunk to FP32 registers in
-// round-to-nearest while the other TMEM buffer takes the next chunk.
-// Relative error against FP64, N = 2048 and K = 24, 512, 4096 segments: 1.7e-7,
-// 1.5e-7, 1.7e-7 on the autos (the sequential sum of the CUDA cores: 2.0e-7, 4.8e-7,
-// 1.4e-6).
+// round-to-nearest while the other TMEM buffer takes the next chunk.  What the
+// cut of one chunk still takes from a sum of positive terms is 1.3e-7 of it
+// (S <= 64; two hi hi' MMAs an accumulator) or 2.2e-7 (four).  The autos are
+// such sums in every job, so they are added apart, in FP32: the F stage's write-out,
+// which holds the FP32 values, sums |X|^2 over its tile of 16 to 64 segments (1/32
+// to 1/128 of the spectra's bytes), and k_split_autos adds those, 8 us for 10 inputs
+// of 4096 segments and 20 for 200 of 2048.  (Squared here, from the operand rows in
+// the ring, by the epilogue's warps or the producer's, 64 inputs took 490 us and not
+// 340, 200 inputs of 2048 segments 1508 and not 1258: their work then sets the pace.)
+//
+// Error against FP64 (inputs that share a tenth of their power; N = 512, 2048,
+// 8192 and 32768, S = 9 .. 200) over that of the CUDA cores' serial sum
+// (cs_xmac_f32), which grows with K: cross products 0.90 to 0.99 at K = 64, 0.40
+// to 0.60 at 512, but 1.00 to 1.09 at 24 and 32, where those are used
+// (CS_SPLIT_MIN_K); autos 0.57 to 0.69 at 64, 0.23 to 0.30 at 512.  Cross products of fully
+// correlated inputs are positive sums as well: up to 1.2 (S <= 64) and 1.6 at 64
+// segments, 1 at 128 and 256, 0.5 and 0.7 at 512.
 //
 // Warp roles: warps 0 .. E-1 epilogue (warp w reads TMEM lanes 32 (w % 4)
 // ..+31), warp E TMA producer, warp E + 1 TMEM owner and MMA issuer.  TMA boxes
@@ -60,11 +73,6 @@ constexpr int BM = 128, BK = 32;                    // tile edge and segments pe
 constexpr int ROW_BYTES = BK * 4;                   // 32 hi and 32 lo halves
 constexpr int MAX_STAGES = 6;
 constexpr long long WAIT_CYCLES = 4000000000LL;     // ~2 s at 2 GHz
-// Mean relative loss of a chunk's positive sums to the accumulator's
-// truncation, given back at the end: measured as the mean error of the autos
-// against FP64 less that of the FP32 transform alone, the same to 0.1e-7 at N = 512,
-// 2048 and 8192, K = 24 .. 1024 (two hi hi' MMAs per chunk and accumulator, four for a tile).
-constexpr float GRAM_BIAS = CS_GRAM_BIAS, TILE_BIAS = 2.17e-7f;
 constexpr unsigned ERR_FULL_WAIT = 1, ERR_EMPTY_WAIT = 2, ERR_ACC_WAIT = 3, ERR_DRAIN_WAIT = 4;
 
 // K-major operand of 128-byte rows; a descriptor's low 14 bits hold the address / 16,
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(2 * R + 64, gram_ctas<R>())
                 const int j = t - i * (i + 1) / 2;
                 const float re = (g[i * GP + j] + g[j * GP + i]) + (g[(R + i) * GP + R + j] + g[(R + j) * GP + R + i]);
                 const float im = (g[(R + i) * GP + j] - g[(R + j) * GP + i]) + (g[j * GP + R + i] - g[i * GP + R + j]);
-                out[t] = make_float2(cs_split_unscale(re, GRAM_BIAS, a.inv) * 0.5f, cs_split_unscale(im, GRAM_BIAS, a.inv) * 0.5f);
+                out[t] = make_float2(re * a.inv * a.inv * 0.5f, im * a.inv * a.inv * 0.5f);
             }
         }
         tc::fence_before();
@@ -407,7 +415,7 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
                     for (int j = 0; j < 16; j++) {
                         float im = acci[cb * 16 + j];
                         if (diag) im -= msh[(col0 + cb * 16 + j) * MP + r];
-                        stg[lane * 17 + j] = make_float2(cs_split_unscale(accr[cb * 16 + j], TILE_BIAS, a.inv), cs_split_unscale(im, TILE_BIAS, a.inv));
+                        stg[lane * 17 + j] = make_float2(accr[cb * 16 + j] * a.inv * a.inv, im * a.inv * a.inv);
                     }
                     __syncwarp();
 #pragma unroll 4
@@ -428,6 +436,28 @@ __global__ void __launch_bounds__(32 * (T_E + 3), 1)
     }
 }
 
+// ---- the autos -------------------------------------------------------------------
+// Input s's auto of 32 channels: eight slices of the F stage's partial sums (32
+// channels of one block are 128 bytes), added in order.
+constexpr int A_SLICES = 8;
+__global__ void __launch_bounds__(32 * A_SLICES)
+    k_split_autos(const float* __restrict__ squares, int S, int C, int c_pitch, int nb, int64_t P, float2* __restrict__ vis)
+{
+    __shared__ float part[A_SLICES][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, s = blockIdx.y;
+    float sum = 0.f;
+    if (c < C) {
+#pragma unroll 8
+        for (int b = slice; b < nb; b += A_SLICES) sum += __ldg(squares + ((int64_t)b * S + s) * c_pitch + c);
+    }
+    part[slice][lane] = sum;
+    __syncthreads();
+    if (slice || c >= C) return;
+#pragma unroll
+    for (int q = 1; q < A_SLICES; q++) sum += part[q][lane];
+    vis[(int64_t)c * P + (int64_t)s * (s + 3) / 2] = make_float2(sum, 0.f);
+}
+
 // stages of `stage` bytes that fit `ctas` CTAs' rings in an SM's shared memory
 int ring_stages(int ctas, uint32_t stage, uint32_t slack)
 {
@@ -446,13 +476,20 @@ int launch_gram(const CUtensorMap& tm, SplitArgs a, int C, cudaStream_t st)
     return (int)cudaGetLastError();
 }
 
+int launch_autos(const float* squares, int nb, const SplitArgs& a, int C, int c_pitch, cudaStream_t st)
+{
+    k_split_autos<<<dim3((C + 31) / 32, a.S), 32 * A_SLICES, 0, st>>>(squares, a.S, C, c_pitch, nb, a.P, a.vis), cs_count_launches(1);
+    return (int)cudaGetLastError();
+}
+
 }  // namespace
 
 float cs_xmac_split_lo(int S) { return S <= 64 ? 2.f : 1.f; }
 
-int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis, float inv_scale, unsigned* err, cudaStream_t st)
+int cs_xmac_split(const void* spectra, const float* squares, int blocks, int S, int C, int c_pitch, int K, int kp,
+                  float2* vis, float inv_scale, unsigned* err, cudaStream_t st)
 {
-    if (!spectra || !vis || !err || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp % BK || kp < K || (uintptr_t)spectra % 16)
+    if (!spectra || !squares || !vis || !err || S > 65535 || S <= 0 || C <= 0 || K <= 0 || C > 65535 || kp % BK || kp < K || (uintptr_t)spectra % 16)
         return CS_ERR_ARG;
     CsEncodeTiledFn enc = cs_encode_tiled();
     if (!enc) return CS_ERR_UNSUPPORTED;
@@ -470,13 +507,15 @@ int cs_xmac_split(const void* spectra, int S, int C, int K, int kp, float2* vis,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return CS_ERR_ARG;
     SplitArgs a{S, K, (int64_t)S * (S + 1) / 2, vis, inv_scale, 0, err, (uint32_t)rows * ROW_BYTES};
-    if (S <= 16) return launch_gram<16>(tm, a, C, st);
-    if (S <= 32) return launch_gram<32>(tm, a, C, st);
-    if (S <= 64) return launch_gram<64>(tm, a, C, st);
+    if (S <= 64) {
+        const int rc = S <= 16 ? launch_gram<16>(tm, a, C, st) : S <= 32 ? launch_gram<32>(tm, a, C, st) : launch_gram<64>(tm, a, C, st);
+        return rc ? rc : launch_autos(squares, blocks, a, C, c_pitch, st);
+    }
     const uint32_t stage = (tiles == 1 ? 2 : 4) * a.plane_bytes, slack = BM * ROW_BYTES - a.plane_bytes;
     a.stages = ring_stages(1, stage, slack);
     const size_t smem = (size_t)a.stages * stage + slack + BAR_BYTES + 1024;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_split), (int)smem));
     k_xmac_split<<<dim3(tiles, C), 32 * (T_E + 3), smem, st>>>(tm, a), cs_count_launches(1);
-    return (int)cudaGetLastError();
+    CS_CUDA_TRY(cudaGetLastError());
+    return launch_autos(squares, blocks, a, C, c_pitch, st);
 }

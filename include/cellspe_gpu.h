@@ -43,7 +43,10 @@ extern "C" {
 
 /* X-stage arithmetic */
 #define CELLSPE_X_FP32     0   /* FP32 precision: CUDA cores, or tensor cores on two FP16 terms a value (FX jobs
-                                * of 9 inputs and 24 segments or more), with no larger error */
+                                * of 9 inputs and 64 segments or more).  Against FP64 the latter's error is the
+                                * smaller one for autos and for weakly correlated inputs; cross products of fully
+                                * correlated inputs lose up to 2.2e-7, as much as the CUDA cores' sums have at 256
+                                * segments (see csrc/xstage_split.cu) */
 #define CELLSPE_X_TC_FP16  1   /* tcgen05 tensor cores, FP16 inputs, FP32 accumulate */
 #define CELLSPE_X_INT8     2   /* int8 spectra (per input and channel max-abs scale),
                                   mma.sync IMMA, int32 accumulate; K % 16 == 0.

@@ -329,3 +329,40 @@ def test_fx_fp32_split_delay_levels(cg, orc, N):
     for q in (i != 3) & (j != 3), (i == 3) & (j != 3):        # the tone's own products do not hide the others
         # the phasor's angle is FP32: up to N/2 dphase rad, 2^-24 of a few hundred rad
         assert _rel(vis[:, q], ref[:, q]) < TOL
+
+
+SPLIT_FORMS = [
+    (9, 512, 64), (16, 1024, 65), (17, 2048, 160), (33, 512, 127), (64, 512, 66),     # a Gram matrix of 16, 32, 64 inputs
+    (9, 4096, 64), (16, 8192, 129), (32, 4096, 95), (40, 4096, 64),                   # segment-major spectra, and 33 inputs on
+    (65, 512, 64), (72, 1024, 257), (128, 512, 300), (129, 512, 64), (200, 512, 287)]     # one tile, several
+
+
+@pytest.mark.parametrize("S,N,K", SPLIT_FORMS + [(16, 512, 63), (65, 512, 63)])
+def test_fx_fp32_split_exact_sums(cg, S, N, K):
+    """Constant inputs, whose products and sums in channel 0 are whole numbers that FP32 holds: bit for bit."""
+    levels = np.array([-3, -1, 1, 3], np.float32)
+    code = np.arange(S) % 4
+    raw = np.repeat((code * 0b01010101).astype(np.uint8)[:, None], N * K // 4 + 16, axis=1)
+    p = cg.fx_params(S, N, K, raw.shape[1], custom_levels=levels)
+    vis = np.full((N // 2, S * (S + 1) // 2), np.nan, np.complex64)
+    cg.fx_correlate(p, raw, vis)
+    i, j = np.tril_indices(S)
+    ref = (levels[code[i]] * levels[code[j]]).astype(np.float64) * K * N * N
+    assert ref.max() < 2.0 ** 24 * N * N                  # multiples of N^2: exact
+    assert np.array_equal(vis[0].real, ref) and not vis[0].imag.any()
+
+
+@pytest.mark.parametrize("S,N,K", SPLIT_FORMS)
+def test_fx_fp32_split_edges(cg, orc, S, N, K):
+    """The two-term forms at their own smallest sizes and partial blocks against FP64, the autos by themselves too."""
+    import synth
+
+    raw = synth.stations_offset_binary(S, (N * K + 63) // 64 * 64, rho=0.2, seed=S + N + 1)
+    vis = np.zeros((N // 2, S * (S + 1) // 2), np.complex64)
+    cg.fx_correlate(cg.fx_params(S, N, K, raw.shape[1]), raw, vis)
+    ref = _vis_f64(orc, raw, S, N, K)
+    # FP32 rounding of an N-point transform and of K-term sums: a few 2^-24, 2e-6 at most
+    assert _rel(vis, ref) < 2e-6
+    i, j = np.tril_indices(S)
+    assert _rel(vis[:, i == j], ref[:, i == j]) < 2e-6
+    assert not vis[:, i == j].imag.any()
