@@ -1544,12 +1544,21 @@ float cs_fstage_split_scale(const CsFStageArgs& a)
     if (a.format != CS_SPECTRA_F32 || a.msb_first) return 0.f;
     const char* gen = getenv("CELLSPE_FSTAGE_GENERIC");
     if (gen && gen[0] == '1') return 0.f;
-    float m = 0.f;
+    float m = 0.f, least = INFINITY;                 // largest and smallest non-zero |level|
+    bool zero = false;
     for (float l : a.lut) {
         if (!std::isfinite(l)) return 0.f;
         m = std::max(m, std::fabs(l));
+        if (l != 0.f) least = std::min(least, std::fabs(l));
+        else zero = true;
     }
     if (!(m > 1e-15f && m < 1e15f)) return 0.f;
+    // The lo term ends at FP16's subnormal step: half of it is 2^-25, at most 2^-39 N m in
+    // the spectra's own units.  Data that never takes the large codes has spectra of rms
+    // least sqrt(N), or of least where most samples may be zero, and keeps FP32's 2^-24
+    // of that only while m is not too far above it (m / least up to 181 at 32768
+    // points, 724 at 2048; the 2-bit tables have 3.3).
+    if ((zero ? (double)a.N : std::sqrt((double)a.N)) * (double)m > 32768.0 * (double)least) return 0.f;
     return std::ldexp(1.f, (int)std::floor(std::log2(32768.0 / ((double)a.N * m))));
 }
 

@@ -366,3 +366,20 @@ def test_fx_fp32_split_edges(cg, orc, S, N, K):
     i, j = np.tril_indices(S)
     assert _rel(vis[:, i == j], ref[:, i == j]) < 2e-6
     assert not vis[:, i == j].imag.any()
+
+
+@pytest.mark.parametrize("S,N,K,levels", [
+    (20, 2048, 70, (-1e6, -1, 1, 1e6)), (70, 512, 80, (-1e4, -1, 1, 1e4)), (12, 4096, 64, (-1, 1e-5, -1e-5, 1)),
+    (20, 1024, 64, (-1e5, 0, 1, 1e5))])
+def test_fx_fp32_levels_rarely_taken(cg, orc, S, N, K, levels):
+    """Custom levels of which the data never takes the large ones: FP32 spectra do not depend on those."""
+    rng = np.random.default_rng(N)
+    codes = rng.integers(1, 3, (S, (N * K + 63) // 64 * 64)).astype(np.uint8).reshape(S, -1, 4)
+    raw = np.ascontiguousarray(codes[..., 0] | codes[..., 1] << 2 | codes[..., 2] << 4 | codes[..., 3] << 6)
+    levels = np.array(levels, np.float32)
+    vis = np.zeros((N // 2, S * (S + 1) // 2), np.complex64)
+    cg.fx_correlate(cg.fx_params(S, N, K, raw.shape[1], custom_levels=levels), raw, vis)
+    ref = _vis_f64(orc, raw, S, N, K, lut=levels)
+    # FP32 rounding of an N-point transform and of K-term sums: a few 2^-24, 2e-6 at most
+    # (channel 0 holds the mean of levels that have one: it does not hide the others)
+    assert _rel(vis[1:], ref[1:]) < 2e-6
