@@ -161,6 +161,73 @@ struct CopyChain {
     bool valid = false;
 };
 
+// Error records of the workspaces' tensor-core kernels: a pair (F stage, X stage)
+// in device memory and the pair of page-locked words it reaches the host through.
+// They come from one pool, in blocks of 256 pairs (10 KB) that stay for the next
+// workspace: freeing a few bytes with each (cudaFree) would wait for the whole
+// device.  The calls that make a block belong to no capture, so the mode in which
+// another thread's capture refuses cudaMalloc is set aside for them.
+struct ErrorPair {
+    CsErrorWord* dev = nullptr;
+    volatile unsigned* host = nullptr;
+};
+class ErrorPool {
+public:
+    cudaError_t take(cudaStream_t stream, ErrorPair* out)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (free_.empty())
+            if (cudaError_t e = grow(stream)) return e;
+        *out = free_.back();
+        free_.pop_back();
+        return cudaSuccess;
+    }
+    // `stream` has no work that uses the pair
+    void give(cudaStream_t stream, ErrorPair p)
+    {
+        cudaMemset2DAsync(p.dev, sizeof(CsErrorWord), 0, sizeof(unsigned), 2, stream);
+        cudaStreamSynchronize(stream);
+        p.host[0] = p.host[1] = 0;
+        std::lock_guard<std::mutex> lk(mu_);
+        free_.push_back(p);
+    }
+
+private:
+    static constexpr int BLOCK = 256;
+    cudaError_t grow(cudaStream_t stream)
+    {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void *d = nullptr, *h = nullptr, *hd = nullptr;
+        cudaError_t e = cudaHostAlloc(&h, BLOCK * 2 * sizeof(unsigned), cudaHostAllocMapped);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&hd, h, 0);
+        if (e == cudaSuccess) e = cudaMalloc(&d, BLOCK * 2 * sizeof(CsErrorWord));
+        if (e == cudaSuccess) {
+            std::memset(h, 0, BLOCK * 2 * sizeof(unsigned));
+            std::vector<CsErrorWord> w(BLOCK * 2);
+            for (int i = 0; i < BLOCK * 2; i++) w[i] = {0, 0, static_cast<unsigned*>(hd) + i};
+            e = cudaMemcpyAsync(d, w.data(), w.size() * sizeof(CsErrorWord), cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        }
+        if (e == cudaSuccess) {
+            for (int i = 0; i < BLOCK; i++) free_.push_back({static_cast<CsErrorWord*>(d) + 2 * i, static_cast<unsigned*>(h) + 2 * i});
+        } else {
+            if (d) cudaFree(d);
+            if (h) cudaFreeHost(h);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return e;
+    }
+    std::mutex mu_;
+    std::vector<ErrorPair> free_;
+};
+// never destroyed: a thread's workspace may go after static objects do
+ErrorPool& error_pool()
+{
+    static ErrorPool* pool = new ErrorPool;
+    return *pool;
+}
+
 struct Workspace {
     CopyChain* chain = nullptr;       // set by the service for its workers
     cudaStream_t stream = nullptr;
@@ -171,10 +238,7 @@ struct Workspace {
     cudaEvent_t ev_legacy = nullptr;  // ordering after the legacy default stream
     Arena arena;
     bool own_stream = true;
-    // error records of the job's tensor-core kernels, F stage and X stage, in
-    // device memory, and the page-locked words they reach the host through
-    CsErrorWord* d_err = nullptr;
-    volatile unsigned* h_err = nullptr;
+    ErrorPair errors;                 // of the job's tensor-core kernels
     bool err_async = false;           // asynchronous jobs were issued since the words were last known clear
     struct Out { void* host; const void* dev; size_t bytes; };
     std::vector<Out> outs;
@@ -192,27 +256,13 @@ struct Workspace {
         for (auto& ev : cev)
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_legacy, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = init_errors();
+        if (e == cudaSuccess) e = error_pool().take(stream, &errors);
         if (e == cudaSuccess) return 0;
         destroy();
         return cuda_fail(e, "stream setup");
     }
-    cudaError_t init_errors()
-    {
-        void *d = nullptr, *h = nullptr, *hd = nullptr;
-        cudaError_t e = cudaHostAlloc(&h, 2 * sizeof(unsigned), cudaHostAllocMapped);
-        if (e != cudaSuccess) return e;
-        h_err = static_cast<unsigned*>(h);
-        h_err[0] = h_err[1] = 0;
-        e = cudaMalloc(&d, 2 * sizeof(CsErrorWord));
-        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&hd, h, 0);
-        d_err = static_cast<CsErrorWord*>(d);
-        const CsErrorWord w[2] = {{0, 0, static_cast<unsigned*>(hd)}, {0, 0, static_cast<unsigned*>(hd) + 1}};
-        if (e == cudaSuccess) e = cudaMemcpy(d, w, sizeof w, cudaMemcpyHostToDevice);
-        return e;
-    }
-    unsigned* f_err() const { return &d_err[0].code; }
-    unsigned* x_err() const { return &d_err[1].code; }
+    unsigned* f_err() const { return &errors.dev[0].code; }
+    unsigned* x_err() const { return &errors.dev[1].code; }
     // Before a job: the words become this job's own.  An asynchronous job is
     // queued, or replayed from a graph, when nobody can tell what an earlier
     // one will have left, so its reset runs on its own stream and is captured
@@ -220,15 +270,15 @@ struct Workspace {
     // the last error's page-locked words still stand.
     void clear_errors(bool sync)
     {
-        if (sync && !err_async && !h_err[0] && !h_err[1]) return;
-        cudaMemset2DAsync(d_err, sizeof(CsErrorWord), 0, sizeof(unsigned), 2, stream);
-        if (sync) h_err[0] = h_err[1] = 0;
+        if (sync && !err_async && !errors.host[0] && !errors.host[1]) return;
+        cudaMemset2DAsync(errors.dev, sizeof(CsErrorWord), 0, sizeof(unsigned), 2, stream);
+        if (sync) errors.host[0] = errors.host[1] = 0;
         err_async = !sync;
     }
     // After a job's stream has synchronised: the error of its tensor-core kernels, cleared.
     int check_errors(const std::string& who)
     {
-        const unsigned f = h_err[0], x = h_err[1];
+        const unsigned f = errors.host[0], x = errors.host[1];
         if (!f && !x) return 0;
         clear_errors(true);
         return set_err(CELLSPE_ERR_CUDA, who + (f ? "F stage" : "X stage") + ": tensor-core pipeline wait timed out (code " +
@@ -259,8 +309,7 @@ struct Workspace {
             if (ev) cudaEventDestroy(ev), ev = nullptr;
         for (auto& ev : cev)
             if (ev) cudaEventDestroy(ev), ev = nullptr;
-        if (d_err) cudaFree(d_err), d_err = nullptr;
-        if (h_err) cudaFreeHost(const_cast<unsigned*>(h_err)), h_err = nullptr;
+        if (errors.dev) error_pool().give(stream, errors), errors = {};
         if (copy) cudaStreamSynchronize(copy), cudaStreamDestroy(copy), copy = nullptr;
         if (stream && own_stream) cudaStreamDestroy(stream);
         stream = nullptr;

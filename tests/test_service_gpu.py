@@ -212,3 +212,42 @@ def test_service_concurrent_small_and_large_x_tiles(cg):
     assert st["failed"] == 0 and st["completed"] == 24
     for a, b in zip(outs[2:], outs):
         assert torch.equal(a, b)
+
+
+def test_service_set_up_and_release_do_not_wait_for_the_device(cg):
+    """Workers' workspaces are made and given back while a kernel of about two
+    seconds runs on another stream."""
+    import time
+
+    import torch
+
+    import synth
+
+    S, N, K = 4, 512, 32
+    raw = synth.stations_offset_binary(S, N * K, rho=0.1, seed=3)
+    p = cg.fx_params(S, N, K, raw.shape[1])
+    ref = np.zeros((N // 2, S * (S + 1) // 2), np.complex64)
+    cg.fx_correlate(p, raw, ref)
+
+    def once():
+        vis = np.zeros_like(ref)
+        t0 = time.perf_counter()
+        svc = cg.Service(max_streams=2)
+        try:
+            svc.wait(svc.submit(p, raw, vis))
+        finally:
+            svc.close()
+        t = time.perf_counter() - t0
+        assert np.array_equal(vis, ref)
+        return t
+
+    once()
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(4_000_000_000)
+        done = torch.cuda.Event()
+        done.record()
+    t = once()
+    assert not done.query(), f"set-up and release took {t:.2f} s"
+    torch.cuda.synchronize()
