@@ -233,7 +233,11 @@ struct Workspace {
     cudaStream_t stream = nullptr;
     cudaStream_t copy = nullptr;      // host <-> device copies overlapping the kernels
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t sev[5] = {};          // stage boundaries of the last FX job
+    // stage boundaries of FX jobs: a job records set `sev_next`, and when it has
+    // succeeded the next one takes the other, so that one that fails half-way
+    // leaves the last good job's events as they are
+    cudaEvent_t sev[2][5] = {};
+    int sev_next = 0;
     cudaEvent_t cev[PIPE_IN + PIPE_OUT + 2] = {};   // copy / compute hand-offs
     cudaEvent_t ev_legacy = nullptr;  // ordering after the legacy default stream
     Arena arena;
@@ -251,8 +255,9 @@ struct Workspace {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&copy, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&ev0);
         if (e == cudaSuccess) e = cudaEventCreate(&ev1);
-        for (auto& ev : sev)
-            if (e == cudaSuccess) e = cudaEventCreate(&ev);
+        for (auto& set : sev)
+            for (auto& ev : set)
+                if (e == cudaSuccess) e = cudaEventCreate(&ev);
         for (auto& ev : cev)
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_legacy, cudaEventDisableTiming);
@@ -305,8 +310,9 @@ struct Workspace {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (ev_legacy) cudaEventDestroy(ev_legacy);
-        for (auto& ev : sev)
-            if (ev) cudaEventDestroy(ev), ev = nullptr;
+        for (auto& set : sev)
+            for (auto& ev : set)
+                if (ev) cudaEventDestroy(ev), ev = nullptr;
         for (auto& ev : cev)
             if (ev) cudaEventDestroy(ev), ev = nullptr;
         if (errors.dev) error_pool().give(stream, errors), errors = {};
@@ -318,18 +324,19 @@ struct Workspace {
 };
 
 thread_local std::unique_ptr<Workspace> t_ws;
-// Stage times of the thread's last blocking FX job (delay model, F stage, X
-// stage, output), read from the events of its workspace when they are asked for.
+// Stage times of the thread's last successful blocking FX job (delay model, F
+// stage, X stage, output).  A job on the thread's own workspace has them read from
+// its events when they are asked for; on others, which may be gone by then, at once.
 thread_local float t_stage_ms[4] = {0, 0, 0, 0};
-thread_local Workspace* t_stage_ws = nullptr;      // set while the events have not been read
+thread_local const cudaEvent_t* t_stage_events = nullptr;      // of t_ws, while they have not been read
 void read_stage_times()
 {
-    if (!t_stage_ws) return;
+    if (!t_stage_events) return;
     for (int i = 0; i < 4; i++) {
         float ms = 0.f;
-        t_stage_ms[i] = cudaEventElapsedTime(&ms, t_stage_ws->sev[i], t_stage_ws->sev[i + 1]) == cudaSuccess ? ms : -1.f;
+        t_stage_ms[i] = cudaEventElapsedTime(&ms, t_stage_events[i], t_stage_events[i + 1]) == cudaSuccess ? ms : -1.f;
     }
-    t_stage_ws = nullptr;
+    t_stage_events = nullptr;
 }
 
 Workspace* thread_ws(int* rc)
@@ -648,7 +655,8 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         }
     }
     ws.clear_errors(sync);
-    if (sync) cudaEventRecord(ws.sev[0], ws.stream);
+    const cudaEvent_t* sev = ws.sev[ws.sev_next];
+    if (sync) cudaEventRecord(sev[0], ws.stream);
     CsFStageArgs fa{};
     fa.err = ws.f_err();
     fa.raw = d_raw;
@@ -693,7 +701,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     // FP16, N = 2048: 128-byte runs per 32 segments, k-blocked (1) or
     // channel-grouped k-blocked (2, the warp-specialised F stage)
     fa.kblock = cs_fstage_layout(fa);
-    if (sync) cudaEventRecord(ws.sev[1], ws.stream);
+    if (sync) cudaEventRecord(sev[1], ws.stream);
     // bytes of one spectra element: F32 rows [C][S][kp] of float2, F16 rows [C][2][S][kp] of half
     const long long el_bytes = fa.format == CS_SPECTRA_F32 ? 8 : 2;
     // 4096-point and longer transforms stage at most 4 segments per CTA, so
@@ -746,7 +754,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             if (rc) j.err = rc;
         }
     }
-    if (sync) cudaEventRecord(ws.sev[2], ws.stream);
+    if (sync) cudaEventRecord(sev[2], ws.stream);
     // X stage into a channel-major buffer
     const bool direct = !host && p->vis_order == CELLSPE_VIS_CHANNEL_MAJOR && !p->accumulate;
     float2* vis_cp = direct ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
@@ -794,7 +802,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         cudaEventRecord(ws.cev[PIPE_IN + PIPE_OUT + 1], ws.copy);
         cudaStreamWaitEvent(ws.stream, ws.cev[PIPE_IN + PIPE_OUT + 1], 0);
     }
-    if (sync) cudaEventRecord(ws.sev[3], ws.stream);
+    if (sync) cudaEventRecord(sev[3], ws.stream);
     if (!direct && !stream_out && !j.err) {
         float2* result = vis_cp;
         if (p->vis_order == CELLSPE_VIS_BASELINE_MAJOR) {
@@ -818,12 +826,16 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
             }
         }
     }
-    if (sync) cudaEventRecord(ws.sev[4], ws.stream);
+    if (sync) cudaEventRecord(sev[4], ws.stream);
     // after a failure the copy stream may still hold copies into the workspace
     if (nsc > 1 && j.err) cudaStreamSynchronize(ws.copy);
     int rc = j.finish(sync);
     if (sync && !rc) rc = ws.check_errors("");
-    if (sync && !rc) t_stage_ws = &ws;
+    if (sync && !rc) {
+        t_stage_events = sev;
+        ws.sev_next ^= 1;
+        if (&ws != t_ws.get()) read_stage_times();
+    }
     return rc;
 }
 

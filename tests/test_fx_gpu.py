@@ -383,3 +383,33 @@ def test_fx_fp32_levels_rarely_taken(cg, orc, S, N, K, levels):
     # FP32 rounding of an N-point transform and of K-term sums: a few 2^-24, 2e-6 at most
     # (channel 0 holds the mean of levels that have one: it does not hide the others)
     assert _rel(vis[1:], ref[1:]) < 2e-6
+
+
+def test_stage_times_are_the_last_good_jobs(cg):
+    """A job that fails after its F stage (the FP16 X stage takes K in multiples of 8) leaves the times of the one before."""
+    import torch
+
+    import synth
+
+    S, N, K = 8, 512, 512
+    raw = synth.device_stations(S, N * K, 0.1, seed=1)
+    vis = torch.zeros((N // 2, S * (S + 1) // 2), dtype=torch.complex64, device="cuda")
+    good = cg.fx_params(S, N, K, raw.shape[1], x_mode=cg.X_TC_FP16)
+    bad = cg.fx_params(S, N, 7, raw.shape[1], x_mode=cg.X_TC_FP16)
+
+    def fail():
+        with pytest.raises(cg.CellspeError):
+            cg.fx_correlate(bad, raw, vis)
+
+    cg.fx_correlate(good, raw, vis)                  # first use: kernels are loaded
+    cg.fx_correlate(good, raw, vis)
+    before = cg.stage_times()
+    assert min(before) >= 0 and before[1] > 0
+    fail()
+    assert cg.stage_times() == before                # read before the failing job
+    cg.fx_correlate(good, raw, vis)
+    cg.fx_correlate(good, raw, vis)
+    fail()
+    fail()
+    t = cg.stage_times()                             # and read only after it
+    assert min(t) >= 0 and t[1] > 0.5 * before[1] and t[2] > 0.5 * before[2]
