@@ -2526,10 +2526,10 @@ cellspe_service* cellspe_service_create(const cellspe_service_config* cfg)
     int n = (cfg && cfg->max_streams > 0) ? cfg->max_streams : 2;
     sv->priority_samples = !cfg || cfg->priority_samples == 0 ? (1LL << 24) : cfg->priority_samples;
     sv->large_samples = cfg ? cfg->large_samples : 0;
-    // batching is on by default (64 inputs); a negative batch_inputs turns it off
-    // (the X stage's forms for more than 64 inputs add in another order than those a
-    // small job runs alone, and a batched job's values are to equal its solo run's)
-    sv->batch_inputs = !cfg || cfg->batch_inputs == 0 ? 64 : std::max(0, std::min(cfg->batch_inputs, 64));
+    // batching is on by default (64 inputs); a negative batch_inputs turns it off.
+    // Up to 128 inputs, one tile of the X stage: its forms up to there (segment-major,
+    // Gram, tile) add in the same order, so a batched job's values equal its solo run's.
+    sv->batch_inputs = !cfg || cfg->batch_inputs == 0 ? 64 : std::max(0, std::min(cfg->batch_inputs, 128));
     for (int i = 0; i < n; i++) sv->workers.emplace_back(service_worker, sv);
     return sv;
 }

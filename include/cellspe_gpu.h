@@ -199,7 +199,7 @@ typedef struct cellspe_service cellspe_service;
 typedef struct {
     long long hbm_budget_bytes;   /* 0: 80% of free device memory            */
     int       max_streams;        /* concurrent jobs (0: 2)                    */
-    int       batch_inputs;       /* small jobs batched up to this many inputs (<= 64); 0: 64; < 0: off */
+    int       batch_inputs;       /* small jobs batched up to this many inputs (<= 128); 0: 64; < 0: off */
     long long priority_samples;   /* 0: 2^24; < 0: one priority for all jobs */
     long long large_samples;      /* <= 0: no limit (large jobs may overlap)  */
 } cellspe_service_config;

@@ -251,3 +251,38 @@ def test_service_set_up_and_release_do_not_wait_for_the_device(cg):
     t = once()
     assert not done.query(), f"set-up and release took {t:.2f} s"
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("N,K", [(512, 64), (512, 72), (2048, 64), (8192, 24)])
+def test_service_batches_of_more_than_64_inputs(cg, N, K):
+    """batch_inputs = 128: twelve jobs of ten inputs that queue behind a large one
+    run in one batch (of 120 inputs, the X stage's tile), each equal to its solo run."""
+    import torch
+
+    import synth
+
+    S, n = 10, 12
+    raws = [synth.device_stations(S, N * K, 0.1, seed=400 + i) for i in range(n)]
+    solo = []
+    for raw in raws:
+        solo.append(torch.empty((N // 2, S * (S + 1) // 2), dtype=torch.complex64, device="cuda"))
+        cg.fx_correlate(cg.fx_params(S, N, K, raw.shape[1], x_mode=cg.X_TC_FP16), raw, solo[-1])
+    big_raw = synth.device_stations(200, 2048 * 2048, 0.02, seed=399)
+    big = torch.empty((1024, 200 * 201 // 2), dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    svc = cg.Service(max_streams=1, batch_inputs=128)
+    try:
+        ids = [svc.submit(cg.fx_params(200, 2048, 2048, big_raw.shape[1], x_mode=cg.X_TC_FP16), big_raw, big) for _ in range(8)]
+        outs = []
+        for raw, v in zip(raws, solo):
+            outs.append(torch.full_like(v, float("nan")))
+            ids.append(svc.submit(cg.fx_params(S, N, K, raw.shape[1], x_mode=cg.X_TC_FP16), raw, outs[-1]))
+        for i in ids:
+            svc.wait(i)
+        st = svc.stats()
+    finally:
+        svc.close()
+    torch.cuda.synchronize()
+    for a, b in zip(outs, solo):
+        assert torch.equal(a.view(torch.float32), b.view(torch.float32))
+    assert st["failed"] == 0 and st["batched_launches"] == 1 and st["batched_jobs"] == n
