@@ -806,8 +806,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     if (!direct && !stream_out && !j.err) {
         float2* result = vis_cp;
         if (p->vis_order == CELLSPE_VIS_BASELINE_MAJOR) {
-            // straight into the caller's device buffer where nothing is added to it
-            float2* t = !host && !p->accumulate ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
+            // straight into the caller's device buffer where nothing is added to it and
+            // 8-byte stores can go there
+            const bool in_place = !host && !p->accumulate && (uintptr_t)vis % sizeof(float2) == 0;
+            float2* t = in_place ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
             if (!j.err) {
                 int rc = map_rc(cs_vis_to_baseline_major(vis_cp, t, C, P, ws.stream), "transpose");
                 if (rc) j.err = rc;
@@ -823,6 +825,9 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
                 }
             } else if (host) {
                 ws.outs.push_back({vis, result, (size_t)C * P * 8});
+            } else if (result != vis) {
+                cudaError_t e = cudaMemcpyAsync(vis, result, (size_t)C * P * 8, cudaMemcpyDeviceToDevice, ws.stream);
+                if (e != cudaSuccess) j.err = cuda_fail(e, "result copy");
             }
         }
     }

@@ -1,4 +1,6 @@
 """Full FX path (K-a + K-b + K-c + K-d1) vs the oracle: FP32 CPU path and FP64 model."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -413,3 +415,21 @@ def test_stage_times_are_the_last_good_jobs(cg):
     fail()
     t = cg.stage_times()                             # and read only after it
     assert min(t) >= 0 and t[1] > 0.5 * before[1] and t[2] > 0.5 * before[2]
+
+
+def test_fx_baseline_major_into_any_address(cg):
+    """Baseline-major visibilities into a device buffer that is no multiple of 8 bytes: by a copy."""
+    import torch
+
+    import synth
+
+    S, N, K = 5, 512, 64
+    raw = synth.device_stations(S, N * K, 0.1, seed=2)
+    n = S * (S + 1) // 2 * (N // 2)
+    p = cg.fx_params(S, N, K, raw.shape[1], vis_order=cg.VIS_BASELINE_MAJOR, memory=cg.MEM_DEVICE)
+    ref = torch.zeros(2 * n, device="cuda")
+    buf = torch.zeros(2 * n + 2, device="cuda")
+    torch.cuda.synchronize()
+    for dst in (ref, buf[1:]):
+        assert cg.lib().cellspe_fx_correlate(ctypes.byref(p), raw.data_ptr(), None, dst.data_ptr()) == 0
+    assert torch.equal(buf[1:-1], ref) and ref.any() and buf[0] == 0 and buf[-1] == 0
