@@ -228,6 +228,7 @@ def lib() -> ctypes.CDLL:
             "cellspe_memcpy": ([V, V, ctypes.c_size_t, I], I),
             "cellspe_debug_inject_failure": ([I, I], I),
             "cellspe_debug_wait_timeout": ([I, I, V], I),
+            "cellspe_debug_workspace_taken": ([], LL),
             "cellspe_kernel_launches": ([], LL),
             "cellspe_last_stage_times": ([ctypes.POINTER(ctypes.c_float), I], I),
             "cellspe_unpack2bit": ([V, LL, I, I, V, V, I], I),

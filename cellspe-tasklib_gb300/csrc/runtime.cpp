@@ -91,6 +91,7 @@ struct Arena {
     std::vector<std::pair<char*, size_t>> blocks;
     size_t used = 0;
     size_t total_taken = 0;
+    size_t last_taken = 0;            // by the job before
     cudaStream_t stream = nullptr;    // the stream the blocks are ordered on
     size_t capacity() const
     {
@@ -134,6 +135,7 @@ struct Arena {
     // a CUDA graph is being captured)
     void rewind()
     {
+        if (total_taken) last_taken = total_taken;
         used = 0;
         total_taken = 0;
     }
@@ -565,34 +567,69 @@ int op_xmac_i8(Workspace& ws, bool host, const void* planes, const float* scale,
 // for the X stage's TMA loads and costs at most 25% memory at K = 256 (1.6%
 // at K = 4096).
 long long spectra_pitch(long long K) { return K >= 256 ? K + 64 : K; }
-// FP32 jobs of 64 segments and more (whose X stage may take its spectra as two
-// FP16 terms in 32-segment blocks) round it up to whole blocks.
-long long spectra_pitch(long long K, int x_mode)
+// What an FX job takes and where it puts it, for its admission and its run alike.
+struct FxPlan {
+    bool host;                  // buffers in host memory
+    bool segmaj;                // spectra written segment-major: transforms of 4096 points and more, which stage
+                                // at most 4 segments per CTA
+    bool seg_x;                 // and read so by the X stage (small arrays); others are transposed in 64 x 64 tiles
+    bool direct;                // the X stage writes the caller's buffer
+    bool in_place;              // the baseline-major transpose does
+    float split;                // FP32: scale of the two FP16 terms, 0 for FP32 rows
+    int kp;                     // row pitch of the spectra in segments
+    long long el_bytes;         // of a complex spectrum value
+};
+
+FxPlan fx_plan(const cellspe_fx_params* p, const void* vis)
 {
-    const long long kp = spectra_pitch(K);
-    return x_mode == CELLSPE_X_FP32 && K >= CS_SPLIT_MIN_K ? (kp + 31) / 32 * 32 : kp;
+    FxPlan f{};
+    const int S = p->n_inputs, N = p->fft_points, K = p->n_segments;
+    f.host = p->memory == CELLSPE_MEM_HOST;
+    f.segmaj = N >= 4096;
+    f.el_bytes = p->x_mode == CELLSPE_X_TC_FP16 ? 4 : 8;     // FP32 spectra for the FP32 and INT8 X stages
+    // FP32 X stage: on the tensor cores from spectra as two FP16 terms, except
+    // for arrays of a few inputs (cs_xmac_f32 reads each row once there: 2 inputs
+    // x 512 channels x 4096 segments 9 us) and for integrations so short that the
+    // CUDA cores' serial sums are the more accurate ones
+    // (an estimate may be asked for a job whose parameters have not been checked)
+    if (p->x_mode == CELLSPE_X_FP32 && S >= CS_SPLIT_MIN_S && K >= CS_SPLIT_MIN_K && N >= 512 && N <= 32768) {
+        CsFStageArgs fa{};
+        fa.N = N;
+        fa.format = CS_SPECTRA_F32;
+        fa.msb_first = (p->levels & CELLSPE_UNPACK_MSB_FIRST) ? 1 : 0;
+        if (pick_levels(p->levels, p->custom_levels, fa.lut)) f.split = cs_fstage_split_scale(fa);
+    }
+    f.seg_x = f.segmaj && (p->x_mode == CELLSPE_X_TC_FP16 || f.split > 0.f) && cs_xmac_seg_supported(S);
+    f.kp = (int)spectra_pitch(K);
+    if (f.split > 0.f) f.kp = (f.kp + 31) / 32 * 32;         // the terms lie in 32-segment blocks
+    const bool add = p->accumulate != 0;
+    f.direct = !f.host && p->vis_order == CELLSPE_VIS_CHANNEL_MAJOR && !add;
+    // nothing is added, and 8-byte stores can go there
+    f.in_place = !f.host && p->vis_order == CELLSPE_VIS_BASELINE_MAJOR && !add && (uintptr_t)vis % sizeof(float2) == 0;
+    return f;
 }
 
 // CsFStageArgs::squares of a job
 long long squares_blocks(int N, int K) { return (K + cs_squares_segs(N) - 1) / cs_squares_segs(N); }
 long long squares_bytes(int S, int N, int K) { return squares_blocks(N, K) * S * (N / 2) * 4; }
 
-long long fx_bytes(const cellspe_fx_params* p, bool with_poly)
+// Device bytes that op_fx takes for the job.
+long long fx_bytes(const cellspe_fx_params* p, bool with_poly, const void* vis)
 {
-    long long S = p->n_inputs, N = p->fft_points, K = p->n_segments, C = N / 2;
-    long long P = S * (S + 1) / 2;
-    bool host = p->memory == CELLSPE_MEM_HOST;
+    const FxPlan f = fx_plan(p, vis);
+    const long long S = p->n_inputs, N = p->fft_points, K = p->n_segments, C = N / 2, P = S * (S + 1) / 2;
+    const long long vis_bytes = align256(C * P * 8);
     long long b = 0;
-    if (host) b += align256(S * p->bytes_per_input);
-    if (with_poly) b += align256(S * 32) + 3 * align256(S * K * 4);
-    const bool f32 = p->x_mode != CELLSPE_X_TC_FP16;   // FP32 spectra (FP32 and INT8 X stages)
-    b += align256(C * S * spectra_pitch(K, p->x_mode) * (f32 ? 8 : 4));
-    if (N >= 4096) b += align256(C * S * K * (f32 ? 8 : 4));   // segment-major spectra
-    if (p->x_mode == CELLSPE_X_FP32 && S >= CS_SPLIT_MIN_S && K >= CS_SPLIT_MIN_K) b += align256(squares_bytes(p->n_inputs, p->fft_points, p->n_segments));
-    if (p->x_mode == CELLSPE_X_INT8) b += align256(C * 2 * S * spectra_pitch(K)) + align256(S * C * 4);
-    bool stage_vis = host || p->vis_order == CELLSPE_VIS_BASELINE_MAJOR || p->accumulate;
-    if (stage_vis) b += 3 * align256(C * P * 8);
-    if (p->x_mode == CELLSPE_X_TC_FP16) b += 2 * align256(S * C * 4);
+    if (f.host) b += align256(S * p->bytes_per_input);
+    if (with_poly) b += (f.host ? align256(S * 32) : 0) + 3 * align256(S * K * 4);
+    if (p->x_mode == CELLSPE_X_TC_FP16 && p->channel_scale) b += (f.host ? 2 : 1) * align256(S * C * 4);
+    if (f.segmaj) b += align256(S * K * C * f.el_bytes);
+    if (!f.seg_x) b += align256(C * S * f.kp * f.el_bytes);
+    if (f.split > 0.f && !f.seg_x) b += align256(squares_bytes(p->n_inputs, p->fft_points, p->n_segments));
+    if (p->x_mode == CELLSPE_X_INT8) b += align256(C * 2 * S * f.kp) + align256(S * C * 4);
+    if (!f.direct) b += vis_bytes;
+    if (p->vis_order == CELLSPE_VIS_BASELINE_MAJOR && !f.in_place) b += vis_bytes;
+    if (p->accumulate && f.host) b += vis_bytes;
     return b;
 }
 
@@ -613,12 +650,13 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     if (poly && !(p->sample_rate_hz > 0)) return set_err(CELLSPE_ERR_ARG, "fx: delay model needs sample_rate_hz");
     float lut[4];
     if (!pick_levels(p->levels, p->custom_levels, lut)) return set_err(CELLSPE_ERR_ARG, "fx: unknown level table");
-    long long need = fx_bytes(p, poly != nullptr);
+    long long need = fx_bytes(p, poly != nullptr, vis);
     long long budget = 0;
     if (over_limit(ws, need, &budget))
         return set_err(CELLSPE_ERR_NOMEM, "fx: job needs " + std::to_string(need) + " device bytes, budget " +
                                               std::to_string(budget));
-    const bool host = p->memory == CELLSPE_MEM_HOST;
+    const FxPlan plan = fx_plan(p, vis);
+    const bool host = plan.host;
     const long long P = (long long)S * (S + 1) / 2;
     const long long bpi = p->bytes_per_input;
     // Host buffers of large jobs move in chunks on the copy stream: input
@@ -690,13 +728,9 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         }
         d_inv_scale = inv;
     }
-    const int kp = (int)spectra_pitch(K, p->x_mode);
+    const int kp = plan.kp;
     fa.kp = kp;
-    // FP32 X stage: on the tensor cores from spectra as two FP16 terms, except
-    // for arrays of a few inputs (cs_xmac_f32 reads each row once there: 2 inputs
-    // x 512 channels x 4096 segments 9 us) and for integrations so short that the
-    // CUDA cores' serial sums are the more accurate ones
-    if (p->x_mode == CELLSPE_X_FP32 && S >= CS_SPLIT_MIN_S && K >= CS_SPLIT_MIN_K) fa.split = cs_fstage_split_scale(fa);
+    fa.split = plan.split;
     fa.split_lo = cs_xmac_split_lo(S);
     // FP16, N = 2048: 128-byte runs per 32 segments, k-blocked (1) or
     // channel-grouped k-blocked (2, the warp-specialised F stage)
@@ -704,14 +738,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     if (sync) cudaEventRecord(sev[1], ws.stream);
     // bytes of one spectra element: F32 rows [C][S][kp] of float2, F16 rows [C][2][S][kp] of half
     const long long el_bytes = fa.format == CS_SPECTRA_F32 ? 8 : 2;
-    // 4096-point and longer transforms stage at most 4 segments per CTA, so
-    // their spectra are written segment-major and transposed in 64 x 64 tiles
-    const bool segmaj = N >= 4096;
-    const long long seg_bytes = fa.format == CS_SPECTRA_F32 ? 8 : 4;       // one channel of one segment
-    // small arrays: the X stage reads the segment-major spectra itself
-    const bool seg_x = segmaj && (fa.format == CS_SPECTRA_F16 || fa.split > 0.f) && cs_xmac_seg_supported(S);
+    const bool segmaj = plan.segmaj, seg_x = plan.seg_x;
+    const long long seg_bytes = plan.el_bytes;             // one channel of one segment
     char* seg_tmp = segmaj ? (char*)j.scratch((size_t)((long long)S * K * C * seg_bytes)) : nullptr;
-    fa.out = seg_x ? seg_tmp : j.scratch((size_t)C * S * kp * (fa.format == CS_SPECTRA_F32 ? 8 : 4));
+    fa.out = seg_x ? seg_tmp : j.scratch((size_t)C * S * kp * plan.el_bytes);
     if (fa.split > 0.f && !seg_x) fa.squares = (float*)j.scratch((size_t)squares_bytes(S, N, K));
     for (int i = 0; i < nsc && !j.err; i++) {
         CsFStageArgs fb = fa;
@@ -756,8 +786,7 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
     }
     if (sync) cudaEventRecord(sev[2], ws.stream);
     // X stage into a channel-major buffer
-    const bool direct = !host && p->vis_order == CELLSPE_VIS_CHANNEL_MAJOR && !p->accumulate;
-    float2* vis_cp = direct ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
+    float2* vis_cp = plan.direct ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
     for (int b = 0; b < ncb && !j.err; b++) {
         // streamed output: a small first block (1/16 of the channels) starts the
         // copy out early; the rest in equal blocks
@@ -803,13 +832,10 @@ int op_fx(Workspace& ws, const cellspe_fx_params* p, const void* raw, const doub
         cudaStreamWaitEvent(ws.stream, ws.cev[PIPE_IN + PIPE_OUT + 1], 0);
     }
     if (sync) cudaEventRecord(sev[3], ws.stream);
-    if (!direct && !stream_out && !j.err) {
+    if (!plan.direct && !stream_out && !j.err) {
         float2* result = vis_cp;
         if (p->vis_order == CELLSPE_VIS_BASELINE_MAJOR) {
-            // straight into the caller's device buffer where nothing is added to it and
-            // 8-byte stores can go there
-            const bool in_place = !host && !p->accumulate && (uintptr_t)vis % sizeof(float2) == 0;
-            float2* t = in_place ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
+            float2* t = plan.in_place ? (float2*)vis : (float2*)j.scratch((size_t)C * P * 8);
             if (!j.err) {
                 int rc = map_rc(cs_vis_to_baseline_major(vis_cp, t, C, P, ws.stream), "transpose");
                 if (rc) j.err = rc;
@@ -2476,7 +2502,7 @@ int cellspe_fx_correlate(const cellspe_fx_params* p, const void* raw, const doub
     return op_fx(*ws, p, raw, delay_poly, vis, true);
 }
 
-long long cellspe_fx_workspace_bytes(const cellspe_fx_params* p) { return p ? fx_bytes(p, true) : -1; }
+long long cellspe_fx_workspace_bytes(const cellspe_fx_params* p) { return p ? fx_bytes(p, true, nullptr) : -1; }
 
 int cellspe_fx_correlate_async(const cellspe_fx_params* p, const void* raw, const double* delay_poly, void* vis,
                                void* stream)
@@ -2490,6 +2516,8 @@ int cellspe_fx_correlate_async(const cellspe_fx_params* p, const void* raw, cons
     ws->stream = saved;
     return rc;
 }
+
+long long cellspe_debug_workspace_taken(void) { return t_ws ? (long long)t_ws->arena.last_taken : 0; }
 
 int cellspe_debug_wait_timeout(int stage, int async, void* stream)
 {
@@ -2548,7 +2576,7 @@ int cellspe_service_submit(cellspe_service* sv, const cellspe_fx_params* p, cons
     j->raw = raw;
     j->poly = delay_poly;
     j->vis = vis;
-    j->footprint = fx_bytes(p, delay_poly != nullptr);
+    j->footprint = fx_bytes(p, delay_poly != nullptr, vis);
     j->large = sv->large_samples > 0 && (long long)p->n_inputs * p->fft_points * p->n_segments >= sv->large_samples;
     if (j->footprint > sv->budget)
         return set_err(CELLSPE_ERR_NOMEM, "service_submit: job footprint exceeds the service HBM budget");

@@ -69,6 +69,8 @@ int  cellspe_memcpy(void* dst, const void* src, size_t bytes, int kind); /* 1 H2
 /* Fault injection for tests: the next `count` tasks or calls on `slot`
  * (-1 = direct calls) fail with CELLSPE_ERR_INJECTED before touching the GPU. */
 int  cellspe_debug_inject_failure(int slot, int count);
+/* For tests: bytes of device scratch that the calling thread's last blocking job took. */
+long long cellspe_debug_workspace_taken(void);
 /* For tests: a kernel whose one wait, on a barrier that nothing arrives at, gives
  * up after about a millisecond and is recorded as an error of the calling thread's
  * F stage (0) or X stage (1).  async = 0: waits for it and returns the error as a

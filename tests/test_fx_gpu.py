@@ -433,3 +433,39 @@ def test_fx_baseline_major_into_any_address(cg):
     for dst in (ref, buf[1:]):
         assert cg.lib().cellspe_fx_correlate(ctypes.byref(p), raw.data_ptr(), None, dst.data_ptr()) == 0
     assert torch.equal(buf[1:-1], ref) and ref.any() and buf[0] == 0 and buf[-1] == 0
+
+
+@pytest.mark.parametrize("S,N,K", [(4, 512, 64), (8, 1024, 100), (24, 2048, 96), (24, 4096, 32), (32, 8192, 64), (33, 4096, 64),
+                                   (40, 8192, 24)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_fx_workspace_estimate_is_what_a_job_takes(cg, mode, S, N, K):
+    """cellspe_fx_workspace_bytes (which counts a delay model) against the scratch
+    that jobs took: host and device buffers, both orders, accumulation, delays, scale."""
+    import torch
+
+    if mode == cg.X_INT8 and K % 16:
+        pytest.skip("the INT8 X stage takes segments in multiples of 16")
+    if mode == cg.X_TC_FP16 and K % 8:
+        K -= K % 8
+    C, P, margin = N // 2, S * (S + 1) // 2, 4096
+    a256 = lambda n: (n + 255) // 256 * 256
+    raw = torch.randint(0, 256, (S, (N * K + 2 * margin) // 4), dtype=torch.uint8)
+    poly = np.zeros((S, 4))
+    poly[:, 0] = np.linspace(-20e-6, 20e-6, S)
+    scale = np.ones((S, C), np.float32) if mode == cg.X_TC_FP16 else None
+    for dev in (False, True):
+        x = raw.cuda() if dev else raw.numpy()
+        for order in (cg.VIS_CHANNEL_MAJOR, cg.VIS_BASELINE_MAJOR):
+            for acc, delays, sc in ((False, False, None), (True, False, None), (False, True, None), (False, False, scale)):
+                shape = (P, C) if order == cg.VIS_BASELINE_MAJOR else (C, P)
+                vis = torch.zeros(shape, dtype=torch.complex64, device="cuda") if dev else np.zeros(shape, np.complex64)
+                if sc is not None and dev:
+                    sc = torch.from_numpy(sc).cuda()
+                p = cg.fx_params(S, N, K, raw.shape[1], x_mode=mode, vis_order=order, start_sample=margin, fs_hz=32e6,
+                                 accumulate=acc, memory=cg.MEM_DEVICE if dev else cg.MEM_HOST, channel_scale=sc)
+                pl = (torch.from_numpy(poly).cuda() if dev else poly) if delays else None
+                cg.fx_correlate(p, x, vis, delay_poly=pl)
+                need = cg.lib().cellspe_fx_workspace_bytes(ctypes.byref(p))
+                if not delays:
+                    need -= 3 * a256(S * K * 4) + (0 if dev else a256(S * 32))
+                assert cg.lib().cellspe_debug_workspace_taken() == need, (dev, order, acc, delays, sc is not None)
