@@ -1212,15 +1212,10 @@ int vdif_spec_mbps(const cellspe_spec_params* p)
     return (r > 0 && r < INT32_MAX && std::fabs(mbps - (double)r) < 1e-6) ? (int)r : 0;
 }
 
-long long spec_bytes(const cellspe_spec_params* p, int ffts_per_chunk = 0)
+// Scratch of spec_planes.
+long long spec_input_bytes(const cellspe_spec_params* p)
 {
-    CsSpecArgs a{};
-    a.ffts_per_chunk = ffts_per_chunk;
-    a.nsub = p->n_subbands; a.N = p->fft_points; a.overlap = p->overlap;
-    a.ffts_per_spectrum = p->ffts_per_spectrum; a.nspec = p->n_spectra; a.tonebins = p->pcal_tonebins;
-    long long b = align256(cs_spectrometer_scratch_floats(a) * 4);
-    bool host = p->memory == CELLSPE_MEM_HOST;
-    if (host) b += align256(p->raw_bytes);
+    long long b = p->memory == CELLSPE_MEM_HOST ? align256(p->raw_bytes) : 0;
     if (p->input_layout == CELLSPE_SPEC_INTERLEAVED && p->n_subbands > 1) b += align256(p->raw_bytes);
     if (p->input_layout == CELLSPE_SPEC_MARK5B_FRAMED) {
         const long long g = m5b_groups(p->raw_bytes, std::max(p->n_subbands, 4));
@@ -1231,8 +1226,25 @@ long long spec_bytes(const cellspe_spec_params* p, int ffts_per_chunk = 0)
         b += align256(g * 4 * p->n_subbands) + align256((g + 1) / 2 * 4) +
              align256(p->raw_bytes / VDIF_SPEC_MIN_FRAME * 8) + 512;
     }
+    return b;
+}
+
+// Scratch of cs_spectrometer; phase_cal_only: of one subband without power spectra.
+long long spec_scratch_bytes(const cellspe_spec_params* p, int ffts_per_chunk, bool phase_cal_only)
+{
+    CsSpecArgs a{};
+    a.ffts_per_chunk = ffts_per_chunk;
+    a.nsub = phase_cal_only ? 1 : p->n_subbands; a.N = p->fft_points; a.overlap = p->overlap;
+    a.ffts_per_spectrum = p->ffts_per_spectrum; a.nspec = p->n_spectra; a.tonebins = p->pcal_tonebins;
+    a.skip_power = phase_cal_only;
+    return align256(cs_spectrometer_scratch_floats(a) * 4);
+}
+
+long long spec_bytes(const cellspe_spec_params* p, int ffts_per_chunk = 0)
+{
+    long long b = spec_input_bytes(p) + spec_scratch_bytes(p, ffts_per_chunk, false);
     long long rows = (long long)p->n_subbands * p->n_spectra;
-    if (host) b += align256(rows * (p->fft_points / 2 + 1) * 4) + 2 * align256(rows * std::max(p->pcal_tonebins, p->pcal_ntones) * 8);
+    if (p->memory == CELLSPE_MEM_HOST) b += align256(rows * (p->fft_points / 2 + 1) * 4) + 2 * align256(rows * std::max(p->pcal_tonebins, p->pcal_ntones) * 8);
     return b;
 }
 
@@ -1395,13 +1407,12 @@ int op_spectrometer(Workspace& ws, const cellspe_spec_params* p, const void* raw
 // windows of one source and the spectra of both.
 long long spec_xpol_bytes(const cellspe_spec_params* p)
 {
-    const long long N = p->fft_points, nb = N / 2 + 1;
-    const long long nwin = (long long)p->n_spectra * (p->overlap * p->ffts_per_spectrum - (p->overlap - 1));
-    cellspe_spec_params one = *p;
-    one.n_subbands = p->n_subbands;
-    long long b = 2 * spec_bytes(&one, CS_SPEC_CHUNK);
-    b += align256(nwin * N * 4) + 2 * align256(nwin * nb * 8);
-    b += align256(3LL * p->n_spectra * nb * 8);
+    const long long N = p->fft_points, nb = N / 2 + 1, nspec = p->n_spectra, tones = p->pcal_tonebins;
+    const long long nwin = nspec * (p->overlap * p->ffts_per_spectrum - (p->overlap - 1));
+    long long b = 2 * spec_input_bytes(p) + align256(nwin * N * 4) + 2 * align256(nwin * nb * 8);
+    if (tones > 0) b += 2 * spec_scratch_bytes(p, 0, true);
+    if (p->memory == CELLSPE_MEM_HOST)
+        b += align256(2 * nspec * nb * 4) + align256(nspec * nb * 8) + (tones > 0 ? align256(2 * nspec * tones * 8) : 0);
     return b;
 }
 

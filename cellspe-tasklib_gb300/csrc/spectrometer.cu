@@ -1216,6 +1216,7 @@ const float* cs_window_table(int type, int n) { return window_table(type, n); }
 // odd, and the phase-cal partials are float2) the phase-cal partials.
 int64_t power_partial_floats(const CsSpecArgs& a)
 {
+    if (a.skip_power) return 0;
     const int64_t power = (int64_t)a.nsub * a.nspec * spec_nchunk(a) * (a.N / 2 + 1);
     return (power + 63) / 64 * 64;
 }

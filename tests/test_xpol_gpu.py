@@ -84,3 +84,35 @@ def test_xpol_rejects(cg):
     p = cg.spec_params(65536, 2, 2, 1, 1, 1, 65536 // 4)
     with pytest.raises(cg.CellspeError):
         cg.spectrometer_xpol(p, r, r, 0, 0, np.zeros((2, 1, 32769), np.float32), np.zeros((1, 32769), np.complex64))
+
+
+@pytest.mark.parametrize("nsub,N,overlap,K,nspec,tb", [(1, 4096, 2, 128, 1, 32), (1, 16384, 2, 32, 2, 32), (4, 2048, 2, 64, 1, 32),
+                                                       (1, 1024, 1, 64, 3, 0)])
+@pytest.mark.parametrize("dev", [False, True])
+def test_xpol_stays_within_its_budget(cg, dev, nsub, N, overlap, K, nspec, tb):
+    """The admission of a cross-polarisation job counts what it takes: an explicit
+    budget of that lets it run, one of 256 bytes less refuses it."""
+    import torch
+
+    T = N * K * nspec
+    recs = [np.random.default_rng(i).integers(0, 256, T * nsub // 4).astype(np.uint8) for i in range(2)]
+    out = [torch.zeros((2, nspec, N // 2 + 1)), torch.zeros((nspec, N // 2 + 1), dtype=torch.complex64),
+           torch.zeros((2, nspec, tb), dtype=torch.complex64) if tb else None]
+    if dev:
+        recs = [torch.from_numpy(r).cuda() for r in recs]
+        out = [o if o is None else o.cuda() for o in out]
+    else:
+        out = [o if o is None else o.numpy() for o in out]
+    p = cg.spec_params(N, overlap, 2, K, nspec, nsub, T * nsub // 4, tonebins=tb, rotatorlen=tb, fs_hz=32e6)
+    cg.spectrometer_xpol(p, recs[0], recs[1], 0, nsub - 1, *out)
+    taken = cg.lib().cellspe_debug_workspace_taken()
+    try:
+        cg.lib().cellspe_set_hbm_budget(taken)
+        cg.spectrometer_xpol(p, recs[0], recs[1], 0, nsub - 1, *out)
+        assert cg.lib().cellspe_debug_workspace_taken() == taken
+        cg.lib().cellspe_set_hbm_budget(taken - 256)
+        with pytest.raises(cg.CellspeError) as e:
+            cg.spectrometer_xpol(p, recs[0], recs[1], 0, nsub - 1, *out)
+        assert e.value.code == cg.ERR_NOMEM
+    finally:
+        cg.lib().cellspe_set_hbm_budget(0)
