@@ -94,17 +94,35 @@ CS_DEV float2 w64c(int m)
     return q ? make_float2(z.y, -z.x) : z;
 }
 
+// v * W8: an eighth turn with cos(pi/4) as two FP32 terms.  The rounded constant alone
+// is 1.7e-8 short in every one of them.
+CS_DEV float2 rot45(float2 v)
+{
+    constexpr float c = 0.70710678118654757f, lo = 1.21016178e-8f;
+    return make_float2(fmaf(v.x, c, fmaf(v.y, c, lo * (v.x + v.y))), fmaf(v.y, c, fmaf(-v.x, c, lo * (v.y - v.x))));
+}
+
 // v * W32^e with the exact quarter turns kept exact (e folds to a constant
-// inside unrolled codelets, so the switch disappears).
-CS_DEV float2 rot32(float2 v, int e)
+// inside unrolled codelets, so the switch disappears); FINE: eighth turns by rot45.
+template <bool FINE = false> CS_DEV float2 rot32(float2 v, int e)
 {
     switch (e & 31) {
         case 0: return v;
         case 8: return make_float2(v.y, -v.x);
         case 16: return make_float2(-v.x, -v.y);
         case 24: return make_float2(-v.y, v.x);
-        default: return cmul(v, w32(e));
+        default: break;
     }
+    if (FINE && (e & 3) == 0) {
+        const float2 r = rot45(v);
+        switch ((e >> 3) & 3) {
+            case 0: return r;
+            case 1: return make_float2(r.y, -r.x);
+            case 2: return make_float2(-r.x, -r.y);
+            default: return make_float2(-r.y, r.x);
+        }
+    }
+    return cmul(v, w32(e));
 }
 
 template <bool PK> CS_DEV void dft2(float2& a, float2& b)
@@ -114,16 +132,17 @@ template <bool PK> CS_DEV void dft2(float2& a, float2& b)
     b = csub<PK>(t, b);
 }
 
-// In-place forward DFT of R points in natural order; PK: packed sums (above).
-template <int R, bool PK = true> struct Dft;
+// In-place forward DFT of R points in natural order; PK: packed sums (above),
+// FINE: eighth turns by rot45.
+template <int R, bool PK = true, bool FINE = false> struct Dft;
 
-template <bool PK> struct Dft<1, PK> {
+template <bool PK, bool FINE> struct Dft<1, PK, FINE> {
     static CS_DEV void run(float2*) {}
 };
-template <bool PK> struct Dft<2, PK> {
+template <bool PK, bool FINE> struct Dft<2, PK, FINE> {
     static CS_DEV void run(float2* a) { dft2<PK>(a[0], a[1]); }
 };
-template <bool PK> struct Dft<4, PK> {
+template <bool PK, bool FINE> struct Dft<4, PK, FINE> {
     static CS_DEV void run(float2* a)
     {
         float2 t0 = cadd<PK>(a[0], a[2]), t1 = csub<PK>(a[0], a[2]);
@@ -135,7 +154,7 @@ template <bool PK> struct Dft<4, PK> {
     }
 };
 // R = R1*R2 split: n = R2*n1 + n2, k = k1 + R1*k2.
-template <int R1, int R2, bool PK> struct DftSplit {
+template <int R1, int R2, bool PK, bool FINE> struct DftSplit {
     static CS_DEV void run(float2* a)
     {
         constexpr int R = R1 * R2;
@@ -144,29 +163,29 @@ template <int R1, int R2, bool PK> struct DftSplit {
         for (int n2 = 0; n2 < R2; n2++) {
 #pragma unroll
             for (int n1 = 0; n1 < R1; n1++) b[n2][n1] = a[R2 * n1 + n2];
-            Dft<R1, PK>::run(b[n2]);
+            Dft<R1, PK, FINE>::run(b[n2]);
 #pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) b[n2][k1] = rot32(b[n2][k1], (n2 * k1) * (32 / R));
+            for (int k1 = 0; k1 < R1; k1++) b[n2][k1] = rot32<FINE>(b[n2][k1], (n2 * k1) * (32 / R));
         }
 #pragma unroll
         for (int k1 = 0; k1 < R1; k1++) {
             float2 c[R2];
 #pragma unroll
             for (int n2 = 0; n2 < R2; n2++) c[n2] = b[n2][k1];
-            Dft<R2, PK>::run(c);
+            Dft<R2, PK, FINE>::run(c);
 #pragma unroll
             for (int k2 = 0; k2 < R2; k2++) a[k1 + R1 * k2] = c[k2];
         }
     }
 };
-template <bool PK> struct Dft<8, PK> {
-    static CS_DEV void run(float2* a) { DftSplit<2, 4, PK>::run(a); }
+template <bool PK, bool FINE> struct Dft<8, PK, FINE> {
+    static CS_DEV void run(float2* a) { DftSplit<2, 4, PK, FINE>::run(a); }
 };
-template <bool PK> struct Dft<16, PK> {
-    static CS_DEV void run(float2* a) { DftSplit<4, 4, PK>::run(a); }
+template <bool PK, bool FINE> struct Dft<16, PK, FINE> {
+    static CS_DEV void run(float2* a) { DftSplit<4, 4, PK, FINE>::run(a); }
 };
-template <bool PK> struct Dft<32, PK> {
-    static CS_DEV void run(float2* a) { DftSplit<4, 8, PK>::run(a); }
+template <bool PK, bool FINE> struct Dft<32, PK, FINE> {
+    static CS_DEV void run(float2* a) { DftSplit<4, 8, PK, FINE>::run(a); }
 };
 
 // Padded shared-memory index: one spare float2 after every 16 elements keeps

@@ -188,23 +188,25 @@ int launch_batch(const void* in, float2* out, int64_t batch, float scale, cudaSt
 // shared-memory transpose, nothing else shared between warps.  Bound by the copy:
 // 65536 real transforms of 2048 points take 181 us a call (1.07 GB, 158 us at the
 // copy rate); the shared-memory radix-16 passes, three of them with CTA barriers,
-// took 346.  2^27 floats as complex transforms of 512 and 1024 points 503 -> 362 and
+// took 346.  Eighth turns take cos(pi/4) as two terms and the split's twiddles come
+// from a table (products of rounded ones cost as much): the error against FP64 is then
+// no larger than those passes' (2048 real points 1.18e-7; 1.25e-7 without either).  2^27 floats as complex transforms of 512 and 1024 points 503 -> 362 and
 // 632 -> 361 us, real ones of 1024 points 282 -> 185.
 constexpr int FW_NT = 256;
 template <int L, int R, bool REAL, bool INV>
 __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict__ in, float2* __restrict__ out, int64_t batch,
                                                        const float2* __restrict__ tw, float scale)
 {
-    using W = WarpFft<L, R, false>;     // bound by the copy, and by registers: no packed sums
+    using W = WarpFft<L, R, false, true>;     // bound by the copy, and by registers: no packed sums
     constexpr int M = W::M, GROUPS = FW_NT / L;
     extern __shared__ __align__(16) unsigned char smem[];
     float2* tab = reinterpret_cast<float2*>(smem);
     const int g = threadIdx.x / L, lane = threadIdx.x % L;
-    float2* tile = tab + W::TWIDDLES + g * W::TILE;
+    float2* half = tab + W::TWIDDLES;                        // REAL: W_N^k / 2, k < M/2
+    float2* tile = half + (REAL ? M / 2 : 0) + g * W::TILE;
     W::fill(tab, tw, 2);
-    float2 wh[W::CPL];
-#pragma unroll
-    for (int c = 0; c < W::CPL; c++) wh[c] = cscale(__ldg(tw + lane + L * c), 0.5f);
+    if constexpr (REAL)
+        for (int k = threadIdx.x; k < M / 2; k += FW_NT) half[k] = cscale(__ldg(tw + k), 0.5f);
     __syncthreads();
     // whole rounds, so that every lane of a warp takes part in its shuffles
     for (int64_t b0 = (int64_t)blockIdx.x * GROUPS; b0 < batch; b0 += (int64_t)gridDim.x * GROUPS) {
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict_
         if constexpr (REAL) {
             float2* o = out + b * (M + 1);
             W::split(
-                v, lane, wh,
+                v, lane, [&](int c, int k2) { return half[lane + L * c + R * k2]; },
                 [&](int, int k, float2 X1, float2 X2) {
                     if (!valid) return;
                     if (k == 0) X1.y = X2.y = 0.f;           // DC and Nyquist
@@ -248,10 +250,10 @@ __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict_
 template <int L, int R, bool REAL, bool INV>
 int launch_warp(const void* in, float2* out, int64_t batch, float scale, cudaStream_t st)
 {
-    using W = WarpFft<L, R, false>;     // bound by the copy, and by registers: no packed sums
+    using W = WarpFft<L, R, false, true>;
     const float2* tw = cs_twiddles(2 * W::M);
     if (!tw) return CS_ERR_ARG;
-    const size_t smem = (size_t)(W::TWIDDLES + FW_NT / L * W::TILE) * sizeof(float2);
+    const size_t smem = (size_t)(W::TWIDDLES + (REAL ? W::M / 2 : 0) + FW_NT / L * W::TILE) * sizeof(float2);
     auto kern = k_fft_warp<L, R, REAL, INV>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));
     const int64_t blocks = (batch + FW_NT / L - 1) / (FW_NT / L);

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(SP_NT, 2) k_spec_power_s(const __grid_constant
         W::run(v, tile, lane, tab);
         const bool valid = j < j_end;
         W::split(
-            v, lane, wh,
+            v, lane, [&](int c, int k2) { return W::rot_half(wh[c], k2); },
             [&](int i, int, float2 X1, float2 X2) {
                 if (!valid) return;
                 acc[2 * i] += X1.x * X1.x + X1.y * X1.y;

@@ -103,3 +103,22 @@ def test_fft_lane_groups(cg, n, batch):
     cg.vis_lags(z, lags, 0.5)
     ref = torch.fft.ifft(z.to(torch.complex128)) * (0.5 * n)
     assert float((lags - ref).norm() / ref.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("real,n,limit", [(True, 128, 9.262e-8), (True, 256, 9.927e-8), (True, 512, 1.065e-7), (True, 1024, 1.133e-7),
+                                          (True, 2048, 1.183e-7), (False, 512, 1.030e-7), (False, 1024, 1.083e-7)])
+def test_register_transforms_error(cg, real, n, limit):
+    """Batched transforms in the registers of a warp against FP64: an error no larger
+    than that of the radix-16 passes through shared memory (measured on Gaussian input,
+    the same to 0.1 % from seed to seed)."""
+    import torch
+
+    b = (1 << 23) // n
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((b, n), generator=g, device="cuda", dtype=torch.float32 if real else torch.complex64)
+    out = torch.empty((b, n // 2 + 1 if real else n), dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    (cg.fft_r2c if real else cg.fft_c2c)(x, out, n, b)
+    ref = torch.fft.rfft(x.double()) if real else torch.fft.fft(x.to(torch.complex128))
+    d = torch.linalg.norm(torch.view_as_real(out.to(torch.complex128) - ref)) / torch.linalg.norm(torch.view_as_real(ref))
+    assert float(d) < 1.005 * limit
