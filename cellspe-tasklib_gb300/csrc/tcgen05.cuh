@@ -134,6 +134,31 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
         : "memory");
 }
 
+// The same into TMEM lanes 0 .. lanes-1 only: the others keep their values, whatever
+// the operand's rows there hold.
+struct LaneMask {
+    uint32_t off[4];
+};
+__device__ __forceinline__ LaneMask first_lanes(int lanes)
+{
+    LaneMask m;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        const int n = lanes - 32 * w;
+        m.off[w] = n <= 0 ? 0xffffffffu : n >= 32 ? 0u : 0xffffffffu << n;
+    }
+    return m;
+}
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc, const LaneMask& m)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+        ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(m.off[0]), "r"(m.off[1]), "r"(m.off[2]), "r"(m.off[3])
+        : "memory");
+}
+
 __device__ __forceinline__ void commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)

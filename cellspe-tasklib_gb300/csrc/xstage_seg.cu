@@ -10,9 +10,9 @@
 // segment of a chunk (32 KB), and each of eight warps' threads turns eight
 // segments of its channels into 16-byte pieces of the swizzled operand rows, up
 // to three chunks behind the copies.  The spectra are read once and nothing is
-// written.  The arithmetic is k_xmac_tc_gram's (FP16: rows Xr, Xi and zeros, Re V
-// and M in one accumulator) and k_xmac_gram's (FP32).  Bound by the read of the
-// spectra, in FP16 also by the MMAs' least cost: those 32 inputs take 474 us in
+// written.  The arithmetic is k_xmac_tc_gram's (FP16: rows Xr and Xi, Re V and M in
+// one accumulator) and k_xmac_gram's (FP32).  Bound by the read of the
+// spectra, in FP16 also by the MMAs' least cost: those 32 inputs take 480 us in
 // FP16 (2.15 GB, 318 us at the copy rate; 512 CTAs are 3.4 waves) and 830 us in
 // FP32, with the transpose 1040 and 2300.  (Register loads instead of TMA: 614 and
 // 1285 us, cp.async 1030 and 1700, both with a single MMA per 16 segments; the F
@@ -110,9 +110,9 @@ template <int RI> struct F16Cfg {
     static constexpr int CB = 8, SEGS = RI == 16 ? 64 : 32, ROWB = 2 * SEGS, KG = SEGS / 8;
     using R = Raw<RI, SEGS>;
     static constexpr int COLS = CB * RI;
-    static constexpr uint32_t TILE = 3 * RI * ROWB, STAGE = CB * TILE;      // 48 KB
-    static constexpr int STAGES = 2, DEPTH = 3;
-    static constexpr uint32_t SLACK = (BM - 2 * RI) * ROWB;                 // operand rows an MMA reads past the ring
+    static constexpr uint32_t TILE = 2 * RI * ROWB, STAGE = CB * TILE;      // 32 KB
+    static constexpr int STAGES = 3, DEPTH = 3;
+    static constexpr uint32_t SLACK = (BM - RI) * ROWB;                     // operand rows an MMA reads past the ring
     static_assert(RI * KG * 2 == LOADERS, "one task per loader");
 };
 
@@ -143,11 +143,6 @@ __global__ void __launch_bounds__(LOADERS + 96, 1)
         tc::mbar_init(accb, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // the zero rows of every tile
-    constexpr uint32_t ZB = RI * F::ROWB;
-    for (uint32_t i = tid; i < F::STAGES * F::CB * ZB / 16; i += LOADERS + 96)
-        *reinterpret_cast<uint4*>(ring + i / (ZB / 16) * F::TILE + 2 * ZB + i % (ZB / 16) * 16) = make_uint4(0, 0, 0, 0);
-    tc::fence_proxy_async();
     if (warp == LOADERS / 32) tc::tmem_alloc(tc::smem_u32(slot), F::COLS);
     tc::fence_before();
     __syncthreads();
@@ -164,6 +159,7 @@ __global__ void __launch_bounds__(LOADERS + 96, 1)
         if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, RI, false, false, false);
             const uint64_t d0 = tc::smem_desc(tc::smem_u32(ring), 16, 8 * F::ROWB, F::ROWB == 128 ? tc::SW128 : tc::SW64);
+            const tc::LaneMask re_lanes = tc::first_lanes(RI);
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % F::STAGES;
                 if (!tc::mbar_wait(full0 + 8 * s, (kc / F::STAGES) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) break;
@@ -175,7 +171,7 @@ __global__ void __launch_bounds__(LOADERS + 96, 1)
 #pragma unroll
                     for (int kk = 0; kk < F::SEGS / 16; kk++) {
                         tc::mma_f16(tmem + c * RI, d + 2 * kk, d + 2 * kk, id, (kc | kk) ? 1u : 0u);
-                        tc::mma_f16(tmem + c * RI, di + 2 * kk, di + 2 * kk, id, 1u);
+                        tc::mma_f16(tmem + c * RI, di + 2 * kk, di + 2 * kk, id, 1u, re_lanes);
                     }
                 }
                 tc::commit(empty0 + 8 * s);

@@ -535,11 +535,12 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_xmac_tc_pair(const __grid_cons
 
 // ---------------------------------------------------------------------------
 // S <= 64: every product of a channel from a few MMAs per 16 segments.
-//   Planes: a stage holds Xr, Xi and zeros, RI rows each (S rounded up to 8).
-//     [Xr; Xi] Xr^T and [Xi; 0] Xi^T go into one accumulator, whose upper rows
-//     are then Re V, added in the order of the tiles below (Re, Im, Re, ... : the
-//     accumulator truncates, so another order would move every auto by parts in
-//     10^5 at thousands of segments), and whose lower rows are M = Xi Xr^T.
+//   Planes: a stage holds Xr and Xi, RI rows each (S rounded up to 8).
+//     [Xr; Xi] Xr^T and, in its upper RI lanes alone, Xi Xi^T go into one accumulator,
+//     whose upper rows are then Re V, added in the order of the tiles below (Re, Im,
+//     Re, ... : the accumulator truncates, so another order would move every auto by
+//     parts in 10^5 at thousands of segments), and whose lower rows are M = Xi Xr^T.
+//     (Rows of zeros under Xi in place of the lane mask make NaN of an infinite Xi.)
 //   k-blocked (BLK): an operand row holds a block's 32 Re and 32 Im halves; Re V
 //     takes two MMAs, M one.
 // Im V = M - M^T is put together at the end through shared memory.  One TMA copy
@@ -554,9 +555,10 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_xmac_tc_pair(const __grid_cons
 // E = COLS / 32 epilogue warps, the TMA producer, the MMA issuer and TMEM owner.
 // ---------------------------------------------------------------------------
 constexpr int G_ROW = 128;                          // operand row bytes
-// Planes take two stages, which leave room for the most CTAs on an SM: 64 inputs, 8192
-// channels of 200 segments 206 us with four stages, 139 with two; 48 inputs 168 and 102.
-template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : 2; }
+// Planes take three stages, and two up to 512 segments, where more CTAs on an SM are
+// worth more: 64 inputs, 1024 channels of 4088 segments 220 us with two, 204 with three;
+// 2048 channels of 200 segments 43 and 49.
+template <int COLS, bool BLK> constexpr int gram_stages() { return BLK ? (COLS == 128 ? 6 : 8) : 3; }
 
 template <int COLS, bool BLK>
 __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constant__ CUtensorMap tmap,
@@ -568,7 +570,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x, S = a.S, RI = a.box_rows, nk = (a.K + SEGS - 1) / SEGS;
-    const uint32_t plane = (uint32_t)RI * G_ROW, stage_bytes = BLK ? plane : 3 * plane;
+    const uint32_t plane = (uint32_t)RI * G_ROW, stage_bytes = BLK ? plane : 2 * plane;
     // columns of an accumulator (BLK: Re V and M side by side)
     const uint32_t n = (uint32_t)((S + 15) & ~15);
     // barriers in front, so that the ring and the rows past it end the buffer
@@ -585,11 +587,6 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
         tc::mbar_init(accb, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
-    }
-    if constexpr (!BLK) {
-        for (uint32_t i = threadIdx.x; i < ST * plane / 16; i += COLS + 64)
-            *reinterpret_cast<uint4*>(ring + i / (plane / 16) * stage_bytes + 2 * plane + i % (plane / 16) * 16) = make_uint4(0, 0, 0, 0);
-        tc::fence_proxy_async();
     }
     if (warp == E + 1) tc::tmem_alloc(smem_u32(tmem_slot), COLS);
     tc::fence_before();
@@ -616,6 +613,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
         if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, n, false, false, false);
             const uint64_t d0 = sw128_desc(sbase);
+            const tc::LaneMask re_lanes = tc::first_lanes(RI);
             for (int kc = 0; kc < nk; kc++) {
                 const int s = kc % ST;
                 if (!tc::mbar_wait(full0 + 8 * s, (kc / ST) & 1, a.err, ERR_FULL_WAIT, WAIT_CYCLES)) break;
@@ -636,7 +634,7 @@ __global__ void __launch_bounds__(COLS + 64) k_xmac_tc_gram(const __grid_constan
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
                         tc::mma_f16(tmem, d + 2 * kk, d + 2 * kk, id, kk ? 1u : acc);
-                        tc::mma_f16(tmem, di + 2 * kk, di + 2 * kk, id, 1u);
+                        tc::mma_f16(tmem, di + 2 * kk, di + 2 * kk, id, 1u, re_lanes);
                     }
                 }
                 tc::commit(empty0 + 8 * s);
@@ -699,13 +697,13 @@ template <int COLS, bool BLK>
 int launch_gram(const CUtensorMap& tm, TcArgs a, cudaStream_t st)
 {
     const int chunks = (a.K + (BLK ? 32 : 64) - 1) / (BLK ? 32 : 64);
-    a.stages = std::min(chunks, gram_stages<COLS, BLK>());
+    a.stages = std::min(chunks, !BLK && chunks <= 8 ? 2 : gram_stages<COLS, BLK>());
     // the ring, the rows past it that an MMA of 128 rows reads (lanes never
     // stored), and after the last MMA the accumulators [rows][columns + 1]
     const size_t plane = (size_t)a.box_rows * G_ROW, rows = (BLK ? 1 : 2) * (size_t)a.box_rows;
     const size_t cols = (BLK ? 2 : 1) * (((size_t)a.S + 15) / 16 * 16);
     // an operand of 128 rows from the last stage's Xr (BLK) or Xi on
-    const size_t ring = a.stages * (BLK ? plane : 3 * plane) + BM * G_ROW - (BLK ? plane : 2 * plane);
+    const size_t ring = a.stages * (BLK ? plane : 2 * plane) + BM * G_ROW - plane;
     const size_t smem = 2048 + std::max(ring, rows * (cols + 1) * sizeof(float));
     auto kern = k_xmac_tc_gram<COLS, BLK>;
     CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(kern), (int)smem));

@@ -308,3 +308,24 @@ def test_fx_segment_major_sizes(cg, orc, S, N, K, mode):
     ref = np.matmul(X, X.conj().transpose(0, 2, 1))[:, i, j]
     # FP16 spectra: 2^-12 per value, less over K; FP32: a few 2^-24
     assert np.linalg.norm(vis - ref) / np.linalg.norm(ref) < (1e-3 if tc else 2e-6)
+
+
+@pytest.mark.parametrize("S,K", [(2, 8), (5, 64), (16, 72), (23, 128), (40, 64), (64, 136), (65, 64), (130, 64)])
+@pytest.mark.parametrize("part", [0, 1])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_xmac_f16_infinite_values(cg, S, K, part, value):
+    """One infinite (or NaN) Re or Im value of one input: what IEEE gives in its
+    products, finite values everywhere else."""
+    rng = np.random.default_rng(S + K)
+    C, s = 3, S // 2
+    x = rng.integers(1, 4, (C, 2, S, K)).astype(np.float16)
+    x[1, part, s, K // 2] = value
+    vis = np.zeros((C, S * (S + 1) // 2), np.complex64)
+    cg.xmac_f16(x, S, C, K, vis)
+    re, im = x[:, 0].astype(np.float64), x[:, 1].astype(np.float64)
+    i, j = np.tril_indices(S)
+    with np.errstate(invalid="ignore"):
+        rr = (re[:, i] * re[:, j] + im[:, i] * im[:, j]).sum(-1)
+        ri = (im[:, i] * re[:, j] - re[:, i] * im[:, j]).sum(-1)
+    assert np.array_equal(vis.real, rr.astype(np.float32), equal_nan=True)
+    assert np.array_equal(vis.imag, ri.astype(np.float32), equal_nan=True)
