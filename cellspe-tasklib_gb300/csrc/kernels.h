@@ -230,6 +230,7 @@ struct CsSpecArgs {
 // budget falls back to.
 constexpr int CS_SPEC_CHUNK = 32;
 int64_t cs_spectrometer_scratch_floats(const CsSpecArgs& a);
+int cs_spec_noalloc_chunk(const CsSpecArgs& a);             // ffts_per_chunk of the no-allocation entry point
 int64_t cs_spectrometer_pcal_floats(const CsSpecArgs& a);   // the phase-cal part of it
 int cs_spectrometer(const CsSpecArgs& a, cudaStream_t st);
 // Window function of TaskCoreIPP::generate_windowfunction, n floats (cached).

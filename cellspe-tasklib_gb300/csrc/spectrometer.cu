@@ -1078,11 +1078,15 @@ bool spec_cta_fft()
 // 220 us with 32, 95 with 4).  Not under 16 where a CTA's 16 or 8 groups
 // take one FFT each, nor under 4; not above 512, and 32 for N >= 4096, whose
 // partial spectra are the larger part of the scratch.
+int64_t spec_slots(const CsSpecArgs& a)              // CTAs (pairs for N = 65536) that run at once
+{
+    const int ctas = a.N <= 2048 ? 2 : a.N == 4096 ? 8 : a.N == 8192 ? 4 : a.N == 16384 ? 2 : 1;   // per SM
+    return (int64_t)152 * ctas / (a.N == 65536 ? 2 : 1);
+}
 int spec_chunk(const CsSpecArgs& a)
 {
     if (a.ffts_per_chunk > 0) return a.ffts_per_chunk;
-    const int ctas = a.N <= 2048 ? 2 : a.N == 4096 ? 8 : a.N == 8192 ? 4 : a.N == 16384 ? 2 : 1;   // per SM
-    const int64_t waves = (int64_t)152 * 3 * ctas / (a.N == 65536 ? 2 : 1);
+    const int64_t waves = 3 * spec_slots(a);
     const int64_t total = (int64_t)(a.overlap * (int64_t)a.ffts_per_spectrum - (a.overlap - 1)) * a.nsub * a.nspec;
     const int64_t ch = (total + waves - 1) / waves;
     if (a.N <= 2048) return (int)(std::min<int64_t>(512, std::max<int64_t>(16, ch) + 15) / 16 * 16);
@@ -1211,6 +1215,18 @@ int spec_nchunk(const CsSpecArgs& a)
 }  // namespace
 
 const float* cs_window_table(int type, int n) { return window_table(type, n); }
+
+// The no-allocation entry point's choice.  Its transforms of 4096 points and more run in
+// k_spec_power and k_spec_power_w, whose CTAs take the same time each: the whole job
+// in one wave where chunks of up to 32 allow it, as 3.4 waves of chunks of 9 cost more
+// (4 x 2044 FFTs of 16384 points 418 us, 390 in chunks of 32, 339 in one wave of 27).
+int cs_spec_noalloc_chunk(const CsSpecArgs& a)
+{
+    if (a.N < 4096) return 0;
+    const int64_t novl = a.overlap * (int64_t)a.ffts_per_spectrum - (a.overlap - 1);
+    const int64_t per_row = std::max<int64_t>(1, spec_slots(a) / ((int64_t)a.nsub * a.nspec));
+    return (int)std::min<int64_t>(SPEC_CH, std::max<int64_t>(4, (novl + per_row - 1) / per_row));
+}
 
 // Scratch layout: chunk partial spectra, then (256-byte aligned: N/2+1 is
 // odd, and the phase-cal partials are float2) the phase-cal partials.

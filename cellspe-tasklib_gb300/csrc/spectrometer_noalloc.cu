@@ -106,7 +106,7 @@ extern "C" int cellspe_spectrometer_noalloc(const cellspe_spec_params* p, const 
     if (!cs_pick_levels(p->levels, p->custom_levels, lut))
         return cs_set_error(CELLSPE_ERR_ARG, "spectrometer_noalloc: unknown level table");
 
-    // Chunking: the default number of FFTs per partial, grown until the
+    // Chunking: FFTs per partial for one wave of CTAs, grown until the
     // partials (plus phase-cal partials) fit the static scratch.
     CsSpecArgs a{};
     a.planes = (const uint8_t*)raw;
@@ -120,7 +120,7 @@ extern "C" int cellspe_spectrometer_noalloc(const cellspe_spec_params* p, const 
     a.pcal_bins = (float2*)pcal_bins;
     a.pcal_tones = (float2*)pcal_tones;
     const long long novl = (long long)p->overlap * p->ffts_per_spectrum - (p->overlap - 1);
-    a.ffts_per_chunk = 0;
+    a.ffts_per_chunk = cs_spec_noalloc_chunk(a);
     if ((size_t)cs_spectrometer_scratch_floats(a) > CS_NOALLOC_SCRATCH_FLOATS) {
         const long long rows = (long long)nsub * p->n_spectra, nb = N / 2 + 1;
         // phase-cal partials + 64 floats of alignment between the two parts
