@@ -601,13 +601,16 @@ def main():
     if x_ms >= f_ms:
         if x_mode == cg.X_FP32:
             pk = peaks["bf16_tflops"] / 3                   # hi hi', hi lo' and lo hi' for each FP32 product
-            roof = {"bound": "tensor", "kernel": "k_xmac_split", "achieved": stages["x_stage_tflops"],
+            roof = {"bound": "tensor", "kernel": "k_xmac_split" if S_run > 64 else "k_xmac_gram", "achieved": stages["x_stage_tflops"],
                     "peak": pk, "unit": "TFLOP/s", "frac": stages["x_stage_tflops"] / pk,
                     "peak_source": f"a third of the {peak_kind} dense bf16 (burst)",
                     "traffic": None}
         else:
             pk = peaks["bf16_tflops"]
-            roof = {"bound": "tensor", "kernel": "k_xmac_tc_pair" if K_run >= 1536 else "k_xmac_tc", "achieved": stages["x_stage_tflops"], "peak": pk,
+            # the X-stage kernel the library picks for this job (xstage_tc.cu's dispatch; N = 2048)
+            xk = ("k_xmac_tc_gram" if S_run <= 64 else "k_xmac_tc_pair" if S_run > 128 and K_run >= max(1536, 8 * S_run)
+                  else "k_xmac_tc")
+            roof = {"bound": "tensor", "kernel": xk, "achieved": stages["x_stage_tflops"], "peak": pk,
                     "unit": "TFLOP/s", "frac": stages["x_stage_tflops"] / pk,
                     "peak_source": f"{peak_kind} dense bf16 (burst)",
                     "traffic": X_TRAFFIC_PER_CHANNEL * C_run}

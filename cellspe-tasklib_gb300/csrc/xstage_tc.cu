@@ -345,9 +345,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_xmac_tc(const __grid_constant
 // producer, TMEM owner and issuer, epilogue): tiles of long integrations, where a
 // ring of three stages each and chunk boundaries that do not meet keep the MMAs
 // busier than one CTA does and the epilogue is a small part.  From where it is
-// faster: 200 inputs of 4096 segments 829 us against 897 (512 inputs 2.97 ms, 3.04),
-// 132 inputs of 960 428 against 402, 300 inputs of 2048 875 against 863.
-constexpr int PAIR_MIN_K = 1536;
+// faster, which moves up with the full tiles' share of the work (us, this form
+// and the persistent one): 1024 channels, 200 inputs 284 and 263 at 1024 segments,
+// 373 and 374 at 1536, 465 and 483 at 2048; 300 inputs 719 and 694 at 1536, 900 and 903
+// at 2048; 512 inputs 1709 and 1656 at 2048, of 256 channels 829 and 818 at 4096, 1569
+// and 1587 at 8192.
+constexpr int pair_min_k(int S) { return S > 192 ? 8 * S : 1536; }
 constexpr int P_STAGES = 3, P_THREADS = 192;
 constexpr size_t P_SMEM = 1024 + P_STAGES * STAGE_BYTES + 256;
 // epilogue shared memory: four warps' 32 x 17 float2 staging blocks, then (on
@@ -802,7 +805,7 @@ int cs_xmac_tc_f16(const void* spectra, int S, int C, int K, int kp, float2* vis
                    accumulate, S < BM ? (S + 7) / 8 * 8 : BM, S <= BM ? 1 : 0, kblock, err};
     CUtensorMap tm;
     if (!encode_map(enc, spectra, kp, BK, a, &tm)) return CS_ERR_ARG;
-    if (S > BM && K >= PAIR_MIN_K) {
+    if (S > BM && K >= pair_min_k(S)) {
         CS_CUDA_TRY(cs_smem_at_least(reinterpret_cast<const void*>(k_xmac_tc_pair), (int)P_SMEM));
         k_xmac_tc_pair<<<dim3((unsigned)ntiles, C), P_THREADS, P_SMEM, st>>>(tm, a), cs_count_launches(1);
         return (int)cudaGetLastError();

@@ -329,3 +329,10 @@ def test_xmac_f16_infinite_values(cg, S, K, part, value):
         ri = (im[:, i] * re[:, j] - re[:, i] * im[:, j]).sum(-1)
     assert np.array_equal(vis.real, rr.astype(np.float32), equal_nan=True)
     assert np.array_equal(vis.imag, ri.astype(np.float32), equal_nan=True)
+
+
+@pytest.mark.parametrize("S,C,K", [(129, 3, 1528), (129, 3, 1536), (192, 3, 1536), (193, 40, 1536), (193, 2, 1544), (257, 2, 2056),
+                                   (300, 1, 2392), (300, 1, 2400)])
+def test_xmac_f16_long_integrations(cg, S, C, K):
+    """Both sides of the line in K, which moves with S, from which every tile has a block of its own."""
+    test_xmac_f16_tile_rounds(cg, S, C, K)
