@@ -438,6 +438,19 @@ def run_reference(args):
     print(json.dumps(line))
 
 
+def _link_gbs(torch, pinned):
+    """GB/s of one plain copy of a pinned host tensor to the device and one back."""
+    dev = torch.empty(pinned.shape, dtype=pinned.dtype, device="cuda")
+    out = []
+    for dst, src in ((dev, pinned), (pinned, dev)):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        dst.copy_(src, non_blocking=True)
+        torch.cuda.synchronize()
+        out.append(pinned.numel() * pinned.element_size() / (time.perf_counter() - t0) / 1e9)
+    return out
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -526,7 +539,7 @@ def main():
     # ---- end to end through the C ABI with host buffers --------------------
     raw_h = np.empty((S_run, T_run // 4), np.uint8)
     raw_h[:] = raw.cpu().numpy()
-    e2e_ms, e2e_value, e2e_sync, e2e_concurrent = None, None, None, None
+    e2e_ms, e2e_value, e2e_sync, e2e_concurrent, e2e_median, e2e_link = None, None, None, None, None, None
     if not args.no_e2e:
         pin_raw = torch.from_numpy(raw_h).pin_memory()
         pin_vis = [torch.empty((C_run, P_run), dtype=torch.complex64).pin_memory() for _ in range(2)]
@@ -563,19 +576,26 @@ def main():
             warm = [svc.submit(jobs[w], raw_np, vis_np[w]) for w in range(2)]
             for jid in warm:
                 svc.wait(jid)
+        # the host link alone, before and after: plain copies of the same pinned samples
+        link = [_link_gbs(torch, pin_raw)]
         barrier()
-        pending = []
+        pending, done = [], []
         t_e2e = time.perf_counter()
         for i in range(args.e2e_steps):
             if len(pending) == 2:
                 svc.wait(pending.pop(0))
+                done.append(time.perf_counter())
             pending.append(svc.submit(jobs[i % 2], raw_np, vis_np[i % 2]))
         for jid in pending:
             svc.wait(jid)
+            done.append(time.perf_counter())
         torch.cuda.synchronize()
         e2e_ms = replicas.max_over_ranks(1e3 * (time.perf_counter() - t_e2e) / args.e2e_steps, dist, device="cuda")
         e2e_value = replicas.aggregate_gsamples(world, S_run * T_run, e2e_ms)
         e2e_concurrent = svc.stats()["max_running"]
+        e2e_median = 1e3 * float(np.median(np.diff(done))) if len(done) > 1 else None
+        link.append(_link_gbs(torch, pin_raw))
+        e2e_link = {"h2d_gbs": [x[0] for x in link], "d2h_gbs": [x[1] for x in link]}
         svc.close()
         del pin_vis, pin_raw
 
@@ -691,7 +711,8 @@ def main():
                     "d2h_bytes_per_step": int(C_run * P_run * 8), "ms_per_step": e2e_ms,
                     "mode": "host buffers through cellspe_service_* (two streams, two jobs in flight; "
                             "wall clock over e2e_steps jobs)",
-                    "max_concurrent_jobs": e2e_concurrent, "sync": e2e_sync},
+                    "max_concurrent_jobs": e2e_concurrent, "median_ms_between_jobs": e2e_median,
+                    "host_link": e2e_link, "sync": e2e_sync},
             "gpu_launches": int(launches),
             "roofline": roof,
             "error": error,
