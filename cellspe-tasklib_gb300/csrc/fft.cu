@@ -190,8 +190,8 @@ int launch_batch(const void* in, float2* out, int64_t batch, float scale, cudaSt
 // copy rate); the shared-memory radix-16 passes, three of them with CTA barriers,
 // took 346.  Eighth turns take cos(pi/4) as two terms and the split's twiddles come
 // from a table (products of rounded ones cost as much): the error against FP64 is then
-// no larger than those passes' (2048 real points 1.18e-7; 1.25e-7 without either).  2^27 floats as complex transforms of 512 and 1024 points 503 -> 362 and
-// 632 -> 361 us, real ones of 1024 points 282 -> 185.
+// no larger than those passes' (2048 real points 1.18e-7; 1.25e-7 without either).
+// 65536 complex transforms of 1024 points 322 -> 197 us, 131072 real ones 282 -> 193.
 constexpr int FW_NT = 256;
 template <int L, int R, bool REAL, bool INV>
 __global__ void __launch_bounds__(FW_NT, 2) k_fft_warp(const float2* __restrict__ in, float2* __restrict__ out, int64_t batch,
@@ -263,7 +263,7 @@ int launch_warp(const void* in, float2* out, int64_t batch, float scale, cudaStr
 }
 
 // Complex transforms of 128 and 256 points stay with the radix-16 groups, whose two
-// passes already run at the copy rate (2^27 floats: 355 and 359 us against 385 and 360).
+// passes already run at the copy rate (2^27 points: 355 and 359 us against 385 and 360).
 template <bool REAL, bool INV>
 int dispatch(const void* in, float2* out, int m, int64_t batch, float scale, cudaStream_t st)
 {

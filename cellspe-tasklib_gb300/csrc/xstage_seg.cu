@@ -13,7 +13,7 @@
 // written.  The arithmetic is k_xmac_tc_gram's (FP16: rows Xr and Xi, Re V and M in
 // one accumulator) and k_xmac_gram's (FP32).  Bound by the read of the
 // spectra, in FP16 also by the MMAs' least cost: those 32 inputs take 480 us in
-// FP16 (2.15 GB, 318 us at the copy rate; 512 CTAs are 3.4 waves) and 830 us in
+// FP16 (2.15 GB, 318 us at the copy rate; 512 CTAs are 3.4 waves) and 870 us in
 // FP32, with the transpose 1040 and 2300.  (Register loads instead of TMA: 614 and
 // 1285 us, cp.async 1030 and 1700, both with a single MMA per 16 segments; the F
 // stage writing blocks of channels for 128-byte TMA rows: 420 and 825, but its
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(LOADERS + 96, 1)
             feed<F::DEPTH, F::SEGS>(&tmap, tc::smem_u32(raw), F::R::BYTES, rfull, rempty, nk, a.err);
     } else if (warp >= LOADERS / 32) {
         // two issuers, four channels each: one thread's instructions took as long
-        // as the MMAs (611 us with one, 512 unrolled, 487 with two; 474 since one lane is elected)
+        // as the MMAs (611 us with one, 512 unrolled, 487 with two; 474 since one lane is elected, 480 with the lane mask)
         const int ca = (warp - LOADERS / 32) * (F::CB / 2);
         if (tc::elect_one()) {
             const uint32_t id = tc::idesc_f16(BM, RI, false, false, false);

@@ -21,10 +21,11 @@
 //     Re V = Xr Xr^T + Xi Xi^T,   Im V = Xi Xr^T - Xr Xi^T,
 // twelve MMAs per 16 segments, nine on a diagonal tile (its Im columns
 // accumulate M = Xi Xr^T and Im V = M - M^T is formed at the end).
-// Bound by the tensor cores: 200 inputs x 1024 channels x 4096 segments 2.59 ms
-// (the CUDA cores 26.6 ms), of which the MMAs are 1.5 ms at 64 cycles each and
-// most of the rest the waits and commits between chunks; one issuer 2.67 ms, and
-// with four 64-byte planes per operand instead of two of 128 bytes 3.17 ms.
+// 200 inputs x 1024 channels x 4096 segments take 2.4 ms (the CUDA cores 26.6 ms), of
+// which the MMAs are 1.5 ms at 64 cycles each and most of the rest the waits and
+// commits between chunks (tensor pipe 46 %, DRAM 29 %).  Before the issuing lanes were
+// elected: 2.59 ms, one issuer 2.67, and with four 64-byte planes per operand
+// instead of two of 128 bytes 3.17.
 //
 // What keeps both at FP32 accuracy is the accumulation: the tensor core adds
 // each MMA to its FP32 accumulator without rounding to nearest, a bias that
